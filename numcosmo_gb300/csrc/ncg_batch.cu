@@ -56,7 +56,7 @@ _tile (const ncg_bprob_t &p, const double *__restrict__ Xq, int bx, int sy, unsi
     constexpr int KC = NcgEv64<DP, KIND>::KC;
     constexpr int S  = NcgEv64<DP, KIND>::S;
 
-    ncg_tile_eval64<DP, KIND, KERN, KC> (p.a, Xq + p.x_off, p.pack64, p.c, p.Vg, (double2 *) p.part, p.kper, bx, sy,
+    ncg_tile_eval64<DP, KIND, KERN, KC, 1> (p.a, Xq + p.x_off, p.pack64, p.c, p.Vg, (double2 *) p.part, p.kper, bx, sy,
                                          (double *) smem, (double *) smem + KC * S);
   }
 }
@@ -85,9 +85,9 @@ _dispatch (const ncg_bprob_t &p, const double *__restrict__ Xq, int bx, int sy, 
   }
 }
 
-/* the slices of point tile bx in slice order, then -2 (gamma + log1p(lambda)
- * - d ln h), the same expression as the one-problem merge kernel.  The pairs
- * were written by other CTAs of this launch: read them past L1 (__ldcg). */
+/* the slices of point tile bx in slice order, then -2 (g + log s - d ln h), as
+ * the one-problem merge kernel.  The pairs were written by other CTAs of this
+ * launch: read them past L1 (__ldcg). */
 __device__ __forceinline__ void
 _merge_tile (const ncg_bprob_t &p, int bx, double *__restrict__ out)
 {
@@ -97,42 +97,19 @@ _merge_tile (const ncg_bprob_t &p, int bx, double *__restrict__ out)
     return;
 
   const bool mixed = p.cls >= NCG_BCLS (1, 4, 0, 0);
-  double G = -CUDART_INF, L = 0.0;
+  double G = NCG_LSE_EMPTY, S = 0.0;
 
   for (int s = 0; s < p.ns; s++)
   {
-    double ms, ls;
+    const double2 q = mixed ? ncg_lse_pair (__ldcg ((const float2 *) p.part + (size_t) s * p.a.m + j))
+                            : __ldcg ((const double2 *) p.part + (size_t) s * p.a.m + j);
+    const double M  = fmax (G, q.x);
 
-    if (mixed)
-    {
-      const float2 q = __ldcg ((const float2 *) p.part + (size_t) s * p.a.m + j);
-
-      ms = (double) q.x;
-      ls = (double) q.y;
-    }
-    else
-    {
-      const double2 q = __ldcg ((const double2 *) p.part + (size_t) s * p.a.m + j);
-
-      ms = q.x;
-      ls = q.y;
-    }
-
-    if (ms > G)
-    {
-      L = (L + 1.0) * exp (G - ms) + ls;
-      G = ms;
-    }
-    else if (ms > -CUDART_INF)
-    {
-      L += (ls + 1.0) * exp (ms - G);
-    }
+    S = S * ncg_exp (G - M) + q.y * ncg_exp (q.x - M);
+    G = M;
   }
 
-  const double gamma = G - p.a.final_shift + (p.dshift ? *p.dshift : 0.0);
-  const double lnp   = gamma + log1p (L) - p.a.d_ln_href;
-
-  out[p.out_off + j] = -2.0 * lnp;
+  out[p.out_off + j] = -2.0 * ncg_lse_lnp (G, S, p.a.final_shift, p.dshift, p.a.d_ln_href);
 }
 
 /* MODE 0: FP64 tiles only; MODE 1: mixed and FP64 tiles (a mixed batch serves

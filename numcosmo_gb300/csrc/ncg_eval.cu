@@ -2,12 +2,10 @@
  * ncg_eval.cu -- eval_m2lnp / eval / compute_IM over (points x kernels) for
  * one problem.
  *
- * Grid: x = tiles of EV_THREADS points (one point per thread), y = slices of
- * the kernel range; each CTA runs one tile of ncg_eval_tiles.cuh and keeps,
- * per point, the reference's (gamma, lambda) pair online: gamma = running
- * maximum of lnt_i, lambda = sum over the other kernels of exp(lnt_i -
- * gamma).  A merge kernel combines the slices in slice order and applies
- * -2 (gamma + log1p(lambda) - d ln h), in FP64 for both forms.
+ * Grid: x = tiles of points, y = slices of the kernel range; each CTA runs one
+ * tile of ncg_eval_tiles.cuh and keeps, per point, the log-sum-exp pair of its
+ * slice online.  A merge kernel combines the slices in a fixed order and
+ * applies -2 (ln sum - d ln h), in FP64 for both forms.
  */
 #include <cuda_runtime.h>
 #include <math_constants.h>
@@ -20,6 +18,37 @@
 /* FP64                                                                     */
 /* ------------------------------------------------------------------------ */
 
+/* warps of a CTA that share 32 points (ncg_tile_eval64's WK): the finest tile,
+ * since the operand traffic (8 S bytes per 32 pairs) is far below what the
+ * FP64 pipes leave room for and fewer points per CTA fill the last wave and
+ * the last tile better */
+#define EV64_WK 4
+#define EV64_FEW 16
+
+__device__ __forceinline__ double2
+_pair (double2 q)
+{
+  return q;
+}
+
+__device__ __forceinline__ double2
+_pair (float2 q)
+{
+  return ncg_lse_pair (q);
+}
+
+__device__ __forceinline__ double
+_pair_g (double2 q)
+{
+  return q.x;
+}
+
+__device__ __forceinline__ double
+_pair_g (float2 q)
+{
+  return (q.x > -CUDART_INF_F) ? (double) q.x : NCG_LSE_EMPTY;
+}
+
 template <int DP, int KIND, int KERN>
 __global__ void __launch_bounds__ (EV_THREADS)
 _eval64_kernel (const ncg_eval_args_t a, const double *__restrict__ Xq, const double *__restrict__ pack,
@@ -28,44 +57,146 @@ _eval64_kernel (const ncg_eval_args_t a, const double *__restrict__ Xq, const do
 {
   constexpr int S  = NcgEv64<DP, KIND>::S;
   constexpr int KC = NcgEv64<DP, KIND>::KC;
-  __shared__ double sm[KC * S];
+  __shared__ __align__ (16) double sm[KC * S];
   __shared__ double sc[KC];
 
-  ncg_tile_eval64<DP, KIND, KERN, KC> (a, Xq, pack, cvec, Vg, part, kper, blockIdx.x, blockIdx.y, sm, sc);
+  ncg_tile_eval64<DP, KIND, KERN, KC, EV64_WK> (a, Xq, pack, cvec, Vg, part, kper, blockIdx.x, blockIdx.y, sm, sc);
 }
 
-/* combine the slices in order; out = -2 (gamma + log1p(lambda) - d ln h) or
- * the linear density exp(gamma + log1p(lambda) - d ln h) */
+/* A few points (EV64_FEW at most): one kernel per thread, grid = (slices,
+ * points).  A warp instruction costs the same 64 cycles for one lane as for
+ * 32, so a lane per point would leave the FP64 pipes idle below a warp of
+ * points: the call with one point against 1000 kernels (KDE, d = 4) took
+ * 306 us when a single lane walked its slice, 36 us like this. */
+template <int DP, int KIND, int KERN>
+__global__ void __launch_bounds__ (EV_THREADS)
+_eval64_few_kernel (const ncg_eval_args_t a, const double *__restrict__ Xq, const double *__restrict__ pack,
+                    const double *__restrict__ cvec, const double *__restrict__ Vg, double2 *__restrict__ part,
+                    int kper)
+{
+  constexpr int S   = NcgEv64<DP, KIND>::S;
+  __shared__ double xs[DP], v[DP];
+  __shared__ double2 ex[EV_THREADS / 32];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int64_t j = blockIdx.y;
+  const int i0    = blockIdx.x * kper, i1 = min (a.n, i0 + kper);
+  double x[DP];
+
+  if (tid < DP)
+    xs[tid] = (tid < a.d) ? Xq[j * a.d + tid] : 0.0;
+
+  __syncthreads ();
+
+  if (KIND == NCG_KDE)
+  {
+    /* row tid of the whitening, in the order of ncg_whiten_point */
+    if (tid < DP)
+    {
+      const double *row = Vg + tid * (tid + 1) / 2;
+      double y          = 0.0;
+
+      for (int c = 0; c <= tid; c++)
+        y = fma (row[c], xs[c], y);
+
+      v[tid] = y;
+    }
+
+    __syncthreads ();
+  }
+
+#pragma unroll
+  for (int c = 0; c < DP; c++)
+    x[c] = (KIND == NCG_KDE) ? v[c] : xs[c];
+
+  double g = NCG_LSE_EMPTY, s = 0.0;
+  const double inv_nu = 1.0 / a.nu;
+
+  for (int i = i0 + tid; i < i1; i += EV_THREADS)
+    ncg_lse_add (ncg_lnt_64<KERN> (ncg_chi2_64<DP, KIND> (pack + (size_t) i * S, x), cvec[i], a.kappa, inv_nu), g, s);
+
+  /* the CTA's pair: the largest g first, then one exp per thread */
+  double G = g;
+
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    G = fmax (G, __shfl_xor_sync (0xffffffffu, G, o));
+
+  s *= ncg_exp (g - G);
+
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    s += __shfl_xor_sync (0xffffffffu, s, o);
+
+  if (lane == 0)
+    ex[w] = make_double2 (G, s);
+
+  __syncthreads ();
+
+  if (tid == 0)
+  {
+#pragma unroll
+    for (int q = 1; q < EV_THREADS / 32; q++)
+    {
+      const double M = fmax (G, ex[q].x);
+
+      s = s * ncg_exp (G - M) + ex[q].y * ncg_exp (ex[q].x - M);
+      G = M;
+    }
+
+    part[(size_t) blockIdx.x * a.m + j] = make_double2 (G, s);
+  }
+}
+
+/* combine the slices; out = -2 (ln sum - d ln h) or the linear density.  One
+ * point per lane, the MG_TH / 32 warps share its slices: the largest g first,
+ * then every slice's exp independently (a serial loop over the slices, each
+ * waiting for the previous one's exp, took 71 us at 24 slices of 8192 points
+ * and 587 us at 316 slices of 256). */
+#define MG_TH 256
+
 template <typename T2>
-__global__ void
+__global__ void __launch_bounds__ (MG_TH)
 _merge_kernel (const T2 *__restrict__ part, int nslices, int64_t m, double shift, const double *dshift,
                double d_ln_href, int linear, double *__restrict__ out)
 {
-  const int64_t j = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
+  __shared__ double red[MG_TH / 32][33];
+  const int lane  = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t j = (int64_t) blockIdx.x * 32 + lane;
+  const bool in   = j < m;
+  double G = NCG_LSE_EMPTY, S = 0.0;
 
-  if (j >= m)
+  if (in)
+    for (int s = w; s < nslices; s += MG_TH / 32)
+      G = fmax (G, _pair_g (part[(size_t) s * m + j]));
+
+  red[w][lane] = G;
+  __syncthreads ();
+
+#pragma unroll
+  for (int q = 0; q < MG_TH / 32; q++)
+    G = fmax (G, red[q][lane]);
+
+  __syncthreads ();
+
+  if (in)
+    for (int s = w; s < nslices; s += MG_TH / 32)
+    {
+      const double2 p = _pair (part[(size_t) s * m + j]);
+
+      S = fma (p.y, ncg_exp (p.x - G), S);
+    }
+
+  red[w][lane] = S;
+  __syncthreads ();
+
+  if (w > 0 || !in)
     return;
 
-  double G = -CUDART_INF, L = 0.0;
+#pragma unroll
+  for (int q = 1; q < MG_TH / 32; q++)
+    S += red[q][lane];
 
-  for (int s = 0; s < nslices; s++)
-  {
-    const T2 p      = part[(size_t) s * m + j];
-    const double ms = (double) p.x, ls = (double) p.y;
-
-    if (ms > G)
-    {
-      L = (L + 1.0) * exp (G - ms) + ls;
-      G = ms;
-    }
-    else if (ms > -CUDART_INF)
-    {
-      L += (ls + 1.0) * exp (ms - G);
-    }
-  }
-
-  const double gamma = G - shift + (dshift ? *dshift : 0.0);
-  const double lnp   = gamma + log1p (L) - d_ln_href;
+  const double lnp = ncg_lse_lnp (G, S, shift, dshift, d_ln_href);
 
   out[j] = linear ? exp (lnp) : -2.0 * lnp;
 }
@@ -73,35 +204,111 @@ _merge_kernel (const T2 *__restrict__ part, int nslices, int64_t m, double shift
 typedef void (*ev64_fn) (const ncg_eval_args_t, const double *, const double *, const double *,
                          const double *, double2 *, int);
 
+#define EV64_PICK(DP) return few ? _eval64_few_kernel<DP, KIND, KERN> : _eval64_kernel<DP, KIND, KERN>
+
 template <int KIND, int KERN>
 static ev64_fn
-_pick64 (int dp)
+_pick64 (int dp, bool few)
 {
   switch (dp)
   {
-    case 4:  return _eval64_kernel<4, KIND, KERN>;
-    case 8:  return _eval64_kernel<8, KIND, KERN>;
-    case 12: return _eval64_kernel<12, KIND, KERN>;
-    case 16: return _eval64_kernel<16, KIND, KERN>;
-    case 20: return _eval64_kernel<20, KIND, KERN>;
-    case 24: return _eval64_kernel<24, KIND, KERN>;
-    case 28: return _eval64_kernel<28, KIND, KERN>;
-    case 32: return _eval64_kernel<32, KIND, KERN>;
+    case 4:  EV64_PICK (4);
+    case 8:  EV64_PICK (8);
+    case 12: EV64_PICK (12);
+    case 16: EV64_PICK (16);
+    case 20: EV64_PICK (20);
+    case 24: EV64_PICK (24);
+    case 28: EV64_PICK (28);
+    case 32: EV64_PICK (32);
     default: return NULL;
   }
 }
 
+static ev64_fn
+_ev64 (const ncg_eval_args_t *a)
+{
+  const bool few = a->m <= EV64_FEW;
+
+  if (a->kind == NCG_VKDE)
+    return (a->kernel == NCG_KERNEL_ST) ? _pick64<NCG_VKDE, NCG_KERNEL_ST> (a->dp, few)
+                                        : _pick64<NCG_VKDE, NCG_KERNEL_GAUSS> (a->dp, few);
+
+  return (a->kernel == NCG_KERNEL_ST) ? _pick64<NCG_KDE, NCG_KERNEL_ST> (a->dp, few)
+                                      : _pick64<NCG_KDE, NCG_KERNEL_GAUSS> (a->dp, few);
+}
+
+/* NcgEv64::KC */
 static int
 _kc64 (int kind, int dp)
 {
-  const int P = dp * (dp + 1) / 2;
-  const int S = (kind == NCG_VKDE) ? dp + P : dp;
-  int kc      = 32768 / ((S + 1) * 8);
+  const int kc = 36864 / ((ncg_pack64_stride (kind, dp) + 1) * 8) / 4 * 4;
 
   return kc < 4 ? 4 : (kc > 256 ? 256 : kc);
 }
 
-/* slices of the kernel range so that the grid fills the GPU several times */
+/* Slices of the FP64 forms.  The work is cut until there are about 48 CTAs
+ * per SM (the last wave then costs a few per cent) but no finer than 8
+ * kernels per warp, where the tile's own set-up and merge reach a tenth of the
+ * loop; a few points take one kernel per thread.  ns_max bounds the slices
+ * (a caller's scratch). */
+static void
+_slicing64 (const ncg_eval_args_t *a, int64_t ns_max, int *nslices, int *kper)
+{
+  const int64_t bx = (a->m + EV_THREADS / EV64_WK - 1) / (EV_THREADS / EV64_WK);
+  const bool few   = a->m <= EV64_FEW;
+  const int unit   = few ? EV_THREADS : 8 * EV64_WK;
+  const int64_t most = (a->n + unit - 1) / unit;
+  int64_t s        = few ? most : (152 * 48 + bx - 1) / bx;
+  int64_t kp;
+
+  if (s > most)
+    s = most;
+
+  if (s > ns_max)
+    s = ns_max;
+
+  if (s < 1)
+    s = 1;
+
+  kp = (a->n + s - 1) / s;
+  kp = (kp + unit - 1) / unit * unit;
+
+  *kper    = (int) kp;
+  *nslices = (int) ((a->n + kp - 1) / kp);
+}
+
+static cudaError_t
+_run64 (const ncg_eval_args_t *a, const double *Xq, const double *pack64, const double *c, const double *Vg,
+        double *out, double2 *part, int64_t ns_max, int linear, cudaStream_t s)
+{
+  ev64_fn fn = _ev64 (a);
+  int ns, kp;
+
+  if (fn == NULL || a->m <= 0 || a->n <= 0)
+    return cudaErrorInvalidValue;
+
+  _slicing64 (a, ns_max, &ns, &kp);
+
+  const int64_t bx = (a->m + EV_THREADS / EV64_WK - 1) / (EV_THREADS / EV64_WK);
+  const dim3 grid  = (a->m <= EV64_FEW) ? dim3 ((unsigned) ns, (unsigned) a->m) : dim3 ((unsigned) bx, (unsigned) ns);
+
+  fn<<<grid, EV_THREADS, 0, s>>> (*a, Xq, pack64, c, Vg, part, kp);
+
+  cudaError_t e = cudaGetLastError ();
+
+  if (e != cudaSuccess)
+    return e;
+
+  _merge_kernel<double2><<<(unsigned) ((a->m + 31) / 32), MG_TH, 0, s>>> (part, ns, a->m, a->final_shift, NULL,
+                                                                          a->d_ln_href, linear, out);
+
+  return cudaGetLastError ();
+}
+
+#define EV64_NS_MAX 4096
+
+/* slices of the kernel range so that the grid fills the GPU several times (the
+ * FP32 form and compute_IM) */
 static void
 _slicing (int64_t m, int n, int kc, int *nslices, int *kper)
 {
@@ -132,43 +339,23 @@ ncg_eval_scratch_bytes (const ncg_eval_args_t *a, int precision)
 {
   int ns, kp;
 
-  _slicing (a->m, a->n, (precision == NCG_PREC_FP64) ? _kc64 (a->kind, a->dp) : 64, &ns, &kp);
+  if (precision == NCG_PREC_FP64)
+  {
+    _slicing64 (a, EV64_NS_MAX, &ns, &kp);
 
-  return (size_t) ns * (size_t) a->m * ((precision == NCG_PREC_FP64) ? sizeof (double2) : sizeof (float2));
+    return (size_t) ns * (size_t) a->m * sizeof (double2);
+  }
+
+  _slicing (a->m, a->n, 64, &ns, &kp);
+
+  return (size_t) ns * (size_t) a->m * sizeof (float2);
 }
 
 extern "C" cudaError_t
 ncg_launch_eval_m2lnp_fp64 (const ncg_eval_args_t *a, const double *Xq, const double *pack64, const double *c,
                             const double *Vg, double *out, void *scratch, int linear, cudaStream_t s)
 {
-  ev64_fn fn;
-
-  if (a->kind == NCG_VKDE)
-    fn = (a->kernel == NCG_KERNEL_ST) ? _pick64<NCG_VKDE, NCG_KERNEL_ST> (a->dp) : _pick64<NCG_VKDE, NCG_KERNEL_GAUSS> (a->dp);
-  else
-    fn = (a->kernel == NCG_KERNEL_ST) ? _pick64<NCG_KDE, NCG_KERNEL_ST> (a->dp) : _pick64<NCG_KDE, NCG_KERNEL_GAUSS> (a->dp);
-
-  if (fn == NULL || a->m <= 0 || a->n <= 0)
-    return cudaErrorInvalidValue;
-
-  int ns, kp;
-
-  _slicing (a->m, a->n, _kc64 (a->kind, a->dp), &ns, &kp);
-
-  const int64_t bx = (a->m + EV_THREADS - 1) / EV_THREADS;
-  dim3 grid ((unsigned) bx, (unsigned) ns);
-
-  fn<<<grid, EV_THREADS, 0, s>>> (*a, Xq, pack64, c, Vg, (double2 *) scratch, kp);
-
-  cudaError_t e = cudaGetLastError ();
-
-  if (e != cudaSuccess)
-    return e;
-
-  _merge_kernel<double2><<<(unsigned) ((a->m + 255) / 256), 256, 0, s>>> (
-    (const double2 *) scratch, ns, a->m, a->final_shift, NULL, a->d_ln_href, linear, out);
-
-  return cudaGetLastError ();
+  return _run64 (a, Xq, pack64, c, Vg, out, (double2 *) scratch, EV64_NS_MAX, linear, s);
 }
 
 /* ------------------------------------------------------------------------ */
@@ -517,7 +704,7 @@ ncg_launch_eval_m2lnp_mixed (const ncg_eval_args_t *a, const double *Xq, const f
   if (e != cudaSuccess)
     return e;
 
-  _merge_kernel<float2><<<(unsigned) ((a->m + 255) / 256), 256, 0, s>>> (
+  _merge_kernel<float2><<<(unsigned) ((a->m + 31) / 32), MG_TH, 0, s>>> (
     (const float2 *) scratch, ns, a->m, a->final_shift, cshift, a->d_ln_href, 0, out);
 
   return cudaGetLastError ();
@@ -560,7 +747,7 @@ _im64_kernel (const ncg_eval_args_t a, const double *__restrict__ X, const doubl
       x[c] = valid ? pack[(size_t) j * S + c] : 0.0;
   }
 
-  const double inv_f = valid ? 1.0 / f[j] : 0.0;
+  const double inv_f = valid ? 1.0 / f[j] : 0.0, inv_nu = 1.0 / a.nu;
   const int i0 = blockIdx.y * a.m;   /* a.m carries the per-slice kernel count here */
   const int i1 = min (n, i0 + (int) a.m);
 
@@ -583,44 +770,9 @@ _im64_kernel (const ncg_eval_args_t a, const double *__restrict__ X, const doubl
 
     for (int kk = 0; kk < kc; kk++)
     {
-      const double *pk = sm + kk * S;
-      double chi2      = 0.0;
-
-      if (KIND == NCG_VKDE)
-      {
-        double dl[DP];
-
-#pragma unroll
-        for (int c = 0; c < DP; c++)
-          dl[c] = x[c] - pk[c];
-
-        const double *W = pk + DP;
-        int p           = 0;
-
-#pragma unroll
-        for (int r = 0; r < DP; r++)
-        {
-          double y = 0.0;
-
-#pragma unroll
-          for (int c = 0; c <= r; c++)
-            y = fma (W[p++], dl[c], y);
-
-          chi2 = fma (y, y, chi2);
-        }
-      }
-      else
-      {
-#pragma unroll
-        for (int c = 0; c < DP; c++)
-        {
-          const double t = pk[c] - x[c];
-
-          chi2 = fma (t, t, chi2);
-        }
-      }
-
-      const double K = (KERN == NCG_KERNEL_ST) ? pow (1.0 + chi2 / a.nu, -0.5 * (a.nu + a.d)) : exp (-0.5 * chi2);
+      const double chi2 = ncg_chi2_64<DP, KIND> (sm + kk * S, x);
+      const double K    = (KERN == NCG_KERNEL_ST) ? ncg_exp_full (-0.5 * (a.nu + a.d) * ncg_log_ge1 (fma (chi2, inv_nu, 1.0)))
+                                                  : ncg_exp_full (-0.5 * chi2);
 
       IM[(size_t) j * n + ic + kk] = (K * sn[kk]) * inv_f;
     }
@@ -683,7 +835,7 @@ extern "C" cudaError_t
 ncg_launch_merge_f2 (const void *part, int nparts, int64_t m, double shift, const double *dshift, double d_ln_href,
                      double *out, cudaStream_t s)
 {
-  _merge_kernel<float2><<<(unsigned) ((m + 255) / 256), 256, 0, s>>> ((const float2 *) part, nparts, m, shift, dshift,
+  _merge_kernel<float2><<<(unsigned) ((m + 31) / 32), MG_TH, 0, s>>> ((const float2 *) part, nparts, m, shift, dshift,
                                                                      d_ln_href, 0, out);
 
   return cudaGetLastError ();
@@ -737,16 +889,10 @@ extern "C" cudaError_t
 ncg_launch_eval_m2lnp_fp64_noalloc (const ncg_eval_args_t *a, const double *Xq, const double *pack64, const double *c,
                                     const double *Vg, double *out, cudaStream_t s)
 {
-  ev64_fn fn;
   int dev = 0;
   cudaError_t e;
 
-  if (a->kind == NCG_VKDE)
-    fn = (a->kernel == NCG_KERNEL_ST) ? _pick64<NCG_VKDE, NCG_KERNEL_ST> (a->dp) : _pick64<NCG_VKDE, NCG_KERNEL_GAUSS> (a->dp);
-  else
-    fn = (a->kernel == NCG_KERNEL_ST) ? _pick64<NCG_KDE, NCG_KERNEL_ST> (a->dp) : _pick64<NCG_KDE, NCG_KERNEL_GAUSS> (a->dp);
-
-  if (fn == NULL || a->m <= 0 || a->n <= 0 || a->m > ncg_noalloc_max_points ())
+  if (a->m <= 0 || a->n <= 0 || a->m > ncg_noalloc_max_points ())
     return cudaErrorInvalidValue;
 
   if ((e = cudaGetDevice (&dev)) != cudaSuccess)
@@ -769,33 +915,9 @@ ncg_launch_eval_m2lnp_fp64_noalloc (const ncg_eval_args_t *a, const double *Xq, 
   }
 
   /* the regular slicing, with the slice count capped by the static size */
-  const int kc = _kc64 (a->kind, a->dp);
-  int ns, kp;
+  const int64_t fit = (int64_t) (NCG_NOALLOC_SCRATCH_BYTES / ((size_t) a->m * sizeof (double2)));
 
-  _slicing (a->m, a->n, kc, &ns, &kp);
-
-  const int64_t ns_max = (int64_t) (NCG_NOALLOC_SCRATCH_BYTES / ((size_t) a->m * sizeof (double2)));
-
-  if (ns > ns_max)
-  {
-    kp = (int) ((a->n + ns_max - 1) / ns_max);
-    kp = ((kp + kc - 1) / kc) * kc;
-    ns = (a->n + kp - 1) / kp;
-  }
-
-  double2 *part    = (double2 *) addr;
-  const int64_t bx = (a->m + EV_THREADS - 1) / EV_THREADS;
-  dim3 grid ((unsigned) bx, (unsigned) ns);
-
-  fn<<<grid, EV_THREADS, 0, s>>> (*a, Xq, pack64, c, Vg, part, kp);
-
-  if ((e = cudaGetLastError ()) != cudaSuccess)
-    return e;
-
-  _merge_kernel<double2><<<(unsigned) ((a->m + 255) / 256), 256, 0, s>>> (part, ns, a->m, a->final_shift, NULL,
-                                                                          a->d_ln_href, 0, out);
-
-  return cudaGetLastError ();
+  return _run64 (a, Xq, pack64, c, Vg, out, (double2 *) addr, fit < EV64_NS_MAX ? fit : EV64_NS_MAX, 0, s);
 }
 
 /* ------------------------------------------------- FP64 pipe measurement */

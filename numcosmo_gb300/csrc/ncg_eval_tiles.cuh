@@ -1,7 +1,8 @@
 /*
- * ncg_eval_tiles.cuh -- the per-CTA work of eval_m2lnp: EV_THREADS points
- * (one per thread) against one slice of the kernel range, leaving per point
- * the reference's (gamma, lambda) pair of the slice.  Shared by the
+ * ncg_eval_tiles.cuh -- the per-CTA work of eval_m2lnp: a tile of points
+ * (one per thread, or one per lane with the warps sharing the kernels)
+ * against one slice of the kernel range, leaving per point the log-sum-exp
+ * pair of the slice.  Shared by the
  * one-problem launches (ncg_eval.cu, grid = point tiles x slices) and the
  * persistent multi-problem launch (ncg_batch.cu, tiles taken from a work
  * list), so a problem gets the same arithmetic in both.
@@ -15,7 +16,13 @@
  * threads read the same kernel: broadcast); the chunk size changes only the
  * staging, never the order of the arithmetic.
  *
- * FP64 form: everything in double.  Mixed form (SIMT): the difference
+ * FP64 form: everything in double; the pair is (g, s) of ncg_fastmath.cuh,
+ * the sum being s exp(g).  One FP64 warp instruction takes 64 cycles of its
+ * SM sub-partition here whatever else happens, so the loop's cost is its count
+ * of FP64 instructions: a branch-free sum on the table-driven exp and log takes
+ * 19 (Student-t) or 10 (Gauss) beyond chi^2, where two library calls in a
+ * divergent online maximum took about 87.  Mixed form (SIMT), which keeps the
+ * reference's (gamma, lambda) pair: the difference
  * x - theta_i is formed from hi/lo float splits of both operands (exact to
  * float rounding of the difference), whitening and chi^2 in FP32 FMA,
  * log-sum-exp in FP32 with the per-kernel constants shifted by their
@@ -29,18 +36,97 @@
 #include <stdint.h>
 
 #include "ncg_internal.h"
+#include "ncg_fastmath.cuh"
 
 #define EV_THREADS 128
 
-/* FP64 operand stride (doubles per kernel) and the one-problem chunk size */
+/* FP64 operand stride (doubles per kernel) and the kernels staged at once: a
+ * multiple of the warps that may share them, within 36 KiB */
 template <int DP, int KIND>
 struct NcgEv64
 {
   static constexpr int P   = DP * (DP + 1) / 2;
   static constexpr int S   = (KIND == NCG_VKDE) ? DP + P : DP;
-  static constexpr int raw = 32768 / ((S + 1) * 8);
+  static constexpr int raw = 36864 / ((S + 1) * 8) / 4 * 4;
   static constexpr int KC  = raw < 4 ? 4 : (raw > 256 ? 256 : raw);
 };
+
+/* y = L x of the packed lower-triangular L (rows in order), zero past d */
+template <int DP>
+__device__ __forceinline__ void
+ncg_whiten_point (const double *__restrict__ Vg, double *x)
+{
+  double v[DP];
+  int p = 0;
+
+#pragma unroll
+  for (int r = 0; r < DP; r++)
+  {
+    double s = 0.0;
+
+#pragma unroll
+    for (int c = 0; c <= r; c++)
+      s = fma (Vg[p++], x[c], s);
+
+    v[r] = s;
+  }
+
+#pragma unroll
+  for (int c = 0; c < DP; c++)
+    x[c] = v[c];
+}
+
+/* chi^2 of the point x against one kernel's operand pk */
+template <int DP, int KIND>
+__device__ __forceinline__ double
+ncg_chi2_64 (const double *pk, const double *x)
+{
+  double chi2 = 0.0;
+
+  if (KIND == NCG_VKDE)
+  {
+    double dl[DP];
+
+#pragma unroll
+    for (int c = 0; c < DP; c++)
+      dl[c] = x[c] - pk[c];
+
+    const double *W = pk + DP;
+    int p           = 0;
+
+#pragma unroll
+    for (int r = 0; r < DP; r++)
+    {
+      double y = 0.0;
+
+#pragma unroll
+      for (int c = 0; c <= r; c++)
+        y = fma (W[p++], dl[c], y);
+
+      chi2 = fma (y, y, chi2);
+    }
+  }
+  else
+  {
+#pragma unroll
+    for (int c = 0; c < DP; c++)
+    {
+      const double t = pk[c] - x[c];
+
+      chi2 = fma (t, t, chi2);
+    }
+  }
+
+  return chi2;
+}
+
+/* ln of the weighted kernel */
+template <int KERN>
+__device__ __forceinline__ double
+ncg_lnt_64 (double chi2, double c, double kappa, double inv_nu)
+{
+  return (KERN == NCG_KERNEL_ST) ? fma (kappa, ncg_log_ge1 (fma (chi2, inv_nu, 1.0)), c) : fma (-0.5, chi2, c);
+}
 
 /* mixed operand stride (floats per kernel, multiple of 4):
  *  VKDE: theta_hi[dp] theta_lo[dp] W[dp(dp+1)/2] c'
@@ -58,16 +144,20 @@ struct NcgEvMx
   static constexpr int KCB = kb < 4 ? 4 : (kb > 64 ? 64 : kb);
 };
 
-template <int DP, int KIND, int KERN, int KC>
+/* WK = 1: EV_THREADS points, one per thread, every warp runs all kernels.
+ * WK = 4: 32 points, one per lane, warp w takes the kernels w mod 4 of each
+ * chunk and the four sums are added at the end (in warp order).  sm holds
+ * KC * S doubles, sc KC. */
+template <int DP, int KIND, int KERN, int KC, int WK>
 __device__ __forceinline__ void
 ncg_tile_eval64 (const ncg_eval_args_t a, const double *__restrict__ Xq, const double *__restrict__ pack,
                  const double *__restrict__ cvec, const double *__restrict__ Vg, double2 *__restrict__ part,
                  int kper, int bx, int sy, double *__restrict__ sm, double *__restrict__ sc)
 {
-  constexpr int S  = NcgEv64<DP, KIND>::S;
-
-  const int64_t j  = (int64_t) bx * EV_THREADS + threadIdx.x;
-  const bool valid = j < a.m;
+  constexpr int S   = NcgEv64<DP, KIND>::S;
+  const int w       = (WK == 1) ? 0 : threadIdx.x >> 5;
+  const int64_t j   = (int64_t) bx * (EV_THREADS / WK) + ((WK == 1) ? threadIdx.x : (threadIdx.x & 31));
+  const bool valid  = j < a.m;
   double x[DP];
 
 #pragma unroll
@@ -75,28 +165,9 @@ ncg_tile_eval64 (const ncg_eval_args_t a, const double *__restrict__ Xq, const d
     x[c] = (valid && c < a.d) ? Xq[j * a.d + c] : 0.0;
 
   if (KIND == NCG_KDE)
-  {
-    double v[DP];
-    int p = 0;
+    ncg_whiten_point<DP> (Vg, x);
 
-#pragma unroll
-    for (int r = 0; r < DP; r++)
-    {
-      double s = 0.0;
-
-#pragma unroll
-      for (int c = 0; c <= r; c++)
-        s = fma (Vg[p++], x[c], s);
-
-      v[r] = s;
-    }
-
-#pragma unroll
-    for (int c = 0; c < DP; c++)
-      x[c] = v[c];
-  }
-
-  double gmax = -CUDART_INF, lam = 0.0;
+  double g = NCG_LSE_EMPTY, s = 0.0;
   const int i0 = sy * kper;
   const int i1 = min (a.n, i0 + kper);
   const double inv_nu = 1.0 / a.nu;
@@ -115,62 +186,37 @@ ncg_tile_eval64 (const ncg_eval_args_t a, const double *__restrict__ Xq, const d
 
     __syncthreads ();
 
-    for (int kk = 0; kk < kc; kk++)
+    for (int kk = w; kk < kc; kk += WK)
+      ncg_lse_add (ncg_lnt_64<KERN> (ncg_chi2_64<DP, KIND> (sm + kk * S, x), sc[kk], a.kappa, inv_nu), g, s);
+  }
+
+  if (WK > 1)
+  {
+    double2 *ex = (double2 *) sm;
+
+    __syncthreads ();
+
+    if (w > 0)
+      ex[threadIdx.x] = make_double2 (g, s);
+
+    __syncthreads ();
+
+    if (w > 0)
+      return;
+
+#pragma unroll
+    for (int q = 1; q < WK; q++)
     {
-      const double *pk = sm + kk * S;
-      double chi2      = 0.0;
+      const double2 o = ex[q * 32 + threadIdx.x];
+      const double G  = fmax (g, o.x);
 
-      if (KIND == NCG_VKDE)
-      {
-        double dl[DP];
-
-#pragma unroll
-        for (int c = 0; c < DP; c++)
-          dl[c] = x[c] - pk[c];
-
-        const double *W = pk + DP;
-        int p           = 0;
-
-#pragma unroll
-        for (int r = 0; r < DP; r++)
-        {
-          double y = 0.0;
-
-#pragma unroll
-          for (int c = 0; c <= r; c++)
-            y = fma (W[p++], dl[c], y);
-
-          chi2 = fma (y, y, chi2);
-        }
-      }
-      else
-      {
-#pragma unroll
-        for (int c = 0; c < DP; c++)
-        {
-          const double t = pk[c] - x[c];
-
-          chi2 = fma (t, t, chi2);
-        }
-      }
-
-      const double lnt = (KERN == NCG_KERNEL_ST) ? fma (a.kappa, log1p (chi2 * inv_nu), sc[kk])
-                                                 : fma (-0.5, chi2, sc[kk]);
-
-      if (lnt > gmax)
-      {
-        lam  = (lam + 1.0) * exp (gmax - lnt);
-        gmax = lnt;
-      }
-      else if (lnt > -CUDART_INF)
-      {
-        lam += exp (lnt - gmax);
-      }
+      s = s * ncg_exp (g - G) + o.y * ncg_exp (o.x - G);
+      g = G;
     }
   }
 
   if (valid)
-    part[(size_t) sy * a.m + j] = make_double2 (gmax, lam);
+    part[(size_t) sy * a.m + j] = make_double2 (g, s);
 }
 
 template <int DP, int KIND, int KERN, int KC>
