@@ -1287,7 +1287,7 @@ ncg_sd_prepare (ncg_sd_t *sd)
   if (sd->cfg.cov_type == NCG_COV_FIXED)
   {
     CK (cudaMemcpyAsync (sd->dcov, sd->cov_fixed, sizeof (double) * d * d, cudaMemcpyHostToDevice, s), "H2D cov");
-    CK (ncg_launch_global_cov_chol (sd->dX, 0, d, sd->dcov, sd->dU, sd->dflag, sd->dst, s), "global_chol");
+    CK (ncg_launch_mean (sd->dX, nkk, d, sd->dmu, s), "mean");
   }
   else if (robust)
   {
@@ -1295,13 +1295,15 @@ ncg_sd_prepare (ncg_sd_t *sd)
     CK (ncg_launch_robust_cov (sd->dX, n, d, NULL, nkk, 1, sd->cfg.cov_type == NCG_COV_ROBUST, sd->drq, sd->dcov,
                                &sd->dst->n_badindex, s),
         "robust global cov");
-    CK (ncg_launch_global_cov_chol (sd->dX, 0, d, sd->dcov, sd->dU, sd->dflag, sd->dst, s), "global_chol");
+    CK (ncg_launch_mean (sd->dX, nkk, d, sd->dmu, s), "mean");
   }
   else
   {
-    CK (ncg_launch_global_cov_chol (sd->dX, nkk, d, sd->dcov, sd->dU, sd->dflag, sd->dst, s), "global_cov_chol");
+    /* the running means and quotients in buffers that are filled later */
+    CK (ncg_launch_global_cov (sd->dX, nkk, d, sd->dcov, sd->dmu, sd->dY, sd->dpack64, s), "global_cov");
   }
 
+  CK (ncg_launch_global_chol (sd->dcov, d, sd->dU, sd->dflag, sd->dst, s), "global_chol");
   CK (cudaMemcpyAsync (&st, sd->dst, sizeof (st), cudaMemcpyDeviceToHost, s), "D2H status");
   CK (cudaStreamSynchronize (s), "sync");
 
@@ -1324,7 +1326,6 @@ ncg_sd_prepare (ncg_sd_t *sd)
 
   CK (ncg_launch_global_lnnorm (sd->dU, d, sd->kernel, sd->nu, sd->dst, s), "global_lnnorm");
   CK (ncg_launch_whiten (sd->dX, sd->dU, n, d, sd->dY, s), "whiten");
-  CK (ncg_launch_mean (sd->dX, nkk, d, sd->dmu, s), "mean");
 
   if (sd->kind == NCG_VKDE)
   {

@@ -82,8 +82,10 @@ typedef struct ncg_eval_args
 int         ncg_fault_take (int fault);
 
 /* ---- prepare (ncg_prepare.cu) ---- */
-cudaError_t ncg_launch_global_cov_chol (const double *X, int n, int d, double *cov, double *U,
-                                        int32_t *flag, ncg_prep_status_t *st, cudaStream_t s);
+cudaError_t ncg_launch_global_cov (const double *X, int n, int d, double *cov, double *mu, double *mean, double *Rq,
+                                   cudaStream_t s);
+cudaError_t ncg_launch_global_chol (const double *cov, int d, double *U, int32_t *flag, ncg_prep_status_t *st,
+                                    cudaStream_t s);
 cudaError_t ncg_launch_nearpd (double *cov_then_U, int count, const int32_t *ids, int d, int maxiter,
                                int32_t *flag, ncg_prep_status_t *st, cudaStream_t s);
 cudaError_t ncg_launch_global_lnnorm (const double *U, int d, int kernel, double nu,

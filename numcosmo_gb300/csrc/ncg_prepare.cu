@@ -1,7 +1,8 @@
 /*
  * ncg_prepare.cu -- device side of NcmStatsDistKDE / NcmStatsDistVKDE prepare.
  *
- *  global_cov_chol  Welford covariance of all centres + upper Cholesky
+ *  global_cov       Welford covariance of all centres
+ *  global_chol      its upper Cholesky
  *                   (numcosmo/ncm/stats/ncm_stats_dist_kde.c:379-450,
  *                    numcosmo/ncm/stats/ncm_stats_vec.c:511-565,2376-2398)
  *  whiten           invUsample = X U^{-1}  (ncm_stats_dist_kde.c:477-480)
@@ -62,18 +63,48 @@ ncg_raise_smem_limit (const void *fn, size_t bytes, int *limit)
   return e;
 }
 
-#define WT 32          /* Welford rows staged per chunk */
 #define PREP_THREADS 128
 
-struct WelfordSmem
+/* ------------------------------------------------------------------------ */
+/* Welford covariance (ncm_stats_vec.c:511-565, get_cov_matrix :2376-2398),   */
+/* bit for bit in the reference's order.  With weight t (rows so far) and     */
+/* mean m, row x does                                                        */
+/*   delta = x - m;  R = delta / (t + 1);  m += R;  var += (t delta) R;        */
+/*   C_rc += (x_r - m_r) delta_c      (m_r updated, delta_c from before).      */
+/*                                                                          */
+/* What bounds it: the running mean is one dependent chain per coordinate,    */
+/* and a dependent FP64 instruction takes 64 cycles here, a division 561      */
+/* (measured).  The divisor t + 1 is known in advance, so the quotient is      */
+/* taken as R = fma (delta, yh, delta * yl) with yh = fl(1 / (t + 1)) and       */
+/* yl = fl((1 - (t + 1) yh) yh): before its one rounding the sum is within      */
+/* 2^-104 of delta / (t + 1), and a quotient by an integer below 2^31 lies at   */
+/* least 2^-32 ulp from the middle of two doubles (and never on it), so this   */
+/* is the correctly rounded quotient.  Deltas outside 2^-895 .. 2^1004 (where   */
+/* yl's product may lose bits) take the division itself.  A row then costs     */
+/* 4 dependent instructions instead of a division and 3.                       */
+/* ------------------------------------------------------------------------ */
+
+__device__ __forceinline__ void
+_recip_pair (double w, double *yh, double *yl)
 {
-  double xs[WT][NCG_DMAX];
-  double mh[WT][NCG_DMAX];
-  double mprev[NCG_DMAX];
-  double A[NCG_DMAX * NCG_DMAX];
-  int    rows[WT];
-  int    info;
-};
+  *yh = __ddiv_rn (1.0, w);
+  *yl = __dmul_rn (__fma_rn (-w, *yh, 1.0), *yh);
+}
+
+/* delta in the range of the product form (or zero) */
+__device__ __forceinline__ bool
+_quot_ok (double delta)
+{
+  const uint32_t hi = (uint32_t) __double2hiint (delta) & 0x7fffffffu;
+
+  return (hi >> 20) - 128u < 1900u || (hi | (uint32_t) __double2loint (delta)) == 0u;
+}
+
+__device__ __forceinline__ double
+_quot (double delta, double yh, double yl)
+{
+  return __fma_rn (delta, yh, __dmul_rn (delta, yl));
+}
 
 /* (r, c), r < c, of the e-th strictly-upper element, row by row */
 __device__ __forceinline__ void
@@ -91,130 +122,158 @@ _upper_rc (int e, int d, int *r, int *c)
   *c = rr + 1 + rem;
 }
 
-/* Unit-weight Welford mean/covariance of X[rows[t]] for t < cnt (rows NULL:
- * row t), restating ncm_stats_vec.c:511-565 and get_cov_matrix :2376-2398.
- * Result (full symmetric, bias-corrected) in sm.A.  All threads call it. */
-__device__ void
-_welford_block (const double *__restrict__ X, const int32_t *__restrict__ rows, int cnt, int d, int nmax,
-                int32_t *bad, WelfordSmem &sm)
+/* The running means of all n rows: one CTA, warp 0 walks the chain (lane =
+ * coordinate, alone on its SM sub-partition's FP64 pipe), warp 1 adds the
+ * rows up in order beside it (the mixed form's anchor mu), warps 2 and 3 stage
+ * the next rows and reciprocals.  mean[t] (after row t) and R[t] go out for
+ * _welford_acc_kernel.  256 cycles a row: n = 8192, d = 16 takes 1.1 ms; one
+ * CTA with divisions, the covariance sums in the same pipes and a kernel of
+ * its own for mu took 7.2 ms. */
+#define WM_ROWS 64
+
+__global__ void __launch_bounds__ (PREP_THREADS)
+_welford_mean_kernel (const double *__restrict__ X, int n, int d, double *__restrict__ mean,
+                      double *__restrict__ Rq, double *__restrict__ mu)
 {
-  const int tid = threadIdx.x, nth = blockDim.x;
-  const int E   = d * (d - 1) / 2;
-  double Cacc[4];
-  int er[4], ec[4];
-  double mean = 0.0, var = 0.0;
+  __shared__ double xs[2][WM_ROWS][NCG_DMAX];
+  __shared__ double yh[2][WM_ROWS], yl[2][WM_ROWS];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int nch = (n + WM_ROWS - 1) / WM_ROWS;
+  double m = 0.0, sum = 0.0;
 
-#pragma unroll
-  for (int q = 0; q < 4; q++)
+  for (int ch = -1; ch < nch; ch++)
   {
-    const int e = tid + q * nth;
-
-    Cacc[q] = 0.0;
-    er[q]   = 0;
-    ec[q]   = 0;
-
-    if (e < E)
-      _upper_rc (e, d, &er[q], &ec[q]);
-  }
-
-  if (tid < d)
-    sm.mprev[tid] = 0.0;
-
-  for (int t0 = 0; t0 < cnt; t0 += WT)
-  {
-    const int tn = min (WT, cnt - t0);
-
-    __syncthreads ();
-
-    if (tid < tn)
+    if (w >= 2 && ch + 1 < nch)
     {
-      int r = rows ? rows[t0 + tid] : t0 + tid;
+      const int t0 = (ch + 1) * WM_ROWS, tn = min (WM_ROWS, n - t0), buf = (ch + 1) & 1;
 
-      if (r < 0 || r >= nmax)
-      {
-        atomicAdd (bad, 1);
-        r = 0;
-      }
+      for (int t = w - 2; t < tn; t += 2)
+        if (lane < d)
+          xs[buf][t][lane] = X[(size_t) (t0 + t) * d + lane];
 
-      sm.rows[tid] = r;
+      if (tid - 64 < tn)
+        _recip_pair ((double) (t0 + tid - 64) + 1.0, &yh[buf][tid - 64], &yl[buf][tid - 64]);
     }
-
-    __syncthreads ();
-
-    for (int idx = tid; idx < tn * d; idx += nth)
+    else if (w < 2 && ch >= 0 && lane < d)
     {
-      const int tt = idx / d, c = idx - tt * d;
+      const int t0 = ch * WM_ROWS, tn = min (WM_ROWS, n - t0), buf = ch & 1;
 
-      sm.xs[tt][c] = X[(size_t) sm.rows[tt] * d + c];
-    }
-
-    __syncthreads ();
-
-    if (tid < d)
-    {
-      for (int tt = 0; tt < tn; tt++)
+      if (w == 0)
       {
-        const double weight    = (double) (t0 + tt);
-        const double curweight = __dadd_rn (weight, 1.0);
-        const double delta     = __dsub_rn (sm.xs[tt][tid], mean);
-        const double R         = __ddiv_rn (delta, curweight);
-        const double dvar      = __dmul_rn (__dmul_rn (weight, delta), R);
+        const double m0 = m;
+        bool ok         = true;
+        double *mo = mean + (size_t) t0 * d + lane, *ro = Rq + (size_t) t0 * d + lane;
 
-        mean            = __dadd_rn (mean, R);
-        var             = __dadd_rn (var, dvar);
-        sm.mh[tt][tid]  = mean;
-      }
-    }
-
-    __syncthreads ();
-
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-    {
-      if (tid + q * nth < E)
-      {
-        const int r = er[q], c = ec[q];
-        double acc  = Cacc[q];
-
-        for (int tt = 0; tt < tn; tt++)
+#pragma unroll 8
+        for (int t = 0; t < tn; t++)
         {
-          const double a = __dsub_rn (sm.xs[tt][r], sm.mh[tt][r]);
-          const double b = __dsub_rn (sm.xs[tt][c], (tt > 0) ? sm.mh[tt - 1][c] : sm.mprev[c]);
+          const double delta = __dsub_rn (xs[buf][t][lane], m);
+          const double R     = _quot (delta, yh[buf][t], yl[buf][t]);
 
-          acc = __dadd_rn (acc, __dmul_rn (a, b));
+          ok = ok && _quot_ok (delta);
+          m  = __dadd_rn (m, R);
+          mo[(size_t) t * d] = m;
+          ro[(size_t) t * d] = R;
         }
 
-        Cacc[q] = acc;
+        if (!ok)
+        {
+          m = m0;
+
+          for (int t = 0; t < tn; t++)
+          {
+            const double delta = __dsub_rn (xs[buf][t][lane], m);
+            const double R     = __ddiv_rn (delta, (double) (t0 + t) + 1.0);
+
+            m = __dadd_rn (m, R);
+            mo[(size_t) t * d] = m;
+            ro[(size_t) t * d] = R;
+          }
+        }
+      }
+      else
+      {
+#pragma unroll 8
+        for (int t = 0; t < tn; t++)
+          sum = __dadd_rn (sum, xs[buf][t][lane]);
       }
     }
 
     __syncthreads ();
-
-    if (tid < d)
-      sm.mprev[tid] = sm.mh[tn - 1][tid];
   }
 
+  if (w == 1 && lane < d)
+    mu[lane] = __ddiv_rn (sum, (double) n);
+}
+
+/* The covariance sums from the running means: a CTA takes 32 of the
+ * d (d + 1) / 2 elements (off-diagonal ones row by row, then the variances).
+ * The products of different rows are independent; only the additions are a
+ * chain, so warp 0 adds (64 cycles a row, alone on its sub-partition: warp 4
+ * idles) what the other six warps multiply one chunk of rows ahead. */
+#define WA_ROWS 64
+#define WA_TH 256
+
+__global__ void __launch_bounds__ (WA_TH)
+_welford_acc_kernel (const double *__restrict__ X, const double *__restrict__ mean, const double *__restrict__ Rq,
+                     int n, int d, double *__restrict__ cov)
+{
+  __shared__ double prod[2][WA_ROWS][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int E    = d * (d - 1) / 2;
+  const int e    = blockIdx.x * 32 + lane;
+  const bool in  = e < E + d;
+  const bool var = e >= E;
+  const int pw   = (w < 4) ? w - 1 : w - 2;     /* producers: warps 1-3, 5-7 */
+  const int nch  = (n + WA_ROWS - 1) / WA_ROWS;
+  int r = 0, c = 0;
+  double acc = 0.0;
+
+  if (in && !var)
+    _upper_rc (e, d, &r, &c);
+  else if (in)
+    r = c = e - E;
+
+  for (int ch = -1; ch < nch; ch++)
   {
-    const double W    = (double) cnt;
-    const double bias = __ddiv_rn (1.0, __dsub_rn (W, __ddiv_rn (W, W)));
-
-#pragma unroll
-    for (int q = 0; q < 4; q++)
+    if (w == 0)
     {
-      if (tid + q * nth < E)
+      if (ch >= 0)
       {
-        const double v = __dmul_rn (Cacc[q], bias);
+        const int tn = min (WA_ROWS, n - ch * WA_ROWS);
 
-        sm.A[er[q] * d + ec[q]] = v;
-        sm.A[ec[q] * d + er[q]] = v;
+#pragma unroll 8
+        for (int t = 0; t < tn; t++)
+          acc = __dadd_rn (acc, prod[ch & 1][t][lane]);
+      }
+    }
+    else if (w != 4 && ch + 1 < nch && in)
+    {
+      const int t0 = (ch + 1) * WA_ROWS, tn = min (WA_ROWS, n - t0);
+
+#pragma unroll 4
+      for (int t = pw; t < tn; t += 6)
+      {
+        const size_t row   = (size_t) (t0 + t) * d;
+        const double delta = __dsub_rn (X[row + c], (t0 + t > 0) ? mean[row - d + c] : 0.0);
+        const double left  = var ? __dmul_rn ((double) (t0 + t), delta) : __dsub_rn (X[row + r], mean[row + r]);
+
+        prod[(ch + 1) & 1][t][lane] = __dmul_rn (left, var ? Rq[row + c] : delta);
       }
     }
 
-    if (tid < d)
-      sm.A[tid * d + tid] = __dmul_rn (var, bias);
+    __syncthreads ();
   }
 
-  __syncthreads ();
+  if (w == 0 && in)
+  {
+    const double W    = (double) n;
+    const double bias = __ddiv_rn (1.0, __dsub_rn (W, __ddiv_rn (W, W)));
+    const double v    = __dmul_rn (acc, bias);
+
+    cov[r * d + c] = v;
+    cov[c * d + r] = v;
+  }
 }
 
 /* In-place upper Cholesky of sm.A (Sigma = U^T U), column by column in the
@@ -274,6 +333,12 @@ _chol_block (double *A, int d, int *info)
   return 0;
 }
 
+struct CholSmem
+{
+  double A[NCG_DMAX * NCG_DMAX];
+  int    info;
+};
+
 /* frexp-guarded 2 ln det (ncm_matrix.c:1158-1186) */
 __device__ double
 _chol_lndet (const double *U, int d, int ld)
@@ -303,38 +368,38 @@ _chol_lndet (const double *U, int d, int ld)
   return 2.0 * (log (detL) + exponent * 0.69314718055994530941723212145818);
 }
 
-/* kernel lnnorm: ncm_stats_dist_kernel_gauss.c:201-207, ncm_stats_dist_kernel_st.c:240-252 */
+/* kernel lnnorm: ncm_stats_dist_kernel_gauss.c:201-207, ncm_stats_dist_kernel_st.c:240-252;
+ * _lnnorm0 is the Student-t form's part without the determinant (two
+ * lgammas), the same for every kernel of a launch */
 __device__ double
-_kernel_lnnorm (int kernel, double nu, int d, double lndet)
+_lnnorm0 (int kernel, double nu, int d)
+{
+  if (kernel == NCG_KERNEL_GAUSS)
+    return 0.0;
+
+  return (lgamma (nu / 2.0) - lgamma ((nu + d) / 2.0)) + (d / 2.0) * (NCG_LNPI + log (nu));
+}
+
+__device__ __forceinline__ double
+_lnnorm_of (int kernel, int d, double ln0, double lndet)
 {
   if (kernel == NCG_KERNEL_GAUSS)
     return 0.5 * (d * NCG_LN2PI + lndet);
 
-  return (lgamma (nu / 2.0) - lgamma ((nu + d) / 2.0)) + (d / 2.0) * (NCG_LNPI + log (nu)) + 0.5 * lndet;
+  return ln0 + 0.5 * lndet;
 }
 
 /* ------------------------------------------------------------------------ */
 
+/* upper Cholesky of the global covariance */
 __global__ void __launch_bounds__ (PREP_THREADS)
-_global_cov_chol_kernel (const double *__restrict__ X, int n, int d, double *cov, double *U,
-                         int32_t *flag, ncg_prep_status_t *st)
+_global_chol_kernel (const double *__restrict__ cov, int d, double *U, int32_t *flag, ncg_prep_status_t *st)
 {
-  __shared__ WelfordSmem sm;
+  __shared__ CholSmem sm;
   const int tid = threadIdx.x;
 
-  if (n > 0)
-  {
-    _welford_block (X, NULL, n, d, n, &st->n_badindex, sm);
-
-    for (int i = tid; i < d * d; i += blockDim.x)
-      cov[i] = sm.A[i];
-  }
-  else
-  {
-    /* fixed covariance supplied in cov (ncm_stats_dist_kde.c:825-845) */
-    for (int i = tid; i < d * d; i += blockDim.x)
-      sm.A[i] = cov[i];
-  }
+  for (int i = tid; i < d * d; i += blockDim.x)
+    sm.A[i] = cov[i];
 
   __syncthreads ();
 
@@ -365,10 +430,20 @@ _global_cov_chol_kernel (const double *__restrict__ X, int n, int d, double *cov
 }
 
 extern "C" cudaError_t
-ncg_launch_global_cov_chol (const double *X, int n, int d, double *cov, double *U, int32_t *flag,
-                            ncg_prep_status_t *st, cudaStream_t s)
+ncg_launch_global_chol (const double *cov, int d, double *U, int32_t *flag, ncg_prep_status_t *st, cudaStream_t s)
 {
-  _global_cov_chol_kernel<<<1, PREP_THREADS, 0, s>>> (X, n, d, cov, U, flag, st);
+  _global_chol_kernel<<<1, PREP_THREADS, 0, s>>> (cov, d, U, flag, st);
+
+  return cudaGetLastError ();
+}
+
+/* the sample covariance of n rows and their mean; mean and Rq: n x d work each */
+extern "C" cudaError_t
+ncg_launch_global_cov (const double *X, int n, int d, double *cov, double *mu, double *mean, double *Rq,
+                       cudaStream_t s)
+{
+  _welford_mean_kernel<<<1, PREP_THREADS, 0, s>>> (X, n, d, mean, Rq, mu);
+  _welford_acc_kernel<<<(d * (d + 1) / 2 + 31) / 32, WA_TH, 0, s>>> (X, mean, Rq, n, d, cov);
 
   return cudaGetLastError ();
 }
@@ -377,7 +452,7 @@ __global__ void
 _global_lnnorm_kernel (const double *U, int d, int kernel, double nu, ncg_prep_status_t *st)
 {
   if (threadIdx.x == 0 && blockIdx.x == 0)
-    st->kernel_lnnorm = _kernel_lnnorm (kernel, nu, d, _chol_lndet (U, d, d));
+    st->kernel_lnnorm = _lnnorm_of (kernel, d, _lnnorm0 (kernel, nu, d), _chol_lndet (U, d, d));
 }
 
 extern "C" cudaError_t
@@ -436,9 +511,22 @@ ncg_launch_whiten (const double *X, const double *U, int n, int d, double *Y, cu
 }
 
 /* ------------------------------------------------------------------------ */
-/* Exact kNN: all squared distances of one query into shared memory (or a    */
-/* per-CTA global slice for large n), MSB-first radix select of the k-th     */
-/* (distance, index) key, ordered compaction of ties, bitonic sort.          */
+/* Exact kNN, ordered by (FP64 squared distance, index).                      */
+/*                                                                          */
+/* FP64 distances to every point would cost 3 d n FP64 operations a query     */
+/* (5.1 of the 6.2 ms at n = 8192, d = 16), so _knn32_kernel screens the       */
+/* points on FP32 distances within a proven error and takes FP64 distances    */
+/* only of the ones that can be among the k nearest.  With v = Y - anchor      */
+/* and N = max |v|, the FP32 coordinates are off by 2^-24 |v| each, so the      */
+/* FP32 difference vector is off by e <= 2^-22 N (conversion of both ends and  */
+/* the subtraction), and the sum of its squares by a relative (d + 1) 2^-24   */
+/* <= g = 2^-18.  If k points have FP32 sums <= T, the k-th FP64 distance is  */
+/* at most sqrt (T (1 + g)) + e, and every point that near has an FP32 sum of  */
+/* at most (sqrt (T (1 + g)) + 2 e)^2 / (1 - g); the code uses 2 e and 2 g,    */
+/* which also covers the FP64 roundings.  T comes from a bisection on counts, */
+/* stopped once the list fits its room, so k plus a few FP64 distances are   */
+/* taken.  A query whose list overflows (many equal or nearly equal            */
+/* distances) or whose coordinates leave the FP32 range goes to _knn_kernel.  */
 /* ------------------------------------------------------------------------ */
 
 #define KNN_THREADS 512
@@ -455,9 +543,13 @@ _pow2_ceil (int k)
   return p;
 }
 
+/* All squared distances of one query in FP64, into shared memory (or a
+ * per-CTA global slice for large n), MSB-first radix select of the k-th
+ * (distance, index) key, ordered compaction of ties, bitonic sort.  The queries
+ * are list[0 .. *count), or all nq (list NULL). */
 __global__ void __launch_bounds__ (KNN_THREADS)
 _knn_kernel (const double *__restrict__ Y, int n, int nq, int d, int k, int kp2, int32_t *__restrict__ out,
-             uint64_t *__restrict__ gkeys)
+             uint64_t *__restrict__ gkeys, const int32_t *__restrict__ list, const int32_t *__restrict__ count)
 {
   extern __shared__ __align__ (16) unsigned char knn_smem[];
   __shared__ double yq[NCG_DMAX];
@@ -471,8 +563,12 @@ _knn_kernel (const double *__restrict__ Y, int n, int nq, int d, int k, int kp2,
   int32_t *seli  = (int32_t *) (selk + kp2);
   uint64_t *keys = gkeys ? gkeys + (size_t) blockIdx.x * n : (uint64_t *) (seli + kp2 + (kp2 & 1));
 
-  for (int q = blockIdx.x; q < nq; q += gridDim.x)
+  const int nlist = list ? *count : nq;
+
+  for (int iq = blockIdx.x; iq < nlist; iq += gridDim.x)
   {
+    const int q = list ? list[iq] : iq;
+
     __syncthreads ();
 
     if (tid < d)
@@ -660,100 +756,599 @@ _knn_kernel (const double *__restrict__ Y, int n, int nq, int d, int k, int kp2,
   }
 }
 
+/* The FP32 coordinates of the screen, Yt[c][j] = fl32 (Y[j][c] - anchor[c]) for
+ * j < npad (0 past n), the anchor being the mean of 32 spread rows, and
+ * nmax2 = the float bits of (an upper bound of) the largest |Y - anchor|^2. */
+#define Y32_TH 256
+
+__global__ void __launch_bounds__ (Y32_TH)
+_y32_kernel (const double *__restrict__ Y, int n, int npad, int d, float *__restrict__ Yt,
+             int32_t *__restrict__ nmax2)
+{
+  __shared__ double an[NCG_DMAX];
+  __shared__ float red[Y32_TH / 32];
+  const int tid = threadIdx.x;
+
+  if (tid < d)
+  {
+    double s = 0.0;
+
+    for (int i = 0; i < 32; i++)
+      s += Y[(size_t) ((int64_t) i * n / 32) * d + tid];
+
+    an[tid] = s * (1.0 / 32.0);
+  }
+
+  __syncthreads ();
+
+  const int j = blockIdx.x * Y32_TH + tid;
+  float s2    = 0.0f;
+
+  if (j < npad)
+    for (int c = 0; c < d; c++)
+    {
+      const float v = (j < n) ? __double2float_rn (Y[(size_t) j * d + c] - an[c]) : 0.0f;
+
+      s2 = fmaf (v, v, s2);
+      Yt[(size_t) c * npad + j] = v;
+    }
+
+  s2 *= 1.0f + 0x1p-17f;
+
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    s2 = fmaxf (s2, __shfl_xor_sync (0xffffffffu, s2, o));
+
+  if ((tid & 31) == 0)
+    red[tid >> 5] = s2;
+
+  __syncthreads ();
+
+  if (tid == 0)
+  {
+    for (int w = 1; w < Y32_TH / 32; w++)
+      s2 = fmaxf (s2, red[w]);
+
+    atomicMax (nmax2, __float_as_int (s2));
+  }
+}
+
+__device__ __forceinline__ void
+_bar_group (int id, int threads)
+{
+  asm volatile ("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+/* QT queries per CTA: their FP32 sums together (each coordinate row is read
+ * once for the QT), then KNN_THREADS / QT threads per query select, measure
+ * and sort. */
+template <int QT>
+__global__ void __launch_bounds__ (KNN_THREADS)
+_knn32_kernel (const double *__restrict__ Y, const float *__restrict__ Yt, int n, int npad, int nq, int d, int k,
+               int cap, const int32_t *__restrict__ nmax2, int32_t *__restrict__ out, int32_t *__restrict__ count,
+               int32_t *__restrict__ list)
+{
+  extern __shared__ __align__ (16) unsigned char knn_smem[];
+  __shared__ float yq[NCG_DMAX][QT];
+  __shared__ int red[2][QT][KNN_THREADS / QT / 32];
+  __shared__ int s_cnt[QT];
+  constexpr int GT = KNN_THREADS / QT, GW = GT / 32;
+  const int tid = threadIdx.x, g = tid / GT, gt = tid - g * GT, gw = gt >> 5, lane = tid & 31;
+  float *keys    = (float *) knn_smem;                                  /* [QT][npad] */
+  uint64_t *selk = (uint64_t *) (keys + (size_t) QT * npad) + (size_t) g * cap;
+  int32_t *seli  = (int32_t *) ((uint64_t *) (keys + (size_t) QT * npad) + (size_t) QT * cap) + (size_t) g * cap;
+
+  const int q0 = blockIdx.x * QT;
+
+  for (int e = tid; e < d * QT; e += KNN_THREADS)
+    yq[e / QT][e % QT] = (q0 + e % QT < nq) ? Yt[(size_t) (e / QT) * npad + q0 + e % QT] : 0.0f;
+
+  if (gt == 0)
+    s_cnt[g] = 0;
+
+  __syncthreads ();
+
+  for (int j = tid * 4; j < npad; j += KNN_THREADS * 4)
+  {
+    float s[QT][4];
+
+#pragma unroll
+    for (int q = 0; q < QT; q++)
+#pragma unroll
+      for (int e = 0; e < 4; e++)
+        s[q][e] = 0.0f;
+
+#pragma unroll 4
+    for (int c = 0; c < d; c++)
+    {
+      const float4 v = *(const float4 *) (Yt + (size_t) c * npad + j);
+
+#pragma unroll
+      for (int q = 0; q < QT; q++)
+      {
+        const float y = yq[c][q];
+        const float t0 = v.x - y, t1 = v.y - y, t2 = v.z - y, t3 = v.w - y;
+
+        s[q][0] = fmaf (t0, t0, s[q][0]);
+        s[q][1] = fmaf (t1, t1, s[q][1]);
+        s[q][2] = fmaf (t2, t2, s[q][2]);
+        s[q][3] = fmaf (t3, t3, s[q][3]);
+      }
+    }
+
+#pragma unroll
+    for (int q = 0; q < QT; q++)
+    {
+#pragma unroll
+      for (int e = 0; e < 4; e++)
+        if (j + e >= n)
+          s[q][e] = CUDART_INF_F;
+
+      *(float4 *) (keys + (size_t) q * npad + j) = make_float4 (s[q][0], s[q][1], s[q][2], s[q][3]);
+    }
+  }
+
+  __syncthreads ();
+
+  const int q = q0 + g;
+
+  if (q >= nq)
+    return;
+
+  const float *kg = keys + (size_t) g * npad;
+  const float nm  = __int_as_float (*nmax2);
+  const double e2 = 2.0 * 0x1p-22 * sqrt ((double) nm), g2 = 2.0 * 0x1p-18;
+  const int slack = (cap - k) / 2;
+  uint32_t lo = 0, hi = 0x7f7fffffu;      /* count (T = lo) < k unless lo = 0; count (hi) >= k once checked */
+  bool have = false;
+
+  /* count of sums <= the float of bits `mid` */
+  for (int it = 0; it < 40 && (lo < hi || !have); it++)
+  {
+    const uint32_t mid = have ? lo + (hi - lo) / 2 : hi;
+    const float T      = __uint_as_float (mid);
+    int cnt            = 0;
+
+    for (int j = gt * 4; j < npad; j += GT * 4)
+    {
+      const float4 v = *(const float4 *) (kg + j);
+
+      cnt += (v.x <= T) + (v.y <= T) + (v.z <= T) + (v.w <= T);
+    }
+
+    cnt = __reduce_add_sync (0xffffffffu, cnt);
+
+    if (lane == 0)
+      red[it & 1][g][gw] = cnt;
+
+    _bar_group (1 + g, GT);
+    cnt = 0;
+
+#pragma unroll
+    for (int w = 0; w < GW; w++)
+      cnt += red[it & 1][g][w];
+
+    if (cnt >= k)
+    {
+      hi   = mid;
+      have = true;
+
+      if (cnt <= k + slack)
+        break;
+    }
+    else if (!have)
+      break;      /* fewer than k finite sums */
+    else
+      lo = mid + 1;
+  }
+
+  /* the bounds hold while no square can leave FP32's normal range unnoticed */
+  bool ok = have && nm >= 0x1p-60f && nm <= 0x1p+100f;
+
+  if (ok)
+  {
+    const double r    = sqrt ((double) __uint_as_float (hi) * (1.0 + g2)) + 2.0 * e2;
+    const double cut  = r * r / (1.0 - g2);
+    const float cutf  = __double2float_ru (cut);
+
+    for (int j = gt; j < n; j += GT)
+      if (kg[j] <= cutf)
+      {
+        const int pos = atomicAdd (&s_cnt[g], 1);
+
+        if (pos < cap)
+          seli[pos] = j;
+      }
+
+    _bar_group (1 + g, GT);
+    ok = s_cnt[g] <= cap;
+  }
+
+  if (!ok)
+  {
+    if (gt == 0)
+      list[atomicAdd (count, 1)] = q;
+
+    return;
+  }
+
+  const int nc = s_cnt[g];
+
+  /* FP64 squared distances summed in coordinate order, candidate minus query */
+  for (int t = gt; t < cap; t += GT)
+  {
+    uint64_t key = ~0ULL;
+
+    if (t < nc)
+    {
+      const double *p = Y + (size_t) seli[t] * d, *yd = Y + (size_t) q * d;
+      double dist     = 0.0;
+
+#pragma unroll 4
+      for (int c = 0; c < d; c++)
+      {
+        const double df = __dsub_rn (p[c], yd[c]);
+
+        dist = __dadd_rn (dist, __dmul_rn (df, df));
+      }
+
+      key = (uint64_t) __double_as_longlong (dist);
+    }
+    else
+      seli[t] = 0x7fffffff;
+
+    selk[t] = key;
+  }
+
+  _bar_group (1 + g, GT);
+
+  /* bitonic sort of (key, index) ascending */
+  for (int size = 2; size <= cap; size <<= 1)
+    for (int stride = size >> 1; stride > 0; stride >>= 1)
+    {
+      for (int h = gt; h < cap / 2; h += GT)
+      {
+        const int t = 2 * h - (h & (stride - 1)), u = t + stride;
+        const uint64_t ka = selk[t], kb = selk[u];
+        const int32_t ia = seli[t], ib = seli[u];
+        const bool gt_ = (ka > kb) || (ka == kb && ia > ib);
+
+        if (gt_ == ((t & size) == 0))
+        {
+          selk[t] = kb;
+          selk[u] = ka;
+          seli[t] = ib;
+          seli[u] = ia;
+        }
+      }
+
+      _bar_group (1 + g, GT);
+    }
+
+  for (int t = gt; t < k; t += GT)
+    out[(size_t) q * k + t] = seli[t];
+}
+
+static inline int
+_knn_npad (int n)
+{
+  return (n + 3) / 4 * 4;
+}
+
+/* room of the screened list: the next power of two with an eighth (32 at
+ * least) to spare */
+static inline int
+_knn_cap (int k)
+{
+  return _pow2_ceil (k + (k / 8 > 32 ? k / 8 : 32));
+}
+
+#define KNN32_SMEM (200 * 1024)
+
+static inline size_t
+_knn32_smem (int qt, int n, int k)
+{
+  return (size_t) qt * ((size_t) _knn_npad (n) * sizeof (float) + (size_t) _knn_cap (k) * 12);
+}
+
+/* [Yt: d npad floats | nmax2, count | list: n ints | pad to 256 | FP64 keys of the large-n form] */
+static inline size_t
+_knn_screen_bytes (int n, int d)
+{
+  return (((size_t) d * _knn_npad (n) + 4 + (size_t) n) * 4 + 255) / 256 * 256;
+}
+
 extern "C" size_t
 ncg_knn_scratch_bytes (int n, int d, int k)
 {
-  (void) d;
   (void) k;
 
-  if (n <= KNN_SMEM_NMAX)
-    return 0;
+  return _knn_screen_bytes (n, d) + (n <= KNN_SMEM_NMAX ? 0 : (size_t) 4 * 152 * (size_t) n * sizeof (uint64_t));
+}
 
-  return (size_t) 4 * 152 * (size_t) n * sizeof (uint64_t);
+template <int QT>
+static cudaError_t
+_run_knn32 (const double *Y, const float *Yt, int n, int nq, int d, int k, const int32_t *meta, int32_t *knn,
+            int32_t *count, int32_t *list, cudaStream_t s)
+{
+  static int limit[NCG_MAX_DEVICES];
+  const size_t smem = _knn32_smem (QT, n, k);
+  cudaError_t e     = ncg_raise_smem_limit ((const void *) _knn32_kernel<QT>, smem, limit);
+
+  if (e != cudaSuccess)
+    return e;
+
+  _knn32_kernel<QT><<<(nq + QT - 1) / QT, KNN_THREADS, smem, s>>> (Y, Yt, n, _knn_npad (n), nq, d, k, _knn_cap (k),
+                                                                  meta, knn, count, list);
+
+  return cudaGetLastError ();
 }
 
 /* the k nearest of the n points Y to each of the first nq of them (the
  * kernels; with a split cross-validation the other observations only enter
- * as neighbours) */
+ * as neighbours); scratch of ncg_knn_scratch_bytes */
 extern "C" cudaError_t
-ncg_launch_knn (const double *Y, int n, int nq, int d, int k, int32_t *knn, uint64_t *keys_scratch, cudaStream_t s)
+ncg_launch_knn (const double *Y, int n, int nq, int d, int k, int32_t *knn, uint64_t *scratch, cudaStream_t s)
 {
   const int kp2      = _pow2_ceil (k);
   const bool in_smem = (n <= KNN_SMEM_NMAX);
   size_t smem        = (size_t) kp2 * (sizeof (uint64_t) + sizeof (int32_t)) + 8;
   int grid           = nq;
+  cudaError_t e;
 
-  if (k > NCG_KNN_KMAX || k > n || nq > n || nq <= 0)
+  if (k > NCG_KNN_KMAX || k > n || nq > n || nq <= 0 || scratch == NULL)
     return cudaErrorInvalidValue;
+
+  float *Yt       = (float *) scratch;
+  int32_t *meta   = (int32_t *) (Yt + (size_t) d * _knn_npad (n)), *list = meta + 4;
+  uint64_t *gkeys = (uint64_t *) ((char *) scratch + _knn_screen_bytes (n, d));
+  /* the screen while one query's sums fit an SM (n <= 46000 or so); four
+   * queries share a pass over the coordinates where four fit */
+  const bool screen = _knn32_smem (1, n, k) <= KNN32_SMEM;
+
+  if (screen)
+  {
+    if ((e = cudaMemsetAsync (meta, 0, 4 * sizeof (int32_t), s)) != cudaSuccess)
+      return e;
+
+    _y32_kernel<<<(_knn_npad (n) + Y32_TH - 1) / Y32_TH, Y32_TH, 0, s>>> (Y, n, _knn_npad (n), d, Yt, meta);
+
+    if ((e = cudaGetLastError ()) != cudaSuccess)
+      return e;
+
+    if (_knn32_smem (4, n, k) <= KNN32_SMEM)
+      e = _run_knn32<4> (Y, Yt, n, nq, d, k, meta, knn, meta + 1, list, s);
+    else if (_knn32_smem (2, n, k) <= KNN32_SMEM)
+      e = _run_knn32<2> (Y, Yt, n, nq, d, k, meta, knn, meta + 1, list, s);
+    else
+      e = _run_knn32<1> (Y, Yt, n, nq, d, k, meta, knn, meta + 1, list, s);
+
+    if (e != cudaSuccess)
+      return e;
+  }
 
   if (in_smem)
     smem += (size_t) n * sizeof (uint64_t);
-  else
-  {
-    if (keys_scratch == NULL)
-      return cudaErrorInvalidValue;
 
-    grid = (nq < 4 * 152) ? nq : 4 * 152;
-  }
+  if ((!in_smem || screen) && grid > 4 * 152)
+    grid = 4 * 152;
 
   /* raised whatever the size: the kernel's static arrays count against the
    * 48 KiB default too */
   static int limit[NCG_MAX_DEVICES];
-  cudaError_t e = ncg_raise_smem_limit ((const void *) _knn_kernel, smem, limit);
+
+  e = ncg_raise_smem_limit ((const void *) _knn_kernel, smem, limit);
 
   if (e != cudaSuccess)
     return e;
 
-  _knn_kernel<<<grid, KNN_THREADS, smem, s>>> (Y, n, nq, d, k, kp2, knn, in_smem ? NULL : keys_scratch);
+  _knn_kernel<<<grid, KNN_THREADS, smem, s>>> (Y, n, nq, d, k, kp2, knn, in_smem ? NULL : gkeys,
+                                               screen ? list : NULL, screen ? meta + 1 : NULL);
 
   return cudaGetLastError ();
 }
 
 /* ------------------------------------------------------------------------ */
 
+/* Local covariances and factors, 4 kpw kernels per CTA.  Rows are staged 16
+ * at a time for all of them; a warp walks the mean chains of kpw kernels (lane
+ * = kernel x coordinate: a warp instruction costs the same however few lanes
+ * work, so d = 16 takes two kernels per warp), then the CTA's threads add
+ * the off-diagonal products, each thread Q elements of the 4 kpw d (d - 1) / 2
+ * in registers, and each warp factors its kernels, lane = column.  Counted in
+ * FP64 warp instructions per kernel and row at d = 16: 4 for the chain and 7.5
+ * for the products, where one CTA per kernel with divisions took 30; the rate
+ * of the FP64 pipes bounds it (n = 8192, k = 409: 7.3 ms before, 2.4 ms now). */
+#define LC_ROWS 16
+
+template <int Q>
 __global__ void __launch_bounds__ (PREP_THREADS)
 _local_cov_chol_kernel (const double *__restrict__ X, const int32_t *__restrict__ knn, int n, int nq, int d, int k,
-                        double *__restrict__ Ui, int32_t *__restrict__ flag, ncg_prep_status_t *st)
+                        int kpw, double *__restrict__ Ui, int32_t *__restrict__ flag, ncg_prep_status_t *st)
 {
-  __shared__ WelfordSmem sm;
-  const int tid = threadIdx.x;
+  __shared__ double buf[2 * 4 * 32 * LC_ROWS];      /* 4 kpw d <= 128 columns of xs and of delta */
+  __shared__ double yh[LC_ROWS], yl[LC_ROWS];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int kb = 4 * kpw, E = d * (d - 1) / 2, kd = LC_ROWS * d;
+  const int i0 = blockIdx.x * kb;
+  double *xs = buf, *dl = buf + kb * kd;
 
-  for (int i = blockIdx.x; i < nq; i += gridDim.x)
+  /* chain lane: kernel gk of the CTA, coordinate gc */
+  const bool chain = lane < kpw * d && i0 + w * kpw + lane / d < nq;
+  const int gk = chain ? w * kpw + lane / d : 0, gc = chain ? lane % d : 0;
+  double m = 0.0, var = 0.0;
+
+  /* product elements */
+  double acc[Q];
+  int oa[Q], ob[Q];
+
+#pragma unroll
+  for (int q = 0; q < Q; q++)
   {
-    double *Uo = Ui + (size_t) i * d * d;
+    const int e = tid + q * PREP_THREADS;
 
-    _welford_block (X, knn + (size_t) i * k, k, d, n, &st->n_badindex, sm);
+    acc[q] = 0.0;
+    oa[q]  = 0;
+    ob[q]  = 0;
 
-    /* keep the covariance in the output slot until the factor succeeds */
-    for (int e = tid; e < d * d; e += blockDim.x)
-      Uo[e] = sm.A[e];
+    if (e < kb * E)
+    {
+      int r, c;
+
+      _upper_rc (e % E, d, &r, &c);
+      oa[q] = (e / E) * kd + r;
+      ob[q] = (e / E) * kd + c;
+    }
+  }
+
+  for (int t0 = 0; t0 < k; t0 += LC_ROWS)
+  {
+    const int tn = min (LC_ROWS, k - t0);
 
     __syncthreads ();
 
-    const int info = _chol_block (sm.A, d, &sm.info);
-
-    if (info != 0)
+    for (int idx = tid; idx < kb * kd; idx += PREP_THREADS)
     {
-      if (tid == 0)
+      const int kk = idx / kd, rem = idx - kk * kd, t = rem / d, c = rem - t * d;
+      double x = 0.0;
+
+      if (t < tn && i0 + kk < nq)
       {
-        flag[i] = 1;
+        int r = knn[(size_t) (i0 + kk) * k + t0 + t];
+
+        if (r < 0 || r >= n)
+        {
+          if (c == 0)
+            atomicAdd (&st->n_badindex, 1);
+
+          r = 0;
+        }
+
+        x = X[(size_t) r * d + c];
+      }
+
+      xs[idx] = x;
+    }
+
+    if (tid < tn)
+      _recip_pair ((double) (t0 + tid) + 1.0, &yh[tid], &yl[tid]);
+
+    __syncthreads ();
+
+    if (chain)
+    {
+      double *px = xs + gk * kd + gc, *pd = dl + gk * kd + gc;
+
+#pragma unroll 4
+      for (int t = 0; t < tn; t++)
+      {
+        const double x     = px[t * d];
+        const double delta = __dsub_rn (x, m);
+        double R           = _quot (delta, yh[t], yl[t]);
+
+        if (!_quot_ok (delta))
+          R = __ddiv_rn (delta, (double) (t0 + t) + 1.0);
+
+        m         = __dadd_rn (m, R);
+        var       = __dadd_rn (var, __dmul_rn (__dmul_rn ((double) (t0 + t), delta), R));
+        px[t * d] = __dsub_rn (x, m);
+        pd[t * d] = delta;
+      }
+    }
+
+    __syncthreads ();
+
+#pragma unroll 2
+    for (int t = 0; t < tn; t++)
+    {
+#pragma unroll
+      for (int q = 0; q < Q; q++)
+        acc[q] = __dadd_rn (acc[q], __dmul_rn (xs[oa[q] + t * d], dl[ob[q] + t * d]));
+    }
+  }
+
+  /* the covariances, d x d per kernel, over the staging buffer */
+  const double W    = (double) k;
+  const double bias = __ddiv_rn (1.0, __dsub_rn (W, __ddiv_rn (W, W)));
+  double *cov       = buf;
+
+  __syncthreads ();
+
+#pragma unroll
+  for (int q = 0; q < Q; q++)
+  {
+    const int e = tid + q * PREP_THREADS;
+
+    if (e < kb * E)
+    {
+      const int kk   = e / E, r = oa[q] - kk * kd, c = ob[q] - kk * kd;
+      const double v = __dmul_rn (acc[q], bias);
+
+      cov[kk * d * d + r * d + c] = v;
+      cov[kk * d * d + c * d + r] = v;
+    }
+  }
+
+  if (chain)
+    cov[gk * d * d + gc * d + gc] = __dmul_rn (var, bias);
+
+  __syncthreads ();
+
+  /* the covariance stays in the output slot unless the factor succeeds */
+  for (int idx = tid; idx < kb * d * d; idx += PREP_THREADS)
+    if (i0 + idx / (d * d) < nq)
+      Ui[(size_t) i0 * d * d + idx] = cov[idx];
+
+  __syncthreads ();
+
+  /* upper Cholesky in the order of _chol_block, row j of every kernel of the
+   * warp at once (idle lanes follow with kernel 0's row) */
+  double *A   = cov + gk * d * d;
+  const int g = (lane / d) * d;     /* first lane of this kernel */
+  bool ok     = true;
+
+  for (int j = 0; j < d; j++)
+  {
+    const bool mine = chain && gc >= j;
+    double v        = mine ? A[j * d + gc] : 1.0;
+
+    if (mine)
+      for (int q = 0; q < j; q++)
+        v = __dsub_rn (v, __dmul_rn (A[q * d + j], A[q * d + gc]));
+
+    const double piv = __shfl_sync (0xffffffffu, v, (g + j) & 31);
+
+    ok = ok && piv > 0.0;
+
+    if (mine && ok)
+    {
+      const double u = __dsqrt_rn (piv);
+
+      A[j * d + gc] = (gc == j) ? u : __ddiv_rn (v, u);
+    }
+
+    __syncwarp ();
+  }
+
+  if (chain)
+  {
+    const int i = i0 + gk;
+
+    if (ok)
+    {
+      double *Uo = Ui + (size_t) i * d * d;
+
+      for (int r = 0; r < d; r++)
+        Uo[r * d + gc] = (gc >= r) ? A[r * d + gc] : 0.0;
+    }
+
+    if (gc == 0)
+    {
+      flag[i] = ok ? 0 : 1;
+
+      if (!ok)
         atomicAdd (&st->n_flagged, 1);
-      }
     }
-    else
-    {
-      for (int e = tid; e < d * d; e += blockDim.x)
-      {
-        const int r = e / d, c = e - r * d;
-
-        Uo[e] = (c >= r) ? sm.A[e] : 0.0;
-      }
-
-      if (tid == 0)
-        flag[i] = 0;
-    }
-
-    __syncthreads ();
   }
 }
 
@@ -763,9 +1358,29 @@ extern "C" cudaError_t
 ncg_launch_local_cov_chol (const double *X, const int32_t *knn, int n, int nq, int d, int k, double *Ui,
                            int32_t *flag, ncg_prep_status_t *st, cudaStream_t s)
 {
-  const int grid = (nq < 152 * 16) ? nq : 152 * 16;
+  int kpw = (d >= 4) ? 32 / d : 8;
 
-  _local_cov_chol_kernel<<<grid, PREP_THREADS, 0, s>>> (X, knn, n, nq, d, k, Ui, flag, st);
+  /* fewer kernels per warp while the CTAs would not give every SM two */
+  while (kpw > 1 && (nq + 4 * kpw - 1) / (4 * kpw) < 2 * 152)
+    kpw = (kpw + 1) / 2;
+
+  const int grid = (nq + 4 * kpw - 1) / (4 * kpw);
+  const int q    = (4 * kpw * (d * (d - 1) / 2) + PREP_THREADS - 1) / PREP_THREADS;
+
+#define LC_RUN(Q) _local_cov_chol_kernel<Q><<<grid, PREP_THREADS, 0, s>>> (X, knn, n, nq, d, k, kpw, Ui, flag, st)
+
+  if (q <= 2)
+    LC_RUN (2);
+  else if (q <= 4)
+    LC_RUN (4);
+  else if (q <= 6)
+    LC_RUN (6);
+  else if (q <= 8)
+    LC_RUN (8);
+  else if (q <= 12)
+    LC_RUN (12);
+  else
+    LC_RUN (16);
 
   return cudaGetLastError ();
 }
@@ -775,7 +1390,7 @@ ncg_launch_local_cov_chol (const double *X, const int32_t *knn, int n, int nq, i
 __global__ void __launch_bounds__ (PREP_THREADS)
 _chol_slots_kernel (double *__restrict__ Ui, int n, int d, int32_t *__restrict__ flag, ncg_prep_status_t *st)
 {
-  __shared__ WelfordSmem sm;
+  __shared__ CholSmem sm;
   const int tid = threadIdx.x;
 
   for (int i = blockIdx.x; i < n; i += gridDim.x)
@@ -1102,6 +1717,7 @@ _vkde_finish_kernel (const double *__restrict__ X, const double *__restrict__ Ui
   const int dp   = ncg_pad_dim (d);
   const int P    = dp * (dp + 1) / 2;
   const int S    = dp + P;
+  const double ln0 = _lnnorm0 (kernel, nu, d);   /* the kernel's constant, with its lgammas, once */
 
   for (int i = blockIdx.x * FIN_WARPS + w; i < n; i += gridDim.x * FIN_WARPS)
   {
@@ -1135,24 +1751,12 @@ _vkde_finish_kernel (const double *__restrict__ X, const double *__restrict__ Ui
     for (int e = lane; e < dp; e += 32)
       pk[e] = (e < d) ? X[(size_t) i * d + e] : 0.0;
 
-    for (int e = lane; e < P; e += 32)
-    {
-      /* e -> (r, c), c <= r, packed by rows */
-      int r = (int) ((sqrt (8.0 * e + 1.0) - 1.0) * 0.5);
-
-      while (r * (r + 1) / 2 > e)
-        r--;
-
-      while ((r + 1) * (r + 2) / 2 <= e)
-        r++;
-
-      const int c = e - r * (r + 1) / 2;
-
-      pk[dp + e] = (r < d && c < d) ? sW[w][r * d + c] * inv_href : 0.0;
-    }
+    for (int r = 0; r < dp; r++)
+      if (lane <= r)
+        pk[dp + r * (r + 1) / 2 + lane] = (r < d && lane < d) ? sW[w][r * d + lane] * inv_href : 0.0;
 
     if (lane == 0)
-      lnnorm[i] = _kernel_lnnorm (kernel, nu, d, _chol_lndet (sU[w], d, d));
+      lnnorm[i] = _lnnorm_of (kernel, d, ln0, _chol_lndet (sU[w], d, d));
 
     __syncwarp ();
   }
@@ -1175,91 +1779,19 @@ ncg_launch_vkde_finish (const double *X, double *Ui, const int32_t *flag, int n,
 
 /* KDE operand: whitened centres / h (dp), and Vg = U^{-T}/h packed lower for
  * whitening the evaluation points. */
-__global__ void
-_kde_finish_kernel (const double *__restrict__ Y, const double *__restrict__ U, int n, int d,
-                    double inv_href, double *__restrict__ pack, double *__restrict__ Vg)
+/* Vg = scale U^{-T}, packed lower by rows with dp padding, by one warp: lane c
+ * computes column c of W = U^{-T}, so the d(d+1)/2 products and the divisions
+ * of a serial inverse (97 us at d = 16, one lane) run d at a time; W: d x d
+ * shared work */
+__device__ __forceinline__ void
+_vg_warp (const double *__restrict__ U, int d, double scale, double *__restrict__ Vg, double *W)
 {
-  const int dp = ncg_pad_dim (d);
-  const int i  = blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31, dp = ncg_pad_dim (d);
 
-  if (i < n)
-    for (int e = 0; e < dp; e++)
-      pack[(size_t) i * dp + e] = (e < d) ? Y[(size_t) i * d + e] * inv_href : 0.0;
-
-  if (blockIdx.x == 0 && threadIdx.x == 0)
+  if (lane < d)
   {
-    double W[NCG_DMAX * NCG_DMAX];
+    const int c = lane;
 
-    for (int c = 0; c < d; c++)
-    {
-      W[c * d + c] = 1.0 / U[c * d + c];
-
-      for (int r = c + 1; r < d; r++)
-      {
-        double s = 0.0;
-
-        for (int m = c; m < r; m++)
-          s += U[m * d + r] * W[m * d + c];
-
-        W[r * d + c] = -s / U[r * d + r];
-      }
-    }
-
-    int e = 0;
-
-    for (int r = 0; r < dp; r++)
-      for (int c = 0; c <= r; c++)
-        Vg[e++] = (r < d && c < d) ? W[r * d + c] * inv_href : 0.0;
-  }
-}
-
-extern "C" cudaError_t
-ncg_launch_kde_finish (const double *Y, const double *U, int n, int d, double href, double *pack64,
-                       double *Vg, cudaStream_t s)
-{
-  _kde_finish_kernel<<<(n + 127) / 128, 128, 0, s>>> (Y, U, n, d, 1.0 / href, pack64, Vg);
-
-  return cudaGetLastError ();
-}
-
-/* mean of the centres, one thread per coordinate (the anchor of the mixed form) */
-__global__ void
-_mean_kernel (const double *__restrict__ X, int n, int d, double *__restrict__ mu)
-{
-  const int c = threadIdx.x;
-
-  if (c >= d)
-    return;
-
-  double s = 0.0;
-
-  for (int i = 0; i < n; i++)
-    s += X[(size_t) i * d + c];
-
-  mu[c] = s / n;
-}
-
-extern "C" cudaError_t
-ncg_launch_mean (const double *X, int n, int d, double *mu, cudaStream_t s)
-{
-  _mean_kernel<<<1, 32, 0, s>>> (X, n, d, mu);
-
-  return cudaGetLastError ();
-}
-
-/* Vg = scale * U^{-T}, packed lower by rows with dp padding (the global
- * whitening of the evaluation points) */
-__global__ void
-_global_vg_kernel (const double *__restrict__ U, int d, double scale, double *__restrict__ Vg)
-{
-  if (blockIdx.x != 0 || threadIdx.x != 0)
-    return;
-
-  const int dp = ncg_pad_dim (d);
-  double W[NCG_DMAX * NCG_DMAX];
-
-  for (int c = 0; c < d; c++)
-  {
     W[c * d + c] = 1.0 / U[c * d + c];
 
     for (int r = c + 1; r < d; r++)
@@ -1273,11 +1805,88 @@ _global_vg_kernel (const double *__restrict__ U, int d, double scale, double *__
     }
   }
 
-  int e = 0;
+  __syncwarp ();
 
   for (int r = 0; r < dp; r++)
-    for (int c = 0; c <= r; c++)
-      Vg[e++] = (r < d && c < d) ? W[r * d + c] * scale : 0.0;
+    if (lane <= r)
+      Vg[r * (r + 1) / 2 + lane] = (r < d && lane < d) ? W[r * d + lane] * scale : 0.0;
+}
+
+__global__ void __launch_bounds__ (128)
+_kde_finish_kernel (const double *__restrict__ Y, const double *__restrict__ U, int n, int d,
+                    double inv_href, double *__restrict__ pack, double *__restrict__ Vg)
+{
+  __shared__ double W[NCG_DMAX * NCG_DMAX];
+  const int dp = ncg_pad_dim (d);
+  const int i  = blockIdx.x * blockDim.x + threadIdx.x;
+
+  if (i < n)
+    for (int e = 0; e < dp; e++)
+      pack[(size_t) i * dp + e] = (e < d) ? Y[(size_t) i * d + e] * inv_href : 0.0;
+
+  if (blockIdx.x == 0 && threadIdx.x < 32)
+    _vg_warp (U, d, inv_href, Vg, W);
+}
+
+extern "C" cudaError_t
+ncg_launch_kde_finish (const double *Y, const double *U, int n, int d, double href, double *pack64,
+                       double *Vg, cudaStream_t s)
+{
+  _kde_finish_kernel<<<(n + 127) / 128, 128, 0, s>>> (Y, U, n, d, 1.0 / href, pack64, Vg);
+
+  return cudaGetLastError ();
+}
+
+/* mean of the centres in row order, lane = coordinate (the anchor of the mixed
+ * form where no sample covariance is taken); the other warps stage the rows */
+__global__ void __launch_bounds__ (PREP_THREADS)
+_mean_kernel (const double *__restrict__ X, int n, int d, double *__restrict__ mu)
+{
+  __shared__ double xs[2][WM_ROWS][NCG_DMAX];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int nch  = (n + WM_ROWS - 1) / WM_ROWS;
+  double sum     = 0.0;
+
+  for (int ch = -1; ch < nch; ch++)
+  {
+    if (w > 0 && ch + 1 < nch && lane < d)
+    {
+      const int t0 = (ch + 1) * WM_ROWS, tn = min (WM_ROWS, n - t0);
+
+      for (int t = w - 1; t < tn; t += 3)
+        xs[(ch + 1) & 1][t][lane] = X[(size_t) (t0 + t) * d + lane];
+    }
+    else if (w == 0 && ch >= 0 && lane < d)
+    {
+      const int tn = min (WM_ROWS, n - ch * WM_ROWS);
+
+#pragma unroll 8
+      for (int t = 0; t < tn; t++)
+        sum = __dadd_rn (sum, xs[ch & 1][t][lane]);
+    }
+
+    __syncthreads ();
+  }
+
+  if (w == 0 && lane < d)
+    mu[lane] = __ddiv_rn (sum, (double) n);
+}
+
+extern "C" cudaError_t
+ncg_launch_mean (const double *X, int n, int d, double *mu, cudaStream_t s)
+{
+  _mean_kernel<<<1, PREP_THREADS, 0, s>>> (X, n, d, mu);
+
+  return cudaGetLastError ();
+}
+
+/* Vg = scale * U^{-T} (the global whitening of the evaluation points) */
+__global__ void __launch_bounds__ (32)
+_global_vg_kernel (const double *__restrict__ U, int d, double scale, double *__restrict__ Vg)
+{
+  __shared__ double W[NCG_DMAX * NCG_DMAX];
+
+  _vg_warp (U, d, scale, Vg, W);
 }
 
 extern "C" cudaError_t
