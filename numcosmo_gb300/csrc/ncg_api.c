@@ -697,7 +697,7 @@ _split_obj (ncg_sd_t *sd, double lnos, double *hbuf, double *f)
   sd->href            = _get_href (sd);
 
   if (sd->kind == NCG_VKDE)
-    CK (ncg_launch_vkde_finish (sd->dX, sd->dUi, sd->dflag, (int) sd->nk, d, sd->kernel, sd->nu, sd->href,
+    CK (ncg_launch_vkde_finish (sd->dX, sd->dUi, sd->dflag, (int) sd->nk, d, sd->kernel, sd->dst, sd->href,
                                 sd->dlnnorm, sd->dpack64, sd->stream), "vkde_finish");
   else
     CK (ncg_launch_kde_finish (sd->dY, sd->dU, (int) sd->n, d, sd->href, sd->dpack64, sd->dVg, sd->stream),
@@ -730,7 +730,7 @@ _href_operand (ncg_sd_t *sd)
   const int d = (int) sd->d;
 
   if (sd->kind == NCG_VKDE)
-    CK (ncg_launch_vkde_finish (sd->dX, sd->dUi, sd->dflag, (int) sd->nk, d, sd->kernel, sd->nu, sd->href,
+    CK (ncg_launch_vkde_finish (sd->dX, sd->dUi, sd->dflag, (int) sd->nk, d, sd->kernel, sd->dst, sd->href,
                                 sd->dlnnorm, sd->dpack64, sd->stream), "vkde_finish");
   else
     CK (ncg_launch_kde_finish (sd->dY, sd->dU, (int) sd->n, d, sd->href, sd->dpack64, sd->dVg, sd->stream),
@@ -1353,7 +1353,7 @@ ncg_sd_prepare (ncg_sd_t *sd)
         return r;
     }
 
-    CK (ncg_launch_vkde_finish (sd->dX, sd->dUi, sd->dflag, nkk, d, sd->kernel, sd->nu, sd->href, sd->dlnnorm,
+    CK (ncg_launch_vkde_finish (sd->dX, sd->dUi, sd->dflag, nkk, d, sd->kernel, sd->dst, sd->href, sd->dlnnorm,
                                 sd->dpack64, s), "vkde_finish");
     /* global whitening of the points for the mixed form (unscaled U^{-T}) */
     CK (ncg_launch_global_vg (sd->dU, d, 1.0, sd->dVg, s), "global_vg");

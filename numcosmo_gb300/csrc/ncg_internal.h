@@ -63,6 +63,7 @@ typedef struct ncg_prep_status
   int32_t n_badindex;     /* neighbour indices outside [0, n) (a bug)   */
   int32_t pad_;
   double  kernel_lnnorm;  /* lnnorm of the global factor                */
+  double  ln0;            /* its part without the determinant (Student-t) */
 } ncg_prep_status_t;
 
 /* Per-launch parameters of the eval kernels. */
@@ -102,8 +103,8 @@ size_t      ncg_robust_work_doubles (int nsets, int d);
 cudaError_t ncg_launch_robust_cov (const double *X, int n, int d, const int32_t *idx, int m, int nsets, int ogk,
                                    double *work, double *out, int32_t *bad, cudaStream_t s);
 cudaError_t ncg_launch_vkde_finish (const double *X, double *Ui, const int32_t *flag, int n, int d,
-                                    int kernel, double nu, double href, double *lnnorm, double *pack64,
-                                    cudaStream_t s);
+                                    int kernel, const ncg_prep_status_t *st, double href, double *lnnorm,
+                                    double *pack64, cudaStream_t s);
 cudaError_t ncg_launch_kde_finish (const double *Y, const double *U, int n, int d, double href,
                                    double *pack64, double *Vg, cudaStream_t s);
 cudaError_t ncg_launch_mean (const double *X, int n, int d, double *mu, cudaStream_t s);

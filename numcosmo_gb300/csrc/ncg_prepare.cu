@@ -97,7 +97,7 @@ _quot_ok (double delta)
 {
   const uint32_t hi = (uint32_t) __double2hiint (delta) & 0x7fffffffu;
 
-  return (hi >> 20) - 128u < 1900u || (hi | (uint32_t) __double2loint (delta)) == 0u;
+  return ((hi >> 20) - 128u < 1900u) | ((hi | (uint32_t) __double2loint (delta)) == 0u);
 }
 
 __device__ __forceinline__ double
@@ -161,7 +161,7 @@ _welford_mean_kernel (const double *__restrict__ X, int n, int d, double *__rest
       if (w == 0)
       {
         const double m0 = m;
-        bool ok         = true;
+        int ok          = 1;
         double *mo = mean + (size_t) t0 * d + lane, *ro = Rq + (size_t) t0 * d + lane;
 
 #pragma unroll 8
@@ -170,8 +170,8 @@ _welford_mean_kernel (const double *__restrict__ X, int n, int d, double *__rest
           const double delta = __dsub_rn (xs[buf][t][lane], m);
           const double R     = _quot (delta, yh[buf][t], yl[buf][t]);
 
-          ok = ok && _quot_ok (delta);
-          m  = __dadd_rn (m, R);
+          ok &= (int) _quot_ok (delta);
+          m   = __dadd_rn (m, R);
           mo[(size_t) t * d] = m;
           ro[(size_t) t * d] = R;
         }
@@ -206,12 +206,16 @@ _welford_mean_kernel (const double *__restrict__ X, int n, int d, double *__rest
     mu[lane] = __ddiv_rn (sum, (double) n);
 }
 
-/* The covariance sums from the running means: a CTA takes 32 of the
- * d (d + 1) / 2 elements (off-diagonal ones row by row, then the variances).
- * The products of different rows are independent; only the additions are a
- * chain, so warp 0 adds (64 cycles a row, alone on its sub-partition: warp 4
- * idles) what the other six warps multiply one chunk of rows ahead. */
-#define WA_ROWS 64
+/* The covariance sums from the running means: a CTA takes 32 off-diagonal
+ * elements (row by row), the last one the variances.  The products of
+ * different rows are independent; only the additions are a chain, so warp 0
+ * adds (64 cycles a row, alone on its sub-partition but for warp 4, which only
+ * writes the row numbers) what the other six warps multiply one chunk of rows
+ * ahead, at three FP64 instructions a row the same 64 cycles on their three
+ * sub-partitions.  Each of them holds its rows of the next chunk in registers
+ * (the loads waited for in place took 1.0 ms at n = 8192, d = 16; 0.4 ms so). */
+#define WA_PER 11
+#define WA_ROWS (6 * WA_PER)
 #define WA_TH 256
 
 __global__ void __launch_bounds__ (WA_TH)
@@ -219,22 +223,25 @@ _welford_acc_kernel (const double *__restrict__ X, const double *__restrict__ me
                      int n, int d, double *__restrict__ cov)
 {
   __shared__ double prod[2][WA_ROWS][32];
+  __shared__ double wt[2][WA_ROWS];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int E    = d * (d - 1) / 2;
-  const int e    = blockIdx.x * 32 + lane;
-  const bool in  = e < E + d;
-  const bool var = e >= E;
+  const bool var = blockIdx.x == gridDim.x - 1;
+  const int e    = var ? lane : blockIdx.x * 32 + lane;
+  const bool in  = e < (var ? d : E);
   const int pw   = (w < 4) ? w - 1 : w - 2;     /* producers: warps 1-3, 5-7 */
   const int nch  = (n + WA_ROWS - 1) / WA_ROWS;
   int r = 0, c = 0;
   double acc = 0.0;
+  double xc[WA_PER], mc[WA_PER], xr[WA_PER], mr[WA_PER];
 
   if (in && !var)
     _upper_rc (e, d, &r, &c);
   else if (in)
-    r = c = e - E;
+    r = c = e;
 
-  for (int ch = -1; ch < nch; ch++)
+  /* step ch: loads of chunk ch + 2, products of chunk ch + 1, sum of chunk ch */
+  for (int ch = -2; ch < nch; ch++)
   {
     if (w == 0)
     {
@@ -242,23 +249,45 @@ _welford_acc_kernel (const double *__restrict__ X, const double *__restrict__ me
       {
         const int tn = min (WA_ROWS, n - ch * WA_ROWS);
 
-#pragma unroll 8
+#pragma unroll 11
         for (int t = 0; t < tn; t++)
           acc = __dadd_rn (acc, prod[ch & 1][t][lane]);
       }
     }
-    else if (w != 4 && ch + 1 < nch && in)
+    else if (w == 4)
     {
-      const int t0 = (ch + 1) * WA_ROWS, tn = min (WA_ROWS, n - t0);
-
-#pragma unroll 4
-      for (int t = pw; t < tn; t += 6)
+      for (int t = lane; t < WA_ROWS; t += 32)
+        wt[ch & 1][t] = (double) ((ch + 2) * WA_ROWS + t);
+    }
+    else
+    {
+      if (ch >= -1 && ch + 1 < nch)
       {
-        const size_t row   = (size_t) (t0 + t) * d;
-        const double delta = __dsub_rn (X[row + c], (t0 + t > 0) ? mean[row - d + c] : 0.0);
-        const double left  = var ? __dmul_rn ((double) (t0 + t), delta) : __dsub_rn (X[row + r], mean[row + r]);
+        /* off-diagonal: (x_r - m_r)(x_c - m'_c), m' the mean before the row;
+         * variance: (t (x_c - m'_c)) R */
+#pragma unroll
+        for (int q = 0; q < WA_PER; q++)
+        {
+          const double delta = __dsub_rn (xc[q], mc[q]);
+          const double left  = var ? __dmul_rn (wt[(ch + 1) & 1][pw + 6 * q], delta) : __dsub_rn (xr[q], mr[q]);
 
-        prod[(ch + 1) & 1][t][lane] = __dmul_rn (left, var ? Rq[row + c] : delta);
+          prod[(ch + 1) & 1][pw + 6 * q][lane] = __dmul_rn (left, var ? mr[q] : delta);
+        }
+      }
+
+      if (ch + 2 < nch)
+      {
+#pragma unroll
+        for (int q = 0; q < WA_PER; q++)
+        {
+          const int t      = min ((ch + 2) * WA_ROWS + pw + 6 * q, n - 1);
+          const size_t row = (size_t) t * d;
+
+          xc[q] = X[row + c];
+          mc[q] = (t > 0) ? mean[row - d + c] : 0.0;
+          xr[q] = X[row + r];
+          mr[q] = var ? Rq[row + c] : mean[row + r];
+        }
       }
     }
 
@@ -443,7 +472,7 @@ ncg_launch_global_cov (const double *X, int n, int d, double *cov, double *mu, d
                        cudaStream_t s)
 {
   _welford_mean_kernel<<<1, PREP_THREADS, 0, s>>> (X, n, d, mean, Rq, mu);
-  _welford_acc_kernel<<<(d * (d + 1) / 2 + 31) / 32, WA_TH, 0, s>>> (X, mean, Rq, n, d, cov);
+  _welford_acc_kernel<<<(d * (d - 1) / 2 + 31) / 32 + 1, WA_TH, 0, s>>> (X, mean, Rq, n, d, cov);
 
   return cudaGetLastError ();
 }
@@ -452,7 +481,10 @@ __global__ void
 _global_lnnorm_kernel (const double *U, int d, int kernel, double nu, ncg_prep_status_t *st)
 {
   if (threadIdx.x == 0 && blockIdx.x == 0)
-    st->kernel_lnnorm = _lnnorm_of (kernel, d, _lnnorm0 (kernel, nu, d), _chol_lndet (U, d, d));
+  {
+    st->ln0           = _lnnorm0 (kernel, nu, d);
+    st->kernel_lnnorm = _lnnorm_of (kernel, d, st->ln0, _chol_lndet (U, d, d));
+  }
 }
 
 extern "C" cudaError_t
@@ -1167,7 +1199,7 @@ _local_cov_chol_kernel (const double *__restrict__ X, const int32_t *__restrict_
                         int kpw, double *__restrict__ Ui, int32_t *__restrict__ flag, ncg_prep_status_t *st)
 {
   __shared__ double buf[2 * 4 * 32 * LC_ROWS];      /* 4 kpw d <= 128 columns of xs and of delta */
-  __shared__ double yh[LC_ROWS], yl[LC_ROWS];
+  __shared__ double yh[LC_ROWS], yl[LC_ROWS], wt[LC_ROWS];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int kb = 4 * kpw, E = d * (d - 1) / 2, kd = LC_ROWS * d;
   const int i0 = blockIdx.x * kb;
@@ -1231,7 +1263,10 @@ _local_cov_chol_kernel (const double *__restrict__ X, const int32_t *__restrict_
     }
 
     if (tid < tn)
-      _recip_pair ((double) (t0 + tid) + 1.0, &yh[tid], &yl[tid]);
+    {
+      wt[tid] = (double) (t0 + tid);
+      _recip_pair (wt[tid] + 1.0, &yh[tid], &yl[tid]);
+    }
 
     __syncthreads ();
 
@@ -1247,10 +1282,10 @@ _local_cov_chol_kernel (const double *__restrict__ X, const int32_t *__restrict_
         double R           = _quot (delta, yh[t], yl[t]);
 
         if (!_quot_ok (delta))
-          R = __ddiv_rn (delta, (double) (t0 + t) + 1.0);
+          R = __ddiv_rn (delta, wt[t] + 1.0);
 
         m         = __dadd_rn (m, R);
-        var       = __dadd_rn (var, __dmul_rn (__dmul_rn ((double) (t0 + t), delta), R));
+        var       = __dadd_rn (var, __dmul_rn (__dmul_rn (wt[t], delta), R));
         px[t * d] = __dsub_rn (x, m);
         pd[t * d] = delta;
       }
@@ -1708,8 +1743,8 @@ ncg_launch_compact_flags (const int32_t *flag, int n, int32_t *ids, int32_t *cou
 
 __global__ void __launch_bounds__ (FIN_WARPS * 32)
 _vkde_finish_kernel (const double *__restrict__ X, const double *__restrict__ Ui, const int32_t *flag,
-                     int n, int d, int kernel, double nu, double inv_href, double *__restrict__ lnnorm,
-                     double *__restrict__ pack)
+                     int n, int d, int kernel, const double *__restrict__ ln0p, double inv_href,
+                     double *__restrict__ lnnorm, double *__restrict__ pack)
 {
   __shared__ double sU[FIN_WARPS][NCG_DMAX * NCG_DMAX];
   __shared__ double sW[FIN_WARPS][NCG_DMAX * NCG_DMAX];
@@ -1717,7 +1752,7 @@ _vkde_finish_kernel (const double *__restrict__ X, const double *__restrict__ Ui
   const int dp   = ncg_pad_dim (d);
   const int P    = dp * (dp + 1) / 2;
   const int S    = dp + P;
-  const double ln0 = _lnnorm0 (kernel, nu, d);   /* the kernel's constant, with its lgammas, once */
+  const double ln0 = *ln0p;
 
   for (int i = blockIdx.x * FIN_WARPS + w; i < n; i += gridDim.x * FIN_WARPS)
   {
@@ -1764,14 +1799,14 @@ _vkde_finish_kernel (const double *__restrict__ X, const double *__restrict__ Ui
 
 extern "C" cudaError_t
 ncg_launch_vkde_finish (const double *X, double *Ui, const int32_t *flag, int n, int d, int kernel,
-                        double nu, double href, double *lnnorm, double *pack64, cudaStream_t s)
+                        const ncg_prep_status_t *st, double href, double *lnnorm, double *pack64, cudaStream_t s)
 {
   int grid = (n + FIN_WARPS - 1) / FIN_WARPS;
 
   if (grid > 152 * 32)
     grid = 152 * 32;
 
-  _vkde_finish_kernel<<<grid, FIN_WARPS * 32, 0, s>>> (X, Ui, flag, n, d, kernel, nu, 1.0 / href, lnnorm,
+  _vkde_finish_kernel<<<grid, FIN_WARPS * 32, 0, s>>> (X, Ui, flag, n, d, kernel, &st->ln0, 1.0 / href, lnnorm,
                                                         pack64);
 
   return cudaGetLastError ();
