@@ -122,7 +122,7 @@ _syrk (const TI *A, int lda, int r0, int r1, int off, int nn, T *C, int ldc, int
   return cudaGetLastError ();
 }
 
-/* FP32 products (the mixed solver's A^T A and its factor's trailing updates):
+/* FP32 products (the mixed solver's A^T A below 1024 columns):
  * 128 x 128 upper tiles, 256 threads of 8 x 8 outputs (rows ty*4 + {0..3} and
  * 64 + ty*4 + {0..3}, columns likewise by tx), contraction rows staged 8 at a
  * time in double-buffered shared memory (the next chunk is loaded into
@@ -134,7 +134,7 @@ _syrk (const TI *A, int lda, int r0, int r1, int off, int nn, T *C, int ldc, int
 template <typename TI>
 __global__ void __launch_bounds__ (256)
 _syrk128_f32_kernel (const TI *__restrict__ A, int lda, int r0, int r1, int off, int nn, float *__restrict__ C,
-                     int ldc, int minus)
+                     int ldc)
 {
   __shared__ __align__ (16) float As[2][SY_KB][SY_T];
   __shared__ __align__ (16) float Bs[2][SY_KB][SY_T];
@@ -225,9 +225,7 @@ _syrk128_f32_kernel (const TI *__restrict__ A, int lda, int r0, int r1, int off,
 
       if (i < end && j < end && j >= i)
       {
-        float *dst = C + (size_t) i * ldc + j;
-
-        *dst = minus ? (*dst - acc[p][q]) : acc[p][q];
+        C[(size_t) i * ldc + j] = acc[p][q];
       }
     }
   }
@@ -235,14 +233,14 @@ _syrk128_f32_kernel (const TI *__restrict__ A, int lda, int r0, int r1, int off,
 
 template <typename TI>
 static cudaError_t
-_syrk128 (const TI *A, int lda, int r0, int r1, int off, int nn, float *C, int ldc, int minus, cudaStream_t s)
+_syrk128 (const TI *A, int lda, int r0, int r1, int off, int nn, float *C, int ldc, cudaStream_t s)
 {
   if (nn <= 0 || r1 <= r0)
     return cudaSuccess;
 
   const int T_ = (nn + SY_T - 1) / SY_T;
 
-  _syrk128_f32_kernel<TI><<<T_ * (T_ + 1) / 2, 256, 0, s>>> (A, lda, r0, r1, off, nn, C, ldc, minus);
+  _syrk128_f32_kernel<TI><<<T_ * (T_ + 1) / 2, 256, 0, s>>> (A, lda, r0, r1, off, nn, C, ldc);
 
   return cudaGetLastError ();
 }
@@ -256,7 +254,7 @@ ncg_launch_syrk_upper (const double *A, int nrows, int ncols, double *M, cudaStr
 extern "C" cudaError_t
 ncg_launch_syrk_upper_f32 (const double *A, int nrows, int ncols, float *M, cudaStream_t s)
 {
-  return _syrk128<double> (A, ncols, 0, nrows, 0, ncols, M, ncols, 0, s);
+  return _syrk128<double> (A, ncols, 0, nrows, 0, ncols, M, ncols, s);
 }
 
 /* ---- gemv --------------------------------------------------------------- */
@@ -554,50 +552,40 @@ _stage_block (T (*S)[B + 1], const T *__restrict__ A, int ld, int r0, int c0, in
   }
 }
 
-/* factor the nb x nb diagonal block at (kb, kb) in place (upper), right-looking
- * inside shared memory: at step j the row j is final, scaled by 1/U_jj, and
- * the trailing block takes the rank-1 update in ascending j order.  Thread
- * (ty, tx) of the 16 x 16 block owns the elements (ty + 16p, tx + 16q), which
- * spreads the shrinking trailing triangle over all threads.  Two barriers a
- * step: the diagonal read and the row scaling, then the update (which also
- * stores U_jj, read by nobody in that phase). */
-template <typename T>
+/* FP64: factor the nb x nb diagonal block at (kb, kb) in place (upper),
+ * right-looking inside shared memory: at step j the row j is final, scaled by
+ * 1/U_jj, and the trailing block takes the rank-1 update in ascending j order.
+ * Thread (ty, tx) of the 16 x 16 block owns the elements (ty + 16p, tx + 16q),
+ * which spreads the shrinking trailing triangle over all threads.  Two
+ * barriers a step: the diagonal read and the row scaling, then the update
+ * (which also stores U_jj, read by nobody in that phase). */
 __global__ void __launch_bounds__ (256)
-_potrf_diag_kernel (T *A, int ld, int kb, int nb, int32_t *info)
+_potrf_diag_f64_kernel (double *A, int ld, int kb, int nb, int32_t *info)
 {
-  __shared__ T S[PB][PB + 1];
+  __shared__ double S[PB][PB + 1];
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   int fail      = 0;
 
   if (*info)
     return;
 
-  _stage_block<T, 256, PB> (S, A, ld, kb, kb, nb, tid);
+  _stage_block<double, 256, PB> (S, A, ld, kb, kb, nb, tid);
 
   __syncthreads ();
 
   for (int j = 0; j < nb; j++)
   {
-    const T ajj = S[j][j];
+    const double ajj = S[j][j];
 
-    if (!(ajj > (T) 0))
+    if (!(ajj > 0.0))
     {
       fail = j + 1;
       break;
     }
 
-    const T ujj = sqrt (ajj);
+    const double ujj = sqrt (ajj);
 
-    /* FP32 (the preconditioner's factor): one reciprocal, then products,
-     * within an ulp of the quotients; FP64 keeps the quotients */
-    if constexpr (sizeof (T) == sizeof (float))
-    {
-      const float ri = __frcp_rn (ujj);
-
-      if (tid > j && tid < nb)
-        S[j][tid] = S[j][tid] * ri;
-    }
-    else if (tid > j && tid < nb)
+    if (tid > j && tid < nb)
       S[j][tid] = S[j][tid] / ujj;
 
     __syncthreads ();
@@ -612,7 +600,7 @@ _potrf_diag_kernel (T *A, int ld, int kb, int nb, int32_t *info)
 
       if (r > j && r < nb)
       {
-        const T sjr = S[j][r];
+        const double sjr = S[j][r];
 
 #pragma unroll
         for (int q = 0; q < PB / 16; q++)
@@ -645,22 +633,21 @@ _potrf_diag_kernel (T *A, int ld, int kb, int nb, int32_t *info)
   }
 }
 
-/* rows kb..kb+nb of the columns right of the block: X = U_kk^{-T} A_panel,
+/* FP64: rows kb..kb+nb of the columns right of the block: X = U_kk^{-T} A_panel,
  * one column per thread held in registers (column sweep in ascending row
  * order) */
 #define TRSM_TH 128
 
-template <typename T>
 __global__ void __launch_bounds__ (TRSM_TH)
-_potrf_trsm_kernel (T *A, int ld, int kb, int nb, int n, const int32_t *info, float *pk)
+_potrf_trsm_f64_kernel (double *A, int ld, int kb, int nb, int n, const int32_t *info)
 {
-  __shared__ T S[PB][PB + 1];
+  __shared__ double S[PB][PB + 1];
   const int tid = threadIdx.x;
 
   if (*info)
     return;
 
-  _stage_block<T, TRSM_TH, PB> (S, A, ld, kb, kb, nb, tid);
+  _stage_block<double, TRSM_TH, PB> (S, A, ld, kb, kb, nb, tid);
 
   __syncthreads ();
 
@@ -669,21 +656,18 @@ _potrf_trsm_kernel (T *A, int ld, int kb, int nb, int n, const int32_t *info, fl
   if (col >= n)
     return;
 
-  T a[PB];
+  double a[PB];
 
 #pragma unroll
   for (int r = 0; r < PB; r++)
-    a[r] = (r < nb) ? A[(size_t) (kb + r) * ld + col] : (T) 0;
+    a[r] = (r < nb) ? A[(size_t) (kb + r) * ld + col] : 0.0;
 
 #pragma unroll
   for (int r = 0; r < PB; r++)
   {
     if (r < nb)
     {
-      if constexpr (sizeof (T) == sizeof (float))
-        a[r] = a[r] * __frcp_rn (S[r][r]);   /* FP32: reciprocal products, as the diagonal factor */
-      else
-        a[r] = a[r] / S[r][r];
+      a[r] = a[r] / S[r][r];
 
 #pragma unroll
       for (int m = r + 1; m < PB; m++)
@@ -695,11 +679,271 @@ _potrf_trsm_kernel (T *A, int ld, int kb, int nb, int n, const int32_t *info, fl
   for (int r = 0; r < PB; r++)
     if (r < nb)
       A[(size_t) (kb + r) * ld + col] = a[r];
+}
 
-  /* the panel as the tensor-core trailing update's operand */
-  if constexpr (sizeof (T) == sizeof (float))
-    if (pk != NULL)
-      _sk_pack_column (pk, col - kb - nb, (const float *) a, nb);
+/* ---- the FP32 preconditioner's panels ---- */
+
+/* The nb x nb diagonal block (upper, in place).  The block lives in registers,
+ * 4 x 4 elements per thread (element (ty + 16p, tx + 16q)); a step publishes
+ * its raw row j through shared memory, one barrier, and every thread takes
+ * s_jr s_jc / a_jj off its elements; the square roots and the rows' own
+ * scaling wait for the end, where all rows take them at once.  It is bound by
+ * the chain of steps: a barrier, two shared-memory trips and a reciprocal
+ * each (24 us with the row scaled and the block updated in shared memory). */
+__device__ __forceinline__ float
+_rcp_approx (float x)
+{
+  float r;
+
+  asm ("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+
+  return r;
+}
+
+__global__ void __launch_bounds__ (256)
+_potrf_diag_f32_kernel (float *A, int ld, int kb, int nb, int32_t *info)
+{
+  __shared__ float row[2][PB];
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  float s[4][4], piv[4];
+  int fail = 0;
+
+  if (*info)
+    return;
+
+  /* the identity past nb */
+#pragma unroll
+  for (int p = 0; p < 4; p++)
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+    {
+      const int r = ty + 16 * p, c = tx + 16 * q;
+
+      s[p][q] = (r < nb && c < nb) ? ((c >= r) ? A[(size_t) (kb + r) * ld + kb + c] : 0.0f) : (r == c ? 1.0f : 0.0f);
+      piv[p]  = 1.0f;
+    }
+
+#pragma unroll
+  for (int p = 0; p < 4; p++)
+    for (int jj = 0; jj < 16; jj++)
+    {
+      const int j = 16 * p + jj;
+      float *rb   = row[j & 1];
+
+      if (fail)
+        break;
+
+      if (ty == jj)
+      {
+#pragma unroll
+        for (int q = p; q < 4; q++)
+          rb[tx + 16 * q] = s[p][q];
+      }
+
+      __syncthreads ();
+
+      const float ajj = rb[j];
+
+      if (!(ajj > 0.0f))
+      {
+        fail = j + 1;
+        break;
+      }
+
+      const float inv = -_rcp_approx (ajj);
+      float rc[4];
+
+      if (ty == jj)
+        piv[p] = ajj;
+
+#pragma unroll
+      for (int q = p; q < 4; q++)
+        rc[q] = rb[tx + 16 * q];
+
+#pragma unroll
+      for (int pp = p; pp < 4; pp++)
+      {
+        const int r   = ty + 16 * pp;
+        const float t = (r > j) ? rb[r] * inv : 0.0f;
+
+#pragma unroll
+        for (int q = pp; q < 4; q++)
+          s[pp][q] = fmaf (t, rc[q], s[pp][q]);
+      }
+    }
+
+  if (fail)
+  {
+    if (tid == 0)
+      atomicCAS (info, 0, kb + fail);
+
+    return;
+  }
+
+#pragma unroll
+  for (int p = 0; p < 4; p++)
+  {
+    const int r    = ty + 16 * p;
+    const float u  = __fsqrt_rn (piv[p]), ri = __frcp_rn (u);
+
+#pragma unroll
+    for (int q = p; q < 4; q++)
+    {
+      const int c = tx + 16 * q;
+
+      if (r < nb && c < nb && c >= r)
+        A[(size_t) (kb + r) * ld + kb + c] = (c == r) ? u : s[p][q] * ri;
+    }
+  }
+}
+
+/* X = U_kk^{-T} A_panel, one column per thread in registers, few columns per
+ * CTA so that the panel covers many SMs; the block's rows are read from shared
+ * memory four at a time (every lane the same), the reciprocals of the diagonal
+ * come once from staging.  27 us -> 11 us at n = 3000, most of it the pack,
+ * whose hi / lo split went through FP64.  pk (may be NULL): the panel as the tensor-core
+ * trailing update's operand. */
+#define TRSM32_TH 64
+
+__global__ void __launch_bounds__ (TRSM32_TH)
+_potrf_trsm_f32_kernel (float *A, int ld, int kb, int nb, int n, const int32_t *info, float *pk)
+{
+  __shared__ __align__ (16) float S[PB][PB];
+  __shared__ float ri[PB];
+  const int tid = threadIdx.x;
+  const int col = kb + nb + blockIdx.x * TRSM32_TH + tid;
+  const bool in = col < n;
+  float a[PB];
+
+  if (*info)
+    return;
+
+#pragma unroll
+  for (int r = 0; r < PB; r++)
+    a[r] = (in && r < nb) ? A[(size_t) (kb + r) * ld + col] : 0.0f;
+
+#pragma unroll 16
+  for (int r = 0; r < PB; r++)
+    S[r][tid] = (r < nb && tid < nb && tid >= r) ? A[(size_t) (kb + r) * ld + kb + tid] : 0.0f;
+
+  ri[tid] = (tid < nb) ? __frcp_rn (S[tid][tid]) : 1.0f;
+  __syncthreads ();
+
+  if (!in)
+    return;
+
+#pragma unroll
+  for (int r = 0; r < PB; r++)
+  {
+    a[r] *= ri[r];
+
+    const float t = -a[r];
+
+#pragma unroll
+    for (int m = (r + 1) / 4 * 4; m < PB; m += 4)
+    {
+      const float4 v = *(const float4 *) &S[r][m];
+
+      if (m + 0 > r)
+        a[m + 0] = fmaf (v.x, t, a[m + 0]);
+      if (m + 1 > r)
+        a[m + 1] = fmaf (v.y, t, a[m + 1]);
+      if (m + 2 > r)
+        a[m + 2] = fmaf (v.z, t, a[m + 2]);
+      if (m + 3 > r)
+        a[m + 3] = fmaf (v.w, t, a[m + 3]);
+    }
+  }
+
+#pragma unroll
+  for (int r = 0; r < PB; r++)
+    if (r < nb)
+      A[(size_t) (kb + r) * ld + col] = a[r];
+
+  if (pk != NULL)
+    _sk_pack_column (pk, col - kb - nb, a, nb);
+}
+
+/* C -= P^T P on the upper tiles of the nn x nn trailing block for a panel of
+ * nb <= 64 rows: 64 x 64 tiles, the whole panel slice of both sides staged at
+ * once, 4 x 4 outputs per thread, C loaded while the panel arrives.  One FMA
+ * chain per output over the rows in ascending order.  11 us on average below
+ * 2560 columns, where the general tile kernel (16 rows a stage) took 18 and the
+ * tensor-core update 13: there its set-up and the traffic of C decide, not the
+ * products. */
+__global__ void __launch_bounds__ (256)
+_potrf_update_f32_kernel (float *A, int ld, int kb, int nb, int off, int nn, const int32_t *info)
+{
+  __shared__ __align__ (16) float As[PB][PB];
+  __shared__ __align__ (16) float Bs[PB][PB];
+  const int T_ = (nn + PB - 1) / PB;
+  int b = blockIdx.x, ti = 0;
+
+  if (*info)
+    return;
+
+  while (b >= T_ - ti)
+  {
+    b -= T_ - ti;
+    ti++;
+  }
+
+  const int tj  = ti + b, i0 = off + ti * PB, j0 = off + tj * PB, end = off + nn;
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int lc  = tid & 63, lr = tid >> 6;
+  float va[16], vb[16], acc[4][4];
+
+#pragma unroll
+  for (int q = 0; q < 16; q++)
+  {
+    const int r = lr + 4 * q;
+
+    va[q] = (r < nb && i0 + lc < end) ? A[(size_t) (kb + r) * ld + i0 + lc] : 0.0f;
+    vb[q] = (r < nb && j0 + lc < end) ? A[(size_t) (kb + r) * ld + j0 + lc] : 0.0f;
+  }
+
+#pragma unroll
+  for (int p = 0; p < 4; p++)
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+    {
+      const int i = i0 + ty * 4 + p, j = j0 + tx * 4 + q;
+
+      acc[p][q] = (i < end && j < end && j >= i) ? A[(size_t) i * ld + j] : 0.0f;
+    }
+
+#pragma unroll
+  for (int q = 0; q < 16; q++)
+  {
+    As[lr + 4 * q][lc] = -va[q];
+    Bs[lr + 4 * q][lc] = vb[q];
+  }
+
+  __syncthreads ();
+
+#pragma unroll 16
+  for (int k = 0; k < PB; k++)
+  {
+    const float4 x = *(const float4 *) &As[k][ty * 4], y = *(const float4 *) &Bs[k][tx * 4];
+    const float xv[4] = { x.x, x.y, x.z, x.w }, yv[4] = { y.x, y.y, y.z, y.w };
+
+#pragma unroll
+    for (int p = 0; p < 4; p++)
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        acc[p][q] = fmaf (xv[p], yv[q], acc[p][q]);
+  }
+
+#pragma unroll
+  for (int p = 0; p < 4; p++)
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+    {
+      const int i = i0 + ty * 4 + p, j = j0 + tx * 4 + q;
+
+      if (i < end && j < end && j >= i)
+        A[(size_t) i * ld + j] = acc[p][q];
+    }
 }
 
 __global__ void
@@ -708,39 +952,24 @@ _zero_int_kernel (int32_t *p)
   *p = 0;
 }
 
-/* trailing blocks at least this wide take the tensor-core update (FP32 with a pack) */
-#define POTRF_TC_MIN 1024
-
-template <typename T>
-static cudaError_t
-_potrf (T *A, int n, int32_t *info, float *pk, cudaStream_t s)
+extern "C" cudaError_t
+ncg_launch_potrf (double *A, int n, int32_t *info, double *work, cudaStream_t s)
 {
+  (void) work;
+
   _zero_int_kernel<<<1, 1, 0, s>>> (info);
 
   for (int kb = 0; kb < n; kb += PB)
   {
-    const int nb = (n - kb < PB) ? n - kb : PB;
+    const int nb = (n - kb < PB) ? n - kb : PB, rest = n - kb - nb;
 
-    _potrf_diag_kernel<T><<<1, 256, 0, s>>> (A, n, kb, nb, info);
+    _potrf_diag_f64_kernel<<<1, 256, 0, s>>> (A, n, kb, nb, info);
 
-    if (kb + nb < n)
+    if (rest > 0)
     {
-      const int rest = n - kb - nb;
-      const bool tc  = sizeof (T) == sizeof (float) && pk != NULL && rest >= POTRF_TC_MIN;
+      _potrf_trsm_f64_kernel<<<(rest + TRSM_TH - 1) / TRSM_TH, TRSM_TH, 0, s>>> (A, n, kb, nb, n, info);
 
-      _potrf_trsm_kernel<T><<<(rest + TRSM_TH - 1) / TRSM_TH, TRSM_TH, 0, s>>> (A, n, kb, nb, n, info,
-                                                                                tc ? pk : NULL);
-
-      cudaError_t e;
-
-      /* FP32: TF32x3 tensor-core tiles for the large updates (pack written by
-       * the panel solve), else 128-wide then 64-wide CUDA-core tiles */
-      if constexpr (sizeof (T) == sizeof (float))
-        e = tc ? ncg_launch_syrk_tc (pk, nb, rest, (float *) A + (size_t) (kb + nb) * n + kb + nb, n, 1, info, s)
-               : (rest >= 2048) ? _syrk128<float> ((const float *) A, n, kb, kb + nb, kb + nb, rest, (float *) A, n, 1, s)
-                                : _syrk<T, T> (A, n, kb, kb + nb, kb + nb, rest, A, n, 1, s);
-      else
-        e = _syrk<T, T> (A, n, kb, kb + nb, kb + nb, rest, A, n, 1, s);
+      const cudaError_t e = _syrk<double, double> (A, n, kb, kb + nb, kb + nb, rest, A, n, 1, s);
 
       if (e != cudaSuccess)
         return e;
@@ -750,18 +979,43 @@ _potrf (T *A, int n, int32_t *info, float *pk, cudaStream_t s)
   return cudaGetLastError ();
 }
 
-extern "C" cudaError_t
-ncg_launch_potrf (double *A, int n, int32_t *info, double *work, cudaStream_t s)
-{
-  (void) work;
-
-  return _potrf<double> (A, n, info, NULL, s);
-}
+/* trailing blocks at least this wide take the tensor-core update */
+#define POTRF_TC_MIN 2560
 
 extern "C" cudaError_t
 ncg_launch_potrf_f32 (float *A, int n, int32_t *info, float *pk, cudaStream_t s)
 {
-  return _potrf<float> (A, n, info, pk, s);
+  _zero_int_kernel<<<1, 1, 0, s>>> (info);
+
+  for (int kb = 0; kb < n; kb += PB)
+  {
+    const int nb  = (n - kb < PB) ? n - kb : PB, rest = n - kb - nb;
+    const bool tc = pk != NULL && rest >= POTRF_TC_MIN;
+
+    _potrf_diag_f32_kernel<<<1, 256, 0, s>>> (A, n, kb, nb, info);
+
+    if (rest > 0)
+    {
+      _potrf_trsm_f32_kernel<<<(rest + TRSM32_TH - 1) / TRSM32_TH, TRSM32_TH, 0, s>>> (A, n, kb, nb, n, info,
+                                                                                       tc ? pk : NULL);
+
+      if (tc)
+      {
+        const cudaError_t e = ncg_launch_syrk_tc (pk, nb, rest, A + (size_t) (kb + nb) * n + kb + nb, n, 1, info, s);
+
+        if (e != cudaSuccess)
+          return e;
+      }
+      else
+      {
+        const int T_ = (rest + PB - 1) / PB;
+
+        _potrf_update_f32_kernel<<<T_ * (T_ + 1) / 2, 256, 0, s>>> (A, n, kb, nb, kb + nb, rest, info);
+      }
+    }
+  }
+
+  return cudaGetLastError ();
 }
 
 /* ---- blocked triangular solves ------------------------------------------- */
@@ -1430,17 +1684,30 @@ _bsolve_chain_kernel (const float *__restrict__ U, const float *__restrict__ V, 
       p[rr] = fmaf (u1[rr], x1, fmaf (u0[rr], x0, p[rr]));
   }
 
+  /* sums over the lanes of 16 values: at each halving a lane keeps the half of
+   * its values that its bit selects and gets their other halves (15 + 1
+   * shuffles; the block waits for this on the chain) */
 #pragma unroll
-  for (int rr = 0; rr < 16; rr++)
+  for (int o = 8; o > 0; o >>= 1)
   {
-    float v = p[rr];
+    const bool up = (lane & (2 * o)) != 0;
 
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-      v += __shfl_xor_sync (0xffffffffu, v, o);
+    for (int q = 0; q < o; q++)
+    {
+      const float send = up ? p[q] : p[q + o], keep = up ? p[q + o] : p[q];
 
-    if (lane == 0)
-      sv[r0 + rr] = (r0 + rr < nb) ? __uint_as_float ((uint32_t) y[kb + r0 + rr]) - v : 0.0f;
+      p[q] = keep + __shfl_xor_sync (0xffffffffu, send, 2 * o);
+    }
+  }
+
+  p[0] += __shfl_xor_sync (0xffffffffu, p[0], 1);
+
+  if ((lane & 1) == 0)
+  {
+    const int r = r0 + (lane >> 1);
+
+    sv[r] = (r < nb) ? __uint_as_float ((uint32_t) y[kb + r]) - p[0] : 0.0f;
   }
 
   __syncthreads ();

@@ -33,6 +33,18 @@ _put_split4 (float *blk, int row, int k4, double v0, double v1, double v2, doubl
                  _tf32 ((float) (v2 - (double) h2)), _tf32 ((float) (v3 - (double) h3)));
 }
 
+/* the same from FP32 values, where v - hi is exact in FP32: no FP64 conversions,
+ * which take 64 cycles of the sub-partition's FP64 pipe each here */
+static __device__ __forceinline__ void
+_put_split4f (float *blk, int row, int k4, float v0, float v1, float v2, float v3)
+{
+  const uint32_t off = _cm_off (row, k4, SK_LBO) >> 2;
+  const float h0 = _tf32 (v0), h1 = _tf32 (v1), h2 = _tf32 (v2), h3 = _tf32 (v3);
+
+  *(float4 *) (blk + off) = make_float4 (h0, h1, h2, h3);
+  *(float4 *) (blk + SK_HALF / 4 + off) = make_float4 (_tf32 (v0 - h0), _tf32 (v1 - h1), _tf32 (v2 - h2), _tf32 (v3 - h3));
+}
+
 /* column rel (0-based past the panel's diagonal block) of a 64-row panel
  * (nkc = 2) whose values are a[0..nb), into the pack pk */
 static __device__ __forceinline__ void
@@ -50,8 +62,8 @@ _sk_pack_column (float *pk, int rel, const float *a, int nb)
     {
       const int k = c * SK_KC + 4 * q;
 
-      _put_split4 (blk, row, 4 * q, (k + 0 < nb) ? a[k + 0] : 0.0f, (k + 1 < nb) ? a[k + 1] : 0.0f,
-                   (k + 2 < nb) ? a[k + 2] : 0.0f, (k + 3 < nb) ? a[k + 3] : 0.0f);
+      _put_split4f (blk, row, 4 * q, (k + 0 < nb) ? a[k + 0] : 0.0f, (k + 1 < nb) ? a[k + 1] : 0.0f,
+                    (k + 2 < nb) ? a[k + 2] : 0.0f, (k + 3 < nb) ? a[k + 3] : 0.0f);
     }
   }
 }
