@@ -248,7 +248,7 @@ _dev_free_all (ncg_sd_t *sd)
     (void **) &sd->dVg, (void **) &sd->dpackmx, (void **) &sd->dknn, (void **) &sd->dflag, (void **) &sd->dids,
     (void **) &sd->dkeys, (void **) &sd->dst, (void **) &sd->dscratch, (void **) &sd->dq,
     (void **) &sd->dqo, (void **) &sd->dqi, (void **) &sd->df, (void **) &sd->dmu, (void **) &sd->dcal, (void **) &sd->dcv, (void **) &sd->dloo,
-    (void **) &sd->drq,
+    (void **) &sd->drq, (void **) &sd->dq64,
   };
 
   for (size_t i = 0; i < sizeof (bufs) / sizeof (bufs[0]); i++)
@@ -695,6 +695,7 @@ _split_obj (ncg_sd_t *sd, double lnos, double *hbuf, double *f)
 
   sd->cfg.over_smooth = exp (lnos);
   sd->href            = _get_href (sd);
+  sd->q64_ready       = 0;
 
   if (sd->kind == NCG_VKDE)
     CK (ncg_launch_vkde_finish (sd->dX, sd->dUi, sd->dflag, (int) sd->nk, d, sd->kernel, sd->dst, sd->href,
@@ -728,6 +729,8 @@ static ncg_status_t
 _href_operand (ncg_sd_t *sd)
 {
   const int d = (int) sd->d;
+
+  sd->q64_ready = 0;
 
   if (sd->kind == NCG_VKDE)
     CK (ncg_launch_vkde_finish (sd->dX, sd->dUi, sd->dflag, (int) sd->nk, d, sd->kernel, sd->dst, sd->href,
@@ -1278,6 +1281,7 @@ ncg_sd_prepare (ncg_sd_t *sd)
   sd->n_fallback     = 0;
   sd->wcum_ready     = 0;
   sd->packmx_ready   = 0;
+  sd->q64_ready      = 0;
   sd->interp_branch  = 0;
   sd->rnorm          = 0.0;
 
@@ -1557,6 +1561,27 @@ _eval_path (ncg_sd_t *sd, int linear, ncg_status_t *r)
   return NCG_PATH_SIMT;
 }
 
+/* The FP64 form's tensor-core operand, built at the first call that takes it
+ * after the kernels or the bandwidth changed (the weights are not in it);
+ * q64_ready = -1 where a kernel is too narrow for its fixed point. */
+static ncg_status_t
+_ensure_q64 (ncg_sd_t *sd, const ncg_eval_args_t *a)
+{
+  int32_t f = 0;
+
+  if (sd->q64_ready)
+    return NCG_OK;
+
+  RESERVE (dq64, q64, ncg_q64_operand_bytes (a->n, a->d));
+  CK (ncg_launch_q64_operand (a, sd->dX, sd->dpack64, sd->dU, sd->dVg, sd->dmu, sd->dq64, sd->stream), "q64 operand");
+  CK (cudaMemcpyAsync (&f, ncg_q64_operand_fmax (sd->dq64, a->n, a->d), sizeof (f), cudaMemcpyDeviceToHost, sd->stream),
+      "D2H q64 range");
+  CK (cudaStreamSynchronize (sd->stream), "sync");
+  sd->q64_ready = (f <= ncg_q64_fmax (a->d)) ? 1 : -1;
+
+  return NCG_OK;
+}
+
 static ncg_status_t
 _eval_device (ncg_sd_t *sd, const double *dXq, uint64_t m, double *dout, int linear)
 {
@@ -1576,6 +1601,23 @@ _eval_device (ncg_sd_t *sd, const double *dXq, uint64_t m, double *dout, int lin
 
   sd->last_path = path;
   ncg_sd_fill_args (sd, m, &a);
+
+  /* (a mixed request that its conditioning guard sends here keeps the plain
+   * form, as in a batch) */
+  if (path == NCG_PATH_FP64 && sd->cfg.precision == NCG_PREC_FP64 && ncg_q64_wanted (&a))
+  {
+    if ((r = _ensure_q64 (sd, &a)) != NCG_OK)
+      return r;
+
+    if (sd->q64_ready == 1)
+    {
+      RESERVE (dscratch, scratch, ncg_q64_scratch_bytes (&a));
+      CK (ncg_launch_eval_q64 (&a, dXq, sd->dq64, sd->dc, sd->dmu, sd->dVg, dout, sd->dscratch, linear,
+                               sd->d_flag_alias, sd->stream), "eval_q64");
+
+      return NCG_OK;
+    }
+  }
 
   if (path == NCG_PATH_FP64)
   {

@@ -12,7 +12,7 @@
 typedef struct ncg_caps
 {
   size_t X, Y, cov, U, Ui, lnnorm, w, c, wcum, pack64, Vg, packmx, knn, flag, ids, keys, st, scratch, q, qo, qi, f,
-         mu, cal, rq, cv, loo;
+         mu, cal, rq, cv, loo, q64;
 } ncg_caps_t;
 
 /* prepare_interp / NNLS device state (ncg_interp.c) */
@@ -71,6 +71,8 @@ struct ncg_sd
   int32_t *d_flag_alias;  /* its device address, written by the merge kernel */
   uint8_t *dtcB;          /* tensor-core kernel tiles */
   size_t cap_tcB;
+  uint8_t *dq64;          /* the FP64 form's tensor-core operand */
+  int q64_ready;          /* 0 not built for this operand state, 1 usable, -1 out of its range */
   uint32_t k;
   uint64_t n_fallback;
   double href, kernel_lnnorm, rnorm;

@@ -157,7 +157,16 @@ _chain_bytes (const ncg_chain_desc_t *c, int mixed)
   b += 8.0 * n * 8.0;                                       /* per-kernel vectors */
   b += 8.0 * 24.0 * n + 8.0 * n * ceil (n / 256.0);         /* NNLS vectors, gemv scratch */
   b += (double) ncg_pcg_trinv_bytes ((int) n) + (double) ncg_syrk_tc_pack_bytes ((int) n, 64);  /* preconditioner */
-  b += 16.0 * 2.0 * n * 16.0;                               /* eval partials (<= 16 slices of 2n) */
+  {
+    /* eval partials of 2n points, and the FP64 form's tensor-core operands */
+    ncg_eval_args_t a = { .kind = (int32_t) c->kind, .kernel = (int32_t) c->kernel, .d = (int32_t) c->dim, .dp = dp,
+                          .n = (int32_t) (c->n / 2), .m = (int64_t) c->n };
+
+    b += (double) ncg_eval_scratch_bytes (&a, NCG_PREC_FP64);
+
+    if (!mixed && ncg_q64_wanted (&a))
+      b += (double) ncg_q64_operand_bytes (a.n, a.d) + (double) ncg_q64_scratch_bytes (&a);
+  }
 
   if (c->kind == NCG_VKDE)
   {
