@@ -29,6 +29,10 @@ typedef struct ncg_nnls_dev
   /* the least-squares fallback's Householder work: A_P (n x np) and f | 3 scalars */
   double *Q, *qy;
   size_t cQ, cqy;
+  /* work of the FP64 normal equations: panel digits, exponents, chain words */
+  uint8_t *w64;
+  int32_t *ex64;
+  size_t cw64, cex64;
   int M64_ready;          /* the FP64 A^T A exists (mixed solver fallback) */
   uint32_t cs_epoch;      /* launches of the chained solves (their words carry it) */
 } ncg_nnls_dev_t;

@@ -229,15 +229,17 @@ cudaError_t ncg_launch_sample_at (int kind, int kernel, int d, double nu, double
 cudaError_t ncg_launch_im_rowsums (const double *IM, int n, double *rowx, double *diag, cudaStream_t s);
 
 /* ---- dense linear algebra for prepare_interp (ncg_linalg.cu) ---- */
-cudaError_t ncg_launch_syrk_upper (const double *A, int nrows, int ncols, double *M, cudaStream_t s);
 size_t      ncg_gemv_t_scratch (int nrows, int ncols);
 cudaError_t ncg_launch_gemv_ex (const double *A, int nrows, int ncols, int trans, double alpha,
                                 const double *x, double beta, double *y, double *part, cudaStream_t s);
 cudaError_t ncg_launch_normalize_weights (double *w, int n, double shrink, int32_t *bad, cudaStream_t s);
 cudaError_t ncg_launch_gather_sub (const double *M, int n, const int32_t *P, int np, double *Msub,
                                    const double *b, double *bsub, cudaStream_t s);
-cudaError_t ncg_launch_potrf (double *A, int n, int32_t *info, double *work, cudaStream_t s);
-cudaError_t ncg_launch_potrs (const double *U, int n, double *b, double *work, cudaStream_t s);
+/* FP64 normal equations on sliced tensor-core products (ncg_posv64.cu) */
+size_t      ncg_posv_work_bytes (int n);
+cudaError_t ncg_launch_posv (double *A, int n, double *b, int32_t *info, void *work, cudaStream_t s);
+cudaError_t ncg_launch_syrk_upper64 (const double *A, int nrows, int ncols, double *M, void *scratch, size_t cap,
+                                     int32_t *ex, int32_t *err, cudaStream_t s);
 /* the NNLS solve's fallbacks: symmetric solve of the upper-stored A (n x n,
  * overwritten) with right-hand side b (overwritten by x), *info = k + 1 at an
  * exactly zero pivot; least squares A[:, P] x = f by Householder QR (Q:

@@ -52,7 +52,7 @@ ncg_nnls_free (ncg_sd_t *sd)
     (void **) &sd->nn.D, (void **) &sd->nn.xv, (void **) &sd->nn.pv, (void **) &sd->nn.qv, (void **) &sd->nn.zv,
     (void **) &sd->nn.rv, (void **) &sd->nn.rp, (void **) &sd->nn.vf, (void **) &sd->nn.yf, (void **) &sd->nn.qf,
     (void **) &sd->nn.sc, (void **) &sd->nn.Vi, (void **) &sd->nn.csync, (void **) &sd->nn.pk32,
-    (void **) &sd->nn.Q, (void **) &sd->nn.qy,
+    (void **) &sd->nn.Q, (void **) &sd->nn.qy, (void **) &sd->nn.w64, (void **) &sd->nn.ex64,
   };
 
   for (size_t i = 0; i < sizeof (bufs) / sizeof (bufs[0]); i++)
@@ -216,17 +216,32 @@ typedef struct
   double rnorm;
 } nnls_t;
 
-/* FP64 A^T A (upper), made on first use by the mixed solver's fallback */
+/* FP64 A^T A (upper): at the start of the FP64 form, on first use by the mixed
+ * solver's fallback.  Its digits go through the factor's buffer, which is free
+ * until the first solve (or the panel work, where that is larger); a wait
+ * that gives up sets info[1]. */
 static ncg_status_t
-_ensure_M64 (nnls_t *s)
+_make_M64 (ncg_sd_t *sd, int nr, int n, int mixed)
 {
-  ncg_sd_t *sd = s->sd;
+  size_t cap;
+  void *scratch;
 
-  if (sd->nn.M64_ready)
-    return NCG_OK;
+  BRES (M, cM, sizeof (double) * (size_t) n * n, !mixed);
+  BRES (Msub, cMsub, sizeof (double) * (size_t) n * n, !mixed);
+  NRES (w64, cw64, ncg_posv_work_bytes (n));
+  NRES (ex64, cex64, sizeof (int32_t) * n);
 
-  BRES (M, cM, sizeof (double) * (size_t) s->n * s->n, 0);
-  CK (ncg_launch_syrk_upper (sd->nn.IM, s->nr, s->n, sd->nn.M, sd->stream), "syrk");
+  cap     = sizeof (double) * (size_t) n * n;
+  scratch = sd->nn.Msub;
+
+  if (cap < ncg_posv_work_bytes (n))
+  {
+    cap     = ncg_posv_work_bytes (n);
+    scratch = sd->nn.w64;
+  }
+
+  CK (ncg_launch_syrk_upper64 (sd->nn.IM, nr, n, sd->nn.M, scratch, cap, sd->nn.ex64, sd->nn.info + 1, sd->stream),
+      "syrk");
   sd->nn.M64_ready = 1;
 
   return NCG_OK;
@@ -242,18 +257,24 @@ _solve_fp64 (nnls_t *s, int np, double *dx)
 {
   ncg_sd_t *sd = s->sd;
   cudaStream_t st = sd->stream;
+  int32_t fi[2] = { 0, 0 };
   int info = 0;
 
-  BRES (Msub, cMsub, sizeof (double) * (size_t) np * np, !s->mixed);
   CK (ncg_launch_gather_sub (sd->nn.M, s->n, sd->nn.P, np, sd->nn.Msub, sd->nn.b, sd->nn.bsub, st), "gather");
-  CK (ncg_launch_potrf (sd->nn.Msub, np, sd->nn.info, NULL, st), "potrf");
-  CK (cudaMemcpyAsync (&info, sd->nn.info, sizeof (int32_t), cudaMemcpyDeviceToHost, st), "D2H info");
+  CK (ncg_launch_posv (sd->nn.Msub, np, sd->nn.bsub, sd->nn.info, sd->nn.w64, st), "posv");
+  CK (cudaMemcpyAsync (fi, sd->nn.info, sizeof (fi), cudaMemcpyDeviceToHost, st), "D2H info");
   CK (cudaStreamSynchronize (st), "sync");
   sd->istats.n_fp64++;
 
-  if (info == 0)
+  if (fi[0] < 0 || fi[1] != 0)
   {
-    CK (ncg_launch_potrs (sd->nn.Msub, np, sd->nn.bsub, sd->nn.xsub, st), "potrs");
+    ncg_set_error ("prepare_interp: a bounded wait of the FP64 normal equations gave up");
+
+    return NCG_ERR_TIMEOUT;
+  }
+
+  if (fi[0] == 0)
+  {
     CK (ncg_launch_scatter_x (sd->nn.bsub, sd->nn.P, np, s->n, dx, st), "scatter");
 
     return NCG_OK;
@@ -410,8 +431,9 @@ _solve_mixed (nnls_t *s, int np, double *dx)
     }
   }
 
+  if (!sd->nn.M64_ready)
   {
-    ncg_status_t r = _ensure_M64 (s);
+    ncg_status_t r = _make_M64 (sd, nr, n, 1);
 
     if (r != NCG_OK)
       return r;
@@ -644,6 +666,8 @@ _nnls_reserve (ncg_sd_t *sd, int nr, int n, int mixed)
   {
     BRES (M, cM, sizeof (double) * (size_t) n * n, 1);
     BRES (Msub, cMsub, sizeof (double) * (size_t) n * n, 1);
+    NRES (w64, cw64, ncg_posv_work_bytes (n));
+    NRES (ex64, cex64, sizeof (int32_t) * n);
   }
 
   return NCG_OK;
@@ -716,8 +740,10 @@ _nnls (ncg_sd_t *sd, int nr, int n, int mixed, double *rnorm_out)
   }
   else
   {
-    CK (ncg_launch_syrk_upper (sd->nn.IM, nr, n, sd->nn.M, st), "syrk");
-    sd->nn.M64_ready = 1;
+    CK (cudaMemsetAsync (sd->nn.info, 0, sizeof (int32_t) * 4, st), "memset info");
+
+    if ((r = _make_M64 (sd, nr, n, 0)) != NCG_OK)
+      return r;
   }
 
   memset (&s, 0, sizeof (s));

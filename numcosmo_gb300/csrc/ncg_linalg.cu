@@ -2,16 +2,15 @@
  * ncg_linalg.cu -- dense kernels behind prepare_interp's NNLS
  * (ncm_nnls_solve, numcosmo/ncm/algebra/ncm_nnls.c:767-871, NORMAL umethod):
  *
- *   syrk_upper    M = A^T A, upper triangle (ncm_matrix_square_to_sym,
- *                 numcosmo/ncm/algebra/ncm_matrix.c:1548-1572); FP64, and an
- *                 FP32 copy for the mixed solver's preconditioner
- *   gemv          y = alpha op(A) x + beta y, deterministic reductions
- *   gather_sub    M[P,P], b[P] for an active set P (ncm_iset_get_submatrix)
- *   potrf         blocked right-looking Cholesky, upper, row-major (dpotrf),
- *                 FP64 and FP32
- *   potrs         U^T U x = b (dposv's solve), blocked over many CTAs
- *   residual_norm res = f - A x and |res|^2 (ncm_nnls.c:700-711)
- *   pcg_*         the FP64 conjugate-gradient refinement of the mixed solver
+ *   syrk_upper_f32  M = A^T A, upper triangle (ncm_matrix_square_to_sym,
+ *                   numcosmo/ncm/algebra/ncm_matrix.c:1548-1572) in FP32 for the
+ *                   mixed solver's preconditioner (FP64: ncg_posv64.cu)
+ *   gemv            y = alpha op(A) x + beta y, deterministic reductions
+ *   gather_sub      M[P,P], b[P] for an active set P (ncm_iset_get_submatrix)
+ *   potrf_f32       blocked right-looking Cholesky, upper, row-major (the FP64
+ *                   solve: ncg_posv64.cu)
+ *   residual_norm   res = f - A x and |res|^2 (ncm_nnls.c:700-711)
+ *   pcg_*           the FP64 conjugate-gradient refinement of the mixed solver
  *
  * Every reduction has a fixed order, so two runs give identical bits.
  */
@@ -20,107 +19,6 @@
 
 #include "ncg_internal.h"
 #include "ncg_syrk_tc.cuh"
-
-#define TB 64     /* output tile */
-#define KB 16     /* rows per smem stage */
-
-/* C[i][j] = (or -=) sum_{r in [r0, r1)} A[r][i] A[r][j] for off <= i <= j < off + nn.
- * TI is the storage type of A, T the arithmetic and output type. */
-template <typename TI, typename T>
-__global__ void __launch_bounds__ (256)
-_syrk_tile_kernel (const TI *__restrict__ A, int lda, int r0, int r1, int off, int nn,
-                   T *__restrict__ C, int ldc, int minus)
-{
-  __shared__ T As[KB][TB];
-  __shared__ T Bs[KB][TB];
-
-  /* map the linear block id onto the upper tiles (ti <= tj) */
-  const int T_ = (nn + TB - 1) / TB;
-  int b = blockIdx.x, ti = 0;
-
-  while (b >= T_ - ti)
-  {
-    b -= T_ - ti;
-    ti++;
-  }
-
-  const int tj  = ti + b;
-  const int i0  = off + ti * TB, j0 = off + tj * TB;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int end = off + nn;
-  T acc[4][4];
-
-#pragma unroll
-  for (int a = 0; a < 4; a++)
-#pragma unroll
-    for (int c = 0; c < 4; c++)
-      acc[a][c] = (T) 0;
-
-  for (int rb = r0; rb < r1; rb += KB)
-  {
-    for (int e = tid; e < KB * TB; e += 256)
-    {
-      const int rr = e / TB, cc = e - rr * TB;
-      const int r  = rb + rr;
-
-      As[rr][cc] = (r < r1 && i0 + cc < end) ? (T) A[(size_t) r * lda + i0 + cc] : (T) 0;
-      Bs[rr][cc] = (r < r1 && j0 + cc < end) ? (T) A[(size_t) r * lda + j0 + cc] : (T) 0;
-    }
-
-    __syncthreads ();
-
-#pragma unroll
-    for (int rr = 0; rr < KB; rr++)
-    {
-      T a[4], bb[4];
-
-#pragma unroll
-      for (int q = 0; q < 4; q++)
-      {
-        a[q]  = As[rr][ty * 4 + q];
-        bb[q] = Bs[rr][tx * 4 + q];
-      }
-
-#pragma unroll
-      for (int p = 0; p < 4; p++)
-#pragma unroll
-        for (int q = 0; q < 4; q++)
-          acc[p][q] = fma (a[p], bb[q], acc[p][q]);
-    }
-
-    __syncthreads ();
-  }
-
-#pragma unroll
-  for (int p = 0; p < 4; p++)
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-    {
-      const int i = i0 + ty * 4 + p, j = j0 + tx * 4 + q;
-
-      if (i < end && j < end && j >= i)
-      {
-        T *dst = C + (size_t) i * ldc + j;
-
-        *dst = minus ? (*dst - acc[p][q]) : acc[p][q];
-      }
-    }
-}
-
-template <typename TI, typename T>
-static cudaError_t
-_syrk (const TI *A, int lda, int r0, int r1, int off, int nn, T *C, int ldc, int minus, cudaStream_t s)
-{
-  if (nn <= 0)
-    return cudaSuccess;
-
-  const int T_      = (nn + TB - 1) / TB;
-  const int nblocks = T_ * (T_ + 1) / 2;
-
-  _syrk_tile_kernel<TI, T><<<nblocks, 256, 0, s>>> (A, lda, r0, r1, off, nn, C, ldc, minus);
-
-  return cudaGetLastError ();
-}
 
 /* FP32 products (the mixed solver's A^T A below 1024 columns):
  * 128 x 128 upper tiles, 256 threads of 8 x 8 outputs (rows ty*4 + {0..3} and
@@ -243,12 +141,6 @@ _syrk128 (const TI *A, int lda, int r0, int r1, int off, int nn, float *C, int l
   _syrk128_f32_kernel<TI><<<T_ * (T_ + 1) / 2, 256, 0, s>>> (A, lda, r0, r1, off, nn, C, ldc);
 
   return cudaGetLastError ();
-}
-
-extern "C" cudaError_t
-ncg_launch_syrk_upper (const double *A, int nrows, int ncols, double *M, cudaStream_t s)
-{
-  return _syrk<double, double> (A, ncols, 0, nrows, 0, ncols, M, ncols, 0, s);
 }
 
 extern "C" cudaError_t
@@ -552,135 +444,6 @@ _stage_block (T (*S)[B + 1], const T *__restrict__ A, int ld, int r0, int c0, in
   }
 }
 
-/* FP64: factor the nb x nb diagonal block at (kb, kb) in place (upper),
- * right-looking inside shared memory: at step j the row j is final, scaled by
- * 1/U_jj, and the trailing block takes the rank-1 update in ascending j order.
- * Thread (ty, tx) of the 16 x 16 block owns the elements (ty + 16p, tx + 16q),
- * which spreads the shrinking trailing triangle over all threads.  Two
- * barriers a step: the diagonal read and the row scaling, then the update
- * (which also stores U_jj, read by nobody in that phase). */
-__global__ void __launch_bounds__ (256)
-_potrf_diag_f64_kernel (double *A, int ld, int kb, int nb, int32_t *info)
-{
-  __shared__ double S[PB][PB + 1];
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  int fail      = 0;
-
-  if (*info)
-    return;
-
-  _stage_block<double, 256, PB> (S, A, ld, kb, kb, nb, tid);
-
-  __syncthreads ();
-
-  for (int j = 0; j < nb; j++)
-  {
-    const double ajj = S[j][j];
-
-    if (!(ajj > 0.0))
-    {
-      fail = j + 1;
-      break;
-    }
-
-    const double ujj = sqrt (ajj);
-
-    if (tid > j && tid < nb)
-      S[j][tid] = S[j][tid] / ujj;
-
-    __syncthreads ();
-
-    if (tid == 0)
-      S[j][j] = ujj;
-
-#pragma unroll
-    for (int p = 0; p < PB / 16; p++)
-    {
-      const int r = ty + 16 * p;
-
-      if (r > j && r < nb)
-      {
-        const double sjr = S[j][r];
-
-#pragma unroll
-        for (int q = 0; q < PB / 16; q++)
-        {
-          const int c = tx + 16 * q;
-
-          if (c >= r && c < nb)
-            S[r][c] = fma (-sjr, S[j][c], S[r][c]);
-        }
-      }
-    }
-
-    __syncthreads ();
-  }
-
-  if (fail)
-  {
-    if (tid == 0)
-      atomicCAS (info, 0, kb + fail);
-
-    return;
-  }
-
-  for (int e = tid; e < nb * nb; e += 256)
-  {
-    const int r = e / nb, c = e - r * nb;
-
-    if (c >= r)
-      A[(size_t) (kb + r) * ld + kb + c] = S[r][c];
-  }
-}
-
-/* FP64: rows kb..kb+nb of the columns right of the block: X = U_kk^{-T} A_panel,
- * one column per thread held in registers (column sweep in ascending row
- * order) */
-#define TRSM_TH 128
-
-__global__ void __launch_bounds__ (TRSM_TH)
-_potrf_trsm_f64_kernel (double *A, int ld, int kb, int nb, int n, const int32_t *info)
-{
-  __shared__ double S[PB][PB + 1];
-  const int tid = threadIdx.x;
-
-  if (*info)
-    return;
-
-  _stage_block<double, TRSM_TH, PB> (S, A, ld, kb, kb, nb, tid);
-
-  __syncthreads ();
-
-  const int col = kb + nb + blockIdx.x * TRSM_TH + tid;
-
-  if (col >= n)
-    return;
-
-  double a[PB];
-
-#pragma unroll
-  for (int r = 0; r < PB; r++)
-    a[r] = (r < nb) ? A[(size_t) (kb + r) * ld + col] : 0.0;
-
-#pragma unroll
-  for (int r = 0; r < PB; r++)
-  {
-    if (r < nb)
-    {
-      a[r] = a[r] / S[r][r];
-
-#pragma unroll
-      for (int m = r + 1; m < PB; m++)
-        a[m] = fma (-S[r][m], a[r], a[m]);
-    }
-  }
-
-#pragma unroll
-  for (int r = 0; r < PB; r++)
-    if (r < nb)
-      A[(size_t) (kb + r) * ld + col] = a[r];
-}
-
 /* ---- the FP32 preconditioner's panels ---- */
 
 /* The nb x nb diagonal block (upper, in place).  The block lives in registers,
@@ -952,33 +715,6 @@ _zero_int_kernel (int32_t *p)
   *p = 0;
 }
 
-extern "C" cudaError_t
-ncg_launch_potrf (double *A, int n, int32_t *info, double *work, cudaStream_t s)
-{
-  (void) work;
-
-  _zero_int_kernel<<<1, 1, 0, s>>> (info);
-
-  for (int kb = 0; kb < n; kb += PB)
-  {
-    const int nb = (n - kb < PB) ? n - kb : PB, rest = n - kb - nb;
-
-    _potrf_diag_f64_kernel<<<1, 256, 0, s>>> (A, n, kb, nb, info);
-
-    if (rest > 0)
-    {
-      _potrf_trsm_f64_kernel<<<(rest + TRSM_TH - 1) / TRSM_TH, TRSM_TH, 0, s>>> (A, n, kb, nb, n, info);
-
-      const cudaError_t e = _syrk<double, double> (A, n, kb, kb + nb, kb + nb, rest, A, n, 1, s);
-
-      if (e != cudaSuccess)
-        return e;
-    }
-  }
-
-  return cudaGetLastError ();
-}
-
 /* trailing blocks at least this wide take the tensor-core update */
 #define POTRF_TC_MIN 2560
 
@@ -1016,191 +752,6 @@ ncg_launch_potrf_f32 (float *A, int n, int32_t *info, float *pk, cudaStream_t s)
   }
 
   return cudaGetLastError ();
-}
-
-/* ---- blocked triangular solves ------------------------------------------- */
-
-#define SB 64     /* diagonal block of the solves */
-#define SV_TH 128
-
-/* U^T y = b, block [kb, kb+nb): every CTA stages the diagonal block in shared
- * memory and solves it from the (final) b_k with one warp (lanes own y_l and
- * y_{l+32}), CTA 0 stores y_k into y, and each CTA subtracts the block's
- * contribution from its slice of b past the block, in ascending row order
- * (the operation order of a plain column sweep).  b_k is read by every CTA
- * and written by none, so the launch has no race. */
-template <typename T>
-__global__ void __launch_bounds__ (SV_TH)
-_trsv_t_kernel (const T *__restrict__ U, int n, int kb, int nb, T *__restrict__ b, T *__restrict__ yout)
-{
-  __shared__ T S[SB][SB + 1];
-  __shared__ T y[SB];
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-
-  _stage_block<T, SV_TH, SB> (S, U, n, kb, kb, nb, tid);
-
-  __syncthreads ();
-
-  if (wid == 0)
-  {
-    T y0 = (lane < nb) ? b[kb + lane] : (T) 0;
-    T y1 = (lane + 32 < nb) ? b[kb + lane + 32] : (T) 0;
-
-    for (int r = 0; r < nb; r++)
-    {
-      const T yraw = __shfl_sync (0xffffffffu, (r < 32) ? y0 : y1, r & 31);
-      const T yr   = yraw / S[r][r];
-
-      if (r < 32)
-      {
-        if (lane == r)
-          y0 = yr;
-      }
-      else if (lane == r - 32)
-      {
-        y1 = yr;
-      }
-
-      if (lane > r && lane < nb)
-        y0 = fma (-S[r][lane], yr, y0);
-
-      if (lane + 32 > r && lane + 32 < nb)
-        y1 = fma (-S[r][lane + 32], yr, y1);
-    }
-
-    y[lane] = y0;
-
-    if (lane + 32 < SB)
-      y[lane + 32] = y1;
-  }
-
-  __syncthreads ();
-
-  if (blockIdx.x == 0 && tid < nb)
-    yout[kb + tid] = y[tid];
-
-  const int i = kb + nb + blockIdx.x * SV_TH + tid;
-
-  if (i < n)
-  {
-    T bi = b[i];
-
-#pragma unroll 16
-    for (int r = 0; r < nb; r++)
-      bi = fma (-U[(size_t) (kb + r) * n + i], y[r], bi);
-
-    b[i] = bi;
-  }
-}
-
-/* U x = y, block [kb, kb+nb) (blocks taken from the last): every CTA stages
- * the diagonal block and solves it by back substitution from the (final)
- * y_k with one warp, CTA 0 stores x_k into x, and the rows of y before the
- * block take the block's contribution, one warp per row. */
-template <typename T>
-__global__ void __launch_bounds__ (SV_TH)
-_trsv_n_kernel (const T *__restrict__ U, int n, int kb, int nb, T *__restrict__ yv, T *__restrict__ xout)
-{
-  __shared__ T S[SB][SB + 1];
-  __shared__ T x[SB];
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-
-  _stage_block<T, SV_TH, SB> (S, U, n, kb, kb, nb, tid);
-
-  __syncthreads ();
-
-  if (wid == 0)
-  {
-    T x0 = (lane < nb) ? yv[kb + lane] : (T) 0;
-    T x1 = (lane + 32 < nb) ? yv[kb + lane + 32] : (T) 0;
-
-    for (int r = nb - 1; r >= 0; r--)
-    {
-      const T xraw = __shfl_sync (0xffffffffu, (r < 32) ? x0 : x1, r & 31);
-      const T xr   = xraw / S[r][r];
-
-      if (r < 32)
-      {
-        if (lane == r)
-          x0 = xr;
-      }
-      else if (lane == r - 32)
-      {
-        x1 = xr;
-      }
-
-      if (lane < r)
-        x0 = fma (-S[lane][r], xr, x0);
-
-      if (lane + 32 < r)
-        x1 = fma (-S[lane + 32][r], xr, x1);
-    }
-
-    x[lane] = x0;
-
-    if (lane + 32 < SB)
-      x[lane + 32] = x1;
-  }
-
-  __syncthreads ();
-
-  if (blockIdx.x == 0 && tid < nb)
-    xout[kb + tid] = x[tid];
-
-  const int row = blockIdx.x * (SV_TH / 32) + wid;
-
-  if (row < kb)
-  {
-    const T *u = U + (size_t) row * n + kb;
-    T s        = (T) 0;
-
-    for (int c = lane; c < nb; c += 32)
-      s = fma (u[c], x[c], s);
-
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-      s += __shfl_xor_sync (0xffffffffu, s, o);
-
-    if (lane == 0)
-      yv[row] -= s;
-  }
-}
-
-/* U^T U x = b: b is the right-hand side on entry and the solution on exit,
- * work an n-long scratch vector */
-template <typename T>
-static cudaError_t
-_potrs (const T *U, int n, T *b, T *work, cudaStream_t s)
-{
-  for (int kb = 0; kb < n; kb += SB)
-  {
-    const int nb   = (n - kb < SB) ? n - kb : SB;
-    const int rest = n - kb - nb;
-    const int g    = (rest + SV_TH - 1) / SV_TH;
-
-    _trsv_t_kernel<T><<<g > 0 ? g : 1, SV_TH, 0, s>>> (U, n, kb, nb, b, work);
-  }
-
-  const int last = ((n - 1) / SB) * SB;
-
-  for (int kb = last; kb >= 0; kb -= SB)
-  {
-    const int nb = (n - kb < SB) ? n - kb : SB;
-    const int g  = (kb + SV_TH / 32 - 1) / (SV_TH / 32);
-
-    _trsv_n_kernel<T><<<g > 0 ? g : 1, SV_TH, 0, s>>> (U, n, kb, nb, work, b);
-  }
-
-  return cudaGetLastError ();
-}
-
-extern "C" cudaError_t
-ncg_launch_potrs (const double *U, int n, double *b, double *work, cudaStream_t s)
-{
-  if (n <= 0)
-    return cudaSuccess;
-
-  return _potrs<double> (U, n, b, work, s);
 }
 
 /* ---- residuals --------------------------------------------------------- */
@@ -1441,6 +992,7 @@ ncg_launch_pcg_matvec (const double *A, int nrows, int n, const int32_t *P, int 
  * launches (the last CTA to finish clears them).  A wait gives up after
  * CS_SPIN polls, sets *err = 1 and sync[2], and the launch goes on with what
  * it has, so it always ends; a later wait that sees sync[2] does not spin. */
+#define SB 64     /* block of the solves */
 #define CS_TH 128
 #define CS_SPIN (1 << 21)
 

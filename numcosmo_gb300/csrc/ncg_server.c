@@ -164,6 +164,9 @@ _chain_bytes (const ncg_chain_desc_t *c, int mixed)
 
     b += (double) ncg_eval_scratch_bytes (&a, NCG_PREC_FP64);
 
+    if (!mixed)
+      b += (double) ncg_posv_work_bytes (a.n);
+
     if (!mixed && ncg_q64_wanted (&a))
       b += (double) ncg_q64_operand_bytes (a.n, a.d) + (double) ncg_q64_scratch_bytes (&a);
   }
