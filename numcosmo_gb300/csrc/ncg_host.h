@@ -23,9 +23,9 @@ typedef struct ncg_nnls_dev
   size_t cIM, cM, cb, cf1, cx, cxsub, cMsub, cbsub, cres, cmg, cpart, cred, cP, cinfo;
   /* mixed solver: FP32 A^T A and factor, FP64 diagonal and CG vectors */
   float *M32, *R32, *t32, *Vi, *pk32;
-  double *diagM, *D, *xv, *pv, *qv, *zv, *rv, *rp, *vf, *yf, *qf, *sc;
+  double *diagM, *D, *xv, *pv, *qv, *zv, *rv, *rp, *yf, *sc;
   int32_t *csync;
-  size_t cM32, cR32, ct32, cVi, cpk32, cdiagM, cD, cxv, cpv, cqv, czv, crv, crp, cvf, cyf, cqf, csc, ccsync;
+  size_t cM32, cR32, ct32, cVi, cpk32, cdiagM, cD, cxv, cpv, cqv, czv, crv, crp, cyf, csc, ccsync;
   /* the least-squares fallback's Householder work: A_P (n x np) and f | 3 scalars */
   double *Q, *qy;
   size_t cQ, cqy;

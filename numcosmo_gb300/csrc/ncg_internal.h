@@ -230,8 +230,8 @@ cudaError_t ncg_launch_im_rowsums (const double *IM, int n, double *rowx, double
 
 /* ---- dense linear algebra for prepare_interp (ncg_linalg.cu) ---- */
 size_t      ncg_gemv_t_scratch (int nrows, int ncols);
-cudaError_t ncg_launch_gemv_ex (const double *A, int nrows, int ncols, int trans, double alpha,
-                                const double *x, double beta, double *y, double *part, cudaStream_t s);
+cudaError_t ncg_launch_gemv_t (const double *A, int nrows, int ncols, const double *x, double *y, double *part,
+                               cudaStream_t s);
 cudaError_t ncg_launch_normalize_weights (double *w, int n, double shrink, int32_t *bad, cudaStream_t s);
 cudaError_t ncg_launch_gather_sub (const double *M, int n, const int32_t *P, int np, double *Msub,
                                    const double *b, double *bsub, cudaStream_t s);
@@ -249,9 +249,9 @@ cudaError_t ncg_launch_gels (const double *A, int nrows, int ncols, const int32_
                              double *Q, double *y, double *sc, double *x, cudaStream_t s);
 
 /* mixed NNLS: FP32 preconditioner, FP64 conjugate-gradient refinement */
-enum { NCG_PCG_RZ = 0, NCG_PCG_PQ, NCG_PCG_RZN, NCG_PCG_ZRP, NCG_PCG_RR, NCG_PCG_BB, NCG_PCG_ERR, NCG_PCG_NSC = 8 };
+enum { NCG_PCG_RZ = 0, NCG_PCG_PQ, NCG_PCG_BE, NCG_PCG_RR, NCG_PCG_BB, NCG_PCG_ERR, NCG_PCG_NSC = 8 };
 cudaError_t ncg_launch_syrk_upper_f32 (const double *A, int nrows, int ncols, float *M, cudaStream_t s);
-cudaError_t ncg_launch_colsumsq (const double *A, int nrows, int ncols, double *out, cudaStream_t s);
+cudaError_t ncg_launch_colsumsq (const double *A, int nrows, int ncols, double *out, double *part, cudaStream_t s);
 cudaError_t ncg_launch_gather_scaled_f32 (const float *M32, int n, const int32_t *P, int np, const double *diagM,
                                           double shift, float *Msub, double *Dsub, const double *b, double *bsub,
                                           cudaStream_t s);
@@ -263,7 +263,7 @@ cudaError_t ncg_launch_syrk_tc (const void *pk, int K, int nn, float *C, int ldc
 cudaError_t ncg_launch_syrk_upper_tc_f64 (const double *A, int nrows, int ncols, float *C, void *scratch,
                                           size_t cap, int *err, cudaStream_t s);
 cudaError_t ncg_launch_pcg_matvec (const double *A, int nrows, int n, const int32_t *P, int np, const double *v,
-                                   double *vf, double *yf, double *qf, double *part, double *q, cudaStream_t s);
+                                   const double *b, double *yf, double *part, double *q, cudaStream_t s);
 size_t      ncg_pcg_trinv_bytes (int n);
 size_t      ncg_pcg_sync_bytes (int n);
 size_t      ncg_pcg_chain_bytes (int n);
@@ -271,12 +271,12 @@ cudaError_t ncg_launch_trinv_diag_f32 (const float *U, int n, float *V, cudaStre
 cudaError_t ncg_launch_pcg_precond (const float *R, const float *V, const double *D, int np, const double *r,
                                     void *chain, uint32_t *epoch, double *z, int32_t *sync, double *err,
                                     cudaStream_t s);
-cudaError_t ncg_launch_pcg_dot (const double *u0, const double *v0, const double *u1, const double *v1,
-                                const double *w, int n, double *sc, int out0, int out1, cudaStream_t s);
+size_t      ncg_pcg_sc_bytes (void);
+cudaError_t ncg_launch_pcg_dots (int mode, const double *u, const double *v, const double *w, const double *D,
+                                 double *p, int n, double *sc, cudaStream_t s);
 cudaError_t ncg_launch_pcg_step (double *x, double *r, double *rprev, const double *p, const double *q, int n,
                                  const double *sc, cudaStream_t s);
 cudaError_t ncg_launch_pcg_dir (double *p, const double *z, int n, double *sc, cudaStream_t s);
-cudaError_t ncg_launch_rsub (const double *b, double *r, int n, cudaStream_t s);
 cudaError_t ncg_launch_scatter_x (const double *xsub, const int32_t *P, int np, int n, double *x,
                                   cudaStream_t s);
 cudaError_t ncg_launch_residual_norm (const double *A, int nrows, int ncols, const double *x,

@@ -50,7 +50,7 @@ ncg_nnls_free (ncg_sd_t *sd)
     (void **) &sd->nn.mg, (void **) &sd->nn.part, (void **) &sd->nn.red, (void **) &sd->nn.P, (void **) &sd->nn.info,
     (void **) &sd->nn.M32, (void **) &sd->nn.R32, (void **) &sd->nn.t32, (void **) &sd->nn.diagM,
     (void **) &sd->nn.D, (void **) &sd->nn.xv, (void **) &sd->nn.pv, (void **) &sd->nn.qv, (void **) &sd->nn.zv,
-    (void **) &sd->nn.rv, (void **) &sd->nn.rp, (void **) &sd->nn.vf, (void **) &sd->nn.yf, (void **) &sd->nn.qf,
+    (void **) &sd->nn.rv, (void **) &sd->nn.rp, (void **) &sd->nn.yf,
     (void **) &sd->nn.sc, (void **) &sd->nn.Vi, (void **) &sd->nn.csync, (void **) &sd->nn.pk32,
     (void **) &sd->nn.Q, (void **) &sd->nn.qy, (void **) &sd->nn.w64, (void **) &sd->nn.ex64,
   };
@@ -359,14 +359,10 @@ _solve_mixed (nnls_t *s, int np, double *dx)
      * precision), r = b - A_P^T A_P x0, z = B^{-1} r, p = z */
     CK (ncg_launch_pcg_precond (nn->R32, nn->Vi, nn->D, np, nn->bsub, nn->t32, &nn->cs_epoch, nn->xv, nn->csync,
                                  nn->sc + NCG_PCG_ERR, st), "precond");
-    CK (ncg_launch_pcg_matvec (nn->IM, nr, n, nn->P, np, nn->xv, nn->vf, nn->yf, nn->qf, nn->part, nn->rv, st), "matvec");
-    CK (ncg_launch_rsub (nn->bsub, nn->rv, np, st), "rsub");
+    CK (ncg_launch_pcg_matvec (nn->IM, nr, n, nn->P, np, nn->xv, nn->bsub, nn->yf, nn->part, nn->rv, st), "matvec");
     CK (ncg_launch_pcg_precond (nn->R32, nn->Vi, nn->D, np, nn->rv, nn->t32, &nn->cs_epoch, nn->zv, nn->csync,
                                  nn->sc + NCG_PCG_ERR, st), "precond");
-    CK (cudaMemcpyAsync (nn->pv, nn->zv, sizeof (double) * np, cudaMemcpyDeviceToDevice, st), "D2D p");
-    CK (ncg_launch_pcg_dot (nn->rv, nn->zv, NULL, NULL, NULL, np, nn->sc, NCG_PCG_RZ, 0, st), "dot");
-    CK (ncg_launch_pcg_dot (nn->bsub, nn->bsub, NULL, NULL, nn->D, np, nn->sc, NCG_PCG_BB, 0, st), "dot");
-    CK (ncg_launch_pcg_dot (nn->rv, nn->rv, NULL, NULL, nn->D, np, nn->sc, NCG_PCG_RR, 0, st), "dot");
+    CK (ncg_launch_pcg_dots (0, nn->rv, nn->zv, nn->bsub, nn->D, nn->pv, np, nn->sc, st), "dots");
 
     for (it = 0;; it++)
     {
@@ -401,24 +397,18 @@ _solve_mixed (nnls_t *s, int np, double *dx)
           !(hs[NCG_PCG_RZ] > 0.0))
         break;
 
-      CK (ncg_launch_pcg_matvec (nn->IM, nr, n, nn->P, np, nn->pv, nn->vf, nn->yf, nn->qf, nn->part, nn->qv, st),
-          "matvec");
-      CK (ncg_launch_pcg_dot (nn->pv, nn->qv, NULL, NULL, NULL, np, nn->sc, NCG_PCG_PQ, 0, st), "dot");
+      CK (ncg_launch_pcg_matvec (nn->IM, nr, n, nn->P, np, nn->pv, NULL, nn->yf, nn->part, nn->qv, st), "matvec");
+      CK (ncg_launch_pcg_dots (1, nn->pv, nn->qv, NULL, NULL, NULL, np, nn->sc, st), "dots");
       CK (ncg_launch_pcg_step (nn->xv, nn->rv, nn->rp, nn->pv, nn->qv, np, nn->sc, st), "step");
 
+      /* every few steps the recurred residual gives way to the true one */
       if ((it + 1) % NCG_PCG_RESTART == 0)
-      {
-        /* replace the recurred residual by the true one */
-        CK (ncg_launch_pcg_matvec (nn->IM, nr, n, nn->P, np, nn->xv, nn->vf, nn->yf, nn->qf, nn->part, nn->rv, st),
-            "matvec");
-        CK (ncg_launch_rsub (nn->bsub, nn->rv, np, st), "rsub");
-      }
+        CK (ncg_launch_pcg_matvec (nn->IM, nr, n, nn->P, np, nn->xv, nn->bsub, nn->yf, nn->part, nn->rv, st), "matvec");
 
       CK (ncg_launch_pcg_precond (nn->R32, nn->Vi, nn->D, np, nn->rv, nn->t32, &nn->cs_epoch, nn->zv, nn->csync,
                                  nn->sc + NCG_PCG_ERR, st), "precond");
-      CK (ncg_launch_pcg_dot (nn->rv, nn->zv, nn->zv, nn->rp, NULL, np, nn->sc, NCG_PCG_RZN, NCG_PCG_ZRP, st), "dot");
+      CK (ncg_launch_pcg_dots (2, nn->rv, nn->zv, nn->rp, nn->D, NULL, np, nn->sc, st), "dots");
       CK (ncg_launch_pcg_dir (nn->pv, nn->zv, np, nn->sc, st), "dir");
-      CK (ncg_launch_pcg_dot (nn->rv, nn->rv, NULL, NULL, nn->D, np, nn->sc, NCG_PCG_RR, 0, st), "dot");
     }
 
     sd->istats.n_cg_iters += it;
@@ -569,7 +559,7 @@ _mgrad (nnls_t *s, const double *dres)
 {
   ncg_sd_t *sd = s->sd;
 
-  CK (ncg_launch_gemv_ex (sd->nn.IM, s->nr, s->n, 1, 1.0, dres, 0.0, sd->nn.mg, sd->nn.part, sd->stream), "mgrad");
+  CK (ncg_launch_gemv_t (sd->nn.IM, s->nr, s->n, dres, sd->nn.mg, sd->nn.part, sd->stream), "mgrad");
   CK (cudaMemcpyAsync (s->mg, sd->nn.mg, sizeof (double) * s->n, cudaMemcpyDeviceToHost, sd->stream), "D2H mgrad");
   CK (cudaStreamSynchronize (sd->stream), "sync");
 
@@ -623,6 +613,10 @@ _add_largest (char *inP, int n, const double *v, double vmin, double add_frac)
   return adds;
 }
 
+/* A^T A of the mixed form goes to the tensor cores from this many columns (n =
+ * 512: 115 us on the CUDA cores) */
+#define NCG_SYRK_TC_MIN 128
+
 /* every device buffer the NNLS of an nr x n system reserves (the large
  * matrices from the caller's arena when one is set, after the interpolation
  * matrix) */
@@ -654,10 +648,8 @@ _nnls_reserve (ncg_sd_t *sd, int nr, int n, int mixed)
     NRES (zv, czv, sizeof (double) * n);
     NRES (rv, crv, sizeof (double) * n);
     NRES (rp, crp, sizeof (double) * n);
-    NRES (vf, cvf, sizeof (double) * n);
     NRES (yf, cyf, sizeof (double) * nr);
-    NRES (qf, cqf, sizeof (double) * n);
-    NRES (sc, csc, sizeof (double) * NCG_PCG_NSC);
+    NRES (sc, csc, ncg_pcg_sc_bytes ());
     NRES (Vi, cVi, ncg_pcg_trinv_bytes (n));
     NRES (csync, ccsync, ncg_pcg_sync_bytes (n));
     NRES (pk32, cpk32, ncg_syrk_tc_pack_bytes (n, 64));
@@ -719,11 +711,11 @@ _nnls (ncg_sd_t *sd, int nr, int n, int mixed, double *rnorm_out)
   memset (&sd->istats, 0, sizeof (sd->istats));
 
   CK (ncg_launch_fill (sd->nn.f1, 1.0, nr, st), "fill");
-  CK (ncg_launch_gemv_ex (sd->nn.IM, nr, n, 1, 1.0, sd->nn.f1, 0.0, sd->nn.b, sd->nn.part, st), "gemv b");
+  CK (ncg_launch_gemv_t (sd->nn.IM, nr, n, sd->nn.f1, sd->nn.b, sd->nn.part, st), "gemv b");
 
   if (mixed)
   {
-    CK (cudaMemsetAsync (sd->nn.sc, 0, sizeof (double) * NCG_PCG_NSC, st), "memset sc");
+    CK (cudaMemsetAsync (sd->nn.sc, 0, ncg_pcg_sc_bytes (), st), "memset sc");
     CK (cudaMemsetAsync (sd->nn.csync, 0, ncg_pcg_sync_bytes (n), st), "memset sync");
     /* the chained solves' words: epoch 0 matches no launch */
     CK (cudaMemsetAsync (sd->nn.t32, 0, ncg_pcg_chain_bytes (n), st), "memset chain");
@@ -731,12 +723,12 @@ _nnls (ncg_sd_t *sd, int nr, int n, int mixed, double *rnorm_out)
 
     /* A^T A on the tensor cores (TF32x3; packed K slabs in the factor's
      * buffer, which is free until the first solve), small n on CUDA cores */
-    if (n >= 1024)
+    if (n >= NCG_SYRK_TC_MIN)
       CK (ncg_launch_syrk_upper_tc_f64 (sd->nn.IM, nr, n, sd->nn.M32, sd->nn.R32, sizeof (float) * (size_t) n * n,
                                         sd->nn.info + 1, st), "syrk tc");
     else
       CK (ncg_launch_syrk_upper_f32 (sd->nn.IM, nr, n, sd->nn.M32, st), "syrk f32");
-    CK (ncg_launch_colsumsq (sd->nn.IM, nr, n, sd->nn.diagM, st), "colsumsq");
+    CK (ncg_launch_colsumsq (sd->nn.IM, nr, n, sd->nn.diagM, sd->nn.part, st), "colsumsq");
   }
   else
   {

@@ -149,12 +149,15 @@ ncg_launch_syrk_upper_f32 (const double *A, int nrows, int ncols, float *M, cuda
   return _syrk128<double> (A, ncols, 0, nrows, 0, ncols, M, ncols, s);
 }
 
-/* ---- gemv --------------------------------------------------------------- */
+/* ---- gemv ---------------------------------------------------------------
+ * Bound by the FP64 pipes from n = 2000 or so (n^2 FMAs, 27 us at n = 4096;
+ * HBM would take 20), by latency below; the products of the refinement run on the
+ * columns P of the active set alone. */
 
-/* y[r] = alpha sum_c A[r][c] x[c] + beta y[r]; one warp per row */
-__global__ void
-_gemv_n_kernel (const double *__restrict__ A, int nrows, int ncols, double alpha, const double *__restrict__ x,
-                double beta, double *__restrict__ y)
+/* y[r] = alpha sum_a A[r][P[a]] x[a] + beta y[r] (P NULL: a itself); one warp per row */
+__global__ void __launch_bounds__ (256)
+_gemv_n_kernel (const double *__restrict__ A, int nrows, int lda, const int32_t *__restrict__ P, int np, double alpha,
+                const double *__restrict__ x, double beta, double *__restrict__ y)
 {
   const int lane = threadIdx.x & 31;
   const int r    = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -162,11 +165,12 @@ _gemv_n_kernel (const double *__restrict__ A, int nrows, int ncols, double alpha
   if (r >= nrows)
     return;
 
-  const double *a = A + (size_t) r * ncols;
-  double s        = 0.0;
+  const double *row = A + (size_t) r * lda;
+  double s          = 0.0;
 
-  for (int c = lane; c < ncols; c += 32)
-    s = fma (a[c], x[c], s);
+#pragma unroll 8
+  for (int a = lane; a < np; a += 32)
+    s = fma (row[P ? P[a] : a], x[a], s);
 
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1)
@@ -176,71 +180,106 @@ _gemv_n_kernel (const double *__restrict__ A, int nrows, int ncols, double alpha
     y[r] = (beta == 0.0) ? alpha * s : fma (beta, y[r], alpha * s);
 }
 
-#define GT_ROWS 256
-
-/* part[rb][c] = sum over rows of block rb of A[r][c] x[r] */
-__global__ void
-_gemv_t_partial_kernel (const double *__restrict__ A, int nrows, int ncols, const double *__restrict__ x,
-                        double *__restrict__ part)
+/* rows of a block of the transposed product: at most 64 blocks, so that their
+ * sums are short, and at least 16 rows (256 rows whatever the size left 8 CTAs
+ * waiting for memory one row after another at n = 512: 62 us, 6 us now) */
+static inline int
+_gt_rows (int nrows)
 {
-  const int c  = blockIdx.x * blockDim.x + threadIdx.x;
-  const int rb = blockIdx.y;
+  const int r = (nrows + 63) / 64;
 
-  if (c >= ncols)
-    return;
-
-  const int r0 = rb * GT_ROWS, r1 = min (nrows, r0 + GT_ROWS);
-  double s     = 0.0;
-
-  for (int r = r0; r < r1; r++)
-    s = fma (A[(size_t) r * ncols + c], x[r], s);
-
-  part[(size_t) rb * ncols + c] = s;
+  return r < 16 ? 16 : r;
 }
 
-__global__ void
-_gemv_t_final_kernel (const double *__restrict__ part, int nrb, int ncols, double alpha, double beta,
+/* part[rb][a] = sum over rows of block rb of A[r][P[a]] x[r], or of
+ * A[r][P[a]]^2 (x NULL) */
+__global__ void __launch_bounds__ (128)
+_gemv_t_partial_kernel (const double *__restrict__ A, int nrows, int lda, const int32_t *__restrict__ P, int np,
+                        const double *__restrict__ x, int rows, double *__restrict__ part)
+{
+  const int a  = blockIdx.x * blockDim.x + threadIdx.x;
+  const int rb = blockIdx.y;
+
+  if (a >= np)
+    return;
+
+  const int r0 = rb * rows, r1 = min (nrows, r0 + rows);
+  const double *col = A + (P ? P[a] : a);
+  double s          = 0.0;
+
+#pragma unroll 8
+  for (int r = r0; r < r1; r++)
+  {
+    const double v = col[(size_t) r * lda];
+
+    s = fma (v, x ? x[r] : v, s);
+  }
+
+  part[(size_t) rb * np + a] = s;
+}
+
+/* y[a] = the blocks' sum, or b[a] less it (b not NULL) */
+__global__ void __launch_bounds__ (128)
+_gemv_t_final_kernel (const double *__restrict__ part, int nrb, int np, const double *__restrict__ b,
                       double *__restrict__ y)
 {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  const int a = blockIdx.x * blockDim.x + threadIdx.x;
 
-  if (c >= ncols)
+  if (a >= np)
     return;
 
   double s = 0.0;
 
+#pragma unroll 8
   for (int rb = 0; rb < nrb; rb++)
-    s += part[(size_t) rb * ncols + c];
+    s += part[(size_t) rb * np + a];
 
-  y[c] = (beta == 0.0) ? alpha * s : fma (beta, y[c], alpha * s);
+  y[a] = b ? b[a] - s : s;
 }
 
 extern "C" size_t
 ncg_gemv_t_scratch (int nrows, int ncols)
 {
-  return (size_t) ((nrows + GT_ROWS - 1) / GT_ROWS) * (size_t) ncols * sizeof (double);
+  const int rows = _gt_rows (nrows);
+
+  return (size_t) ((nrows + rows - 1) / rows) * (size_t) ncols * sizeof (double);
 }
 
-extern "C" cudaError_t
-ncg_launch_gemv_ex (const double *A, int nrows, int ncols, int trans, double alpha, const double *x, double beta,
-                    double *y, double *part, cudaStream_t s)
+/* y = (A[:, P])^T x, or b less it */
+static cudaError_t
+_gemv_t (const double *A, int nrows, int lda, const int32_t *P, int np, const double *x, const double *b, double *y,
+         double *part, cudaStream_t s)
 {
-  if (!trans)
-  {
-    const int th = 256;
+  const int rows = _gt_rows (nrows), nrb = (nrows + rows - 1) / rows;
 
-    _gemv_n_kernel<<<(unsigned) (((size_t) nrows * 32 + th - 1) / th), th, 0, s>>> (A, nrows, ncols, alpha, x, beta, y);
-  }
-  else
-  {
-    const int nrb = (nrows + GT_ROWS - 1) / GT_ROWS;
-    dim3 g ((ncols + 127) / 128, nrb);
-
-    _gemv_t_partial_kernel<<<g, 128, 0, s>>> (A, nrows, ncols, x, part);
-    _gemv_t_final_kernel<<<(ncols + 255) / 256, 256, 0, s>>> (part, nrb, ncols, alpha, beta, y);
-  }
+  _gemv_t_partial_kernel<<<dim3 ((np + 127) / 128, nrb), 128, 0, s>>> (A, nrows, lda, P, np, x, rows, part);
+  _gemv_t_final_kernel<<<(np + 127) / 128, 128, 0, s>>> (part, nrb, np, b, y);
 
   return cudaGetLastError ();
+}
+
+static cudaError_t
+_gemv_n (const double *A, int nrows, int lda, const int32_t *P, int np, double alpha, const double *x, double beta,
+         double *y, cudaStream_t s)
+{
+  _gemv_n_kernel<<<(unsigned) (((size_t) nrows * 32 + 255) / 256), 256, 0, s>>> (A, nrows, lda, P, np, alpha, x, beta,
+                                                                                y);
+
+  return cudaGetLastError ();
+}
+
+/* y = A^T x */
+extern "C" cudaError_t
+ncg_launch_gemv_t (const double *A, int nrows, int ncols, const double *x, double *y, double *part, cudaStream_t s)
+{
+  return _gemv_t (A, nrows, ncols, NULL, ncols, x, NULL, y, part, s);
+}
+
+/* diagM[c] = sum_r A[r][c]^2, the FP64 diagonal of A^T A */
+extern "C" cudaError_t
+ncg_launch_colsumsq (const double *A, int nrows, int ncols, double *out, double *part, cudaStream_t s)
+{
+  return _gemv_t (A, nrows, ncols, NULL, ncols, NULL, NULL, out, part, s);
 }
 
 /* ---- active-set gather / scatter ----------------------------------------- */
@@ -338,35 +377,6 @@ ncg_launch_gather_scaled_f32 (const float *M32, int n, const int32_t *P, int np,
   return cudaGetLastError ();
 }
 
-/* diagM[c] = sum_r A[r][c]^2, the FP64 diagonal of A^T A */
-__global__ void
-_colsumsq_kernel (const double *__restrict__ A, int nrows, int ncols, double *__restrict__ out)
-{
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-
-  if (c >= ncols)
-    return;
-
-  double s = 0.0;
-
-  for (int r = 0; r < nrows; r++)
-  {
-    const double v = A[(size_t) r * ncols + c];
-
-    s = fma (v, v, s);
-  }
-
-  out[c] = s;
-}
-
-extern "C" cudaError_t
-ncg_launch_colsumsq (const double *A, int nrows, int ncols, double *out, cudaStream_t s)
-{
-  _colsumsq_kernel<<<(ncols + 127) / 128, 128, 0, s>>> (A, nrows, ncols, out);
-
-  return cudaGetLastError ();
-}
-
 __global__ void
 _scatter_kernel (const double *__restrict__ xsub, const int32_t *__restrict__ P, int np, int n, double *__restrict__ x)
 {
@@ -394,15 +404,6 @@ ncg_launch_scatter_x (const double *xsub, const int32_t *P, int np, int n, doubl
     _scatter2_kernel<<<(np + 255) / 256, 256, 0, s>>> (xsub, P, np, x);
 
   return cudaGetLastError ();
-}
-
-__global__ void
-_gather_vec_kernel (const double *__restrict__ xf, const int32_t *__restrict__ P, int np, double *__restrict__ xs)
-{
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-
-  if (a < np)
-    xs[a] = xf[P[a]];
 }
 
 /* ---- blocked Cholesky ------------------------------------------------------ */
@@ -789,7 +790,7 @@ ncg_launch_residual_norm (const double *A, int nrows, int ncols, const double *x
   if (e != cudaSuccess)
     return e;
 
-  e = ncg_launch_gemv_ex (A, nrows, ncols, 0, -1.0, x, 1.0, res, NULL, s);
+  e = _gemv_n (A, nrows, ncols, NULL, ncols, -1.0, x, 1.0, res, s);
 
   if (e != cudaSuccess)
     return e;
@@ -801,26 +802,38 @@ ncg_launch_residual_norm (const double *A, int nrows, int ncols, const double *x
 
 /* ---- weight normalisation (ncm_stats_dist.c:1086-1093) ------------------- */
 
-__global__ void
+/* one CTA; the total as a tree (one thread's chain of n additions took 243 us at
+ * n = 4096) */
+__global__ void __launch_bounds__ (1024)
 _normalize_weights_kernel (double *w, int n, double shrink, int32_t *bad)
 {
-  __shared__ double sc, ad;
+  __shared__ double red[32];
+  const int tid = threadIdx.x, lane = tid & 31;
+  double t      = 0.0;
 
-  if (threadIdx.x == 0)
-  {
-    double total = 0.0;
+  for (int i = tid; i < n; i += 1024)
+    t += w[i];
 
-    for (int i = 0; i < n; i++)
-      total += w[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    t += __shfl_xor_sync (0xffffffffu, t, o);
 
-    *bad = !(total > 0.0);
-    sc   = (1.0 - shrink) / total;
-    ad   = shrink / n;
-  }
+  if (lane == 0)
+    red[tid >> 5] = t;
 
   __syncthreads ();
+  t = red[lane];
 
-  for (int i = threadIdx.x; i < n; i += blockDim.x)
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    t += __shfl_xor_sync (0xffffffffu, t, o);
+
+  const double sc = (1.0 - shrink) / t, ad = shrink / n;
+
+  if (tid == 0)
+    *bad = !(t > 0.0);
+
+  for (int i = tid; i < n; i += 1024)
     w[i] = __dadd_rn (__dmul_rn (w[i], sc), ad);
 }
 
@@ -844,57 +857,113 @@ ncg_launch_normalize_weights (double *w, int n, double shrink, int32_t *bad, cud
  * sc[PCG_RR] to decide when to stop.
  */
 
-#define PCG_THREADS 1024
+#define DOT_TH 256
+#define DOT_CTAS 64
 
-/* sc[out0] = <u0, v0> (and sc[out1] = <u1, v1> when u1 != NULL); one CTA,
- * fixed reduction order */
-__global__ void __launch_bounds__ (PCG_THREADS)
-_dot2_kernel (const double *__restrict__ u0, const double *__restrict__ v0, const double *__restrict__ u1,
-              const double *__restrict__ v1, const double *__restrict__ w, int n, double *sc, int out0, int out1)
+/* The scalars of one point of the iteration, as many dot products as it needs
+ * in one launch: the CTAs leave partial sums and the last one to finish (a
+ * counter, cleared again) adds them up in CTA order.  (One CTA of 1024 threads
+ * per product took 8 to 10 us each.)
+ *  MODE 0 (start): RZ = <r, z>, BB = |D b|^2, RR = |D r|^2, and p = z
+ *  MODE 1: PQ = <p, q>
+ *  MODE 2: RZ' = <r, z>, <z, r_prev>, RR = |D r|^2; BE = (RZ' - <z, r_prev>) / RZ
+ *          (Polak-Ribiere), then RZ = RZ' */
+template <int MODE>
+__global__ void __launch_bounds__ (DOT_TH)
+_pcg_dots_kernel (const double *__restrict__ u, const double *__restrict__ v, const double *__restrict__ w,
+                  const double *__restrict__ D, double *__restrict__ p, int n, double *__restrict__ sc,
+                  double *__restrict__ part, int32_t *__restrict__ count)
 {
-  __shared__ double r0[PCG_THREADS / 32], r1[PCG_THREADS / 32];
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  double s0 = 0.0, s1 = 0.0;
+  __shared__ double red[3][DOT_TH / 32];
+  __shared__ int last;
+  const int tid = threadIdx.x, lane = tid & 31;
+  double s[3]   = { 0.0, 0.0, 0.0 };
 
-  for (int i = tid; i < n; i += PCG_THREADS)
+  for (int i = blockIdx.x * DOT_TH + tid; i < n; i += gridDim.x * DOT_TH)
   {
-    const double wi = (w != NULL) ? w[i] * w[i] : 1.0;
+    const double ui = u[i], vi = v[i];
 
-    s0 = fma (u0[i] * wi, v0[i], s0);
+    s[0] = fma (ui, vi, s[0]);
 
-    if (u1 != NULL)
-      s1 = fma (u1[i], v1[i], s1);
+    if (MODE != 1)
+    {
+      const double wi = w[i], di = D[i] * ui, b = (MODE == 0) ? D[i] * wi : vi;
+
+      s[1] = fma (b, (MODE == 0) ? b : wi, s[1]);
+      s[2] = fma (di, di, s[2]);
+    }
+
+    if (MODE == 0)
+      p[i] = vi;
   }
 
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
+  for (int k = 0; k < (MODE == 1 ? 1 : 3); k++)
   {
-    s0 += __shfl_xor_sync (0xffffffffu, s0, o);
-    s1 += __shfl_xor_sync (0xffffffffu, s1, o);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      s[k] += __shfl_xor_sync (0xffffffffu, s[k], o);
+
+    if (lane == 0)
+      red[k][tid >> 5] = s[k];
   }
 
-  if (lane == 0)
+  __syncthreads ();
+
+  if (tid < 3)
   {
-    r0[wid] = s0;
-    r1[wid] = s1;
+    double t = red[tid][0];
+
+    for (int k = 1; k < DOT_TH / 32; k++)
+      t += red[tid][k];
+
+    part[tid * DOT_CTAS + blockIdx.x] = t;
+    __threadfence ();
   }
 
   __syncthreads ();
 
   if (tid == 0)
+    last = atomicAdd (count, 1) == (int) gridDim.x - 1;
+
+  __syncthreads ();
+
+  if (!last || tid >= 32)
+    return;
+
+  __threadfence ();
+
+  if (tid < 3)
   {
-    double t0 = 0.0, t1 = 0.0;
+    double t = 0.0;
 
-    for (int k = 0; k < PCG_THREADS / 32; k++)
+    for (int k = 0; k < (int) gridDim.x; k++)
+      t += __ldcg (part + tid * DOT_CTAS + k);
+
+    s[0] = t;
+  }
+
+  const double t0 = __shfl_sync (0xffffffffu, s[0], 0), t1 = __shfl_sync (0xffffffffu, s[0], 1),
+               t2 = __shfl_sync (0xffffffffu, s[0], 2);
+
+  if (tid == 0)
+  {
+    *count = 0;
+
+    if (MODE == 0)
     {
-      t0 += r0[k];
-      t1 += r1[k];
+      sc[NCG_PCG_RZ] = t0;
+      sc[NCG_PCG_BB] = t1;
+      sc[NCG_PCG_RR] = t2;
     }
-
-    sc[out0] = t0;
-
-    if (u1 != NULL)
-      sc[out1] = t1;
+    else if (MODE == 1)
+      sc[NCG_PCG_PQ] = t0;
+    else
+    {
+      sc[NCG_PCG_BE] = (t0 - t1) / sc[NCG_PCG_RZ];
+      sc[NCG_PCG_RZ] = t0;
+      sc[NCG_PCG_RR] = t2;
+    }
   }
 }
 
@@ -916,60 +985,27 @@ _pcg_step_kernel (double *__restrict__ x, double *__restrict__ r, double *__rest
   r[i]     = fma (-al, q[i], ri);
 }
 
-/* p = z + beta p with beta = (sc[RZN] - sc[ZRP]) / sc[RZ]; the following
- * _pcg_shift_kernel launch then sets sc[RZ] = sc[RZN] */
+/* p = z + BE p */
 __global__ void
 _pcg_dir_kernel (double *__restrict__ p, const double *__restrict__ z, int n, const double *sc)
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
 
-  if (i >= n)
-    return;
-
-  const double be = (sc[NCG_PCG_RZN] - sc[NCG_PCG_ZRP]) / sc[NCG_PCG_RZ];
-
-  p[i] = fma (be, p[i], z[i]);
-}
-
-__global__ void
-_pcg_shift_kernel (double *sc)
-{
-  sc[NCG_PCG_RZ] = sc[NCG_PCG_RZN];
-}
-
-/* r = b - r (turns r = A_P^T A_P x into the residual) */
-__global__ void
-_rsub_kernel (const double *__restrict__ b, double *__restrict__ r, int n)
-{
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-
   if (i < n)
-    r[i] = b[i] - r[i];
+    p[i] = fma (sc[NCG_PCG_BE], p[i], z[i]);
 }
 
 #define VB(n) (((n) + 255) / 256), 256
 
-/* q = A_P^T (A_P v) for a compact v on the set P (np entries), A nrows x n;
- * vf and qf are n-long work vectors, yf nrows-long, part the transposed-gemv
- * scratch */
+/* q = A_P^T (A_P v) for a compact v on the set P (np entries), or b less it; A
+ * nrows x n; yf: nrows-long work, part the transposed product's scratch */
 extern "C" cudaError_t
-ncg_launch_pcg_matvec (const double *A, int nrows, int n, const int32_t *P, int np, const double *v, double *vf,
-                       double *yf, double *qf, double *part, double *q, cudaStream_t s)
+ncg_launch_pcg_matvec (const double *A, int nrows, int n, const int32_t *P, int np, const double *v, const double *b,
+                       double *yf, double *part, double *q, cudaStream_t s)
 {
-  cudaError_t e = ncg_launch_scatter_x (v, P, np, n, vf, s);
+  const cudaError_t e = _gemv_n (A, nrows, n, P, np, 1.0, v, 0.0, yf, s);
 
-  if (e == cudaSuccess)
-    e = ncg_launch_gemv_ex (A, nrows, n, 0, 1.0, vf, 0.0, yf, NULL, s);
-
-  if (e == cudaSuccess)
-    e = ncg_launch_gemv_ex (A, nrows, n, 1, 1.0, yf, 0.0, qf, part, s);
-
-  if (e != cudaSuccess)
-    return e;
-
-  _gather_vec_kernel<<<VB (np), 0, s>>> (qf, P, np, q);
-
-  return cudaGetLastError ();
+  return (e == cudaSuccess) ? _gemv_t (A, nrows, n, P, np, yf, b, q, part, s) : e;
 }
 
 /* ---- chained triangular solves of the FP32 preconditioner ----------------
@@ -1063,39 +1099,54 @@ _cs_finish (int32_t *sync, int tid)
 
 /* V_i = (U_ii^T)^{-1}, lower triangular, for each 64 x 64 diagonal block of the
  * upper factor U (zero outside the nb x nb triangle of a partial last block);
- * thread c computes column c by forward substitution */
+ * thread c solves for column c in registers, as the panel solve does (36 us
+ * with the column in shared memory and a division per row) */
 __global__ void __launch_bounds__ (SB)
 _trinv_diag_kernel (const float *__restrict__ U, int n, float *__restrict__ V)
 {
-  __shared__ float S[SB][SB + 1];
-  __shared__ float X[SB][SB + 1];
+  __shared__ __align__ (16) float S[SB][SB];
+  __shared__ float ri[SB];
   const int i = blockIdx.x, kb = i * SB, nb = (n - kb < SB) ? n - kb : SB, c = threadIdx.x;
+  float x[SB];
 
-  _stage_block<float, SB, SB> (S, U, n, kb, kb, nb, c);
+#pragma unroll 16
+  for (int r = 0; r < SB; r++)
+    S[r][c] = (r < nb && c < nb && c >= r) ? U[(size_t) (kb + r) * n + kb + c] : 0.0f;
+
+  ri[c] = (c < nb) ? __frcp_rn (S[c][c]) : 0.0f;
+
+#pragma unroll
+  for (int r = 0; r < SB; r++)
+    x[r] = (r == c) ? 1.0f : 0.0f;
 
   __syncthreads ();
 
+#pragma unroll
   for (int r = 0; r < SB; r++)
   {
-    float v = 0.0f;
+    x[r] *= ri[r];
 
-    if (c < nb && r < nb && r >= c)
+    const float t = -x[r];
+
+#pragma unroll
+    for (int m = (r + 1) / 4 * 4; m < SB; m += 4)
     {
-      float acc = (r == c) ? 1.0f : 0.0f;
+      const float4 v = *(const float4 *) &S[r][m];
 
-      for (int k = c; k < r; k++)
-        acc = fmaf (-S[k][r], X[k][c], acc);
-
-      v = acc / S[r][r];
+      if (m + 0 > r)
+        x[m + 0] = fmaf (v.x, t, x[m + 0]);
+      if (m + 1 > r)
+        x[m + 1] = fmaf (v.y, t, x[m + 1]);
+      if (m + 2 > r)
+        x[m + 2] = fmaf (v.z, t, x[m + 2]);
+      if (m + 3 > r)
+        x[m + 3] = fmaf (v.w, t, x[m + 3]);
     }
-
-    X[r][c] = v;
   }
 
-  __syncthreads ();
-
-  for (int e = c; e < SB * SB; e += SB)
-    V[(size_t) i * SB * SB + e] = X[e / SB][e % SB];
+#pragma unroll
+  for (int r = 0; r < SB; r++)
+    V[(size_t) i * SB * SB + r * SB + c] = x[r];
 }
 
 /* U^T y = (float) (D r): block i, y_i = V_i ((D r)_i - sum_{j<i} U_ji^T y_j);
@@ -1336,11 +1387,28 @@ ncg_launch_pcg_precond (const float *R, const float *V, const double *D, int np,
   return cudaGetLastError ();
 }
 
-extern "C" cudaError_t
-ncg_launch_pcg_dot (const double *u0, const double *v0, const double *u1, const double *v1, const double *w, int n,
-                    double *sc, int out0, int out1, cudaStream_t s)
+extern "C" size_t
+ncg_pcg_sc_bytes (void)
 {
-  _dot2_kernel<<<1, PCG_THREADS, 0, s>>> (u0, v0, u1, v1, w, n, sc, out0, out1);
+  return sizeof (double) * (NCG_PCG_NSC + 3 * DOT_CTAS + 1);
+}
+
+/* the scalars sc of the start (mode 0: u = r, v = z, w = b, p = z), <p, q> (mode 1:
+ * u = p, v = q) or the next direction (mode 2: u = r, v = z, w = r_prev) */
+extern "C" cudaError_t
+ncg_launch_pcg_dots (int mode, const double *u, const double *v, const double *w, const double *D, double *p, int n,
+                     double *sc, cudaStream_t s)
+{
+  double *part   = sc + NCG_PCG_NSC;
+  int32_t *count = (int32_t *) (part + 3 * DOT_CTAS);
+  const int g    = (n + DOT_TH - 1) / DOT_TH < DOT_CTAS ? (n + DOT_TH - 1) / DOT_TH : DOT_CTAS;
+
+  if (mode == 0)
+    _pcg_dots_kernel<0><<<g, DOT_TH, 0, s>>> (u, v, w, D, p, n, sc, part, count);
+  else if (mode == 1)
+    _pcg_dots_kernel<1><<<g, DOT_TH, 0, s>>> (u, v, w, D, p, n, sc, part, count);
+  else
+    _pcg_dots_kernel<2><<<g, DOT_TH, 0, s>>> (u, v, w, D, p, n, sc, part, count);
 
   return cudaGetLastError ();
 }
@@ -1358,15 +1426,6 @@ extern "C" cudaError_t
 ncg_launch_pcg_dir (double *p, const double *z, int n, double *sc, cudaStream_t s)
 {
   _pcg_dir_kernel<<<VB (n), 0, s>>> (p, z, n, sc);
-  _pcg_shift_kernel<<<1, 1, 0, s>>> (sc);
-
-  return cudaGetLastError ();
-}
-
-extern "C" cudaError_t
-ncg_launch_rsub (const double *b, double *r, int n, cudaStream_t s)
-{
-  _rsub_kernel<<<VB (n), 0, s>>> (b, r, n);
 
   return cudaGetLastError ();
 }

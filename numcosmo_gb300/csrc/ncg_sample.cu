@@ -3,8 +3,8 @@
  *
  *  wcum            the reference's lazily built cumulative weights: a
  *                  sequential FP64 prefix sum then a multiplication by the
- *                  reciprocal of the total (numcosmo/ncm/stats/ncm_stats_dist.c:1565-1590).
- *                  One thread, same operation order, so the table is
+ *                  reciprocal of the total (numcosmo/ncm/stats/ncm_stats_dist.c:1565-1590),
+ *                  in the same operation order, so the table is
  *                  bit-identical and the chosen indices are exact.
  *  kernel_choose   binary search of p on wcum (ncm_stats_dist.c:1592-1606).
  *  sample          x = theta_i + s U_i^T (h z), s = 1 (Gauss) or
@@ -17,32 +17,68 @@
 
 #include "ncg_internal.h"
 
-__global__ void
+/* One CTA: lane 0 of warp 0 adds, 64 cycles a weight and the bound, the others
+ * bring the next weights to shared memory, write the last sums out and at the
+ * end take all the products (a thread alone that waited for every weight
+ * and multiplied them one by one took 68 us at n = 512). */
+#define WC_TH 256
+#define WC_CH 256
+
+__global__ void __launch_bounds__ (WC_TH)
 _wcum_kernel (const double *__restrict__ w, int n, double *__restrict__ wcum)
 {
-  if (blockIdx.x != 0 || threadIdx.x != 0)
-    return;
+  __shared__ double in[2][WC_CH], out[2][WC_CH];
+  __shared__ double total;
+  const int tid = threadIdx.x, nch = (n + WC_CH - 1) / WC_CH;
+  double cum    = 0.0;
 
-  double cum = 0.0;
-
-  wcum[0] = cum;
-
-  for (int i = 0; i < n; i++)
+  /* step ch: chunk ch + 1 in, chunk ch added up, chunk ch - 1 out */
+  for (int ch = -1; ch <= nch; ch++)
   {
-    cum         = __dadd_rn (cum, w[i]);
-    wcum[i + 1] = cum;
+    if (tid == 0 && ch >= 0 && ch < nch)
+    {
+      const int m = min (WC_CH, n - ch * WC_CH);
+
+#pragma unroll 8
+      for (int i = 0; i < m; i++)
+      {
+        cum             = __dadd_rn (cum, in[ch & 1][i]);
+        out[ch & 1][i]  = cum;
+      }
+    }
+    else if (tid >= 32)
+    {
+      for (int i = tid - 32; i < WC_CH; i += WC_TH - 32)
+      {
+        if ((ch + 1) * WC_CH + i < n && ch + 1 < nch)
+          in[(ch + 1) & 1][i] = w[(ch + 1) * WC_CH + i];
+
+        if (ch >= 1 && (ch - 1) * WC_CH + i < n)
+          wcum[(ch - 1) * WC_CH + i + 1] = out[(ch - 1) & 1][i];
+      }
+    }
+
+    __syncthreads ();
   }
 
-  const double s = __ddiv_rn (1.0, cum);
+  if (tid == 0)
+  {
+    total   = cum;
+    wcum[0] = 0.0;
+  }
 
-  for (int i = 0; i <= n; i++)
+  __syncthreads ();
+
+  const double s = __ddiv_rn (1.0, total);
+
+  for (int i = tid; i <= n; i += WC_TH)
     wcum[i] = __dmul_rn (wcum[i], s);
 }
 
 extern "C" cudaError_t
 ncg_launch_wcum (const double *w, int n, double *wcum, cudaStream_t s)
 {
-  _wcum_kernel<<<1, 32, 0, s>>> (w, n, wcum);
+  _wcum_kernel<<<1, WC_TH, 0, s>>> (w, n, wcum);
 
   return cudaGetLastError ();
 }
