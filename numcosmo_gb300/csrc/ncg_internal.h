@@ -253,12 +253,15 @@ enum { NCG_PCG_RZ = 0, NCG_PCG_PQ, NCG_PCG_BE, NCG_PCG_RR, NCG_PCG_BB, NCG_PCG_E
 cudaError_t ncg_launch_syrk_upper_f32 (const double *A, int nrows, int ncols, float *M, cudaStream_t s);
 cudaError_t ncg_launch_colsumsq (const double *A, int nrows, int ncols, double *out, double *part, cudaStream_t s);
 cudaError_t ncg_launch_gather_scaled_f32 (const float *M32, int n, const int32_t *P, int np, const double *diagM,
-                                          double shift, float *Msub, double *Dsub, const double *b, double *bsub,
-                                          cudaStream_t s);
-cudaError_t ncg_launch_potrf_f32 (float *A, int n, int32_t *info, float *pk, cudaStream_t s);
+                                          double shift, float *Msub, float *dg, double *Dsub, const double *b,
+                                          double *bsub, cudaStream_t s);
+/* work of ncg_potrf_f32_work_bytes (cap), cap >= n; its diagonal block (ncg_potrf_f32_dg) holds the leading one of A */
+size_t      ncg_potrf_f32_work_bytes (int n);
+float      *ncg_potrf_f32_dg (float *work, int cap);
+cudaError_t ncg_launch_potrf_f32 (float *A, int n, int32_t *info, float *work, int cap, cudaStream_t s);
 /* tensor-core (TF32x3) symmetric rank-K updates, ncg_syrk_tc.cu */
 size_t      ncg_syrk_tc_pack_bytes (int nn, int K);
-cudaError_t ncg_launch_syrk_tc (const void *pk, int K, int nn, float *C, int ldc, int mode, int *err,
+cudaError_t ncg_launch_syrk_tc (const void *pk, int K, int nn, float *C, int ldc, int mode, float *dg, int *err,
                                 cudaStream_t s);
 cudaError_t ncg_launch_syrk_upper_tc_f64 (const double *A, int nrows, int ncols, float *C, void *scratch,
                                           size_t cap, int *err, cudaStream_t s);

@@ -334,9 +334,9 @@ _solve_mixed (nnls_t *s, int np, double *dx)
     if (a > 0)
       sd->istats.n_shifted++;
 
-    CK (ncg_launch_gather_scaled_f32 (nn->M32, n, nn->P, np, nn->diagM, shifts[a], nn->R32, nn->D, nn->b, nn->bsub,
-                                      st), "gather scaled");
-    CK (ncg_launch_potrf_f32 (nn->R32, np, nn->info, nn->pk32, st), "potrf f32");
+    CK (ncg_launch_gather_scaled_f32 (nn->M32, n, nn->P, np, nn->diagM, shifts[a], nn->R32,
+                                      ncg_potrf_f32_dg (nn->pk32, n), nn->D, nn->b, nn->bsub, st), "gather scaled");
+    CK (ncg_launch_potrf_f32 (nn->R32, np, nn->info, nn->pk32, n, st), "potrf f32");
     CK (ncg_launch_trinv_diag_f32 (nn->R32, np, nn->Vi, st), "diagonal inverses");
     CK (cudaMemcpyAsync (info, nn->info, sizeof (info), cudaMemcpyDeviceToHost, st), "D2H info");
     CK (cudaStreamSynchronize (st), "sync");
@@ -652,7 +652,7 @@ _nnls_reserve (ncg_sd_t *sd, int nr, int n, int mixed)
     NRES (sc, csc, ncg_pcg_sc_bytes ());
     NRES (Vi, cVi, ncg_pcg_trinv_bytes (n));
     NRES (csync, ccsync, ncg_pcg_sync_bytes (n));
-    NRES (pk32, cpk32, ncg_syrk_tc_pack_bytes (n, 64));
+    NRES (pk32, cpk32, ncg_potrf_f32_work_bytes (n));
   }
   else
   {

@@ -320,7 +320,8 @@ ncg_launch_gather_sub (const double *M, int n, const int32_t *P, int np, double 
 /* The mixed solver's preconditioner operand, in two launches: Dsub[a] =
  * 1/sqrt(diagM[P_a]) (Jacobi scaling, FP64) and bsub[a] = b[P_a]; then
  * Msub[a][b] = D_a M32[P_a][P_b] D_b in FP32, upper triangle only, with the
- * unit diagonal raised by `shift`. */
+ * unit diagonal raised by `shift`; its leading 64 x 64 block in dg as well, where
+ * the factorisation reads it. */
 __global__ void
 _scale_vec_kernel (const int32_t *__restrict__ P, int np, const double *__restrict__ diagM,
                    double *__restrict__ Dsub, const double *__restrict__ b, double *__restrict__ bsub)
@@ -338,7 +339,8 @@ _scale_vec_kernel (const int32_t *__restrict__ P, int np, const double *__restri
 
 __global__ void
 _gather_scaled_kernel (const float *__restrict__ M32, int n, const int32_t *__restrict__ P, int np,
-                       const double *__restrict__ Dsub, float shift, float *__restrict__ Msub)
+                       const double *__restrict__ Dsub, float shift, float *__restrict__ Msub,
+                       float *__restrict__ dg)
 {
   const int a = blockIdx.y;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -359,12 +361,15 @@ _gather_scaled_kernel (const float *__restrict__ M32, int n, const int32_t *__re
       v = (Da * row[P[bb]]) * Da * (1.0f + shift);
 
     Msub[(size_t) a * np + bb] = v;
+
+    if (a < 64 && bb < 64)
+      dg[a * 64 + bb] = v;
   }
 }
 
 extern "C" cudaError_t
 ncg_launch_gather_scaled_f32 (const float *M32, int n, const int32_t *P, int np, const double *diagM, double shift,
-                              float *Msub, double *Dsub, const double *b, double *bsub, cudaStream_t s)
+                              float *Msub, float *dg, double *Dsub, const double *b, double *bsub, cudaStream_t s)
 {
   if (np <= 0)
     return cudaSuccess;
@@ -372,7 +377,7 @@ ncg_launch_gather_scaled_f32 (const float *M32, int n, const int32_t *P, int np,
   dim3 g ((np + 255) / 256 < 8 ? (np + 255) / 256 : 8, np);
 
   _scale_vec_kernel<<<(np + 255) / 256, 256, 0, s>>> (P, np, diagM, Dsub, b, bsub);
-  _gather_scaled_kernel<<<g, 256, 0, s>>> (M32, n, P, np, Dsub, (float) shift, Msub);
+  _gather_scaled_kernel<<<g, 256, 0, s>>> (M32, n, P, np, Dsub, (float) shift, Msub, dg);
 
   return cudaGetLastError ();
 }
@@ -447,13 +452,17 @@ _stage_block (T (*S)[B + 1], const T *__restrict__ A, int ld, int r0, int c0, in
 
 /* ---- the FP32 preconditioner's panels ---- */
 
-/* The nb x nb diagonal block (upper, in place).  The block lives in registers,
- * 4 x 4 elements per thread (element (ty + 16p, tx + 16q)); a step publishes
- * its raw row j through shared memory, one barrier, and every thread takes
- * s_jr s_jc / a_jj off its elements; the square roots and the rows' own
- * scaling wait for the end, where all rows take them at once.  It is bound by
- * the chain of steps: a barrier, two shared-memory trips and a reciprocal
- * each (24 us with the row scaled and the block updated in shared memory). */
+/* One panel: the diagonal block (raw in dg, 64 x 64) and 64 of the columns to
+ * its right per CTA, eliminated in the same steps.  Both live in registers,
+ * 4 x 4 elements each per thread (element (ty + 16p, tx + 16q)); a step
+ * publishes its raw row j of both through shared memory, one barrier, and every
+ * thread takes s_jr s_jc / a_jj off its elements; the square roots and the
+ * rows' scaling wait for the end, where all rows take them at once.  CTA 0 writes
+ * the factored block.  It is bound by the chain of 64 steps (a barrier, two
+ * shared-memory trips and a reciprocal each), which every CTA walks for itself:
+ * as two launches, the factor and then the columns against it, a panel took
+ * 10 + 11 us (24 + 27 with the row scaled on the chain and a pack through FP64);
+ * 12 us so.  pk (may be NULL): the panel as the tensor-core update's operand. */
 __device__ __forceinline__ float
 _rcp_approx (float x)
 {
@@ -465,14 +474,18 @@ _rcp_approx (float x)
 }
 
 __global__ void __launch_bounds__ (256)
-_potrf_diag_f32_kernel (float *A, int ld, int kb, int nb, int32_t *info)
+_potrf_panel_f32_kernel (float *A, int ld, int kb, int nb, int n, const float *__restrict__ dg, int32_t *info,
+                         float *pk)
 {
-  __shared__ float row[2][PB];
+  __shared__ float row[2][2 * PB];
+  __shared__ float X[PB][PB + 1];
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  float s[4][4], piv[4];
+  const int c0  = kb + nb + blockIdx.x * PB;
+  float s[4][4], a[4][4], piv[4];
   int fail = 0;
 
-  if (*info)
+  /* agreed on by the CTA: CTA 0 may be writing it */
+  if (__syncthreads_or (*(volatile int32_t *) info))
     return;
 
   /* the identity past nb */
@@ -483,7 +496,8 @@ _potrf_diag_f32_kernel (float *A, int ld, int kb, int nb, int32_t *info)
     {
       const int r = ty + 16 * p, c = tx + 16 * q;
 
-      s[p][q] = (r < nb && c < nb) ? ((c >= r) ? A[(size_t) (kb + r) * ld + kb + c] : 0.0f) : (r == c ? 1.0f : 0.0f);
+      s[p][q] = (r < nb && c < nb) ? ((c >= r) ? dg[r * PB + c] : 0.0f) : (r == c ? 1.0f : 0.0f);
+      a[p][q] = (r < nb && c0 + c < n) ? A[(size_t) (kb + r) * ld + c0 + c] : 0.0f;
       piv[p]  = 1.0f;
     }
 
@@ -500,8 +514,13 @@ _potrf_diag_f32_kernel (float *A, int ld, int kb, int nb, int32_t *info)
       if (ty == jj)
       {
 #pragma unroll
-        for (int q = p; q < 4; q++)
-          rb[tx + 16 * q] = s[p][q];
+        for (int q = 0; q < 4; q++)
+        {
+          if (q >= p)
+            rb[tx + 16 * q] = s[p][q];
+
+          rb[PB + tx + 16 * q] = a[p][q];
+        }
       }
 
       __syncthreads ();
@@ -515,14 +534,17 @@ _potrf_diag_f32_kernel (float *A, int ld, int kb, int nb, int32_t *info)
       }
 
       const float inv = -_rcp_approx (ajj);
-      float rc[4];
+      float rc[4], ac[4];
 
       if (ty == jj)
         piv[p] = ajj;
 
 #pragma unroll
-      for (int q = p; q < 4; q++)
-        rc[q] = rb[tx + 16 * q];
+      for (int q = 0; q < 4; q++)
+      {
+        rc[q] = (q >= p) ? rb[tx + 16 * q] : 0.0f;
+        ac[q] = rb[PB + tx + 16 * q];
+      }
 
 #pragma unroll
       for (int pp = p; pp < 4; pp++)
@@ -533,12 +555,17 @@ _potrf_diag_f32_kernel (float *A, int ld, int kb, int nb, int32_t *info)
 #pragma unroll
         for (int q = pp; q < 4; q++)
           s[pp][q] = fmaf (t, rc[q], s[pp][q]);
+
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+          a[pp][q] = fmaf (t, ac[q], a[pp][q]);
       }
     }
 
   if (fail)
   {
-    if (tid == 0)
+    /* every CTA finds the same step */
+    if (tid == 0 && blockIdx.x == 0)
       atomicCAS (info, 0, kb + fail);
 
     return;
@@ -547,96 +574,53 @@ _potrf_diag_f32_kernel (float *A, int ld, int kb, int nb, int32_t *info)
 #pragma unroll
   for (int p = 0; p < 4; p++)
   {
-    const int r    = ty + 16 * p;
-    const float u  = __fsqrt_rn (piv[p]), ri = __frcp_rn (u);
+    const int r   = ty + 16 * p;
+    const float u = __fsqrt_rn (piv[p]), ri = __frcp_rn (u);
 
 #pragma unroll
-    for (int q = p; q < 4; q++)
+    for (int q = 0; q < 4; q++)
     {
       const int c = tx + 16 * q;
 
-      if (r < nb && c < nb && c >= r)
+      a[p][q] *= ri;
+      X[r][c]  = a[p][q];
+
+      if (r < nb && c0 + c < n)
+        A[(size_t) (kb + r) * ld + c0 + c] = a[p][q];
+
+      if (blockIdx.x == 0 && r < nb && c < nb && c >= r)
         A[(size_t) (kb + r) * ld + kb + c] = (c == r) ? u : s[p][q] * ri;
     }
   }
-}
 
-/* X = U_kk^{-T} A_panel, one column per thread in registers, few columns per
- * CTA so that the panel covers many SMs; the block's rows are read from shared
- * memory four at a time (every lane the same), the reciprocals of the diagonal
- * come once from staging.  27 us -> 11 us at n = 3000, most of it the pack,
- * whose hi / lo split went through FP64.  pk (may be NULL): the panel as the tensor-core
- * trailing update's operand. */
-#define TRSM32_TH 64
-
-__global__ void __launch_bounds__ (TRSM32_TH)
-_potrf_trsm_f32_kernel (float *A, int ld, int kb, int nb, int n, const int32_t *info, float *pk)
-{
-  __shared__ __align__ (16) float S[PB][PB];
-  __shared__ float ri[PB];
-  const int tid = threadIdx.x;
-  const int col = kb + nb + blockIdx.x * TRSM32_TH + tid;
-  const bool in = col < n;
-  float a[PB];
-
-  if (*info)
+  if (pk == NULL)
     return;
 
-#pragma unroll
-  for (int r = 0; r < PB; r++)
-    a[r] = (in && r < nb) ? A[(size_t) (kb + r) * ld + col] : 0.0f;
-
-#pragma unroll 16
-  for (int r = 0; r < PB; r++)
-    S[r][tid] = (r < nb && tid < nb && tid >= r) ? A[(size_t) (kb + r) * ld + kb + tid] : 0.0f;
-
-  ri[tid] = (tid < nb) ? __frcp_rn (S[tid][tid]) : 1.0f;
   __syncthreads ();
 
-  if (!in)
-    return;
+  /* units of four rows of a column */
+  float *blk = pk + (size_t) (blockIdx.x / 2) * 2 * (SK_BLOCK / 4);
 
-#pragma unroll
-  for (int r = 0; r < PB; r++)
+  for (int e = tid; e < PB * 16; e += 256)
   {
-    a[r] *= ri[r];
+    const int c = e & 63, k = (e >> 6) * 4;
 
-    const float t = -a[r];
-
-#pragma unroll
-    for (int m = (r + 1) / 4 * 4; m < PB; m += 4)
-    {
-      const float4 v = *(const float4 *) &S[r][m];
-
-      if (m + 0 > r)
-        a[m + 0] = fmaf (v.x, t, a[m + 0]);
-      if (m + 1 > r)
-        a[m + 1] = fmaf (v.y, t, a[m + 1]);
-      if (m + 2 > r)
-        a[m + 2] = fmaf (v.z, t, a[m + 2]);
-      if (m + 3 > r)
-        a[m + 3] = fmaf (v.w, t, a[m + 3]);
-    }
+    _put_split4f (blk + (size_t) (k / SK_KC) * (SK_BLOCK / 4), (blockIdx.x & 1) * PB + c, k % SK_KC, X[k][c], X[k + 1][c],
+                  X[k + 2][c], X[k + 3][c]);
   }
-
-#pragma unroll
-  for (int r = 0; r < PB; r++)
-    if (r < nb)
-      A[(size_t) (kb + r) * ld + col] = a[r];
-
-  if (pk != NULL)
-    _sk_pack_column (pk, col - kb - nb, a, nb);
 }
 
 /* C -= P^T P on the upper tiles of the nn x nn trailing block for a panel of
  * nb <= 64 rows: 64 x 64 tiles, the whole panel slice of both sides staged at
  * once, 4 x 4 outputs per thread, C loaded while the panel arrives.  One FMA
- * chain per output over the rows in ascending order.  11 us on average below
+ * chain per output over the rows in ascending order.  The leading tile also
+ * goes to dg, the next panel's raw diagonal block.  11 us on average below
  * 2560 columns, where the general tile kernel (16 rows a stage) took 18 and the
  * tensor-core update 13: there its set-up and the traffic of C decide, not the
  * products. */
 __global__ void __launch_bounds__ (256)
-_potrf_update_f32_kernel (float *A, int ld, int kb, int nb, int off, int nn, const int32_t *info)
+_potrf_update_f32_kernel (float *A, int ld, int kb, int nb, int off, int nn, float *__restrict__ dg,
+                          const int32_t *info)
 {
   __shared__ __align__ (16) float As[PB][PB];
   __shared__ __align__ (16) float Bs[PB][PB];
@@ -707,6 +691,9 @@ _potrf_update_f32_kernel (float *A, int ld, int kb, int nb, int off, int nn, con
 
       if (i < end && j < end && j >= i)
         A[(size_t) i * ld + j] = acc[p][q];
+
+      if (blockIdx.x == 0)
+        dg[(ty * 4 + p) * PB + tx * 4 + q] = acc[p][q];
     }
 }
 
@@ -719,36 +706,49 @@ _zero_int_kernel (int32_t *p)
 /* trailing blocks at least this wide take the tensor-core update */
 #define POTRF_TC_MIN 2560
 
-extern "C" cudaError_t
-ncg_launch_potrf_f32 (float *A, int n, int32_t *info, float *pk, cudaStream_t s)
+/* work of potrf_f32 on n columns: the panel's tensor-core operand, then the raw
+ * diagonal block */
+extern "C" size_t
+ncg_potrf_f32_work_bytes (int n)
 {
+  return ncg_syrk_tc_pack_bytes (n, PB) + sizeof (float) * PB * PB;
+}
+
+extern "C" float *
+ncg_potrf_f32_dg (float *work, int n)
+{
+  return work + ncg_syrk_tc_pack_bytes (n, PB) / sizeof (float);
+}
+
+/* upper Cholesky of A (n x n, in place); work's diagonal block holds the leading
+ * 64 x 64 of A already (ncg_launch_gather_scaled_f32 leaves it there) */
+extern "C" cudaError_t
+ncg_launch_potrf_f32 (float *A, int n, int32_t *info, float *work, int cap, cudaStream_t s)
+{
+  float *dg = ncg_potrf_f32_dg (work, cap);
+
   _zero_int_kernel<<<1, 1, 0, s>>> (info);
 
   for (int kb = 0; kb < n; kb += PB)
   {
     const int nb  = (n - kb < PB) ? n - kb : PB, rest = n - kb - nb;
-    const bool tc = pk != NULL && rest >= POTRF_TC_MIN;
+    const bool tc = rest >= POTRF_TC_MIN;
 
-    _potrf_diag_f32_kernel<<<1, 256, 0, s>>> (A, n, kb, nb, info);
+    _potrf_panel_f32_kernel<<<rest > 0 ? (rest + PB - 1) / PB : 1, 256, 0, s>>> (A, n, kb, nb, n, dg, info,
+                                                                                tc ? work : NULL);
 
-    if (rest > 0)
+    if (tc)
     {
-      _potrf_trsm_f32_kernel<<<(rest + TRSM32_TH - 1) / TRSM32_TH, TRSM32_TH, 0, s>>> (A, n, kb, nb, n, info,
-                                                                                       tc ? pk : NULL);
+      const cudaError_t e = ncg_launch_syrk_tc (work, nb, rest, A + (size_t) (kb + nb) * n + kb + nb, n, 1, dg, info, s);
 
-      if (tc)
-      {
-        const cudaError_t e = ncg_launch_syrk_tc (pk, nb, rest, A + (size_t) (kb + nb) * n + kb + nb, n, 1, info, s);
+      if (e != cudaSuccess)
+        return e;
+    }
+    else if (rest > 0)
+    {
+      const int T_ = (rest + PB - 1) / PB;
 
-        if (e != cudaSuccess)
-          return e;
-      }
-      else
-      {
-        const int T_ = (rest + PB - 1) / PB;
-
-        _potrf_update_f32_kernel<<<T_ * (T_ + 1) / 2, 256, 0, s>>> (A, n, kb, nb, kb + nb, rest, info);
-      }
+      _potrf_update_f32_kernel<<<T_ * (T_ + 1) / 2, 256, 0, s>>> (A, n, kb, nb, kb + nb, rest, dg, info);
     }
   }
 

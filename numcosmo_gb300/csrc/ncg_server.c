@@ -156,7 +156,7 @@ _chain_bytes (const ncg_chain_desc_t *c, int mixed)
   b += 8.0 * n * ncg_pack64_stride (c->kind, dp);           /* pack64         */
   b += 8.0 * n * 8.0;                                       /* per-kernel vectors */
   b += 8.0 * 24.0 * n + (double) ncg_gemv_t_scratch ((int) (c->n / 2), (int) (c->n / 2));   /* NNLS vectors, gemv scratch */
-  b += (double) ncg_pcg_trinv_bytes ((int) n) + (double) ncg_syrk_tc_pack_bytes ((int) n, 64);  /* preconditioner */
+  b += (double) ncg_pcg_trinv_bytes ((int) n) + (double) ncg_potrf_f32_work_bytes ((int) n);  /* preconditioner */
   {
     /* eval partials of 2n points, and the FP64 form's tensor-core operands */
     ncg_eval_args_t a = { .kind = (int32_t) c->kind, .kernel = (int32_t) c->kernel, .d = (int32_t) c->dim, .dp = dp,

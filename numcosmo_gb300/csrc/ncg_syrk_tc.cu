@@ -105,10 +105,11 @@ _pack_f64_kernel (const double *__restrict__ A, int lda, int r0, int r1, int c0,
   }
 }
 
-/* mode: 0 C = A^T A, 1 C -= A^T A, 2 C += A^T A (upper, i <= j) */
+/* mode: 0 C = A^T A, 1 C -= A^T A, 2 C += A^T A (upper, i <= j); dg (may be NULL):
+ * the leading 64 x 64 of the result */
 __global__ void __launch_bounds__ (SK_THREADS, 1)
 _syrk_tc_kernel (const uint8_t *__restrict__ pk, int nkc, int nn, float *__restrict__ C, int ldc, int mode,
-                 int *__restrict__ err_out)
+                 float *__restrict__ dg, int *__restrict__ err_out)
 {
   extern __shared__ uint8_t smem_raw[];
   SkSmem &sm = *(SkSmem *) (((uintptr_t) smem_raw + 1023) & ~(uintptr_t) 1023);
@@ -347,6 +348,11 @@ _syrk_tc_kernel (const uint8_t *__restrict__ pk, int nkc, int nn, float *__restr
           for (int r = 0; r < 32; r++)
             if (SK_IN (r, j))
               C[(size_t) (i0 + r) * ldc + j] = nv[r];
+
+          if (dg != NULL && i0 < 64 && j < 64)
+#pragma unroll
+            for (int r = 0; r < 32; r++)
+              dg[(i0 + r) * 64 + j] = nv[r];
         }
       }
 
@@ -398,7 +404,7 @@ ncg_syrk_tc_pack_bytes (int nn, int K)
 }
 
 extern "C" cudaError_t
-ncg_launch_syrk_tc (const void *pk, int K, int nn, float *C, int ldc, int mode, int *err, cudaStream_t s)
+ncg_launch_syrk_tc (const void *pk, int K, int nn, float *C, int ldc, int mode, float *dg, int *err, cudaStream_t s)
 {
   if (nn <= 0 || K <= 0)
     return cudaSuccess;
@@ -414,7 +420,7 @@ ncg_launch_syrk_tc (const void *pk, int K, int nn, float *C, int ldc, int mode, 
   const int grid   = (ntiles < nsm) ? ntiles : nsm;
 
   _syrk_tc_kernel<<<grid, SK_THREADS, SK_SMEM_BYTES, s>>> ((const uint8_t *) pk, (K + SK_KC - 1) / SK_KC, nn, C,
-                                                           ldc, mode, err);
+                                                           ldc, mode, dg, err);
 
   return cudaGetLastError ();
 }
@@ -443,7 +449,7 @@ ncg_launch_syrk_upper_tc_f64 (const double *A, int nrows, int ncols, float *C, v
 
     _pack_f64_kernel<<<T_ * nkc, 256, 0, s>>> (A, ncols, r0, r1, 0, ncols, nkc, (float *) scratch);
 
-    cudaError_t e = ncg_launch_syrk_tc (scratch, r1 - r0, ncols, C, ncols, (r0 == 0) ? 0 : 2, err, s);
+    cudaError_t e = ncg_launch_syrk_tc (scratch, r1 - r0, ncols, C, ncols, (r0 == 0) ? 0 : 2, NULL, err, s);
 
     if (e != cudaSuccess)
       return e;

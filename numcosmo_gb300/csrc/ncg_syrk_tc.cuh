@@ -45,27 +45,4 @@ _put_split4f (float *blk, int row, int k4, float v0, float v1, float v2, float v
   *(float4 *) (blk + SK_HALF / 4 + off) = make_float4 (_tf32 (v0 - h0), _tf32 (v1 - h1), _tf32 (v2 - h2), _tf32 (v3 - h3));
 }
 
-/* column rel (0-based past the panel's diagonal block) of a 64-row panel
- * (nkc = 2) whose values are a[0..nb), into the pack pk */
-static __device__ __forceinline__ void
-_sk_pack_column (float *pk, int rel, const float *a, int nb)
-{
-  const int t = rel >> 7, row = rel & 127;
-
-#pragma unroll
-  for (int c = 0; c < 2; c++)
-  {
-    float *blk = pk + (size_t) (t * 2 + c) * (SK_BLOCK / 4);
-
-#pragma unroll
-    for (int q = 0; q < 8; q++)
-    {
-      const int k = c * SK_KC + 4 * q;
-
-      _put_split4f (blk, row, 4 * q, (k + 0 < nb) ? a[k + 0] : 0.0f, (k + 1 < nb) ? a[k + 1] : 0.0f,
-                    (k + 2 < nb) ? a[k + 2] : 0.0f, (k + 3 < nb) ? a[k + 3] : 0.0f);
-    }
-  }
-}
-
 #endif /* NCG_SYRK_TC_CUH */
