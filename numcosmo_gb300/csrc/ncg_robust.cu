@@ -13,11 +13,12 @@
  * m/(m+3.8) for even m above).  One CTA (large sets) or one warp (the VKDE
  * neighbourhoods) computes one Qn: a bitonic sort of the m values in shared
  * memory on order-preserving integer keys, then the k-th smallest pairwise
- * difference found exactly by bisection over the bit patterns of
- * non-negative doubles (their order is the integer order):
- * count(t) = #{a < b : x_b - x_a <= t}, and the smallest t with
- * count(t) >= k is the order statistic itself (a difference of two sample
- * values, computed as the reference computes it).
+ * difference found exactly: bisection over the bit patterns of non-negative
+ * doubles (their order is the integer order) with
+ * count(t) = #{a < b : x_b - x_a <= t} until the bracket holds few differences,
+ * and those ranked by value.  The smallest t with count(t) >= k is the order
+ * statistic itself (a difference of two sample values, computed as the
+ * reference computes it).
  *
  * Each test fl64(x_b - x_a) <= t of the count is first decided on FP32
  * copies of the sorted values less their median c (FP64 runs at 1/64 of the
@@ -50,11 +51,13 @@
 #include "ncg_internal.h"
 #include "ncg_jacobi.cuh"
 
-#define RQ_TH 256
+#define RQ_TH 256        /* CTAs of a warp per Qn, at most */
+#define RQ_CTA_TH 1024   /* the CTA per Qn: 32 warps, one sum per lane in _rq_block_sum */
 
-/* -------------------------------------------------------------- Qn on a CTA */
+/* ------------------------------------------------------------ the estimator */
 
-__device__ __forceinline__ double
+/* (host: a division per Qn would be a tenth of its FP64 work) */
+static double
 _qn_dn (int m)
 {
   /* small-sample factors for m = 2..9, Croux & Rousseeuw (1992) */
@@ -74,15 +77,13 @@ _qn_dn (int m)
   return (m & 1) ? m / (m + 1.4) : m / (m + 3.8);
 }
 
-__device__ __forceinline__ long long
-_rq_block_sum (long long v, long long *red)
+/* sum over the CTA of RQ_CTA_TH threads (red: RQ_CTA_TH / 32 values) */
+__device__ __forceinline__ int
+_rq_block_sum (int v, int *red)
 {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-    v += __shfl_xor_sync (0xffffffffu, v, o);
-
+  v = __reduce_add_sync (0xffffffffu, v);
   __syncthreads ();
 
   if (lane == 0)
@@ -90,13 +91,7 @@ _rq_block_sum (long long v, long long *red)
 
   __syncthreads ();
 
-  long long t = 0;
-
-#pragma unroll
-  for (int w = 0; w < RQ_TH / 32; w++)
-    t += red[w];
-
-  return t;
+  return __reduce_add_sync (0xffffffffu, red[lane]);
 }
 
 /* order-preserving map of a double's bits to a signed integer (its own
@@ -127,20 +122,16 @@ _qn_sort (double *v, float *f, int m, int mpad, int t0, int nt, Sync sync)
   for (int k = 2; k <= mpad; k <<= 1)
     for (int j = k >> 1; j > 0; j >>= 1)
     {
-      for (int t = t0; t < mpad; t += nt)
+      /* the stage's pairs, one per thread */
+      for (int p = t0; p < mpad / 2; p += nt)
       {
-        const int u = t ^ j;
+        const int t       = 2 * p - (p & (j - 1)), u = t + j;
+        const long long a = kv[t], b = kv[u];
 
-        if (u > t)
+        if ((a > b) == ((t & k) == 0))
         {
-          const long long a = kv[t], b = kv[u];
-          const bool up     = (t & k) == 0;
-
-          if ((a > b) == up)
-          {
-            kv[t] = b;
-            kv[u] = a;
-          }
+          kv[t] = b;
+          kv[u] = a;
         }
       }
 
@@ -191,6 +182,15 @@ _qn_row (const double *v, const float *f, int a, float tf, bool fast)
   return r;
 }
 
+/* fl64(y - x) <= t, as a call: inlined, the two FP64 instructions are predicated
+ * and go through their pipe (64 cycles each) for every test, also where no lane
+ * needs them.  They were what bound the counts: 75 % of the pipe's cycles */
+__device__ __noinline__ bool
+_qn_le64 (double y, double x, double t)
+{
+  return y - x <= t;
+}
+
 /* fl64(v[j] - r.x) <= t, for j past the row (v[j] >= r.x) */
 __device__ __forceinline__ bool
 _qn_le (const double *v, const float *f, int j, const QnRow &r, double t)
@@ -203,7 +203,7 @@ _qn_le (const double *v, const float *f, int j, const QnRow &r, double t)
   if (y > r.hi)
     return false;
 
-  return v[j] - r.x <= t;
+  return _qn_le64 (v[j], r.x, t);
 }
 
 /* the FP32 band holds for the set: every |v - v[m/2]| < 2^100 (v sorted) */
@@ -215,55 +215,189 @@ _qn_fast (const double *v, int m)
   return fabs (v[0] - c) < 0x1p100 && fabs (v[m - 1] - c) < 0x1p100;
 }
 
-/* Qn of v[0..m) (v holds mpad >= m slots, mpad a power of two; sorted on
- * return; f holds mpad floats); every thread gets the value */
-__device__ double
-_qn_cta (double *v, float *f, int m, int mpad, long long *red)
+/* The k-th smallest difference is bracketed by bisection, and the bracket's last
+ * few differences are ranked.  A count over threshold t moves lo or hi (bit
+ * patterns of non-negative doubles); cL and cH, the counts below lo and up to
+ * hi, say how many differences the bracket still holds, and the steps end when
+ * those fit the ranking.  While nothing is known to lie below, the threshold
+ * steps down from hi by octaves (3, 6, 12, ...): a scale estimate is within a few of
+ * the range, where halving the patterns of [0, hi] spends its first steps near
+ * 1e-154 and takes ten to reach the right octave.  Bisecting all 62 bits took 62
+ * counts; now about 9 for 100 values and 16 for 2000: with the FP64 tests off the
+ * counts (_qn_le64) the pairs of 2048 sets of 102 rows, d = 8, took 2550 -> 950 us
+ * and those of one set of 2048 rows 860 -> 150 us. */
+struct QnBracket
 {
-  const int tid = threadIdx.x;
+  unsigned long long lo, hi;
+  int cL, cH, kk;
+  unsigned long long down;
 
-  _qn_sort (v, f, m, mpad, tid, RQ_TH, [] () { __syncthreads (); });
-
-  const long long h = m / 2 + 1, kk = h * (h - 1) / 2;
-  const double span = v[m - 1] - v[0];
-  const bool fast   = _qn_fast (v, m);
-  unsigned long long lo = 0ull, hi = (unsigned long long) __double_as_longlong (span > 0.0 ? span : 0.0);
-
-  while (lo < hi)
+  __device__ QnBracket (const double *v, int m)
   {
-    const unsigned long long mid = lo + ((hi - lo) >> 1);
-    const double t = __longlong_as_double ((long long) mid);
-    const float tf = __double2float_rn (t);
-    long long c    = 0;
+    const int h       = m / 2 + 1;
+    const double span = v[m - 1] - v[0];
 
-    for (int i = tid; i < m - 1; i += RQ_TH)
-    {
-      const QnRow r = _qn_row (v, f, i, tf, fast);
-      int a = i, b = m - 1;
-
-      /* largest j in [i, m) with v[j] - v[i] <= t (monotone in j) */
-      while (a < b)
-      {
-        const int md = (a + b + 1) >> 1;
-
-        if (_qn_le (v, f, md, r, t))
-          a = md;
-        else
-          b = md - 1;
-      }
-
-      c += a - i;
-    }
-
-    c = _rq_block_sum (c, red);
-
-    if (c >= kk)
-      hi = mid;
-    else
-      lo = mid + 1;
+    lo   = 0ull;
+    hi   = (unsigned long long) __double_as_longlong (span > 0.0 ? span : 0.0);
+    cL   = 0;
+    cH   = m * (m - 1) / 2;
+    kk   = h * (h - 1) / 2;
+    down = 3ull << 52;
   }
 
-  return 2.21914 * _qn_dn (m) * __longlong_as_double ((long long) lo);
+  __device__ bool open (int cap) const
+  {
+    return lo < hi && cH - cL > cap;
+  }
+
+  __device__ unsigned long long mid ()
+  {
+    if (lo == 0ull && hi > down)
+    {
+      const unsigned long long t = hi - down;
+
+      down *= 2;
+
+      return t;
+    }
+
+    return lo + ((hi - lo) >> 1);
+  }
+
+  /* count c at threshold t; true when the bracket's upper end moved */
+  __device__ bool take (unsigned long long t, int c)
+  {
+    if (c >= kk)
+    {
+      hi = t;
+      cH = c;
+
+      return true;
+    }
+
+    lo = t + 1;
+    cL = c;
+
+    return false;
+  }
+
+  /* the difference's ranking key; one that is no number sorts at the bracket's end */
+  __device__ unsigned long long key (double dif) const
+  {
+    const unsigned long long b = (unsigned long long) __double_as_longlong (dif);
+
+    return b < hi ? b : hi;
+  }
+};
+
+/* how many differences are ranked: one per lane, one per thread of 8 warps */
+#define QN_WARP_CAP 32
+#define QN_CTA_CAP 256
+
+/* largest j in [i, m) with fl64(v[j] - v[i]) <= t (monotone in j) */
+__device__ __forceinline__ int
+_qn_reach (const double *v, const float *f, int i, int m, double t, float tf, bool fast)
+{
+  const QnRow r = _qn_row (v, f, i, tf, fast);
+  int a = i, b = m - 1;
+
+  while (a < b)
+  {
+    const int md = (a + b + 1) >> 1;
+
+    if (_qn_le (v, f, md, r, t))
+      a = md;
+    else
+      b = md - 1;
+  }
+
+  return a;
+}
+
+/* Qn of v[0..m) (v holds mpad >= m slots, mpad a power of two; sorted on
+ * return; f holds mpad floats); every thread gets the value.  The row searches
+ * are dependent shared-memory trips, so the CTA is as wide as it can be: one
+ * global estimate has 8 to 28 of them for d = 8, on 152 SMs */
+__device__ double
+_qn_cta (double *v, float *f, int m, int mpad, double cq, int *red)
+{
+  __shared__ unsigned long long cand[QN_CTA_CAP];
+  __shared__ unsigned long long sel;
+  __shared__ int ncand;
+  const int tid = threadIdx.x;
+
+  _qn_sort (v, f, m, mpad, tid, RQ_CTA_TH, [] () { __syncthreads (); });
+
+  const bool fast = _qn_fast (v, m);
+  QnBracket q (v, m);
+
+  while (q.open (QN_CTA_CAP))
+  {
+    const unsigned long long mid = q.mid ();
+    const double t = __longlong_as_double ((long long) mid);
+    const float tf = __double2float_rn (t);
+    int c          = 0;
+
+    for (int i = tid; i < m - 1; i += RQ_CTA_TH)
+      c += _qn_reach (v, f, i, m, t, tf, fast) - i;
+
+    q.take (mid, _rq_block_sum (c, red));
+  }
+
+  if (q.lo < q.hi)
+  {
+    const int nc     = q.cH - q.cL;
+    const double th  = __longlong_as_double ((long long) q.hi);
+    const double tl  = __longlong_as_double ((long long) (q.lo > 0ull ? q.lo - 1 : 0ull));
+    const float thf  = __double2float_rn (th), tlf = __double2float_rn (tl);
+    const bool below = q.lo > 0ull;
+
+    if (tid < QN_CTA_CAP)
+      cand[tid] = q.hi;
+
+    if (tid == 0)
+    {
+      ncand = 0;
+      sel   = q.hi;
+    }
+
+    __syncthreads ();
+
+    for (int i = tid; i < m - 1; i += RQ_CTA_TH)
+    {
+      const int H = _qn_reach (v, f, i, m, th, thf, fast);
+      const int L = below ? _qn_reach (v, f, i, m, tl, tlf, fast) : i;
+
+      if (H > L)
+      {
+        const int o = atomicAdd (&ncand, H - L);
+
+        for (int j = L + 1; j <= H; j++)
+          if (o + j - L - 1 < QN_CTA_CAP)
+            cand[o + j - L - 1] = q.key (v[j] - v[i]);
+      }
+    }
+
+    __syncthreads ();
+
+    if (tid < nc)
+    {
+      const unsigned long long own = cand[tid];
+      int rank = 0;
+
+      for (int k = 0; k < nc; k++)
+        rank += cand[k] < own || (cand[k] == own && k < tid);
+
+      if (rank == q.kk - q.cL - 1)
+        sel = own;
+    }
+
+    __syncthreads ();
+    q.lo = sel;
+    __syncthreads ();
+  }
+
+  return cq * __longlong_as_double ((long long) q.lo);
 }
 
 /* row a of set s; an index outside [0, n) is counted in *bad and replaced by 0 */
@@ -295,29 +429,26 @@ _rq_row (const int32_t *idx, int s, int m, int a, int n, int32_t *bad)
 #define RQ_WARP_MPAD 1024
 
 __device__ double
-_qn_warp (double *v, float *f, uint32_t *bnd, int m, int mpad)
+_qn_warp (double *v, float *f, uint32_t *bnd, int m, int mpad, double cq)
 {
   const int lane = threadIdx.x & 31;
 
   _qn_sort (v, f, m, mpad, lane, 32, [] () { __syncwarp (); });
 
-  const long long h = m / 2 + 1, kk = h * (h - 1) / 2;
-  const double span = v[m - 1] - v[0];
-  const bool fast   = _qn_fast (v, m);
+  const bool fast = _qn_fast (v, m);
   const int chunk = (m - 1 + 31) / 32, r0 = lane * chunk, r1 = min (m - 1, r0 + chunk);
-  unsigned long long lo = 0ull, hi = (unsigned long long) __double_as_longlong (span > 0.0 ? span : 0.0);
+  QnBracket q (v, m);
   int pend = 0;   /* the last step's verdict, applied as each row is read: 1 L := a, 2 H := a */
 
   for (int i = r0; i < r1; i++)
     bnd[i] = (uint32_t) i | ((uint32_t) (m - 1) << 10);
 
-  while (lo < hi)
+  while (q.open (QN_WARP_CAP))
   {
-    const unsigned long long mid = lo + ((hi - lo) >> 1);
+    const unsigned long long mid = q.mid ();
     const double t = __longlong_as_double ((long long) mid);
     const float tf = __double2float_rn (t);
-    long long c    = 0;
-    int a          = -1;
+    int c = 0, a = -1;
 
     for (int i = r0; i < r1; i++)
     {
@@ -359,23 +490,66 @@ _qn_warp (double *v, float *f, uint32_t *bnd, int m, int mpad)
       bnd[i] = (uint32_t) L | ((uint32_t) H << 10) | ((uint32_t) a << 20);
     }
 
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-      c += __shfl_xor_sync (0xffffffffu, c, o);
-
-    if (c >= kk)
-    {
-      hi   = mid;
-      pend = 2;
-    }
-    else
-    {
-      lo   = mid + 1;
-      pend = 1;
-    }
+    pend = q.take (mid, __reduce_add_sync (0xffffffffu, c)) ? 2 : 1;
   }
 
-  return 2.21914 * _qn_dn (m) * __longlong_as_double ((long long) lo);
+  if (q.lo < q.hi)
+  {
+    /* the bracket's differences, one per lane, through the copies' room */
+    unsigned long long *cand = (unsigned long long *) f;
+    const int nc             = q.cH - q.cL;
+    int cnt = 0, o;
+
+    for (int i = r0; i < r1; i++)
+    {
+      const uint32_t wd = bnd[i];
+      const int L       = (int) ((pend == 1) ? wd >> 20 : wd & 1023u);
+      const int H       = (int) ((pend == 2) ? wd >> 20 : (wd >> 10) & 1023u);
+
+      cnt += max (H - L, 0);
+    }
+
+    o = cnt;
+
+#pragma unroll
+    for (int k = 1; k < 32; k <<= 1)
+    {
+      const int t = __shfl_up_sync (0xffffffffu, o, k);
+
+      if (lane >= k)
+        o += t;
+    }
+
+    o -= cnt;
+    __syncwarp ();
+    cand[lane] = q.hi;
+    __syncwarp ();
+
+    for (int i = r0; i < r1; i++)
+    {
+      const uint32_t wd = bnd[i];
+      const int L       = (int) ((pend == 1) ? wd >> 20 : wd & 1023u);
+      const int H       = (int) ((pend == 2) ? wd >> 20 : (wd >> 10) & 1023u);
+
+      for (int j = L + 1; j <= H; j++, o++)
+        if (o < QN_WARP_CAP)
+          cand[o] = q.key (v[j] - v[i]);
+    }
+
+    __syncwarp ();
+
+    const unsigned long long own = cand[lane];
+    int rank = 0;
+
+    for (int k = 0; k < nc; k++)
+      rank += cand[k] < own || (cand[k] == own && k < lane);
+
+    const unsigned w = __ballot_sync (0xffffffffu, lane < nc && rank == q.kk - q.cL - 1);
+
+    q.lo = w ? __shfl_sync (0xffffffffu, own, __ffs (w) - 1) : q.hi;
+  }
+
+  return cq * __longlong_as_double ((long long) q.lo);
 }
 
 /* ------------------------------------------------------------------ stages */
@@ -384,6 +558,13 @@ _qn_warp (double *v, float *f, uint32_t *bnd, int m, int mpad)
  * one warp with its own slice of the shared values (W = true; CTAs of 2 to
  * RQ_WPB such warps, as many as keep the most warps resident). */
 #define RQ_WPB (RQ_TH / 32)
+
+/* floats of a worker's copies: room for the ranked differences of a small set */
+__host__ __device__ __forceinline__ int
+_rq_fpad (int mpad)
+{
+  return mpad < 2 * QN_WARP_CAP ? 2 * QN_WARP_CAP : mpad;
+}
 
 template <bool W>
 struct RqWorker
@@ -395,14 +576,14 @@ struct RqWorker
 
   __device__ RqWorker (double *smem, int mpad)
   {
-    const int warp = threadIdx.x >> 5, wpb = W ? (int) (blockDim.x >> 5) : 1;
+    const int warp = threadIdx.x >> 5, wpb = W ? (int) (blockDim.x >> 5) : 1, fpad = _rq_fpad (mpad);
 
     id  = W ? blockIdx.x * wpb + warp : blockIdx.x;
     t   = W ? (threadIdx.x & 31) : threadIdx.x;
-    nt  = W ? 32 : RQ_TH;
+    nt  = W ? 32 : RQ_CTA_TH;
     v   = W ? smem + (size_t) warp * mpad : smem;
-    f   = (float *) (smem + (size_t) mpad * wpb) + (W ? (size_t) warp * mpad : 0);
-    bnd = W ? (uint32_t *) ((float *) (smem + (size_t) mpad * wpb) + (size_t) mpad * wpb) + (size_t) warp * mpad
+    f   = (float *) (smem + (size_t) mpad * wpb) + (W ? (size_t) warp * fpad : 0);
+    bnd = W ? (uint32_t *) ((float *) (smem + (size_t) mpad * wpb) + (size_t) fpad * wpb) + (size_t) warp * mpad
             : NULL;
   }
 
@@ -414,9 +595,9 @@ struct RqWorker
       __syncthreads ();
   }
 
-  __device__ double qn (int m, int mpad, long long *red) const
+  __device__ double qn (int m, int mpad, double cq, int *red) const
   {
-    return W ? _qn_warp (v, f, bnd, m, mpad) : _qn_cta (v, f, m, mpad, red);
+    return W ? _qn_warp (v, f, bnd, m, mpad, cq) : _qn_cta (v, f, m, mpad, cq, red);
   }
 };
 
@@ -424,13 +605,13 @@ struct RqWorker
  * row i is written (sigma^2 on the diagonal), else C's row i (1 on the
  * diagonal) */
 template <bool W>
-__global__ void __launch_bounds__ (RQ_TH)
+__global__ void __launch_bounds__ (W ? RQ_TH : RQ_CTA_TH)
 _rq_sigma_kernel (const double *__restrict__ X, int n, int d, int32_t *__restrict__ bad,
-                  const int32_t *__restrict__ idx, int m, int mpad, int ntasks, double *__restrict__ sig,
+                  const int32_t *__restrict__ idx, int m, int mpad, double cq, int ntasks, double *__restrict__ sig,
                   double *__restrict__ out, int diag)
 {
   extern __shared__ double rq_v[];
-  __shared__ long long red[RQ_TH / 32];
+  __shared__ int red[RQ_CTA_TH / 32];
   const RqWorker<W> w (rq_v, mpad);
 
   if (w.id >= ntasks)   /* whole warps (W) or the whole CTA leave together */
@@ -443,7 +624,7 @@ _rq_sigma_kernel (const double *__restrict__ X, int n, int d, int32_t *__restric
 
   w.sync ();
 
-  const double q = w.qn (m, mpad, red);
+  const double q = w.qn (m, mpad, cq, red);
 
   if (w.t == 0)
     sig[(size_t) s * d + i] = q;
@@ -454,13 +635,13 @@ _rq_sigma_kernel (const double *__restrict__ X, int n, int d, int32_t *__restric
 
 /* 2. C[s][i][j] = C[s][j][i] = (Qn(y_i + y_j)^2 - Qn(y_i - y_j)^2) / 4 */
 template <bool W>
-__global__ void __launch_bounds__ (RQ_TH)
+__global__ void __launch_bounds__ (W ? RQ_TH : RQ_CTA_TH)
 _rq_pair_kernel (const double *__restrict__ X, int n, int d, int32_t *__restrict__ bad,
-                 const int32_t *__restrict__ idx, int m, int mpad, int ntasks, const double *__restrict__ sig,
+                 const int32_t *__restrict__ idx, int m, int mpad, double cq, int ntasks, const double *__restrict__ sig,
                  double *__restrict__ C)
 {
   extern __shared__ double rq_v[];
-  __shared__ long long red[RQ_TH / 32];
+  __shared__ int red[RQ_CTA_TH / 32];
   const RqWorker<W> w (rq_v, mpad);
 
   if (w.id >= ntasks)
@@ -477,7 +658,9 @@ _rq_pair_kernel (const double *__restrict__ X, int n, int d, int32_t *__restrict
   }
 
   const int j = i + 1 + p;
-  const double ri = 1.0 / sig[(size_t) s * d + i], rj = 1.0 / sig[(size_t) s * d + j];
+  /* both reciprocals in one division */
+  const double rl = 1.0 / sig[(size_t) s * d + ((threadIdx.x & 1) ? j : i)];
+  const double ri = __shfl_sync (0xffffffffu, rl, 0), rj = __shfl_sync (0xffffffffu, rl, 1);
   double sq0 = 0.0, sq1 = 0.0;
 
   for (int pass = 0; pass < 2; pass++)
@@ -492,7 +675,7 @@ _rq_pair_kernel (const double *__restrict__ X, int n, int d, int32_t *__restrict
 
     w.sync ();
 
-    const double q = w.qn (m, mpad, red);
+    const double q = w.qn (m, mpad, cq, red);
 
     if (pass)
       sq1 = q * q;
@@ -563,13 +746,13 @@ _rq_eig_kernel (const double *__restrict__ C, int d, double *__restrict__ E)
 
 /* 4. sigz[s][i] = Qn of z_i = E_i . y over the set */
 template <bool W>
-__global__ void __launch_bounds__ (RQ_TH)
+__global__ void __launch_bounds__ (W ? RQ_TH : RQ_CTA_TH)
 _rq_z_kernel (const double *__restrict__ X, int n, int d, int32_t *__restrict__ bad,
-              const int32_t *__restrict__ idx, int m, int mpad, int ntasks, const double *__restrict__ sig,
+              const int32_t *__restrict__ idx, int m, int mpad, double cq, int ntasks, const double *__restrict__ sig,
               const double *__restrict__ E, double *__restrict__ sigz)
 {
   extern __shared__ double rq_v[];
-  __shared__ long long red[RQ_TH / 32];
+  __shared__ int red[RQ_CTA_TH / 32];
   __shared__ double eis[RQ_WPB][NCG_DMAX], rss[RQ_WPB][NCG_DMAX];
   const RqWorker<W> w (rq_v, mpad);
 
@@ -600,7 +783,7 @@ _rq_z_kernel (const double *__restrict__ X, int n, int d, int32_t *__restrict__ 
 
   w.sync ();
 
-  const double q = w.qn (m, mpad, red);
+  const double q = w.qn (m, mpad, cq, red);
 
   if (w.t == 0)
     sigz[(size_t) s * d + i] = q;
@@ -680,10 +863,11 @@ _robust_launch (const double *X, int n, int d, const int32_t *idx, int m, int ns
                 double *sigz, double *C, double *E, double *out, int32_t *bad, cudaStream_t s)
 {
   const int mpad        = _pow2_at_least (m);
-  const size_t per_warp = (W ? sizeof (double) + sizeof (float) + sizeof (uint32_t) : sizeof (double) + sizeof (float)) *
-                          (size_t) mpad;
+  const size_t per_warp = (W ? sizeof (double) + sizeof (uint32_t) : sizeof (double)) * (size_t) mpad +
+                          sizeof (float) * (size_t) _rq_fpad (mpad);
   const size_t smax     = per_warp * (W ? RQ_WPB : 1);
   const int t1 = nsets * d, t2 = nsets * (d * (d - 1) / 2);
+  const double cq = 2.21914 * _qn_dn (m);
   cudaError_t e;
 
   /* raised whatever the size: the kernels' static arrays (up to 4 KiB) count
@@ -699,17 +883,17 @@ _robust_launch (const double *X, int n, int d, const int32_t *idx, int m, int ns
   const int w2 = W ? _rq_wpb ((const void *) _rq_pair_kernel<W>, per_warp) : 1;
   const int w3 = W ? _rq_wpb ((const void *) _rq_z_kernel<W>, per_warp) : 1;
 
-  _rq_sigma_kernel<W><<<(t1 + w1 - 1) / w1, W ? 32 * w1 : RQ_TH, per_warp * w1, s>>> (X, n, d, bad, idx, m, mpad, t1,
-                                                                                      sig, ogk ? C : out, !ogk);
+  _rq_sigma_kernel<W><<<(t1 + w1 - 1) / w1, W ? 32 * w1 : RQ_CTA_TH, per_warp * w1, s>>> (X, n, d, bad, idx, m, mpad, cq,
+                                                                                          t1, sig, ogk ? C : out, !ogk);
 
   if (ogk)
   {
     if (d > 1)
-      _rq_pair_kernel<W><<<(t2 + w2 - 1) / w2, W ? 32 * w2 : RQ_TH, per_warp * w2, s>>> (X, n, d, bad, idx, m, mpad,
-                                                                                         t2, sig, C);
+      _rq_pair_kernel<W><<<(t2 + w2 - 1) / w2, W ? 32 * w2 : RQ_CTA_TH, per_warp * w2, s>>> (X, n, d, bad, idx, m, mpad,
+                                                                                             cq, t2, sig, C);
 
     _rq_eig_kernel<<<nsets, NPD_THREADS, 0, s>>> (C, d, E);
-    _rq_z_kernel<W><<<(t1 + w3 - 1) / w3, W ? 32 * w3 : RQ_TH, per_warp * w3, s>>> (X, n, d, bad, idx, m, mpad, t1,
+    _rq_z_kernel<W><<<(t1 + w3 - 1) / w3, W ? 32 * w3 : RQ_CTA_TH, per_warp * w3, s>>> (X, n, d, bad, idx, m, mpad, cq, t1,
                                                                                     sig, E, sigz);
     _rq_final_kernel<<<nsets, 128, 0, s>>> (E, d, sig, sigz, out);
   }
