@@ -277,8 +277,8 @@ cudaError_t ncg_launch_pcg_precond (const float *R, const float *V, const double
 size_t      ncg_pcg_sc_bytes (void);
 cudaError_t ncg_launch_pcg_dots (int mode, const double *u, const double *v, const double *w, const double *D,
                                  double *p, int n, double *sc, cudaStream_t s);
-cudaError_t ncg_launch_pcg_step (double *x, double *r, double *rprev, const double *p, const double *q, int n,
-                                 const double *sc, cudaStream_t s);
+cudaError_t ncg_launch_pcg_step (double *x, double *r, double *rprev, const double *p, const double *q, const double *D,
+                                 int n, double *sc, cudaStream_t s);
 cudaError_t ncg_launch_pcg_dir (double *p, const double *z, int n, double *sc, cudaStream_t s);
 cudaError_t ncg_launch_scatter_x (const double *xsub, const int32_t *P, int np, int n, double *x,
                                   cudaStream_t s);

@@ -397,18 +397,24 @@ _solve_mixed (nnls_t *s, int np, double *dx)
           !(hs[NCG_PCG_RZ] > 0.0))
         break;
 
+      if (it > 0)
+      {
+        CK (ncg_launch_pcg_precond (nn->R32, nn->Vi, nn->D, np, nn->rv, nn->t32, &nn->cs_epoch, nn->zv, nn->csync,
+                                     nn->sc + NCG_PCG_ERR, st), "precond");
+        CK (ncg_launch_pcg_dots (2, nn->rv, nn->zv, nn->rp, NULL, NULL, np, nn->sc, st), "dots");
+        CK (ncg_launch_pcg_dir (nn->pv, nn->zv, np, nn->sc, st), "dir");
+      }
+
       CK (ncg_launch_pcg_matvec (nn->IM, nr, n, nn->P, np, nn->pv, NULL, nn->yf, nn->part, nn->qv, st), "matvec");
       CK (ncg_launch_pcg_dots (1, nn->pv, nn->qv, NULL, NULL, NULL, np, nn->sc, st), "dots");
-      CK (ncg_launch_pcg_step (nn->xv, nn->rv, nn->rp, nn->pv, nn->qv, np, nn->sc, st), "step");
+      CK (ncg_launch_pcg_step (nn->xv, nn->rv, nn->rp, nn->pv, nn->qv, nn->D, np, nn->sc, st), "step");
 
       /* every few steps the recurred residual gives way to the true one */
       if ((it + 1) % NCG_PCG_RESTART == 0)
+      {
         CK (ncg_launch_pcg_matvec (nn->IM, nr, n, nn->P, np, nn->xv, nn->bsub, nn->yf, nn->part, nn->rv, st), "matvec");
-
-      CK (ncg_launch_pcg_precond (nn->R32, nn->Vi, nn->D, np, nn->rv, nn->t32, &nn->cs_epoch, nn->zv, nn->csync,
-                                 nn->sc + NCG_PCG_ERR, st), "precond");
-      CK (ncg_launch_pcg_dots (2, nn->rv, nn->zv, nn->rp, nn->D, NULL, np, nn->sc, st), "dots");
-      CK (ncg_launch_pcg_dir (nn->pv, nn->zv, np, nn->sc, st), "dir");
+        CK (ncg_launch_pcg_dots (3, nn->rv, NULL, NULL, nn->D, NULL, np, nn->sc, st), "dots");
+      }
     }
 
     sd->istats.n_cg_iters += it;

@@ -860,45 +860,19 @@ ncg_launch_normalize_weights (double *w, int n, double shrink, int32_t *bad, cud
 #define DOT_TH 256
 #define DOT_CTAS 64
 
-/* The scalars of one point of the iteration, as many dot products as it needs
- * in one launch: the CTAs leave partial sums and the last one to finish (a
- * counter, cleared again) adds them up in CTA order.  (One CTA of 1024 threads
- * per product took 8 to 10 us each.)
- *  MODE 0 (start): RZ = <r, z>, BB = |D b|^2, RR = |D r|^2, and p = z
- *  MODE 1: PQ = <p, q>
- *  MODE 2: RZ' = <r, z>, <z, r_prev>, RR = |D r|^2; BE = (RZ' - <z, r_prev>) / RZ
- *          (Polak-Ribiere), then RZ = RZ' */
-template <int MODE>
-__global__ void __launch_bounds__ (DOT_TH)
-_pcg_dots_kernel (const double *__restrict__ u, const double *__restrict__ v, const double *__restrict__ w,
-                  const double *__restrict__ D, double *__restrict__ p, int n, double *__restrict__ sc,
-                  double *__restrict__ part, int32_t *__restrict__ count)
+/* K sums over all threads of the grid (part: 3 DOT_CTAS, count: zero): the CTAs
+ * leave partial sums and the last one to finish (a counter, cleared again) adds
+ * them up in CTA order.  True in one thread of the grid, which then has them in s */
+template <int K>
+__device__ bool
+_dots_sum (double (&s)[3], double *part, int32_t *count)
 {
   __shared__ double red[3][DOT_TH / 32];
   __shared__ int last;
   const int tid = threadIdx.x, lane = tid & 31;
-  double s[3]   = { 0.0, 0.0, 0.0 };
-
-  for (int i = blockIdx.x * DOT_TH + tid; i < n; i += gridDim.x * DOT_TH)
-  {
-    const double ui = u[i], vi = v[i];
-
-    s[0] = fma (ui, vi, s[0]);
-
-    if (MODE != 1)
-    {
-      const double wi = w[i], di = D[i] * ui, b = (MODE == 0) ? D[i] * wi : vi;
-
-      s[1] = fma (b, (MODE == 0) ? b : wi, s[1]);
-      s[2] = fma (di, di, s[2]);
-    }
-
-    if (MODE == 0)
-      p[i] = vi;
-  }
 
 #pragma unroll
-  for (int k = 0; k < (MODE == 1 ? 1 : 3); k++)
+  for (int k = 0; k < K; k++)
   {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
@@ -910,7 +884,7 @@ _pcg_dots_kernel (const double *__restrict__ u, const double *__restrict__ v, co
 
   __syncthreads ();
 
-  if (tid < 3)
+  if (tid < K)
   {
     double t = red[tid][0];
 
@@ -929,60 +903,113 @@ _pcg_dots_kernel (const double *__restrict__ u, const double *__restrict__ v, co
   __syncthreads ();
 
   if (!last || tid >= 32)
-    return;
+    return false;
 
   __threadfence ();
 
-  if (tid < 3)
-  {
-    double t = 0.0;
+  double t = 0.0;
 
+  if (tid < K)
     for (int k = 0; k < (int) gridDim.x; k++)
       t += __ldcg (part + tid * DOT_CTAS + k);
 
-    s[0] = t;
-  }
-
-  const double t0 = __shfl_sync (0xffffffffu, s[0], 0), t1 = __shfl_sync (0xffffffffu, s[0], 1),
-               t2 = __shfl_sync (0xffffffffu, s[0], 2);
+#pragma unroll
+  for (int k = 0; k < K; k++)
+    s[k] = __shfl_sync (0xffffffffu, t, k);
 
   if (tid == 0)
-  {
     *count = 0;
+
+  return tid == 0;
+}
+
+/* The scalars of one point of the iteration, as many dot products as it needs
+ * in one launch (one CTA of 1024 threads per product took 8 to 10 us each).
+ *  MODE 0 (start): RZ = <r, z>, BB = |D b|^2, RR = |D r|^2, and p = z
+ *  MODE 1: PQ = <p, q>
+ *  MODE 2: RZ' = <r, z>, <z, r_prev>; BE = (RZ' - <z, r_prev>) / RZ
+ *          (Polak-Ribiere), then RZ = RZ'
+ *  MODE 3: RR = |D r|^2 */
+template <int MODE>
+__global__ void __launch_bounds__ (DOT_TH)
+_pcg_dots_kernel (const double *__restrict__ u, const double *__restrict__ v, const double *__restrict__ w,
+                  const double *__restrict__ D, double *__restrict__ p, int n, double *__restrict__ sc,
+                  double *__restrict__ part, int32_t *__restrict__ count)
+{
+  double s[3] = { 0.0, 0.0, 0.0 };
+
+  for (int i = blockIdx.x * DOT_TH + threadIdx.x; i < n; i += gridDim.x * DOT_TH)
+  {
+    const double ui = u[i];
+
+    if (MODE == 3)
+    {
+      const double di = D[i] * ui;
+
+      s[0] = fma (di, di, s[0]);
+      continue;
+    }
+
+    const double vi = v[i];
+
+    s[0] = fma (ui, vi, s[0]);
 
     if (MODE == 0)
     {
-      sc[NCG_PCG_RZ] = t0;
-      sc[NCG_PCG_BB] = t1;
-      sc[NCG_PCG_RR] = t2;
+      const double di = D[i] * ui, b = D[i] * w[i];
+
+      s[1] = fma (b, b, s[1]);
+      s[2] = fma (di, di, s[2]);
+      p[i] = vi;
     }
-    else if (MODE == 1)
-      sc[NCG_PCG_PQ] = t0;
-    else
-    {
-      sc[NCG_PCG_BE] = (t0 - t1) / sc[NCG_PCG_RZ];
-      sc[NCG_PCG_RZ] = t0;
-      sc[NCG_PCG_RR] = t2;
-    }
+    else if (MODE == 2)
+      s[1] = fma (vi, w[i], s[1]);
   }
-}
 
-/* x += alpha p, r_prev = r, r -= alpha q with alpha = sc[RZ] / sc[PQ] */
-__global__ void
-_pcg_step_kernel (double *__restrict__ x, double *__restrict__ r, double *__restrict__ rprev,
-                  const double *__restrict__ p, const double *__restrict__ q, int n, const double *sc)
-{
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-
-  if (i >= n)
+  if (!_dots_sum<(MODE == 0) ? 3 : (MODE == 2) ? 2 : 1> (s, part, count))
     return;
 
-  const double al = sc[NCG_PCG_RZ] / sc[NCG_PCG_PQ];
-  const double ri = r[i];
+  if (MODE == 0)
+  {
+    sc[NCG_PCG_RZ] = s[0];
+    sc[NCG_PCG_BB] = s[1];
+    sc[NCG_PCG_RR] = s[2];
+  }
+  else if (MODE == 1)
+    sc[NCG_PCG_PQ] = s[0];
+  else if (MODE == 2)
+  {
+    sc[NCG_PCG_BE] = (s[0] - s[1]) / sc[NCG_PCG_RZ];
+    sc[NCG_PCG_RZ] = s[0];
+  }
+  else
+    sc[NCG_PCG_RR] = s[0];
+}
 
-  x[i]     = fma (al, p[i], x[i]);
-  rprev[i] = ri;
-  r[i]     = fma (-al, q[i], ri);
+/* x += alpha p, r_prev = r, r -= alpha q with alpha = sc[RZ] / sc[PQ], and RR =
+ * |D r|^2 of the new r, so that the host can stop before the next
+ * preconditioning (two triangular solves, 160 us at n = 3000, per solve).  A
+ * direction with RZ not above zero is not taken: the host stops at RZ */
+__global__ void __launch_bounds__ (DOT_TH)
+_pcg_step_kernel (double *__restrict__ x, double *__restrict__ r, double *__restrict__ rprev,
+                  const double *__restrict__ p, const double *__restrict__ q, const double *__restrict__ D, int n,
+                  double *__restrict__ sc, double *__restrict__ part, int32_t *__restrict__ count)
+{
+  const double rz = sc[NCG_PCG_RZ], al = (rz > 0.0) ? rz / sc[NCG_PCG_PQ] : 0.0;
+  double s[3] = { 0.0, 0.0, 0.0 };
+
+  for (int i = blockIdx.x * DOT_TH + threadIdx.x; i < n; i += gridDim.x * DOT_TH)
+  {
+    const double ri = r[i], rn = fma (-al, q[i], ri), di = D[i] * rn;
+
+    x[i]     = fma (al, p[i], x[i]);
+    rprev[i] = ri;
+    r[i]     = rn;
+    s[0]     = fma (di, di, s[0]);
+  }
+
+  if (_dots_sum<1> (s, part, count))
+    sc[NCG_PCG_RR] = s[0];
 }
 
 /* p = z + BE p */
@@ -1393,31 +1420,46 @@ ncg_pcg_sc_bytes (void)
   return sizeof (double) * (NCG_PCG_NSC + 3 * DOT_CTAS + 1);
 }
 
+/* CTAs of a launch that sums over n entries */
+static int
+_dots_grid (int n)
+{
+  const int g = (n + DOT_TH - 1) / DOT_TH;
+
+  return g < DOT_CTAS ? g : DOT_CTAS;
+}
+
 /* the scalars sc of the start (mode 0: u = r, v = z, w = b, p = z), <p, q> (mode 1:
- * u = p, v = q) or the next direction (mode 2: u = r, v = z, w = r_prev) */
+ * u = p, v = q), the next direction (mode 2: u = r, v = z, w = r_prev) or the
+ * residual alone (mode 3: u = r) */
 extern "C" cudaError_t
 ncg_launch_pcg_dots (int mode, const double *u, const double *v, const double *w, const double *D, double *p, int n,
                      double *sc, cudaStream_t s)
 {
   double *part   = sc + NCG_PCG_NSC;
   int32_t *count = (int32_t *) (part + 3 * DOT_CTAS);
-  const int g    = (n + DOT_TH - 1) / DOT_TH < DOT_CTAS ? (n + DOT_TH - 1) / DOT_TH : DOT_CTAS;
+  const int g    = _dots_grid (n);
 
   if (mode == 0)
     _pcg_dots_kernel<0><<<g, DOT_TH, 0, s>>> (u, v, w, D, p, n, sc, part, count);
   else if (mode == 1)
     _pcg_dots_kernel<1><<<g, DOT_TH, 0, s>>> (u, v, w, D, p, n, sc, part, count);
-  else
+  else if (mode == 2)
     _pcg_dots_kernel<2><<<g, DOT_TH, 0, s>>> (u, v, w, D, p, n, sc, part, count);
+  else
+    _pcg_dots_kernel<3><<<g, DOT_TH, 0, s>>> (u, v, w, D, p, n, sc, part, count);
 
   return cudaGetLastError ();
 }
 
 extern "C" cudaError_t
-ncg_launch_pcg_step (double *x, double *r, double *rprev, const double *p, const double *q, int n, const double *sc,
-                     cudaStream_t s)
+ncg_launch_pcg_step (double *x, double *r, double *rprev, const double *p, const double *q, const double *D, int n,
+                     double *sc, cudaStream_t s)
 {
-  _pcg_step_kernel<<<VB (n), 0, s>>> (x, r, rprev, p, q, n, sc);
+  double *part   = sc + NCG_PCG_NSC;
+  int32_t *count = (int32_t *) (part + 3 * DOT_CTAS);
+
+  _pcg_step_kernel<<<_dots_grid (n), DOT_TH, 0, s>>> (x, r, rprev, p, q, D, n, sc, part, count);
 
   return cudaGetLastError ();
 }
