@@ -455,14 +455,15 @@ _stage_block (T (*S)[B + 1], const T *__restrict__ A, int ld, int r0, int c0, in
 /* One panel: the diagonal block (raw in dg, 64 x 64) and 64 of the columns to
  * its right per CTA, eliminated in the same steps.  Both live in registers,
  * 4 x 4 elements each per thread (element (ty + 16p, tx + 16q)); a step
- * publishes its raw row j of both through shared memory, one barrier, and every
- * thread takes s_jr s_jc / a_jj off its elements; the square roots and the
- * rows' scaling wait for the end, where all rows take them at once.  CTA 0 writes
- * the factored block.  It is bound by the chain of 64 steps (a barrier, two
- * shared-memory trips and a reciprocal each), which every CTA walks for itself:
+ * publishes two raw rows j, j + 1 of both through shared memory, one barrier, and
+ * every thread works out row j + 1 as row j leaves it where it needs it, then takes
+ * s_jr s_jc / a_jj of both rows off its elements; the square roots and the rows'
+ * scaling wait for the end, where all rows take them at once.  CTA 0 writes the
+ * factored block.  It is bound by the chain of 32 steps (a barrier, two
+ * shared-memory trips and two reciprocals each), which every CTA walks for itself:
  * as two launches, the factor and then the columns against it, a panel took
- * 10 + 11 us (24 + 27 with the row scaled on the chain and a pack through FP64);
- * 12 us so.  pk (may be NULL): the panel as the tensor-core update's operand. */
+ * 10 + 11 us (24 + 27 with the row scaled on the chain and a pack through FP64),
+ * row by row in one 14.7 us; 10.8 us so (mean over the panels at n = 3000).  pk (may be NULL): the panel as the tensor-core update's operand. */
 __device__ __forceinline__ float
 _rcp_approx (float x)
 {
@@ -477,7 +478,7 @@ __global__ void __launch_bounds__ (256)
 _potrf_panel_f32_kernel (float *A, int ld, int kb, int nb, int n, const float *__restrict__ dg, int32_t *info,
                          float *pk)
 {
-  __shared__ float row[2][2 * PB];
+  __shared__ float row[2][2][2 * PB];
   __shared__ float X[PB][PB + 1];
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const int c0  = kb + nb + blockIdx.x * PB;
@@ -503,16 +504,18 @@ _potrf_panel_f32_kernel (float *A, int ld, int kb, int nb, int n, const float *_
 
 #pragma unroll
   for (int p = 0; p < 4; p++)
-    for (int jj = 0; jj < 16; jj++)
+    for (int jj = 0; jj < 16; jj += 2)
     {
       const int j = 16 * p + jj;
-      float *rb   = row[j & 1];
+      float *r0 = row[(jj >> 1) & 1][0], *r1 = row[(jj >> 1) & 1][1];
 
       if (fail)
         break;
 
-      if (ty == jj)
+      if ((ty & ~1) == jj)
       {
+        float *rb = (ty & 1) ? r1 : r0;
+
 #pragma unroll
         for (int q = 0; q < 4; q++)
         {
@@ -525,40 +528,43 @@ _potrf_panel_f32_kernel (float *A, int ld, int kb, int nb, int n, const float *_
 
       __syncthreads ();
 
-      const float ajj = rb[j];
+      const float a0 = r0[j], b0 = r0[j + 1], i0 = -_rcp_approx (a0), l = b0 * i0, a1 = fmaf (l, b0, r1[j + 1]);
 
-      if (!(ajj > 0.0f))
+      if (!(a0 > 0.0f) || !(a1 > 0.0f))
       {
-        fail = j + 1;
+        fail = (a0 > 0.0f) ? j + 2 : j + 1;
         break;
       }
 
-      const float inv = -_rcp_approx (ajj);
-      float rc[4], ac[4];
+      const float i1 = -_rcp_approx (a1);
+      float c0v[4], c1v[4], d0v[4], d1v[4];
 
-      if (ty == jj)
-        piv[p] = ajj;
+      if ((ty & ~1) == jj)
+        piv[p] = (ty & 1) ? a1 : a0;
 
 #pragma unroll
       for (int q = 0; q < 4; q++)
       {
-        rc[q] = (q >= p) ? rb[tx + 16 * q] : 0.0f;
-        ac[q] = rb[PB + tx + 16 * q];
+        c0v[q] = (q >= p) ? r0[tx + 16 * q] : 0.0f;
+        c1v[q] = (q >= p) ? fmaf (l, c0v[q], r1[tx + 16 * q]) : 0.0f;
+        d0v[q] = r0[PB + tx + 16 * q];
+        d1v[q] = fmaf (l, d0v[q], r1[PB + tx + 16 * q]);
       }
 
 #pragma unroll
       for (int pp = p; pp < 4; pp++)
       {
-        const int r   = ty + 16 * pp;
-        const float t = (r > j) ? rb[r] * inv : 0.0f;
+        const int r    = ty + 16 * pp;
+        const float v0 = r0[r], v1 = fmaf (l, v0, r1[r]);
+        const float t0 = (r > j) ? v0 * i0 : 0.0f, t1 = (r > j + 1) ? v1 * i1 : 0.0f;
 
 #pragma unroll
         for (int q = pp; q < 4; q++)
-          s[pp][q] = fmaf (t, rc[q], s[pp][q]);
+          s[pp][q] = fmaf (t1, c1v[q], fmaf (t0, c0v[q], s[pp][q]));
 
 #pragma unroll
         for (int q = 0; q < 4; q++)
-          a[pp][q] = fmaf (t, ac[q], a[pp][q]);
+          a[pp][q] = fmaf (t1, d1v[q], fmaf (t0, d0v[q], a[pp][q]));
       }
     }
 
