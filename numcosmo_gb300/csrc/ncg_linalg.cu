@@ -463,7 +463,8 @@ _stage_block (T (*S)[B + 1], const T *__restrict__ A, int ld, int r0, int c0, in
  * shared-memory trips and two reciprocals each), which every CTA walks for itself:
  * as two launches, the factor and then the columns against it, a panel took
  * 10 + 11 us (24 + 27 with the row scaled on the chain and a pack through FP64),
- * row by row in one 14.7 us; 10.8 us so (mean over the panels at n = 3000).  pk (may be NULL): the panel as the tensor-core update's operand. */
+ * row by row in one 14.7 us; 10.8 us so (mean over the panels at n = 3000).  pk
+ * (may be NULL): the panel as the tensor-core update's operand. */
 __device__ __forceinline__ float
 _rcp_approx (float x)
 {
@@ -1044,13 +1045,13 @@ ncg_launch_pcg_matvec (const double *A, int nrows, int n, const int32_t *P, int 
 /* ---- chained triangular solves of the FP32 preconditioner ----------------
  *
  * z = D (R^T R)^{-1} D r, one launch per triangular solve instead of one per
- * 64-row block.  Each CTA takes the next block from a ticket counter, so every
+ * block of SB rows.  Each CTA takes the next block from a ticket counter, so every
  * block it waits for belongs to a CTA that is already running and the launch
  * cannot deadlock whatever the residency.  While the blocks before its own
- * finish, a CTA streams its off-diagonal 64 x 64 tiles of R (the loads do not
+ * finish, a CTA streams its off-diagonal SB x SB tiles of R (the loads do not
  * depend on the waits), then applies the inverse of its diagonal block
  * (ncg_launch_trinv_diag_f32, once per factorisation).  A block publishes
- * each of its 64 values as one 64-bit word (value, epoch): a single-copy
+ * each of its values as one 64-bit word (value, epoch): a single-copy
  * atomic store that carries its own validity, so a reader polls the value
  * itself (one memory round trip, no flag and no fence).  The epoch is unique
  * to the launch (the host counts launches; the words are zeroed when the
@@ -1061,8 +1062,12 @@ ncg_launch_pcg_matvec (const double *A, int nrows, int n, const int32_t *P, int 
  * launches (the last CTA to finish clears them).  A wait gives up after
  * CS_SPIN polls, sets *err = 1 and sync[2], and the launch goes on with what
  * it has, so it always ends; a later wait that sees sync[2] does not spin. */
-#define SB 64     /* block of the solves */
-#define CS_TH 128
+/* The block of the solves.  A step is a memory round trip and two small products
+ * whatever the block: with 64 rows, 71 and 87 us at n = 3000 (17 and 18 at 512),
+ * with 128 and the half rows of the inverse in registers 40 and 44 us (10 and
+ * 10); the inverses then take 16 instead of 9 us, once per factorisation. */
+#define SB 128
+#define CS_TH 256
 #define CS_SPIN (1 << 21)
 
 __device__ __forceinline__ unsigned long long
@@ -1116,6 +1121,42 @@ _cs_get (const unsigned long long *w, uint32_t epoch, int32_t *sync, double *err
   return __uint_as_float ((uint32_t) x);
 }
 
+/* the values of words w[0], w[32], w[64] and w[96] below w[n], polled together: one
+ * after the other each costs a memory round trip */
+__device__ __forceinline__ void
+_cs_get4 (const unsigned long long *w, int n, float (&v)[4], uint32_t epoch, int32_t *sync, double *err)
+{
+  unsigned long long x[4];
+  int k = 0;
+
+  for (;;)
+  {
+    bool all = true;
+
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      x[q] = (32 * q < n) ? _ld_relaxed64 (w + 32 * q) : (unsigned long long) epoch << 32;
+
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      all = all && (uint32_t) (x[q] >> 32) == epoch;
+
+    if (all)
+      break;
+
+    if (++k > CS_SPIN || ((k & 255) == 0 && _ld_relaxed32 (sync + 2) != 0))
+    {
+      atomicExch (sync + 2, 1);
+      *err = 1.0;
+      break;
+    }
+  }
+
+#pragma unroll
+  for (int q = 0; q < 4; q++)
+    v[q] = __uint_as_float ((uint32_t) x[q]);
+}
+
 /* count the CTA as finished; the last one clears the ticket and the counters */
 __device__ __forceinline__ void
 _cs_finish (int32_t *sync, int tid)
@@ -1130,68 +1171,174 @@ _cs_finish (int32_t *sync, int tid)
   }
 }
 
-/* V_i = (U_ii^T)^{-1}, lower triangular, for each 64 x 64 diagonal block of the
- * upper factor U (zero outside the nb x nb triangle of a partial last block);
- * thread c solves for column c in registers, as the panel solve does (36 us
- * with the column in shared memory and a division per row) */
-__global__ void __launch_bounds__ (SB)
+/* V_i = (U_ii^T)^{-1}, lower triangular, for each SB x SB diagonal block of the
+ * upper factor U (zero outside the nb x nb triangle of a partial last block).
+ * With U_ii = [U11 U12; 0 U22]: V11 and V22 by substitution, thread c column c
+ * in registers as the panel solve does it (36 us with the column in shared
+ * memory and a division per row), then V21 = -V22 (U12^T V11), two 64 x 64
+ * products of 4 x 4 outputs a thread. */
+#define TI 64
+
+__global__ void __launch_bounds__ (256)
 _trinv_diag_kernel (const float *__restrict__ U, int n, float *__restrict__ V)
 {
-  __shared__ __align__ (16) float S[SB][SB];
-  __shared__ float ri[SB];
-  const int i = blockIdx.x, kb = i * SB, nb = (n - kb < SB) ? n - kb : SB, c = threadIdx.x;
-  float x[SB];
+  __shared__ __align__ (16) float S[2][TI][TI];   /* U11, U22, then V11, V22^T */
+  __shared__ __align__ (16) float T[TI][TI];      /* 1 / diagonal, then U12, then U12^T V11 */
+  const int i = blockIdx.x, kb = i * SB, nb = (n - kb < SB) ? n - kb : SB, tid = threadIdx.x;
+  float *Vi   = V + (size_t) i * SB * SB;
 
 #pragma unroll 16
-  for (int r = 0; r < SB; r++)
-    S[r][c] = (r < nb && c < nb && c >= r) ? U[(size_t) (kb + r) * n + kb + c] : 0.0f;
+  for (int e = tid; e < 2 * TI * TI; e += 256)
+  {
+    const int h = e / (TI * TI), r = (e / TI) % TI, c = e % TI;
 
-  ri[c] = (c < nb) ? __frcp_rn (S[c][c]) : 0.0f;
-
-#pragma unroll
-  for (int r = 0; r < SB; r++)
-    x[r] = (r == c) ? 1.0f : 0.0f;
+    S[h][r][c] = (h * TI + c < nb && c >= r) ? U[(size_t) (kb + h * TI + r) * n + kb + h * TI + c] : 0.0f;
+  }
 
   __syncthreads ();
 
-#pragma unroll
-  for (int r = 0; r < SB; r++)
+  if (tid < SB)
+    T[0][tid] = (tid < nb) ? __frcp_rn (S[tid / TI][tid % TI][tid % TI]) : 0.0f;
+
+  __syncthreads ();
+
+  const int h = (tid / TI) & 1, c = tid % TI;
+  float x[TI];
+
+  if (tid < SB)
   {
-    x[r] *= ri[r];
-
-    const float t = -x[r];
+#pragma unroll
+    for (int r = 0; r < TI; r++)
+      x[r] = (r == c) ? 1.0f : 0.0f;
 
 #pragma unroll
-    for (int m = (r + 1) / 4 * 4; m < SB; m += 4)
+    for (int r = 0; r < TI; r++)
     {
-      const float4 v = *(const float4 *) &S[r][m];
+      x[r] *= T[0][h * TI + r];
 
-      if (m + 0 > r)
-        x[m + 0] = fmaf (v.x, t, x[m + 0]);
-      if (m + 1 > r)
-        x[m + 1] = fmaf (v.y, t, x[m + 1]);
-      if (m + 2 > r)
-        x[m + 2] = fmaf (v.z, t, x[m + 2]);
-      if (m + 3 > r)
-        x[m + 3] = fmaf (v.w, t, x[m + 3]);
+      const float t = -x[r];
+
+#pragma unroll
+      for (int m = (r + 1) / 4 * 4; m < TI; m += 4)
+      {
+        const float4 v = *(const float4 *) &S[h][r][m];
+
+        if (m + 0 > r)
+          x[m + 0] = fmaf (v.x, t, x[m + 0]);
+        if (m + 1 > r)
+          x[m + 1] = fmaf (v.y, t, x[m + 1]);
+        if (m + 2 > r)
+          x[m + 2] = fmaf (v.z, t, x[m + 2]);
+        if (m + 3 > r)
+          x[m + 3] = fmaf (v.w, t, x[m + 3]);
+      }
     }
   }
 
+  __syncthreads ();
+
+  if (tid < SB)
+  {
 #pragma unroll
-  for (int r = 0; r < SB; r++)
-    V[(size_t) i * SB * SB + r * SB + c] = x[r];
+    for (int r = 0; r < TI; r++)
+    {
+      Vi[(size_t) (h * TI + r) * SB + h * TI + c] = x[r];
+
+      if (h == 0)
+        S[0][r][c] = x[r];
+    }
+
+    /* V22 by columns, for the product's reads along a row */
+    if (h == 1)
+#pragma unroll
+      for (int r = 0; r < TI; r += 4)
+        *(float4 *) &S[1][c][r] = make_float4 (x[r], x[r + 1], x[r + 2], x[r + 3]);
+  }
+
+#pragma unroll
+  for (int e = tid; e < TI * TI; e += 256)
+  {
+    const int r = e / TI, cc = e % TI;
+
+    T[r][cc]                            = (TI + cc < nb) ? U[(size_t) (kb + r) * n + kb + TI + cc] : 0.0f;
+    Vi[(size_t) r * SB + TI + cc]       = 0.0f;
+  }
+
+  __syncthreads ();
+
+  /* rows 4 ty.., columns 4 tx..: first T = U12^T V11, then V21 = -V22 T */
+  const int tx = tid & 15, ty = tid >> 4;
+  float acc[4][4];
+
+  for (int pass = 0; pass < 2; pass++)
+  {
+    const float (*L)[TI] = pass ? S[1] : T, (*R)[TI] = pass ? T : S[0];
+
+#pragma unroll
+    for (int p = 0; p < 4; p++)
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        acc[p][q] = 0.0f;
+
+#pragma unroll 8
+    for (int k = 0; k < TI; k++)
+    {
+      const float4 l = *(const float4 *) &L[k][4 * ty], r = *(const float4 *) &R[k][4 * tx];
+      const float lv[4] = { l.x, l.y, l.z, l.w }, rv[4] = { r.x, r.y, r.z, r.w };
+
+#pragma unroll
+      for (int p = 0; p < 4; p++)
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+          acc[p][q] = fmaf (lv[p], rv[q], acc[p][q]);
+    }
+
+    __syncthreads ();
+
+#pragma unroll
+    for (int p = 0; p < 4; p++)
+    {
+      if (pass == 0)
+        *(float4 *) &T[4 * ty + p][4 * tx] = make_float4 (acc[p][0], acc[p][1], acc[p][2], acc[p][3]);
+      else
+        *(float4 *) &Vi[(size_t) (TI + 4 * ty + p) * SB + 4 * tx] =
+          make_float4 (-acc[p][0], -acc[p][1], -acc[p][2], -acc[p][3]);
+    }
+
+    __syncthreads ();
+  }
+}
+
+/* sv . Vr over 64 entries, four chains */
+__device__ __forceinline__ float
+_cs_dot (const float (&Vr)[SB / 2], const float *sv)
+{
+  float acc[4] = { 0.0f, 0.0f, 0.0f, 0.0f };
+
+#pragma unroll
+  for (int c = 0; c < SB / 2; c += 4)
+  {
+    const float4 b = *(const float4 *) (sv + c);
+
+    acc[0] = fmaf (Vr[c + 0], b.x, acc[0]);
+    acc[1] = fmaf (Vr[c + 1], b.y, acc[1]);
+    acc[2] = fmaf (Vr[c + 2], b.z, acc[2]);
+    acc[3] = fmaf (Vr[c + 3], b.w, acc[3]);
+  }
+
+  return (acc[0] + acc[1]) + (acc[2] + acc[3]);
 }
 
 /* U^T y = (float) (D r): block i, y_i = V_i ((D r)_i - sum_{j<i} U_ji^T y_j);
- * warp w owns rows 16w..16w+15 of each tile, lanes its two columns */
+ * warp w owns rows 16w..16w+15 of each tile, lanes four of its columns; thread
+ * (row, half) holds its half row of V_i in registers before its turn comes */
 __global__ void __launch_bounds__ (CS_TH)
 _fsolve_chain_kernel (const float *__restrict__ U, const float *__restrict__ V, const double *__restrict__ D,
                       const double *__restrict__ r, int n, unsigned long long *__restrict__ y, uint32_t epoch,
                       uint32_t pepoch, int32_t *__restrict__ sync, double *__restrict__ err)
 {
-  __shared__ float Vs[SB][SB + 1];
   __shared__ float part[CS_TH / 32][SB];
-  __shared__ float sv[SB];
+  __shared__ __align__ (16) float sv[SB];
   __shared__ int blk;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
 
@@ -1200,25 +1347,33 @@ _fsolve_chain_kernel (const float *__restrict__ U, const float *__restrict__ V, 
 
   __syncthreads ();
 
-  const int i = blk, kb = i * SB, nb = (n - kb < SB) ? n - kb : SB;
+  const int i = blk, kb = i * SB, nb = (n - kb < SB) ? n - kb : SB, vrow = tid >> 1, vh = (tid & 1) * (SB / 2);
+  float Vr[SB / 2];
 
-  for (int e = tid; e < SB * SB; e += CS_TH)
-    Vs[e / SB][e % SB] = V[(size_t) i * SB * SB + e];
+#pragma unroll
+  for (int c = 0; c < SB / 2; c += 4)
+  {
+    const float4 v = *(const float4 *) (V + (size_t) i * SB * SB + vrow * SB + vh + c);
 
-  const bool v0 = lane < nb, v1 = lane + 32 < nb;
-  float a0 = 0.0f, a1 = 0.0f;
+    Vr[c + 0] = v.x;
+    Vr[c + 1] = v.y;
+    Vr[c + 2] = v.z;
+    Vr[c + 3] = v.w;
+  }
+
+  const double bd = (tid < nb) ? D[kb + tid] * r[kb + tid] : 0.0;
+  float a[4]      = { 0.0f, 0.0f, 0.0f, 0.0f };
 
   for (int j = 0; j < i; j++)
   {
     const float *row = U + (size_t) (j * SB + wid * 16) * n + kb + lane;
-    float u0[16], u1[16];
+    float u[4][16];
 
 #pragma unroll
     for (int rr = 0; rr < 16; rr++)
-    {
-      u0[rr] = v0 ? row[(size_t) rr * n] : 0.0f;
-      u1[rr] = v1 ? row[(size_t) rr * n + 32] : 0.0f;
-    }
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        u[q][rr] = (lane + 32 * q < nb) ? row[(size_t) rr * n + 32 * q] : 0.0f;
 
     /* y_j of this warp's 16 rows: lane rr waits for row rr, then shares it */
     const float ym = (lane < 16) ? _cs_get (y + j * SB + wid * 16 + lane, epoch, sync, err) : 0.0f;
@@ -1228,41 +1383,44 @@ _fsolve_chain_kernel (const float *__restrict__ U, const float *__restrict__ V, 
     {
       const float yv = __shfl_sync (0xffffffffu, ym, rr);
 
-      a0 = fmaf (u0[rr], yv, a0);
-      a1 = fmaf (u1[rr], yv, a1);
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        a[q] = fmaf (u[q][rr], yv, a[q]);
     }
   }
 
-  part[wid][lane]      = a0;
-  part[wid][lane + 32] = a1;
+#pragma unroll
+  for (int q = 0; q < 4; q++)
+    part[wid][lane + 32 * q] = a[q];
 
   __syncthreads ();
 
   if (tid < SB)
   {
-    float b = 0.0f;
+    float b = (float) bd;
 
     if (tid < nb)
-      b = (float) (D[kb + tid] * r[kb + tid]) - (((part[0][tid] + part[1][tid]) + part[2][tid]) + part[3][tid]);
+    {
+      float t = 0.0f;
+
+#pragma unroll
+      for (int w = 0; w < CS_TH / 32; w++)
+        t += part[w][tid];
+
+      b -= t;
+    }
 
     sv[tid] = b;
   }
 
   __syncthreads ();
 
-  {
-    const int row = tid >> 1, h = (tid & 1) * 32;
-    float acc = 0.0f;
+  float acc = _cs_dot (Vr, sv + vh);
 
-#pragma unroll 8
-    for (int c = 0; c < 32; c++)
-      acc = fmaf (Vs[row][h + c], sv[h + c], acc);
+  acc += __shfl_xor_sync (0xffffffffu, acc, 1);
 
-    acc += __shfl_xor_sync (0xffffffffu, acc, 1);
-
-    if (h == 0 && row < nb)
-      _cs_put (y + kb + row, acc, pepoch);
-  }
+  if (vh == 0 && vrow < nb)
+    _cs_put (y + kb + vrow, acc, pepoch);
 
   _cs_finish (sync, tid);
 }
@@ -1274,8 +1432,8 @@ _bsolve_chain_kernel (const float *__restrict__ U, const float *__restrict__ V, 
                       uint32_t epoch, uint32_t pepoch, double *__restrict__ z, int32_t *__restrict__ sync,
                       double *__restrict__ err)
 {
-  __shared__ float Vs[SB][SB + 1];
-  __shared__ float sv[SB];
+  __shared__ __align__ (16) float sv[SB];
+  __shared__ float half[SB];
   __shared__ int blk;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int nbk = (n + SB - 1) / SB;
@@ -1285,39 +1443,45 @@ _bsolve_chain_kernel (const float *__restrict__ U, const float *__restrict__ V, 
 
   __syncthreads ();
 
+  /* column vrow of V_i, entries vh.. (the halves in warps of their own, so that
+   * the loads of V run along its rows) */
   const int i = blk, kb = i * SB, nb = (n - kb < SB) ? n - kb : SB, r0 = wid * 16;
+  const int vrow = tid & (SB - 1), vh = (tid / SB) * (SB / 2);
+  float Vr[SB / 2], p[16];
 
-  for (int e = tid; e < SB * SB; e += CS_TH)
-    Vs[e / SB][e % SB] = V[(size_t) i * SB * SB + e];
-
-  float p[16];
+#pragma unroll
+  for (int c = 0; c < SB / 2; c++)
+    Vr[c] = V[(size_t) i * SB * SB + (vh + c) * SB + vrow];
 
 #pragma unroll
   for (int rr = 0; rr < 16; rr++)
     p[rr] = 0.0f;
 
+  const double dz = (vrow < nb) ? D[kb + vrow] : 0.0;
+
   for (int j = nbk - 1; j > i; j--)
   {
     const int jb = j * SB, nbj = (n - jb < SB) ? n - jb : SB;
-    const bool v0 = lane < nbj, v1 = lane + 32 < nbj;
     const float *row = U + (size_t) (kb + r0) * n + jb + lane;
-    float u0[16], u1[16];
+    float u[4][16], xv[4];
 
 #pragma unroll
     for (int rr = 0; rr < 16; rr++)
     {
-      const bool ok = r0 + rr < nb;
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        u[q][rr] = (r0 + rr < nb && lane + 32 * q < nbj) ? row[32 * q] : 0.0f;
 
-      u0[rr] = (ok && v0) ? row[(size_t) rr * n] : 0.0f;
-      u1[rr] = (ok && v1) ? row[(size_t) rr * n + 32] : 0.0f;
+      row += n;
     }
 
-    const float x0 = v0 ? _cs_get (x + jb + lane, epoch, sync, err) : 0.0f;
-    const float x1 = v1 ? _cs_get (x + jb + lane + 32, epoch, sync, err) : 0.0f;
+    _cs_get4 (x + jb + lane, nbj - lane, xv, epoch, sync, err);
 
 #pragma unroll
     for (int rr = 0; rr < 16; rr++)
-      p[rr] = fmaf (u1[rr], x1, fmaf (u0[rr], x0, p[rr]));
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        p[rr] = fmaf (u[q][rr], xv[q], p[rr]);
   }
 
   /* sums over the lanes of 16 values: at each halving a lane keeps the half of
@@ -1348,21 +1512,18 @@ _bsolve_chain_kernel (const float *__restrict__ U, const float *__restrict__ V, 
 
   __syncthreads ();
 
+  float acc = _cs_dot (Vr, sv + vh);
+
+  if (vh != 0)
+    half[vrow] = acc;
+
+  __syncthreads ();
+
+  if (vh == 0 && vrow < nb)
   {
-    const int row = tid >> 1, h = (tid & 1) * 32;
-    float acc = 0.0f;
-
-#pragma unroll 8
-    for (int c = 0; c < 32; c++)
-      acc = fmaf (Vs[h + c][row], sv[h + c], acc);
-
-    acc += __shfl_xor_sync (0xffffffffu, acc, 1);
-
-    if (h == 0 && row < nb)
-    {
-      _cs_put (x + kb + row, acc, pepoch);
-      z[kb + row] = D[kb + row] * (double) acc;
-    }
+    acc += half[vrow];
+    _cs_put (x + kb + vrow, acc, pepoch);
+    z[kb + vrow] = dz * (double) acc;
   }
 
   _cs_finish (sync, tid);
@@ -1394,7 +1555,7 @@ ncg_launch_trinv_diag_f32 (const float *U, int n, float *V, cudaStream_t s)
   if (n <= 0)
     return cudaSuccess;
 
-  _trinv_diag_kernel<<<(n + SB - 1) / SB, SB, 0, s>>> (U, n, V);
+  _trinv_diag_kernel<<<(n + SB - 1) / SB, 256, 0, s>>> (U, n, V);
 
   return cudaGetLastError ();
 }
