@@ -18,6 +18,7 @@
 #include <stdint.h>
 
 #include "ncg_internal.h"
+#include "ncg_pdl.cuh"
 #include "ncg_syrk_tc.cuh"
 
 /* FP32 products (the mixed solver's A^T A below 1024 columns):
@@ -159,6 +160,12 @@ __global__ void __launch_bounds__ (256)
 _gemv_n_kernel (const double *__restrict__ A, int nrows, int lda, const int32_t *__restrict__ P, int np, double alpha,
                 const double *__restrict__ x, double beta, double *__restrict__ y)
 {
+  const size_t pdl0 = ncg_pdl_enter ();
+
+  A += pdl0;
+  P += pdl0;
+  x += pdl0;
+
   const int lane = threadIdx.x & 31;
   const int r    = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
 
@@ -197,6 +204,12 @@ __global__ void __launch_bounds__ (128)
 _gemv_t_partial_kernel (const double *__restrict__ A, int nrows, int lda, const int32_t *__restrict__ P, int np,
                         const double *__restrict__ x, int rows, double *__restrict__ part)
 {
+  const size_t pdl0 = ncg_pdl_enter ();
+
+  A += pdl0;
+  P += pdl0;
+  x += pdl0;
+
   const int a  = blockIdx.x * blockDim.x + threadIdx.x;
   const int rb = blockIdx.y;
 
@@ -223,6 +236,11 @@ __global__ void __launch_bounds__ (128)
 _gemv_t_final_kernel (const double *__restrict__ part, int nrb, int np, const double *__restrict__ b,
                       double *__restrict__ y)
 {
+  const size_t pdl0 = ncg_pdl_enter ();
+
+  part += pdl0;
+  b += pdl0;
+
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
 
   if (a >= np)
@@ -252,8 +270,8 @@ _gemv_t (const double *A, int nrows, int lda, const int32_t *P, int np, const do
 {
   const int rows = _gt_rows (nrows), nrb = (nrows + rows - 1) / rows;
 
-  _gemv_t_partial_kernel<<<dim3 ((np + 127) / 128, nrb), 128, 0, s>>> (A, nrows, lda, P, np, x, rows, part);
-  _gemv_t_final_kernel<<<(np + 127) / 128, 128, 0, s>>> (part, nrb, np, b, y);
+  ncg_pdl_launch (_gemv_t_partial_kernel, dim3 ((np + 127) / 128, nrb), 128, 0, s, A, nrows, lda, P, np, x, rows, part);
+  ncg_pdl_launch (_gemv_t_final_kernel, (np + 127) / 128, 128, 0, s, part, nrb, np, b, y);
 
   return cudaGetLastError ();
 }
@@ -262,8 +280,8 @@ static cudaError_t
 _gemv_n (const double *A, int nrows, int lda, const int32_t *P, int np, double alpha, const double *x, double beta,
          double *y, cudaStream_t s)
 {
-  _gemv_n_kernel<<<(unsigned) (((size_t) nrows * 32 + 255) / 256), 256, 0, s>>> (A, nrows, lda, P, np, alpha, x, beta,
-                                                                                y);
+  ncg_pdl_launch (_gemv_n_kernel, (unsigned) (((size_t) nrows * 32 + 255) / 256), 256, 0, s, A, nrows, lda, P, np,
+                  alpha, x, beta, y);
 
   return cudaGetLastError ();
 }
@@ -326,6 +344,12 @@ __global__ void
 _scale_vec_kernel (const int32_t *__restrict__ P, int np, const double *__restrict__ diagM,
                    double *__restrict__ Dsub, const double *__restrict__ b, double *__restrict__ bsub)
 {
+  const size_t pdl0 = ncg_pdl_enter ();
+
+  P += pdl0;
+  diagM += pdl0;
+  b += pdl0;
+
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
 
   if (a < np)
@@ -342,6 +366,12 @@ _gather_scaled_kernel (const float *__restrict__ M32, int n, const int32_t *__re
                        const double *__restrict__ Dsub, float shift, float *__restrict__ Msub,
                        float *__restrict__ dg)
 {
+  const size_t pdl0 = ncg_pdl_enter ();
+
+  M32 += pdl0;
+  P += pdl0;
+  Dsub += pdl0;
+
   const int a = blockIdx.y;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
 
@@ -376,8 +406,8 @@ ncg_launch_gather_scaled_f32 (const float *M32, int n, const int32_t *P, int np,
 
   dim3 g ((np + 255) / 256 < 8 ? (np + 255) / 256 : 8, np);
 
-  _scale_vec_kernel<<<(np + 255) / 256, 256, 0, s>>> (P, np, diagM, Dsub, b, bsub);
-  _gather_scaled_kernel<<<g, 256, 0, s>>> (M32, n, P, np, Dsub, (float) shift, Msub, dg);
+  ncg_pdl_launch (_scale_vec_kernel, (np + 255) / 256, 256, 0, s, P, np, diagM, Dsub, b, bsub);
+  ncg_pdl_launch (_gather_scaled_kernel, g, 256, 0, s, M32, n, P, np, Dsub, (float) shift, Msub, dg);
 
   return cudaGetLastError ();
 }
@@ -479,6 +509,10 @@ __global__ void __launch_bounds__ (256)
 _potrf_panel_f32_kernel (float *A, int ld, int kb, int nb, int n, const float *__restrict__ dg, int32_t *info,
                          float *pk)
 {
+  const size_t pdl0 = ncg_pdl_enter ();
+
+  dg += pdl0;
+
   __shared__ float row[2][2][2 * PB];
   __shared__ float X[PB][PB + 1];
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
@@ -629,6 +663,8 @@ __global__ void __launch_bounds__ (256)
 _potrf_update_f32_kernel (float *A, int ld, int kb, int nb, int off, int nn, float *__restrict__ dg,
                           const int32_t *info)
 {
+  (void) ncg_pdl_enter ();
+
   __shared__ __align__ (16) float As[PB][PB];
   __shared__ __align__ (16) float Bs[PB][PB];
   const int T_ = (nn + PB - 1) / PB;
@@ -741,8 +777,8 @@ ncg_launch_potrf_f32 (float *A, int n, int32_t *info, float *work, int cap, cuda
     const int nb  = (n - kb < PB) ? n - kb : PB, rest = n - kb - nb;
     const bool tc = rest >= POTRF_TC_MIN;
 
-    _potrf_panel_f32_kernel<<<rest > 0 ? (rest + PB - 1) / PB : 1, 256, 0, s>>> (A, n, kb, nb, n, dg, info,
-                                                                                tc ? work : NULL);
+    ncg_pdl_launch (_potrf_panel_f32_kernel, rest > 0 ? (rest + PB - 1) / PB : 1, 256, 0, s, A, n, kb, nb, n, dg, info,
+                    tc ? work : NULL);
 
     if (tc)
     {
@@ -755,7 +791,7 @@ ncg_launch_potrf_f32 (float *A, int n, int32_t *info, float *work, int cap, cuda
     {
       const int T_ = (rest + PB - 1) / PB;
 
-      _potrf_update_f32_kernel<<<T_ * (T_ + 1) / 2, 256, 0, s>>> (A, n, kb, nb, kb + nb, rest, dg, info);
+      ncg_pdl_launch (_potrf_update_f32_kernel, T_ * (T_ + 1) / 2, 256, 0, s, A, n, kb, nb, kb + nb, rest, dg, info);
     }
   }
 
@@ -943,6 +979,13 @@ _pcg_dots_kernel (const double *__restrict__ u, const double *__restrict__ v, co
                   const double *__restrict__ D, double *__restrict__ p, int n, double *__restrict__ sc,
                   double *__restrict__ part, int32_t *__restrict__ count)
 {
+  const size_t pdl0 = ncg_pdl_enter ();
+
+  u += pdl0;
+  v += pdl0;
+  w += pdl0;
+  D += pdl0;
+
   double s[3] = { 0.0, 0.0, 0.0 };
 
   for (int i = blockIdx.x * DOT_TH + threadIdx.x; i < n; i += gridDim.x * DOT_TH)
@@ -1002,6 +1045,12 @@ _pcg_step_kernel (double *__restrict__ x, double *__restrict__ r, double *__rest
                   const double *__restrict__ p, const double *__restrict__ q, const double *__restrict__ D, int n,
                   double *__restrict__ sc, double *__restrict__ part, int32_t *__restrict__ count)
 {
+  const size_t pdl0 = ncg_pdl_enter ();
+
+  p += pdl0;
+  q += pdl0;
+  D += pdl0;
+
   const double rz = sc[NCG_PCG_RZ], al = (rz > 0.0) ? rz / sc[NCG_PCG_PQ] : 0.0;
   double s[3] = { 0.0, 0.0, 0.0 };
 
@@ -1023,13 +1072,15 @@ _pcg_step_kernel (double *__restrict__ x, double *__restrict__ r, double *__rest
 __global__ void
 _pcg_dir_kernel (double *__restrict__ p, const double *__restrict__ z, int n, const double *sc)
 {
+  const size_t pdl0 = ncg_pdl_enter ();
+
+  z += pdl0;
+
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
 
   if (i < n)
     p[i] = fma (sc[NCG_PCG_BE], p[i], z[i]);
 }
-
-#define VB(n) (((n) + 255) / 256), 256
 
 /* q = A_P^T (A_P v) for a compact v on the set P (np entries), or b less it; A
  * nrows x n; yf: nrows-long work, part the transposed product's scratch */
@@ -1182,6 +1233,10 @@ _cs_finish (int32_t *sync, int tid)
 __global__ void __launch_bounds__ (256)
 _trinv_diag_kernel (const float *__restrict__ U, int n, float *__restrict__ V)
 {
+  const size_t pdl0 = ncg_pdl_enter ();
+
+  U += pdl0;
+
   __shared__ __align__ (16) float S[2][TI][TI];   /* U11, U22, then V11, V22^T */
   __shared__ __align__ (16) float T[TI][TI];      /* 1 / diagonal, then U12, then U12^T V11 */
   const int i = blockIdx.x, kb = i * SB, nb = (n - kb < SB) ? n - kb : SB, tid = threadIdx.x;
@@ -1337,6 +1392,13 @@ _fsolve_chain_kernel (const float *__restrict__ U, const float *__restrict__ V, 
                       const double *__restrict__ r, int n, unsigned long long *__restrict__ y, uint32_t epoch,
                       uint32_t pepoch, int32_t *__restrict__ sync, double *__restrict__ err)
 {
+  const size_t pdl0 = ncg_pdl_enter ();
+
+  U += pdl0;
+  V += pdl0;
+  D += pdl0;
+  r += pdl0;
+
   __shared__ float part[CS_TH / 32][SB];
   __shared__ __align__ (16) float sv[SB];
   __shared__ int blk;
@@ -1432,6 +1494,13 @@ _bsolve_chain_kernel (const float *__restrict__ U, const float *__restrict__ V, 
                       uint32_t epoch, uint32_t pepoch, double *__restrict__ z, int32_t *__restrict__ sync,
                       double *__restrict__ err)
 {
+  const size_t pdl0 = ncg_pdl_enter ();
+
+  U += pdl0;
+  V += pdl0;
+  D += pdl0;
+  y += pdl0;
+
   __shared__ __align__ (16) float sv[SB];
   __shared__ float half[SB];
   __shared__ int blk;
@@ -1555,7 +1624,7 @@ ncg_launch_trinv_diag_f32 (const float *U, int n, float *V, cudaStream_t s)
   if (n <= 0)
     return cudaSuccess;
 
-  _trinv_diag_kernel<<<(n + SB - 1) / SB, 256, 0, s>>> (U, n, V);
+  ncg_pdl_launch (_trinv_diag_kernel, (n + SB - 1) / SB, 256, 0, s, U, n, V);
 
   return cudaGetLastError ();
 }
@@ -1575,8 +1644,8 @@ ncg_launch_pcg_precond (const float *R, const float *V, const double *D, int np,
    * so its first dependent wait runs out (CS_SPIN polls) and reports */
   const uint32_t py = ncg_fault_take (NCG_FAULT_CHAIN_WAIT) ? ey ^ 0x80000000u : ey;
 
-  _fsolve_chain_kernel<<<nbk, CS_TH, 0, s>>> (R, V, D, r, np, y, ey, py, sync, err);
-  _bsolve_chain_kernel<<<nbk, CS_TH, 0, s>>> (R, V, D, y, np, x, ex, ex, z, sync, err);
+  ncg_pdl_launch (_fsolve_chain_kernel, nbk, CS_TH, 0, s, R, V, D, r, np, y, ey, py, sync, err);
+  ncg_pdl_launch (_bsolve_chain_kernel, nbk, CS_TH, 0, s, R, V, D, y, np, x, ex, ex, z, sync, err);
 
   return cudaGetLastError ();
 }
@@ -1608,13 +1677,13 @@ ncg_launch_pcg_dots (int mode, const double *u, const double *v, const double *w
   const int g    = _dots_grid (n);
 
   if (mode == 0)
-    _pcg_dots_kernel<0><<<g, DOT_TH, 0, s>>> (u, v, w, D, p, n, sc, part, count);
+    ncg_pdl_launch (_pcg_dots_kernel<0>, g, DOT_TH, 0, s, u, v, w, D, p, n, sc, part, count);
   else if (mode == 1)
-    _pcg_dots_kernel<1><<<g, DOT_TH, 0, s>>> (u, v, w, D, p, n, sc, part, count);
+    ncg_pdl_launch (_pcg_dots_kernel<1>, g, DOT_TH, 0, s, u, v, w, D, p, n, sc, part, count);
   else if (mode == 2)
-    _pcg_dots_kernel<2><<<g, DOT_TH, 0, s>>> (u, v, w, D, p, n, sc, part, count);
+    ncg_pdl_launch (_pcg_dots_kernel<2>, g, DOT_TH, 0, s, u, v, w, D, p, n, sc, part, count);
   else
-    _pcg_dots_kernel<3><<<g, DOT_TH, 0, s>>> (u, v, w, D, p, n, sc, part, count);
+    ncg_pdl_launch (_pcg_dots_kernel<3>, g, DOT_TH, 0, s, u, v, w, D, p, n, sc, part, count);
 
   return cudaGetLastError ();
 }
@@ -1626,7 +1695,7 @@ ncg_launch_pcg_step (double *x, double *r, double *rprev, const double *p, const
   double *part   = sc + NCG_PCG_NSC;
   int32_t *count = (int32_t *) (part + 3 * DOT_CTAS);
 
-  _pcg_step_kernel<<<_dots_grid (n), DOT_TH, 0, s>>> (x, r, rprev, p, q, D, n, sc, part, count);
+  ncg_pdl_launch (_pcg_step_kernel, _dots_grid (n), DOT_TH, 0, s, x, r, rprev, p, q, D, n, sc, part, count);
 
   return cudaGetLastError ();
 }
@@ -1634,7 +1703,7 @@ ncg_launch_pcg_step (double *x, double *r, double *rprev, const double *p, const
 extern "C" cudaError_t
 ncg_launch_pcg_dir (double *p, const double *z, int n, double *sc, cudaStream_t s)
 {
-  _pcg_dir_kernel<<<VB (n), 0, s>>> (p, z, n, sc);
+  ncg_pdl_launch (_pcg_dir_kernel, (n + 255) / 256, 256, 0, s, p, z, n, sc);
 
   return cudaGetLastError ();
 }

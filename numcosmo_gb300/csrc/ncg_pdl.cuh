@@ -1,0 +1,56 @@
+/*
+ * ncg_pdl.cuh -- launches that overlap the end of the kernel before them in the
+ * stream (programmatic dependent launch): in the chains of short kernels of the
+ * mixed weight fit the start of a grid, 1 to 2 us, is hidden behind its predecessor
+ * (fit d=12 N=4096 41.5 -> 38.4 ms, half-move d=8 N=512 3.8 -> 3.3 ms).  Kernels with
+ * most of an SM's shared memory are launched plainly: so launched, the FP64 fit's
+ * product and panel kernels took 38.4 instead of 32.7 ms, d=12 N=2048.
+ *
+ * A kernel launched by ncg_pdl_launch begins with ncg_pdl_enter (before any access
+ * to global memory): it returns once every kernel before it in the stream has
+ * finished and its writes can be seen, since each of those waited in the same way
+ * before it let the next one start.  Loads through `const T *__restrict__` may be
+ * moved by the compiler as if nothing could write there, also ahead of that wait:
+ * the zero that ncg_pdl_enter returns, added to such a pointer, ties its loads to
+ * the wait and leaves the pointer what it is to the compiler (hidden pointers cost
+ * the inverses' kernel twice its time, its loads no longer ran ahead of its stores).
+ */
+#ifndef NCG_PDL_CUH
+#define NCG_PDL_CUH
+
+#include <cuda_runtime.h>
+
+static __device__ __forceinline__ size_t
+ncg_pdl_enter (void)
+{
+  size_t zero;
+
+  asm volatile ("griddepcontrol.wait;\n\t"
+                "griddepcontrol.launch_dependents;\n\t"
+                "mov.u64 %0, 0;"
+                : "=l"(zero)::"memory");
+
+  return zero;
+}
+
+template <typename... K, typename... A>
+static cudaError_t
+ncg_pdl_launch (void (*kernel) (K...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args)
+{
+  cudaLaunchAttribute at[1];
+  cudaLaunchConfig_t cfg = {};
+
+  at[0].id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+
+  cfg.gridDim          = grid;
+  cfg.blockDim         = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream           = s;
+  cfg.attrs            = at;
+  cfg.numAttrs         = 1;
+
+  return cudaLaunchKernelEx (&cfg, kernel, args...);
+}
+
+#endif /* NCG_PDL_CUH */
