@@ -985,6 +985,36 @@ _nonfinite_kernel (const double *__restrict__ X, int64_t n, int32_t *flag)
     *(volatile int32_t *) flag = 1;
 }
 
+/* the same while the values move to dst (src: mapped host memory) */
+__global__ void __launch_bounds__ (256)
+_stage_points_kernel (const double *__restrict__ src, int64_t n, double *__restrict__ dst, int32_t *flag)
+{
+  const int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
+  int bad = 0;
+
+  if (i < n)
+  {
+    const double v = src[i];
+
+    dst[i] = v;
+    bad    = !isfinite (v);
+  }
+
+  if (__syncthreads_or (bad) && threadIdx.x == 0)
+    *(volatile int32_t *) flag = 1;
+}
+
+extern "C" cudaError_t
+ncg_launch_stage_points (const double *src, int64_t n, double *dst, int32_t *flag, cudaStream_t s)
+{
+  if (n <= 0)
+    return cudaSuccess;
+
+  _stage_points_kernel<<<(unsigned) ((n + 255) / 256), 256, 0, s>>> (src, n, dst, flag);
+
+  return cudaGetLastError ();
+}
+
 extern "C" cudaError_t
 ncg_launch_nonfinite (const double *X, int64_t n, int32_t *flag, cudaStream_t s)
 {

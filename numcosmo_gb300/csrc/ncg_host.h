@@ -9,6 +9,13 @@
 
 #include "ncg_internal.h"
 
+/* doubles of the points and of the results in a handle's mapped host memory, and
+ * where they lie behind its flags */
+#define NCG_IO_IN 8192
+#define NCG_IO_OUT 2048
+#define NCG_IO_OFFSET 64
+#define NCG_IO_BYTES (sizeof (double) * (NCG_IO_IN + NCG_IO_OUT))
+
 typedef struct ncg_caps
 {
   size_t X, Y, cov, U, Ui, lnnorm, w, c, wcum, pack64, Vg, packmx, knn, flag, ids, keys, st, scratch, q, qo, qi, f,
@@ -73,6 +80,8 @@ struct ncg_sd
   double tc_err;          /* its measured error on the kernel centres */
   int32_t *h_flag;        /* mapped pinned: error word of the last tensor-core launch */
   int32_t *d_flag_alias;  /* its device address, written by the merge kernel */
+  double *h_io;           /* mapped pinned: points (NCG_IO_IN) and results (NCG_IO_OUT) of a small host eval */
+  double *d_io;           /* its device address */
   uint8_t *dtcB;          /* tensor-core kernel tiles */
   size_t cap_tcB;
   uint8_t *dq64;          /* the FP64 form's tensor-core operand */

@@ -140,6 +140,7 @@ cudaError_t ncg_launch_dfma_peak (double *out, int blocks, int iters, cudaStream
 #define NCG_MAX_DEVICES 64
 cudaError_t ncg_raise_smem_limit (const void *fn, size_t bytes, int *limit);
 cudaError_t ncg_launch_nonfinite (const double *X, int64_t n, int32_t *flag, cudaStream_t s);
+cudaError_t ncg_launch_stage_points (const double *src, int64_t n, double *dst, int32_t *flag, cudaStream_t s);
 
 /* The mixed form whitens with FP32 arithmetic; its chi^2 error grows with the
  * infinity-norm condition number of the per-kernel whitening W'_i.  Above this
