@@ -1761,7 +1761,7 @@ ncg_sd_eval_m2lnp_device_noalloc (ncg_sd_t *sd, const double *d_X, uint64_t m, d
  * third of a call).  Up to NCG_IO_DIRECT points the FP64 kernel reads its few
  * coordinates there and the host looks for non-finite ones; more are moved by
  * the kernel that checks them.  One point, KDE d=4 n=1000: 36 -> 27 us; 1000
- * points 104 -> 97 us. */
+ * points 104 -> 97 us (24 and 93 with the launches overlapped, ncg_pdl.cuh). */
 #define NCG_IO_DIRECT 16
 
 static ncg_status_t

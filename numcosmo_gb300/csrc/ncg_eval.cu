@@ -12,6 +12,7 @@
 #include <stdint.h>
 
 #include "ncg_internal.h"
+#include "ncg_pdl.cuh"
 #include "ncg_eval_tiles.cuh"
 
 /* ------------------------------------------------------------------------ */
@@ -59,6 +60,12 @@ _eval64_kernel (const ncg_eval_args_t a, const double *__restrict__ Xq, const do
   constexpr int KC = NcgEv64<DP, KIND>::KC;
   __shared__ __align__ (16) double sm[KC * S];
   __shared__ double sc[KC];
+  const size_t pdl0 = ncg_pdl_enter ();
+
+  Xq   += pdl0;
+  pack += pdl0;
+  cvec += pdl0;
+  Vg   += pdl0;
 
   ncg_tile_eval64<DP, KIND, KERN, KC, EV64_WK> (a, Xq, pack, cvec, Vg, part, kper, blockIdx.x, blockIdx.y, sm, sc);
 }
@@ -80,7 +87,13 @@ _eval64_few_kernel (const ncg_eval_args_t a, const double *__restrict__ Xq, cons
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int64_t j = blockIdx.y;
   const int i0    = blockIdx.x * kper, i1 = min (a.n, i0 + kper);
+  const size_t pdl0 = ncg_pdl_enter ();
   double x[DP];
+
+  Xq   += pdl0;
+  pack += pdl0;
+  cvec += pdl0;
+  Vg   += pdl0;
 
   if (tid < DP)
     xs[tid] = (tid < a.d) ? Xq[j * a.d + tid] : 0.0;
@@ -164,6 +177,8 @@ _merge_kernel (const T2 *__restrict__ part, int nslices, int64_t m, double shift
   const int64_t j = (int64_t) blockIdx.x * 32 + lane;
   const bool in   = j < m;
   double G = NCG_LSE_EMPTY, S = 0.0;
+
+  part += ncg_pdl_enter ();
 
   if (in)
     for (int s = w; s < nslices; s += MG_TH / 32)
@@ -292,17 +307,13 @@ _run64 (const ncg_eval_args_t *a, const double *Xq, const double *pack64, const 
   const int64_t bx = (a->m + EV_THREADS / EV64_WK - 1) / (EV_THREADS / EV64_WK);
   const dim3 grid  = (a->m <= EV64_FEW) ? dim3 ((unsigned) ns, (unsigned) a->m) : dim3 ((unsigned) bx, (unsigned) ns);
 
-  fn<<<grid, EV_THREADS, 0, s>>> (*a, Xq, pack64, c, Vg, part, kp);
-
-  cudaError_t e = cudaGetLastError ();
+  cudaError_t e = ncg_pdl_launch (fn, grid, EV_THREADS, 0, s, *a, Xq, pack64, c, Vg, part, kp);
 
   if (e != cudaSuccess)
     return e;
 
-  _merge_kernel<double2><<<(unsigned) ((a->m + 31) / 32), MG_TH, 0, s>>> (part, ns, a->m, a->final_shift, NULL,
-                                                                          a->d_ln_href, linear, out);
-
-  return cudaGetLastError ();
+  return ncg_pdl_launch (_merge_kernel<double2>, (unsigned) ((a->m + 31) / 32), MG_TH, 0, s, part, ns, a->m,
+                         a->final_shift, (const double *) NULL, a->d_ln_href, linear, out);
 }
 
 #define EV64_NS_MAX 4096

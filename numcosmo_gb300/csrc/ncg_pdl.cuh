@@ -2,7 +2,9 @@
  * ncg_pdl.cuh -- launches that overlap the end of the kernel before them in the
  * stream (programmatic dependent launch): in the chains of short kernels of the
  * mixed weight fit the start of a grid, 1 to 2 us, is hidden behind its predecessor
- * (fit d=12 N=4096 41.5 -> 38.4 ms, half-move d=8 N=512 3.8 -> 3.3 ms).  Kernels with
+ * (fit d=12 N=4096 41.5 -> 38.4 ms, half-move d=8 N=512 3.8 -> 3.3 ms), and between
+ * the FP64 eval and its merge (one point 27.0 -> 24.4 us, 1000 points 97.0 -> 92.7 us,
+ * KDE d=4 n=1000).  Kernels with
  * most of an SM's shared memory are launched plainly: so launched, the FP64 fit's
  * product and panel kernels took 38.4 instead of 32.7 ms, d=12 N=2048.
  *
