@@ -23,11 +23,11 @@
  * the first tile, factors the next diagonal block while the others update.  The
  * right-hand side rides along as one more column, which leaves U^{-T} b at the
  * end; _posv_back_kernel solves U x = U^{-T} b in one launch.
- * Measured at n = 1700 (n = 4096): panel 12 us, update 23 us with the diagonal
- * block's 30 beside it (82 us), U x = y 182 us (431 us); the whole solve 2.5 ms
- * (7.4 ms).  The plain form took 90 (diagonal) + 120 (panel) + 110 us (update)
- * per 64 rows at n = 1700 and 33 us per 64 rows for each triangle, 10 ms.  Left:
- * the chain of 32 pivots (30 us, the bound below n = 1500), the epilogue of the
+ * Measured at n = 1700 (n = 4096): panel 10 us (12), update 23 us with the
+ * diagonal block's 27 beside it (78 us), U x = y 175 us (413 us); the whole solve
+ * 2.0 ms (6.5 ms).  The plain form took 90 (diagonal) + 120 (panel) + 110 us
+ * (update) per 64 rows at n = 1700 and 33 us per 64 rows for each triangle, 10 ms.
+ * Left: the chain of 32 pivots (the bound below n = 1900), the epilogue of the
  * update above.
  */
 #include <cuda_fp16.h>
@@ -164,20 +164,41 @@ _pack63_kernel (const double *__restrict__ A, int r0, int r1, int ncols, int nch
 
 /* ---------------------------------------------------------- diagonal blocks */
 
-/* The 32 x 32 diagonal block of a panel, factored by four warps (one per SM
- * sub-partition).  Warp w holds the rows w mod 4, lane = column; step j publishes
- * row j, one barrier, and every row r below takes t_r = s_jr / s_jj times it
- * off.  The quotient comes from the FP32 reciprocal of the pivot, a Newton step
- * and one correction by its remainder, so it is rounded like a division (the
- * pivot of a repeated column is then exactly zero) at 5 FP64 instructions, 4 of
- * them on the chain; the moves between FP32 and FP64 are integer instructions
+/* The 32 x 32 diagonal block of a panel, factored by 16 warps, lane = column.
+ * Warp 0 walks the chain of pivots: with row j finished it publishes the row and
+ * the multipliers t_r = s_jr / s_jj, and takes t_(j+1) times it off row j + 1.  Ten
+ * others, on the SM's other three sub-partitions so that their FP64 instructions
+ * do not hold up the chain's, keep three rows each and take every step off them;
+ * row r goes back to the chain after step r - 2.  So the chain is a reciprocal and 4
+ * FP64 instructions (of 64 cycles each) per pivot, and the updates run beside it.
+ * The quotient comes from the pivot's reciprocal in FP32 and one correction by its
+ * remainder, so it is rounded like a division (the pivot of a repeated column is
+ * then exactly zero); the moves between FP32 and FP64 are integer instructions
  * (conversions, divisions and square roots hold the FP64 pipe).  The rows are
- * scaled by 1 / sqrt (s_jj) at the end. */
+ * scaled by 1 / sqrt (s_jj) at the end.  16 us from the first tile's end to the
+ * stores (19 with four warps that each took their share of every step before the
+ * next pivot). */
+#define DG_WARPS 16
+
 struct DiagSmem
 {
-  double S[P_K][P_K + 1];
-  double row[2][P_K], piv[P_K], root[P_K], rinv[P_K];
+  double S[P_K][P_K + 1];           /* the block; row j as it is handed back, then final */
+  double T[P_K][P_K];               /* the multipliers of row j */
+  double root[P_K], rinv[P_K];
+  uint64_t full[P_K], next[P_K];    /* row j final, with its multipliers; row j taken through step j - 2 */
+  int stop;                         /* not positive, or a wait that gave up */
 };
+
+/* by at least 64 threads, before the CTA's next barrier */
+__device__ __forceinline__ void
+_diag_init (DiagSmem &d, int tid)
+{
+  if (tid < 2 * P_K)
+    _mbar_init (tid < P_K ? &d.full[tid] : &d.next[tid - P_K], 1);
+
+  if (tid == 0)
+    d.stop = 0;
+}
 
 __device__ __forceinline__ void
 _bar_named (int id, int threads)
@@ -185,26 +206,33 @@ _bar_named (int id, int threads)
   asm volatile ("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
-/* near 1 / x (22 bits) for a positive x */
+/* 1 / x to 2^-43 for a positive x, in FP32 and integer instructions: the FP32
+ * reciprocal r0 of the mantissa's leading 24 bits, its residual with the next 23
+ * taken in, and r1 = r0 (1 - f r0) added to r0 in units of its binade as a double
+ * (1 / f stays in [1/2, 1], so the sum leaves that binade by the error only).  A
+ * Newton step in FP64 gave as much for two more instructions of 64 cycles on the
+ * pivots' chain. */
 __device__ __forceinline__ double
-_recip22 (double x)
+_recip44 (double x)
 {
-  const int hi = __double2hiint (x), ef = (hi >> 20) & 0x7ff;
+  const int hi = __double2hiint (x), lo = __double2loint (x), ef = (hi >> 20) & 0x7ff;
 
   if (ef < 64 || ef > 1980)
     return 1.0 / x;
 
-  /* mantissa in [1, 2) as a float, truncated */
-  const float f = __int_as_float (0x3f800000 | ((hi & 0xfffff) << 3) | (int) ((uint32_t) __double2loint (x) >> 29));
-  float r;
+  /* mantissa in [1, 2): f + g, f its leading 24 bits */
+  const float f = __int_as_float (0x3f800000 | ((hi & 0xfffff) << 3) | (int) ((uint32_t) lo >> 29));
+  const float g = (__int_as_float (0x3f800000 | ((lo >> 6) & 0x7fffff)) - 1.0f) * 0x1p-23f;
+  float r0;
 
-  asm ("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(f));
+  asm ("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(f));
+  r0 = fminf (r0, 0x1.fffffep-1f);
 
-  /* r in (0.5, 1] as a double, times 2^(1023 - ef) */
-  const int rb = __float_as_int (r);
-  const int re = ((rb >> 23) & 0xff) - 127 + 1023 + (1023 - ef);
+  const float r1 = r0 * fmaf (-g, r0, fmaf (-f, r0, 1.0f));
+  const int rb   = __float_as_int (r0);
 
-  return __hiloint2double ((re << 20) | ((rb & 0x7fffff) >> 3), rb << 29);
+  return __longlong_as_double (__double_as_longlong (__hiloint2double (((2045 - ef) << 20) | ((rb & 0x7fffff) >> 3), rb << 29)) +
+                               __float2int_rn (r1 * 0x1p+53f));
 }
 
 /* a / u from ri near 1 / u, its remainder put right once: rounded like a division */
@@ -218,78 +246,146 @@ _scaled (double a, double u, double ri)
 
 /* d.S in, the factor (nb x nb, at A with leading dimension ld) out; Lt[j][r] =
  * s_jr / s_jj for r > j, root and rd (1 / root) for the panel's other columns.
- * Threads w = 0..3 x 32 lanes with named barrier `bar`. */
+ * DG_WARPS warps w with named barrier `bar`; d set up by _diag_init. */
 __device__ __forceinline__ void
 _diag_factor (DiagSmem &d, int w, int lane, int bar, int nb, double *__restrict__ A, int ld, double *__restrict__ Lt,
               double *__restrict__ root, double *__restrict__ rd, int col0, int32_t *__restrict__ info)
 {
-  double s[8];
+  volatile int *stop = &d.stop;
+  const int b        = (w >> 2) * 3 + (w & 3) - 1;
   int fail = 0;
 
   /* the identity past nb */
-#pragma unroll
-  for (int p = 0; p < 8; p++)
+  auto in = [&] (int r) -> double {
+    return (r < nb && lane < nb) ? ((lane >= r) ? d.S[r][lane] : 0.0) : (r == lane ? 1.0 : 0.0);
+  };
+
+  if (w == 0)
   {
-    const int r = w + 4 * p;
+    double row = in (0);
 
-    s[p] = (r < nb && lane < nb) ? ((lane >= r) ? d.S[r][lane] : 0.0) : (r == lane ? 1.0 : 0.0);
-  }
-
-#pragma unroll
-  for (int p0 = 0; p0 < 8; p0++)
-    for (int wj = 0; wj < 4; wj++)
+#pragma unroll 1
+    for (int j = 0; j < P_K; j++)
     {
-      const int j = 4 * p0 + wj;
-      double *rb  = d.row[j & 1];
-
-      if (fail)
-        break;
-
-      if (w == wj)
-        rb[lane] = s[p0];
-
-      _bar_named (bar, 128);
-
-      const double pv = rb[j], dj = rb[lane];
+      const double pv = __shfl_sync (0xffffffffu, row, j);
       const int ph    = __double2hiint (pv);
 
       /* not positive, inf or NaN, by the high word (an FP64 compare is 64 cycles) */
       if ((uint32_t) (ph - 1) >= 0x7fefffffu && !(ph == 0 && __double2loint (pv) != 0))
       {
-        fail = j + 1;
+        fail  = j + 1;
+        *stop = 1;
+        __syncwarp ();
+
+        /* nobody waits for what does not come */
+        if (lane >= j)
+          _mbar_arrive (&d.full[lane]);
+
         break;
       }
 
-      const double y0 = _recip22 (pv), q = dj * y0, e = fma (-pv, y0, 1.0), t0 = fma (q, e, q);
-      const double t  = fma (fma (-t0, pv, dj), y0, t0);
+      const double y0 = _recip44 (pv), q = row * y0, t = fma (fma (-q, pv, row), y0, q);
+      double nx       = 0.0;
 
-      if (w == wj)
+      /* only here: row j + 1 comes back a step's update after row j - 1 went out,
+       * while this step's quotient is worked out */
+      if (j == 0)
+        nx = in (1);
+      else if (j < P_K - 1)
       {
-        Lt[j * P_K + lane] = t;
+        if (!__all_sync (0xffffffffu, _mbar_wait (&d.next[j + 1], 0, stop)))
+          break;
 
-        if (lane == 0)
-          d.piv[j] = pv;
+        nx = d.S[j + 1][lane];
       }
 
-#pragma unroll
-      for (int p = p0; p < 8; p++)
-        if (p > p0 || w > wj)
-          s[p] = fma (-__shfl_sync (0xffffffffu, t, w + 4 * p), dj, s[p]);
+      const double rn = fma (-__shfl_sync (0xffffffffu, t, (j + 1) & 31), row, nx);
+
+      d.S[j][lane] = row;
+      d.T[j][lane] = t;
+      __syncwarp ();
+
+      if (lane == 0)
+        _mbar_arrive (&d.full[j]);
+
+      Lt[j * P_K + lane] = t;
+      row                = rn;
+    }
+  }
+  else if ((w & 3) != 0 && b < 10)
+  {
+    const int ra = 2 + b, rb = 21 - b, rc = 22 + b;
+    double sa = in (ra), sb = in (rb), sc = in (rc), dj = 0.0;
+    int j   = 0;
+    bool go = true;
+
+    auto wait = [&] () {
+      go = __all_sync (0xffffffffu, _mbar_wait (&d.full[j], 0, stop) && !*stop);
+      dj = d.S[j][lane];
+    };
+
+    auto back = [&] (int r, double v) {
+      d.S[r][lane] = v;
+      __syncwarp ();
+
+      if (lane == 0)
+        _mbar_arrive (&d.next[r]);
+    };
+
+#pragma unroll 1
+    for (; j <= ra - 2 && go; j++)
+    {
+      wait ();
+      sa = fma (-d.T[j][ra], dj, sa);
+
+      if (j == ra - 2)
+        back (ra, sa);
+
+      sb = fma (-d.T[j][rb], dj, sb);
+      sc = fma (-d.T[j][rc], dj, sc);
     }
 
-  if (fail)
+#pragma unroll 1
+    for (; j <= rb - 2 && go; j++)
+    {
+      wait ();
+      sb = fma (-d.T[j][rb], dj, sb);
+
+      if (j == rb - 2)
+        back (rb, sb);
+
+      sc = fma (-d.T[j][rc], dj, sc);
+    }
+
+#pragma unroll 1
+    for (; j <= rc - 2 && go; j++)
+    {
+      wait ();
+      sc = fma (-d.T[j][rc], dj, sc);
+    }
+
+    if (go)
+      back (rc, sc);
+  }
+
+  _bar_named (bar, DG_WARPS * 32);
+
+  if (*stop)
   {
     if (w == 0 && lane == 0)
-      atomicCAS (info, 0, col0 + fail);
+    {
+      if (fail)
+        atomicCAS (info, 0, col0 + fail);
+      else
+        atomicExch (info, -1);
+    }
 
     return;
   }
 
-  _bar_named (bar, 128);
-
   if (w == 0)
   {
-    const double u = sqrt (d.piv[lane]), ri = 1.0 / u;
+    const double u = sqrt (d.S[lane][lane]), ri = 1.0 / u;
 
     d.root[lane] = u;
     d.rinv[lane] = ri;
@@ -299,16 +395,12 @@ _diag_factor (DiagSmem &d, int w, int lane, int bar, int nb, double *__restrict_
       rd[lane] = ri;
   }
 
-  _bar_named (bar, 128);
+  _bar_named (bar, DG_WARPS * 32);
 
 #pragma unroll
-  for (int p = 0; p < 8; p++)
-  {
-    const int r = w + 4 * p;
-
+  for (int r = w; r < P_K; r += DG_WARPS)
     if (r < nb && lane < nb && lane >= r)
-      A[(size_t) r * ld + lane] = (lane == r) ? d.root[r] : _scaled (s[p], d.root[r], d.rinv[r]);
-  }
+      A[(size_t) r * ld + lane] = (lane == r) ? d.root[r] : _scaled (d.S[r][lane], d.root[r], d.rinv[r]);
 }
 
 /* ----------------------------------------------------- the symmetric product */
@@ -319,7 +411,7 @@ _diag_factor (DiagSmem &d, int w, int lane, int bar, int nb, double *__restrict_
 #define S_B_LBO (P_NS * S_B_UNIT)
 #define S_B_BYTES (4 * S_B_LBO)
 #define S_EPI_WARP0 2
-#define S_EPI_WARPS 16
+#define S_EPI_WARPS 16                       /* DG_WARPS of them factor the diagonal block */
 #define S_THREADS ((S_EPI_WARP0 + S_EPI_WARPS) * 32)
 #define S_TMEM (P_NS * P_N)                  /* 224 columns, two accumulators */
 
@@ -461,8 +553,13 @@ _syrk64_kernel (const S64Params p)
     }
 
     _mbar_init (&sm.done, 1);
-    asm volatile ("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+
+  if (p.Lt != NULL && blockIdx.x == 0 && warp >= S_EPI_WARP0)
+    _diag_init (sm.diag, threadIdx.x - S_EPI_WARP0 * 32);
+
+  if (warp != 1)
+    asm volatile ("fence.mbarrier_init.release.cluster;" ::: "memory");
 
   if (warp == 1)
   {
@@ -706,7 +803,7 @@ _syrk64_kernel (const S64Params p)
 
         _bar_named (1, S_EPI_WARPS * 32);
 
-        if (wg == 0 && *(volatile int *) &sm.ndiag == S_EPI_WARPS)
+        if (*(volatile int *) &sm.ndiag == S_EPI_WARPS)
           _diag_factor (sm.diag, warp - S_EPI_WARP0, lane, 2, min (p.nn, P_K), p.C, p.ldc, p.Lt, p.root, p.rd, p.col0,
                         p.err);
       }
@@ -729,67 +826,77 @@ _syrk64_kernel (const S64Params p)
 /* ------------------------------------------------------------------ panels */
 
 /* One panel: rows kb .. kb + nb of the columns right of its diagonal block
- * (and of b, column n), from the block's multipliers Lt.  32 columns per CTA,
- * lane = column, warp w holds the rows w mod 4; step j publishes the finished row j
- * and the rows below take it off.  Then the rows are scaled, written and packed
- * as digits with their columns' exponents. */
+ * (and of b, column n), from the block's multipliers Lt.  16 columns per CTA: a
+ * lane has column lane mod 16 and the rows 2w + lane / 16 mod 8, so that an FP64
+ * instruction takes two rows and the columns spread over twice as many SMs (32
+ * columns with a row per instruction: 13 us, now 10 us at n = 1700).  Step j
+ * publishes the finished row j and the rows below take it off.  Then the rows are
+ * scaled, written and packed as digits with their columns' exponents. */
 #define PP_TH 128
+#define PP_C 16
 
 __global__ void __launch_bounds__ (PP_TH)
 _posv_panel_kernel (double *__restrict__ A, int n, double *__restrict__ b, int kb, int nb,
                     const double *__restrict__ Lt, const double *__restrict__ root, uint8_t *__restrict__ pk,
                     int32_t *__restrict__ ex, const int32_t *__restrict__ info)
 {
-  __shared__ double L[P_K][P_K], row[2][32];
-  __shared__ int exm[4][32];
-  __shared__ __align__ (16) uint16_t dig[P_NS][32][P_K + 8];
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int rel = blockIdx.x * 32 + lane, col = kb + nb + rel;
-  double a[8];
+  __shared__ double L[P_K][P_K], row[2][PP_C];
+  __shared__ int exm[8][PP_C];
+  __shared__ __align__ (16) uint16_t dig[P_NS][PP_C][P_K + 8];
+  const int tid = threadIdx.x, lane = tid & 31, c = tid & (PP_C - 1), r0 = tid / PP_C;
+  const int rel = blockIdx.x * PP_C + c, col = kb + nb + rel;
+  double a[4];
 
   if (*(volatile const int32_t *) info)
     return;
 
 #pragma unroll
-  for (int p = 0; p < 8; p++)
+  for (int p = 0; p < 4; p++)
   {
-    const int r = w + 4 * p;
+    const int r = r0 + 8 * p;
 
     a[p] = (r < nb && col <= n) ? ((col < n) ? A[(size_t) (kb + r) * n + col] : b[kb + r]) : 0.0;
   }
 
 #pragma unroll
   for (int p = 0; p < 8; p++)
-    L[w + 4 * p][lane] = Lt[(w + 4 * p) * P_K + lane];
+    L[(tid >> 5) + 4 * p][lane] = Lt[((tid >> 5) + 4 * p) * P_K + lane];
 
 #pragma unroll
-  for (int p0 = 0; p0 < 8; p0++)
+  for (int p0 = 0; p0 < 4; p0++)
 #pragma unroll
-    for (int wj = 0; wj < 4; wj++)
+    for (int jj = 0; jj < 8; jj++)
     {
-      const int j = 4 * p0 + wj;
+      const int j = 8 * p0 + jj;
 
-      if (w == wj)
-        row[j & 1][lane] = a[p0];
+      if (r0 == jj)
+        row[j & 1][c] = a[p0];
 
       __syncthreads ();
 
-      const double aj = row[j & 1][lane];
+      const double aj = row[j & 1][c];
+
+      /* the warp's two rows may lie on either side of row j */
+      if ((r0 | 1) > jj)
+      {
+        const double v = fma (-L[j][r0 + 8 * p0], aj, a[p0]);
+
+        a[p0] = (r0 > jj) ? v : a[p0];
+      }
 
 #pragma unroll
-      for (int p = p0; p < 8; p++)
-        if (p > p0 || w > wj)
-          a[p] = fma (-L[j][w + 4 * p], aj, a[p]);
+      for (int p = p0 + 1; p < 4; p++)
+        a[p] = fma (-L[j][r0 + 8 * p], aj, a[p]);
     }
 
-  /* row r = lane's root and near its reciprocal (44 bits) */
-  const double ur = root[lane], y0 = _recip22 (ur), rr = y0 * fma (-ur, y0, 2.0);
+  /* row r = lane's root and near its reciprocal */
+  const double ur = root[lane], rr = _recip44 (ur);
   int e = P_ZERO;
 
 #pragma unroll
-  for (int p = 0; p < 8; p++)
+  for (int p = 0; p < 4; p++)
   {
-    const int r = w + 4 * p;
+    const int r = r0 + 8 * p;
 
     a[p] = _scaled (a[p], __shfl_sync (0xffffffffu, ur, r), __shfl_sync (0xffffffffu, rr, r));
     e    = max (e, _above (a[p]));
@@ -804,39 +911,46 @@ _posv_panel_kernel (double *__restrict__ A, int n, double *__restrict__ b, int k
   }
 
   /* the columns' digits */
-  exm[w][lane] = e;
+  exm[r0][c] = e;
   __syncthreads ();
-  e = max (max (exm[0][lane], exm[1][lane]), max (exm[2][lane], exm[3][lane]));
 
-  if (w == 0 && col <= n)
+#pragma unroll
+  for (int q = 0; q < 8; q++)
+    e = max (e, exm[q][c]);
+
+  if (r0 == 0 && col <= n)
     ex[rel] = e;
 
 #pragma unroll
-  for (int p = 0; p < 8; p++)
-    _digits63 (a[p], e, &dig[0][lane][w + 4 * p], 32 * (P_K + 8));
+  for (int p = 0; p < 4; p++)
+    _digits63 (a[p], e, &dig[0][c][r0 + 8 * p], PP_C * (P_K + 8));
 
   __syncthreads ();
 
-  uint8_t *blk = pk + (size_t) (blockIdx.x / 4) * P_CHUNK;
+  uint8_t *blk = pk + (size_t) (blockIdx.x / (P_T / PP_C)) * P_CHUNK;
 
-  for (int u = tid; u < 4 * P_NS * 32; u += PP_TH)
+  for (int u = tid; u < 4 * P_NS * PP_C; u += PP_TH)
   {
-    const int c = u & 31, qs = u >> 5, sl = qs % P_NS, q = qs / P_NS, r = (blockIdx.x & 3) * 32 + c;
+    const int cc = u % PP_C, qs = u / PP_C, sl = qs % P_NS, q = qs / P_NS;
+    const int r  = (blockIdx.x % (P_T / PP_C)) * PP_C + cc;
 
     *(uint4 *) (blk + (size_t) q * P_LBO + (size_t) sl * P_UNIT + (r >> 3) * 128 + (r & 7) * 16) =
-      *(const uint4 *) &dig[sl][c][q * 8];
+      *(const uint4 *) &dig[sl][cc][q * 8];
   }
 }
 
 /* the first diagonal block; info = 0 */
-__global__ void __launch_bounds__ (128)
+__global__ void __launch_bounds__ (DG_WARPS * 32)
 _posv_begin_kernel (double *__restrict__ A, int n, double *__restrict__ Lt, double *__restrict__ root,
                     double *__restrict__ rd, int32_t *info)
 {
   __shared__ DiagSmem d;
   const int tid = threadIdx.x, nb = min (n, P_K);
 
-  for (int e = tid; e < P_K * P_K; e += 128)
+  _diag_init (d, tid);
+  asm volatile ("fence.mbarrier_init.release.cluster;" ::: "memory");
+
+  for (int e = tid; e < P_K * P_K; e += DG_WARPS * 32)
   {
     const int r = e / P_K, c = e % P_K;
 
@@ -1078,13 +1192,13 @@ ncg_launch_posv (double *A, int n, double *b, int32_t *info, void *work, cudaStr
   if ((e = cudaMemsetAsync (pk + o.words, 0, o.total - o.words, s)) != cudaSuccess)
     return e;
 
-  _posv_begin_kernel<<<1, 128, 0, s>>> (A, n, Lt, root, rd, info);
+  _posv_begin_kernel<<<1, DG_WARPS * 32, 0, s>>> (A, n, Lt, root, rd, info);
 
   for (int kb = 0; kb < n; kb += P_K)
   {
     const int nb = (n - kb < P_K) ? n - kb : P_K, rest = n - kb - nb;
 
-    _posv_panel_kernel<<<(rest + 1 + 31) / 32, PP_TH, 0, s>>> (A, n, b, kb, nb, Lt, root, pk, ex, info);
+    _posv_panel_kernel<<<(rest + 1 + PP_C - 1) / PP_C, PP_TH, 0, s>>> (A, n, b, kb, nb, Lt, root, pk, ex, info);
 
     if ((e = cudaGetLastError ()) != cudaSuccess)
       return e;
