@@ -14,11 +14,13 @@
 #define NPD_THREADS 128
 #define NPD_LD (NCG_DMAX + 1)
 
-/* player at seat i of round r of the round-robin schedule over m (even) */
+/* player at seat i < m of round r < m - 1 of the round-robin schedule over m (even) */
 static __device__ __forceinline__ int
 _rr_seat (int i, int r, int m)
 {
-  return (i == 0) ? 0 : ((i - 1 + r) % (m - 1)) + 1;
+  const int x = i + r;
+
+  return (i == 0) ? 0 : (x < m ? x : x - (m - 1));
 }
 
 /* sum over the threads of the CTA in a fixed order */

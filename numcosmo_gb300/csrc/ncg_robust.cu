@@ -694,53 +694,190 @@ _rq_pair_kernel (const double *__restrict__ X, int n, int d, int32_t *__restrict
   }
 }
 
-/* 3. E[s] rows = eigenvectors of C[s], eigenvalues ascending */
-__global__ void __launch_bounds__ (NPD_THREADS)
-_rq_eig_kernel (const double *__restrict__ C, int d, double *__restrict__ E)
-{
-  __shared__ double W[NCG_DMAX][NPD_LD];
-  __shared__ double V[NCG_DMAX][NPD_LD];
-  __shared__ double eva[NCG_DMAX];
-  __shared__ double2 cs[NCG_DMAX / 2 + 1];
-  __shared__ double red[NPD_THREADS / 32];
-  __shared__ int perm[NCG_DMAX];
-  const int s = blockIdx.x, tid = threadIdx.x;
+#define EIG_TH 256
+#define EIG_SETS 8
 
-  for (int e = tid; e < d * d; e += NPD_THREADS)
-    W[e / d][e % d] = C[(size_t) s * d * d + e];
+/* 3. E[s] rows = eigenvectors of C[s], eigenvalues ascending: cyclic Jacobi as
+ * _npd_jacobi does it, for several sets at once.  A round's angles (two square
+ * roots and three divisions, some 50 FP64 instructions of 64 cycles) cost the
+ * same for the d / 2 rotations of one set as for a warp full of them: 2048 sets of
+ * 8 x 8 with a CTA each took 466 us, 8 sets to a CTA 206 us (one set 145, now 120).
+ * A set that has converged is left as it is while the others of its CTA go on.
+ * G: sets per CTA, a power of two. */
+__global__ void __launch_bounds__ (EIG_TH)
+_rq_eig_kernel (const double *__restrict__ C, int d, int nsets, int G, double *__restrict__ E)
+{
+  extern __shared__ double rq_wv[];   /* per set W, then V: d rows of ld */
+  __shared__ double2 cs[32], part[EIG_TH / 32];
+  __shared__ int live[EIG_SETS], perm[EIG_SETS][NCG_DMAX];
+  const int tps = EIG_TH / G, ld = d | 1, m = d + (d & 1), np = m / 2;
+  const int tid = threadIdx.x, s0 = blockIdx.x * G, ng = min (G, nsets - s0);
+  const int mat = d * ld;
+  /* divisions by d (of e < 2^12) and np (of at most 32) as products */
+  const int dinv = (1 << 20) / d + 1, npinv = (1 << 16) / np + 1;
+
+  for (int e = tid; e < G * d * d; e += EIG_TH)
+  {
+    const int g = e / (d * d), r = e / d % d, c = e % d;
+    double *W   = rq_wv + 2 * g * mat;
+
+    W[r * ld + c]       = (g < ng) ? C[(size_t) (s0 + g) * d * d + r * d + c] : 0.0;
+    W[mat + r * ld + c] = (r == c) ? 1.0 : 0.0;
+  }
 
   __syncthreads ();
 
-  _npd_jacobi (W, V, d, eva, cs, red);
-
-  if (tid == 0)
+  for (int sweep = 0; sweep < 100; sweep++)
   {
+    {
+      const double *W = rq_wv + 2 * (tid / tps) * mat;
+      double off = 0.0, dg = 0.0;
+
+      for (int e = tid % tps; e < d * d; e += tps)
+      {
+        const int r = e / d, c = e % d;
+        const double v = W[r * ld + c];
+
+        if (c > r)
+          off += v * v;
+        else if (c == r)
+          dg += v * v;
+      }
+
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+      {
+        off += __shfl_xor_sync (0xffffffffu, off, o);
+        dg  += __shfl_xor_sync (0xffffffffu, dg, o);
+      }
+
+      /* tps is a multiple of 32 */
+      if ((tid & 31) == 0)
+        part[tid >> 5] = make_double2 (off, dg);
+    }
+
+    __syncthreads ();
+
+    int on = 0;
+
+    if (tid < G)
+    {
+      double off = 0.0, dg = 0.0;
+
+      for (int t = 0; t < tps / 32; t++)
+      {
+        off += part[tid * (tps / 32) + t].x;
+        dg  += part[tid * (tps / 32) + t].y;
+      }
+
+      on        = tid < ng && !(off <= 1.0e-30 * dg || off == 0.0);
+      live[tid] = on;
+    }
+
+    if (!__syncthreads_or (on))
+      break;
+
+    for (int r = 0; r < m - 1; r++)
+    {
+      if (tid < G * np)
+      {
+        const int g     = tid / np, k = tid % np;
+        const double *W = rq_wv + 2 * g * mat;
+        const int x = _rr_seat (k, r, m), y = _rr_seat (m - 1 - k, r, m), p = min (x, y), q = max (x, y);
+        double c = 1.0, sn = 0.0;
+
+        if (q < d && live[g])
+        {
+          const double apq = W[p * ld + q];
+
+          if (apq != 0.0)
+          {
+            const double theta = (W[q * ld + q] - W[p * ld + p]) / (2.0 * apq);
+            const double t     = (theta >= 0.0 ? 1.0 : -1.0) / (fabs (theta) + sqrt (theta * theta + 1.0));
+
+            c  = 1.0 / sqrt (t * t + 1.0);
+            sn = t * c;
+          }
+        }
+
+        cs[tid] = make_double2 (c, sn);
+      }
+
+      __syncthreads ();
+
+      /* W J and V J: columns p, q of every row (V's rows follow W's) */
+      for (int e = tid; e < G * np * 2 * d; e += EIG_TH)
+      {
+        const int gk = (e * dinv) >> 21, row = e - gk * 2 * d;
+        const int s = (gk * npinv) >> 16, k = gk - s * np;
+        const int x = _rr_seat (k, r, m), y = _rr_seat (m - 1 - k, r, m), p = min (x, y), q = max (x, y);
+        const double2 g = cs[gk];
+
+        if (q >= d || g.y == 0.0)
+          continue;
+
+        double *Z       = rq_wv + 2 * s * mat + row * ld;
+        const double zp = Z[p], zq = Z[q];
+
+        Z[p] = g.x * zp - g.y * zq;
+        Z[q] = g.y * zp + g.x * zq;
+      }
+
+      __syncthreads ();
+
+      /* J^T (W J): rows p, q of every column */
+      for (int e = tid; e < G * np * d; e += EIG_TH)
+      {
+        const int gk = (e * dinv) >> 20, col = e - gk * d;
+        const int s = (gk * npinv) >> 16, k = gk - s * np;
+        const int x = _rr_seat (k, r, m), y = _rr_seat (m - 1 - k, r, m), p = min (x, y), q = max (x, y);
+        const double2 g = cs[gk];
+
+        if (q >= d || g.y == 0.0)
+          continue;
+
+        double *W       = rq_wv + 2 * s * mat + col;
+        const double wp = W[p * ld], wq = W[q * ld];
+
+        W[p * ld] = g.x * wp - g.y * wq;
+        W[q * ld] = g.y * wp + g.x * wq;
+      }
+
+      __syncthreads ();
+    }
+  }
+
+  if (tid < ng)
+  {
+    const double *W = rq_wv + 2 * tid * mat;
+    int *pm         = perm[tid];
+
     for (int a = 0; a < d; a++)
-      perm[a] = a;
+      pm[a] = a;
 
     /* ascending eigenvalues (ties keep their index order) */
     for (int a = 1; a < d; a++)
     {
-      const int pa = perm[a];
+      const int pa = pm[a];
       int b        = a - 1;
 
-      while (b >= 0 && eva[perm[b]] > eva[pa])
+      while (b >= 0 && W[pm[b] * (ld + 1)] > W[pa * (ld + 1)])
       {
-        perm[b + 1] = perm[b];
+        pm[b + 1] = pm[b];
         b--;
       }
 
-      perm[b + 1] = pa;
+      pm[b + 1] = pa;
     }
   }
 
   __syncthreads ();
 
-  for (int e = tid; e < d * d; e += NPD_THREADS)
+  for (int e = tid; e < ng * d * d; e += EIG_TH)
   {
-    const int r = e / d, c = e % d;
+    const int g = e / (d * d), r = e / d % d, c = e % d;
 
-    E[(size_t) s * d * d + e] = V[c][perm[r]];
+    E[(size_t) s0 * d * d + e] = rq_wv[(2 * g + 1) * mat + c * ld + perm[g][r]];
   }
 }
 
@@ -869,6 +1006,12 @@ _robust_launch (const double *X, int n, int d, const int32_t *idx, int m, int ns
   const int t1 = nsets * d, t2 = nsets * (d * (d - 1) / 2);
   const double cq = 2.21914 * _qn_dn (m);
   cudaError_t e;
+  /* sets per CTA of the eigenvectors: as many as fill a warp with angles, but
+   * not fewer CTAs than SMs */
+  int G = d <= 8 ? EIG_SETS : (d <= 16 ? EIG_SETS / 2 : EIG_SETS / 4);
+
+  while (G > 1 && nsets < 152 * G)
+    G /= 2;
 
   /* raised whatever the size: the kernels' static arrays (up to 4 KiB) count
    * against the 48 KiB default too */
@@ -892,7 +1035,7 @@ _robust_launch (const double *X, int n, int d, const int32_t *idx, int m, int ns
       _rq_pair_kernel<W><<<(t2 + w2 - 1) / w2, W ? 32 * w2 : RQ_CTA_TH, per_warp * w2, s>>> (X, n, d, bad, idx, m, mpad,
                                                                                              cq, t2, sig, C);
 
-    _rq_eig_kernel<<<nsets, NPD_THREADS, 0, s>>> (C, d, E);
+    _rq_eig_kernel<<<(nsets + G - 1) / G, EIG_TH, sizeof (double) * 2 * G * d * (d | 1), s>>> (C, d, nsets, G, E);
     _rq_z_kernel<W><<<(t1 + w3 - 1) / w3, W ? 32 * w3 : RQ_CTA_TH, per_warp * w3, s>>> (X, n, d, bad, idx, m, mpad, cq, t1,
                                                                                     sig, E, sigz);
     _rq_final_kernel<<<nsets, 128, 0, s>>> (E, d, sig, sigz, out);
