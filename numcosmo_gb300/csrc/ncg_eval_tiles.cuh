@@ -41,12 +41,14 @@
 #define EV_THREADS 128
 
 /* FP64 operand stride (doubles per kernel) and the kernels staged at once: a
- * multiple of the warps that may share them, within 36 KiB */
+ * multiple of the warps that may share them, within 36 KiB.  KDE: DP may be any
+ * even number of coordinates within the operand's multiple of 4 (the rest are
+ * zeros on both sides and add nothing) */
 template <int DP, int KIND>
 struct NcgEv64
 {
   static constexpr int P   = DP * (DP + 1) / 2;
-  static constexpr int S   = (KIND == NCG_VKDE) ? DP + P : DP;
+  static constexpr int S   = (KIND == NCG_VKDE) ? DP + P : (DP + 3) / 4 * 4;
   static constexpr int raw = 36864 / ((S + 1) * 8) / 4 * 4;
   static constexpr int KC  = raw < 4 ? 4 : (raw > 256 ? 256 : raw);
 };
