@@ -25,7 +25,7 @@
  * end; _posv_back_kernel solves U x = U^{-T} b in one launch.
  * Measured at n = 1700 (n = 4096): panel 10 us (12), update 23 us with the
  * diagonal block's 27 beside it (78 us), U x = y 175 us (413 us); the whole solve
- * 2.0 ms (6.5 ms).  The plain form took 90 (diagonal) + 120 (panel) + 110 us
+ * 1.76 ms (5.9 ms), the starts of its launches behind their predecessors.  The plain form took 90 (diagonal) + 120 (panel) + 110 us
  * (update) per 64 rows at n = 1700 and 33 us per 64 rows for each triangle, 10 ms.
  * Left: the chain of 32 pivots (the bound below n = 1900), the epilogue of the
  * update above.
@@ -36,6 +36,7 @@
 #include <stdint.h>
 
 #include "ncg_internal.h"
+#include "ncg_pdl.cuh"
 #include "ncg_tc_ptx.cuh"
 
 #define P_NS 7                        /* slices and orders                   */
@@ -383,6 +384,8 @@ _diag_factor (DiagSmem &d, int w, int lane, int bar, int nb, double *__restrict_
     return;
   }
 
+  ncg_pdl_next ();
+
   if (w == 0)
   {
     const double u = sqrt (d.S[lane][lane]), ri = 1.0 / u;
@@ -532,12 +535,9 @@ _syrk64_kernel (const S64Params p)
   const bool lone = p.Lt != NULL && gridDim.x > 1;
   const int ustep = !lone ? (int) gridDim.x : (blockIdx.x == 0 ? (1 << 28) : (int) gridDim.x - 1);
   volatile int *err = &sm.err;
-  /* a factorisation that already failed (or timed out) needs no more updates */
-  const bool skip = *(volatile int32_t *) p.err != 0;
 
   if (threadIdx.x == 0)
   {
-    sm.err   = skip ? 1 : 0;
     sm.ndiag = 0;
 
     for (int s = 0; s < S_STAGES; s++)
@@ -568,6 +568,14 @@ _syrk64_kernel (const S64Params p)
                   : "memory");
     asm volatile ("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+
+  (void) ncg_pdl_wait ();
+
+  /* a factorisation that already failed (or timed out) needs no more updates */
+  const bool skip = *(volatile int32_t *) p.err != 0;
+
+  if (threadIdx.x == 0)
+    sm.err = skip ? 1 : 0;
 
   _tc_fence_before ();
   __syncthreads ();
@@ -847,6 +855,11 @@ _posv_panel_kernel (double *__restrict__ A, int n, double *__restrict__ b, int k
   const int rel = blockIdx.x * PP_C + c, col = kb + nb + rel;
   double a[4];
 
+  const size_t pdl0 = ncg_pdl_wait ();
+
+  Lt   += pdl0;
+  root += pdl0;
+
   if (*(volatile const int32_t *) info)
     return;
 
@@ -888,6 +901,8 @@ _posv_panel_kernel (double *__restrict__ A, int n, double *__restrict__ b, int k
       for (int p = p0 + 1; p < 4; p++)
         a[p] = fma (-L[j][r0 + 8 * p], aj, a[p]);
     }
+
+  ncg_pdl_next ();
 
   /* row r = lane's root and near its reciprocal */
   const double ur = root[lane], rr = _recip44 (ur);
@@ -1136,7 +1151,7 @@ _run_syrk64 (const S64Params &p, int nsm, cudaStream_t s)
   for (int i = 0; i < (p.nn + P_T - 1) / P_T && tiles < nsm; i++)
     tiles += Tn - P_T / P_N * i;
 
-  _syrk64_kernel<<<tiles < nsm ? tiles : nsm, S_THREADS, S64_SMEM_BYTES, s>>> (p);
+  ncg_pdl_launch (_syrk64_kernel, tiles < nsm ? tiles : nsm, S_THREADS, S64_SMEM_BYTES, s, p);
 
   return cudaGetLastError ();
 }
@@ -1198,7 +1213,7 @@ ncg_launch_posv (double *A, int n, double *b, int32_t *info, void *work, cudaStr
   {
     const int nb = (n - kb < P_K) ? n - kb : P_K, rest = n - kb - nb;
 
-    _posv_panel_kernel<<<(rest + 1 + PP_C - 1) / PP_C, PP_TH, 0, s>>> (A, n, b, kb, nb, Lt, root, pk, ex, info);
+    ncg_pdl_launch (_posv_panel_kernel, (rest + 1 + PP_C - 1) / PP_C, PP_TH, 0, s, A, n, b, kb, nb, Lt, root, pk, ex, info);
 
     if ((e = cudaGetLastError ()) != cudaSuccess)
       return e;
