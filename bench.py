@@ -387,7 +387,8 @@ def run_gpu(args):
                  "speedup_mixed_over_fp64": value / v64,
                  "roofline": {"bound": "fp64", "achieved": v64 / ws * FLOP_PER_PAIR / 1e12, "peak": fp64_peak,
                               "unit": "TFLOP/s", "frac": v64 / ws * FLOP_PER_PAIR / 1e12 / fp64_peak,
-                              "note": "peak = FP64 FMA rate measured on this device (ncg_measure_fp64_peak)"}},
+                              "note": "peak = FP64 FMA rate measured on this device (ncg_measure_fp64_peak); above 1 because "
+                                      "chi^2 runs as exact FP16 digit products on the tensor cores"}},
         "mixed_simt": {"value": ws * pairs * len(tsimt) / sum(tsimt), "unit": "pairs/s",
                        "ms_per_step": 1e3 * sum(tsimt) / len(tsimt), "max_rel_err_vs_fp64": err_simt},
         "mixed_max_rel_err_vs_fp64": err_mx,

@@ -4,15 +4,15 @@
  * mixed weight fit the start of a grid, 1 to 2 us, is hidden behind its predecessor
  * (fit d=12 N=4096 41.5 -> 38.4 ms, half-move d=8 N=512 3.8 -> 3.3 ms), and between
  * the FP64 eval and its merge (one point 27.0 -> 24.4 us, 1000 points 97.0 -> 92.7 us,
- * KDE d=4 n=1000).  Kernels
- * that fill an SM let the next grid in only as they leave: the FP64 fit's product
- * and panel kernels, d=12 N=2048, took 38.4 instead of 32.7 ms with the next
- * grid's CTAs resident from their start, and 26.1 instead of 29.6 ms like this.
+ * KDE d=4 n=1000).  Kernels that fill an SM let the next grid in only as they
+ * leave: the FP64 fit's product and panel kernels, d=12 N=2048, took 38.4 instead
+ * of 32.7 ms with the next grid's CTAs resident from their start, and 26.1 instead
+ * of 29.6 ms like this.
  *
  * A kernel launched by ncg_pdl_launch begins with ncg_pdl_enter or ncg_pdl_wait
- * (before any access to global memory): it returns once every kernel before it in the stream has
- * finished and its writes can be seen, since each of those waited in the same way
- * before it let the next one start.  Loads through `const T *__restrict__` may be
+ * (before any access to global memory): it returns once every kernel before it in
+ * the stream has finished and its writes can be seen, since each of those waited in
+ * the same way before it let the next one start.  Loads through `const T *__restrict__` may be
  * moved by the compiler as if nothing could write there, also ahead of that wait:
  * the zero that they return, added to such a pointer, ties its loads to
  * the wait and leaves the pointer what it is to the compiler (hidden pointers cost

@@ -25,10 +25,10 @@
  * end; _posv_back_kernel solves U x = U^{-T} b in one launch.
  * Measured at n = 1700 (n = 4096): panel 10 us (12), update 23 us with the
  * diagonal block's 27 beside it (78 us), U x = y 175 us (413 us); the whole solve
- * 1.76 ms (5.9 ms), the starts of its launches behind their predecessors.  The plain form took 90 (diagonal) + 120 (panel) + 110 us
- * (update) per 64 rows at n = 1700 and 33 us per 64 rows for each triangle, 10 ms.
- * Left: the chain of 32 pivots (the bound below n = 1900), the epilogue of the
- * update above.
+ * 1.76 ms (5.9 ms), the starts of its launches behind their predecessors.  The
+ * plain form took 90 (diagonal) + 120 (panel) + 110 us (update) per 64 rows at
+ * n = 1700 and 33 us per 64 rows for each triangle, 10 ms.  Left: the chain of 32
+ * pivots (the bound below n = 1900), the epilogue of the update above.
  */
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
