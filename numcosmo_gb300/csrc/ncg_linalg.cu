@@ -663,7 +663,7 @@ __global__ void __launch_bounds__ (256)
 _potrf_update_f32_kernel (float *A, int ld, int kb, int nb, int off, int nn, float *__restrict__ dg,
                           const int32_t *info)
 {
-  (void) ncg_pdl_enter ();
+  (void) ncg_pdl_wait ();
 
   __shared__ __align__ (16) float As[PB][PB];
   __shared__ __align__ (16) float Bs[PB][PB];
@@ -724,6 +724,8 @@ _potrf_update_f32_kernel (float *A, int ld, int kb, int nb, int off, int nn, flo
       for (int q = 0; q < 4; q++)
         acc[p][q] = fmaf (xv[p], yv[q], acc[p][q]);
   }
+
+  ncg_pdl_next ();
 
 #pragma unroll
   for (int p = 0; p < 4; p++)

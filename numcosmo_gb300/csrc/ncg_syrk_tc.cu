@@ -32,6 +32,7 @@
 #include <stdint.h>
 
 #include "ncg_internal.h"
+#include "ncg_pdl.cuh"
 #include "ncg_tc_ptx.cuh"
 #include "ncg_syrk_tc.cuh"
 
@@ -116,13 +117,9 @@ _syrk_tc_kernel (const uint8_t *__restrict__ pk, int nkc, int nn, float *__restr
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int T_ = (nn + SK_T - 1) / SK_T, ntiles = T_ * (T_ + 1) / 2;
   volatile int *err = &sm.err;
-  /* a factorisation that already failed (or timed out) needs no more updates */
-  const bool skip = *(volatile int *) err_out != 0;
 
   if (threadIdx.x == 0)
   {
-    sm.err = skip ? 1 : 0;
-
     for (int s = 0; s < SK_STAGES; s++)
     {
       _mbar_init (&sm.full[s], 1);
@@ -146,6 +143,14 @@ _syrk_tc_kernel (const uint8_t *__restrict__ pk, int nkc, int nn, float *__restr
                   : "memory");
     asm volatile ("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+
+  pk += ncg_pdl_wait ();
+
+  /* a factorisation that already failed (or timed out) needs no more updates */
+  const bool skip = *(volatile int *) err_out != 0;
+
+  if (threadIdx.x == 0)
+    sm.err = skip ? 1 : 0;
 
   _tc_fence_before ();
   __syncthreads ();
@@ -361,6 +366,7 @@ _syrk_tc_kernel (const uint8_t *__restrict__ pk, int nkc, int nn, float *__restr
     }
   }
 
+  ncg_pdl_next ();
   _tc_fence_before ();
   __syncthreads ();
 
@@ -419,10 +425,8 @@ ncg_launch_syrk_tc (const void *pk, int K, int nn, float *C, int ldc, int mode, 
   const int ntiles = T_ * (T_ + 1) / 2;
   const int grid   = (ntiles < nsm) ? ntiles : nsm;
 
-  _syrk_tc_kernel<<<grid, SK_THREADS, SK_SMEM_BYTES, s>>> ((const uint8_t *) pk, (K + SK_KC - 1) / SK_KC, nn, C,
-                                                           ldc, mode, dg, err);
-
-  return cudaGetLastError ();
+  return ncg_pdl_launch (_syrk_tc_kernel, grid, SK_THREADS, SK_SMEM_BYTES, s, (const uint8_t *) pk,
+                         (K + SK_KC - 1) / SK_KC, nn, C, ldc, mode, dg, err);
 }
 
 /* C = A^T A over the ncols x ncols upper triangle (A FP64, nrows x ncols,
