@@ -1,8 +1,8 @@
 /*
  * ncg_jacobi.cuh -- CTA-parallel cyclic Jacobi eigen-decomposition of a small
- * symmetric matrix (d <= NCG_DMAX) in shared memory, NPD_THREADS threads:
- * used by the nearPD fallback (ncg_prepare.cu) and the OGK robust covariance
- * (ncg_robust.cu), where the reference calls LAPACK dsyevr.
+ * symmetric matrix (d <= NCG_DMAX) in shared memory, NPD_THREADS threads, for
+ * the nearPD fallback (ncg_prepare.cu), where the reference calls LAPACK dsyevr; the
+ * OGK robust covariance (ncg_robust.cu) uses its schedule for several matrices at once.
  */
 #ifndef NCG_JACOBI_CUH
 #define NCG_JACOBI_CUH
