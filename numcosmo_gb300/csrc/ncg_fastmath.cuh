@@ -315,7 +315,7 @@ static __device__ __forceinline__ double
 ncg_log_ge1 (double u)
 {
   const int hi    = __double2hiint (u);
-  const int E     = (hi >> 20) - 1023;
+  const int E     = ((hi >> 20) & 0x7ff) - 1023;   /* a NaN of either sign: 1024 */
   const double2 c = __ldg (ncg_log_tab + ((hi >> 12) & 255));
   const double m  = __hiloint2double ((hi & 0x000fffff) | 0x3ff00000, __double2loint (u));
   const double r  = fma (m, c.x, -1.0);
