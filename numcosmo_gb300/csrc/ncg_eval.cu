@@ -125,7 +125,8 @@ _eval64_few_kernel (const ncg_eval_args_t a, const double *__restrict__ Xq, cons
   const double inv_nu = 1.0 / a.nu;
 
   for (int i = i0 + tid; i < i1; i += EV_THREADS)
-    ncg_lse_add (ncg_lnt_64<KERN> (ncg_chi2_64<DP, KIND> (pack + (size_t) i * S, x), cvec[i], a.kappa, inv_nu), g, s);
+    ncg_lse_add (ncg_lnt_64<KERN> (ncg_chi2_64<DP, KIND> (pack + (size_t) i * S, x), cvec[i], a.kappa, inv_nu, false),
+                 g, s);
 
   /* the CTA's pair: the largest g first, then one exp per thread */
   double G = g;
@@ -267,11 +268,15 @@ _ev64 (const ncg_eval_args_t *a)
 {
   const bool few = a->m <= EV64_FEW;
 
-  if (a->kind == NCG_VKDE)
-    return (a->kernel == NCG_KERNEL_ST) ? _pick64<NCG_VKDE, NCG_KERNEL_ST> (a->dp, few)
-                                        : _pick64<NCG_VKDE, NCG_KERNEL_GAUSS> (a->dp, few);
+  if (a->kernel == NCG_KERNEL_GAUSS)
+    return (a->kind == NCG_VKDE) ? _pick64<NCG_VKDE, NCG_KERNEL_GAUSS> (a->dp, few)
+                                 : _pick64_kde<NCG_KERNEL_GAUSS> (a->d, few);
 
-  return (a->kernel == NCG_KERNEL_ST) ? _pick64_kde<NCG_KERNEL_ST> (a->d, few) : _pick64_kde<NCG_KERNEL_GAUSS> (a->d, few);
+  if (ncg_nu_wide (a->nu, a->d))
+    return (a->kind == NCG_VKDE) ? _pick64<NCG_VKDE, NCG_KERNEL_ST_WIDE> (a->dp, few)
+                                 : _pick64_kde<NCG_KERNEL_ST_WIDE> (a->d, few);
+
+  return (a->kind == NCG_VKDE) ? _pick64<NCG_VKDE, NCG_KERNEL_ST> (a->dp, few) : _pick64_kde<NCG_KERNEL_ST> (a->d, few);
 }
 
 /* NcgEv64::KC */

@@ -884,8 +884,9 @@ _eval_q64_kernel (const QParams p)
                             : (ex > 0x7fe)  ? __hiloint2double ((hs & 0x80000000) | 0x7ff00000, 0)
                                             : __hiloint2double ((hs & 0x800fffff) | (ex << 20), __double2loint (sk));
 
-          ncg_lse_add ((KERN == NCG_KERNEL_ST) ? fma (p.kappa, ncg_log_ge1 (fma (x[k], sc, 1.0)), c)
-                                               : fma (x[k], sc, c), g, s);
+          ncg_lse_add ((KERN == NCG_KERNEL_GAUSS)     ? fma (x[k], sc, c)
+                       : (KERN == NCG_KERNEL_ST_WIDE) ? ncg_lnt_wide (x[k] * sc, p.kappa, c)
+                                                      : fma (p.kappa, ncg_log_ge1 (fma (x[k], sc, 1.0)), c), g, s);
         }
       }
 
@@ -1048,6 +1049,13 @@ _run_q64 (const QParams &p, int grid, cudaStream_t s)
   return cudaGetLastError ();
 }
 
+template <int KERN>
+static cudaError_t
+_run_q64_bits (const QParams &p, int d, int grid, cudaStream_t s)
+{
+  return (d <= 16) ? _run_q64<KERN, 8> (p, grid, s) : _run_q64<KERN, 7> (p, grid, s);
+}
+
 extern "C" cudaError_t
 ncg_launch_eval_q64 (const ncg_eval_args_t *a, const double *Xq, const uint8_t *op, const double *c,
                      const double *mu, const double *Vg, double *out, void *scratch, int linear, int *flag_host,
@@ -1101,10 +1109,9 @@ ncg_launch_eval_q64 (const ncg_eval_args_t *a, const double *Xq, const uint8_t *
 
     const int units = p.npt * p.nslices, grid = units < nsm ? units : nsm;
 
-    if (a->kernel == NCG_KERNEL_ST)
-      e = (a->d <= 16) ? _run_q64<NCG_KERNEL_ST, 8> (p, grid, s) : _run_q64<NCG_KERNEL_ST, 7> (p, grid, s);
-    else
-      e = (a->d <= 16) ? _run_q64<NCG_KERNEL_GAUSS, 8> (p, grid, s) : _run_q64<NCG_KERNEL_GAUSS, 7> (p, grid, s);
+    e = (a->kernel == NCG_KERNEL_GAUSS)  ? _run_q64_bits<NCG_KERNEL_GAUSS> (p, a->d, grid, s)
+        : ncg_nu_wide (a->nu, a->d)      ? _run_q64_bits<NCG_KERNEL_ST_WIDE> (p, a->d, grid, s)
+                                         : _run_q64_bits<NCG_KERNEL_ST> (p, a->d, grid, s);
 
     if (e == cudaSuccess)
       e = ncg_launch_merge_d2 (p.part, Q_WG * o.ns, mc, a->final_shift, a->d_ln_href, linear, out + j0, s);

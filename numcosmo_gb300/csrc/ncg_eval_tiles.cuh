@@ -122,12 +122,18 @@ ncg_chi2_64 (const double *pk, const double *x)
   return chi2;
 }
 
-/* ln of the weighted kernel */
+/* ln of the weighted kernel (NCG_KERNEL_ST with wide set: as NCG_KERNEL_ST_WIDE) */
 template <int KERN>
 __device__ __forceinline__ double
-ncg_lnt_64 (double chi2, double c, double kappa, double inv_nu)
+ncg_lnt_64 (double chi2, double c, double kappa, double inv_nu, bool wide)
 {
-  return (KERN == NCG_KERNEL_ST) ? fma (kappa, ncg_log_ge1 (fma (chi2, inv_nu, 1.0)), c) : fma (-0.5, chi2, c);
+  if (KERN == NCG_KERNEL_GAUSS)
+    return fma (-0.5, chi2, c);
+
+  if (KERN == NCG_KERNEL_ST_WIDE || wide)
+    return ncg_lnt_wide (chi2 * inv_nu, kappa, c);
+
+  return fma (kappa, ncg_log_ge1 (fma (chi2, inv_nu, 1.0)), c);
 }
 
 /* mixed operand stride (floats per kernel, multiple of 4):
@@ -173,6 +179,8 @@ ncg_tile_eval64 (const ncg_eval_args_t a, const double *__restrict__ Xq, const d
   const int i0 = sy * kper;
   const int i1 = min (a.n, i0 + kper);
   const double inv_nu = 1.0 / a.nu;
+  /* (the batch's kernel serves both nu) */
+  const bool wide     = KERN == NCG_KERNEL_ST && WK == 1 && ncg_nu_wide (a.nu, a.d);
 
   for (int ic = i0; ic < i1; ic += KC)
   {
@@ -189,7 +197,7 @@ ncg_tile_eval64 (const ncg_eval_args_t a, const double *__restrict__ Xq, const d
     __syncthreads ();
 
     for (int kk = w; kk < kc; kk += WK)
-      ncg_lse_add (ncg_lnt_64<KERN> (ncg_chi2_64<DP, KIND> (sm + kk * S, x), sc[kk], a.kappa, inv_nu), g, s);
+      ncg_lse_add (ncg_lnt_64<KERN> (ncg_chi2_64<DP, KIND> (sm + kk * S, x), sc[kk], a.kappa, inv_nu, wide), g, s);
   }
 
   if (WK > 1)

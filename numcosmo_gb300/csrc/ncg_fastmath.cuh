@@ -331,6 +331,143 @@ ncg_log_ge1 (double u)
   return fma ((double) E, 0x1.62e42fefa39efp-1, c.y) + p;
 }
 
+/* -log c_j less its double in ncg_log_tab */
+static __device__ const double ncg_log_lo_tab[256] = {
+  0x1.e29e3a153e432p-64, 0x1.3c2d23a074505p-63, 0x1.600d65eebbc60p-61, -0x1.7b4213447a4ccp-61,
+  0x1.2be019c2d240ep-61, -0x1.885b61f610d84p-63, -0x1.cbf63e207e981p-60, 0x1.4b2c67dcd0956p-60,
+  -0x1.c5bc089e0b23bp-59, 0x1.042b74e00f373p-60, -0x1.9d6a40b6e333bp-59, 0x1.19f3f276b596dp-59,
+  -0x1.284d2b1a4a1edp-60, -0x1.4502014926cd6p-59, -0x1.4d9501f1df1d3p-59, 0x1.a66e7585e8241p-59,
+  0x1.ba13162a9c44ep-60, 0x1.1e4add513114dp-58, 0x1.7d7a7a2605718p-58, -0x1.34d66a3f7a2b6p-58,
+  0x1.44d6a6b9dad0cp-58, -0x1.9308973e22a83p-61, -0x1.42a375515892ep-58, 0x1.d2da7bd644829p-59,
+  0x1.cff28ef6a5931p-58, -0x1.f491a5df236ecp-58, -0x1.e463f9e4dd91fp-59, 0x1.76df97bcb1787p-60,
+  -0x1.89f383dad0d65p-58, 0x1.d248382a5ecffp-62, -0x1.64af228bcf63ap-60, -0x1.9d4a8f3f05aa5p-59,
+  0x1.a227143a5a99ap-58, 0x1.38176812fe880p-59, -0x1.652e70072e4b1p-57, -0x1.aae2afa34f48ap-58,
+  0x1.cf798d39f1b7dp-58, -0x1.f52f6c3723f80p-57, 0x1.837097648f581p-58, 0x1.14f176448b993p-60,
+  0x1.dcdca01dc0febp-57, 0x1.f28bf9ca923d6p-58, 0x1.bbbeaea81ece2p-57, -0x1.1e103f093930dp-58,
+  0x1.b1391fb1b4b22p-57, 0x1.24140543648f3p-58, -0x1.4644b3703041cp-57, -0x1.1919a4664319dp-57,
+  -0x1.0ea8fd38a2c66p-58, 0x1.28891a29eac08p-57, -0x1.de12ad4822814p-57, 0x1.440d1e78f44cep-57,
+  -0x1.d9f13877e61b9p-57, -0x1.16fa715e8d38bp-59, 0x1.610816ebe4976p-57, -0x1.f28442017473fp-57,
+  0x1.0593750fffe78p-58, -0x1.9fb3f9cdff9d3p-57, -0x1.966bc4ca8938dp-57, 0x1.2b1a83b18de21p-58,
+  0x1.1adf25feae309p-57, 0x1.9990bc47005e0p-59, -0x1.beb83c874aaf3p-57, -0x1.44269756071afp-58,
+  0x1.cd329bc9d42b1p-64, -0x1.204a2aa97ac8ep-58, 0x1.d01e4d9c3e3a7p-57, -0x1.4f486fc6e8c8ap-64,
+  -0x1.daf3c7a62832cp-57, -0x1.9987ee52650b9p-60, -0x1.98a0bf20f9d99p-59, 0x1.8d2b5b2204b4cp-57,
+  0x1.6e32d5e8c7080p-57, -0x1.6bb183e51ec40p-56, 0x1.e9432dc9528f1p-56, 0x1.2140c5a328e6dp-56,
+  -0x1.2333a23204a40p-56, 0x1.0b5e955ff414ep-59, 0x1.97b8198d22e05p-56, 0x1.a6880da1b13e4p-58,
+  0x1.1458b5d97ba9dp-56, -0x1.b26dc55e2d052p-56, 0x1.154d86a4ff98bp-59, -0x1.3a2eb579e2857p-59,
+  -0x1.99bae06a5c863p-61, -0x1.0e09ea9b4c4a4p-56, 0x1.895c18aa47a54p-57, 0x1.f3ee1106a6ca7p-57,
+  -0x1.95d2280d51407p-58, -0x1.263d5c1f755e9p-56, 0x1.8d8af2d5b0557p-59, 0x1.2d733ea6502f0p-56,
+  0x1.06d1e3224d3e9p-57, -0x1.0c4f82601ebfap-60, -0x1.8027c87f91214p-57, -0x1.430c8309edcfcp-56,
+  -0x1.1c0f372f6825bp-57, -0x1.51d7e6a892849p-57, 0x1.cb3fe83434321p-56, -0x1.bc78b7cdae677p-56,
+  -0x1.c4826ceaff1c8p-56, -0x1.81de37d2989eep-56, -0x1.24f586adeb499p-57, 0x1.ec1e3016fc9f5p-58,
+  -0x1.fa7088c705f8ap-56, -0x1.e15bd0fed391dp-56, -0x1.d617f8a08338cp-58, 0x1.b9b7b9e219186p-56,
+  -0x1.fc80d000b4083p-57, -0x1.5e8e76dd346a0p-56, -0x1.fc083df227104p-59, 0x1.4caf721f626aap-57,
+  0x1.a748662fc4171p-56, -0x1.29943804dfbeep-56, -0x1.9a576c0601322p-58, -0x1.58f8f27d8e90fp-57,
+  -0x1.306488dd76781p-58, -0x1.dc45997fbc413p-56, 0x1.7cab36811fa33p-57, -0x1.f4419b612c65ap-57,
+  0x1.9f4fca257a85dp-57, -0x1.51ec4c14526a6p-56, 0x1.dd8e962c0c0adp-56, -0x1.02711f5645823p-57,
+  -0x1.f3c3fbbc738aap-57, -0x1.951ec6ae7473ep-58, 0x1.6ef49cf67f73bp-56, 0x1.0f947c24d6d15p-57,
+  -0x1.66f70bc45a4eap-56, 0x1.a254f268e3b77p-57, -0x1.83875c3d29410p-56, 0x1.11178481c3254p-57,
+  0x1.027ed837c8098p-56, 0x1.db9250ec7d6c0p-56, 0x1.49cdf84b4963bp-59, 0x1.2d4ebe6b64659p-57,
+  0x1.46b9d39edb329p-56, 0x1.46a03ad42b053p-58, -0x1.b230b0b86cdb3p-56, -0x1.b575624ae2937p-56,
+  0x1.42e6254debd1ap-56, -0x1.7f81655ffb866p-57, 0x1.6a615815805b6p-56, 0x1.b5ac6bcf865f1p-60,
+  0x1.490f7d8320aa6p-56, 0x1.555ccfd34e773p-56, -0x1.392469ec4f2d1p-57, 0x1.6b1ca5b4c2326p-57,
+  0x1.894972adf9532p-58, -0x1.f73153d5f3576p-58, -0x1.5033e78d17001p-56, -0x1.fc1498cd5f810p-59,
+  0x1.866ba1f8898b2p-58, 0x1.0af58040358ccp-56, -0x1.f2180135bc9e9p-57, -0x1.e1ea13f7bb73cp-56,
+  -0x1.2c2a607f4211fp-56, -0x1.ae71b7919fe41p-62, -0x1.f987ff7ff1891p-56, 0x1.7694d500702eep-56,
+  -0x1.a045e49ba251ep-56, 0x1.259465d63197dp-57, -0x1.746e0614b6c54p-60, -0x1.a1d4ac924a114p-56,
+  -0x1.4070d99441964p-56, -0x1.91c292bb5006ep-57, -0x1.ac9a15ed191cdp-56, -0x1.4059e632f810ep-59,
+  0x1.01637cd0c6322p-55, 0x1.b3ca7518f79eep-55, 0x1.3956e356c4427p-55, -0x1.09c4075c537f5p-57,
+  0x1.b3b5da204f2b4p-56, 0x1.cbfa8aba6b01bp-56, -0x1.637129e8e65d6p-55, 0x1.9f7b2c890500ap-57,
+  0x1.12b0a6bece97ep-55, 0x1.fe2b7fa595f64p-55, -0x1.d8d54bbb0dd12p-58, -0x1.a6e6efd578cdfp-57,
+  0x1.e6178fa93d276p-57, -0x1.8dc202e52373bp-55, 0x1.3fd142b10a7d5p-57, -0x1.c3f0e01a37834p-55,
+  -0x1.dcf909e3864ebp-58, 0x1.97a882bf8aad4p-56, -0x1.df40f54d1f054p-55, -0x1.f81c49a23f756p-58,
+  -0x1.92db65c2b36abp-55, -0x1.5ff40c85bc439p-58, 0x1.f38426184f32ap-56, 0x1.5f5b45b30e302p-55,
+  -0x1.abfa36e2d19f9p-55, -0x1.5cbe32567e6afp-57, 0x1.a1afa4aeb598ap-64, -0x1.3e6cde2013e20p-55,
+  0x1.4d0496643f035p-55, -0x1.5dd121bc42e34p-55, -0x1.6534a9a0dcbbdp-57, -0x1.97f4edb1f37cbp-56,
+  0x1.c3fb96be5d640p-57, 0x1.9899fca1425e8p-56, -0x1.5d299abea2437p-55, 0x1.d1ff94a792f17p-55,
+  -0x1.d9becbb0e4322p-56, 0x1.0f3ef07774574p-55, -0x1.e9ae735118099p-55, 0x1.dbf08ade6a75ep-55,
+  -0x1.1d5ba1424b05ap-58, 0x1.d7f1bd5fda3d6p-55, 0x1.ef8b734c91c5dp-56, -0x1.2ac7fe2a95992p-56,
+  -0x1.7f9c5ae27b58ap-57, -0x1.45dac4b904390p-58, 0x1.bcade2e600649p-58, 0x1.24677c50b4f2fp-57,
+  -0x1.c5ab543639f33p-55, 0x1.05d28c1ee028bp-58, 0x1.5f5078dc66fcap-55, 0x1.6ff71a5d46072p-55,
+  -0x1.e1b74bd7dc57dp-56, -0x1.aa1f2821f7e80p-57, 0x1.e8eac4149d261p-56, 0x1.df8a528db9e2cp-57,
+  -0x1.7c4d58c23cd48p-56, 0x1.32539ce2355b0p-55, -0x1.3f8369cbbe59cp-57, -0x1.a785f94848c6cp-55,
+  0x1.52017a9a0ae4fp-58, -0x1.288675d0fb1f9p-55, -0x1.dbad233fb591cp-59, -0x1.4b98fa670a3fbp-58,
+  -0x1.0f6379c6918c0p-55, 0x1.f7a9713105cedp-55, 0x1.284f66c1ee3bap-59, -0x1.c9dd3f2c57232p-55,
+  -0x1.6ebac541fb222p-55, -0x1.f6f07ea5faf41p-56, 0x1.dc3c55b9ff703p-56, -0x1.df05830ea2cf0p-55,
+  -0x1.d864d52029c26p-55, 0x1.df1ab56bd0694p-56, 0x1.addbe1cefeccdp-63, -0x1.8997c4a22e891p-55,
+  -0x1.75638d706fc01p-55, -0x1.b91f884591919p-56, -0x1.1adfd04bb2ed0p-55, -0x1.38d3c3ffe9f6ep-58,
+  0x1.b46dbddbb1f4dp-56, 0x1.82ea1d0142b6cp-61, -0x1.20a591b0ba580p-55, 0x1.10c88f64cc285p-55,
+  -0x1.2591e1e383d79p-55, 0x1.c6a443e72f437p-57, 0x1.5c7e902d91dc0p-56, -0x1.a40dee0981e4cp-58,
+};
+
+/* log (1 + t) as x + y for t + dt >= 0 (dt far below t; t + dt may be inf or NaN): the
+ * rounding of 1 + t is taken along, below 2^-8 the series runs in t itself, and above
+ * it the table's and the sums' low parts are kept.  Against quadruple precision over t =
+ * 2^-60 .. 2^1010 within 2^-53 of itself just above 2^-8 and 2^-61 absolutely from there on
+ * (2^-58 relative below it). */
+static __device__ __forceinline__ double2
+ncg_log1p_dd (double t, double dt)
+{
+  double h, l;
+
+  if ((uint32_t) __double2hiint (t) < 0x3f700000u)
+  {
+    const double a = fma (t, fma (t, 0x1.2492492492492p-3, -0x1.5555555555555p-3), 0x1.999999999999ap-3);
+
+    h = t;
+    l = fma (t * t, fma (t, fma (t, fma (t, a, -0.25), 0x1.5555555555555p-2), -0.5), dt);
+  }
+  else
+  {
+    const double u  = 1.0 + t;
+    const int hi    = __double2hiint (u);
+    const int E     = ((hi >> 20) & 0x7ff) - 1023;
+    const double2 c = __ldg (ncg_log_tab + ((hi >> 12) & 255));
+
+    if (E == 1024)
+      return make_double2 (u, 0.0);   /* inf, NaN */
+
+    /* 1 + t - u, exact, in units of 2^E (nothing from 2^64) */
+    const double du = ((E == 0) ? t - (u - 1.0) : 1.0 - (u - t)) + dt;
+    const double d  = (E < 64) ? du * __hiloint2double ((1023 - E) << 20, 0) : 0.0;
+    const double m  = __hiloint2double ((hi & 0x000fffff) | 0x3ff00000, __double2loint (u));
+    const double r  = fma (m, c.x, -1.0);
+    const double a  = fma (r, fma (r, -0x1.5555555555555p-3, 0x1.999999999999ap-3), -0.25);
+    const double q  = fma (r, fma (r, a, 0x1.5555555555555p-2), -0.5);
+    /* ln2 as 42 bits and the rest: E times the first is exact */
+    const double e0 = E * 0x1.62e42fefa3800p-1, s0 = e0 + c.y, f0 = c.y - (s0 - e0);
+    const double s1 = s0 + r, b1 = s1 - s0, f1 = (s0 - (s1 - b1)) + (r - b1);
+
+    h = s1;
+    l = fma (r * r, q, fma (d, c.x, fma ((double) E, 0x1.ef35793c76730p-45, __ldg (ncg_log_lo_tab + ((hi >> 12) & 255)) + (f0 + f1))));
+  }
+
+  const double x = h + l;
+
+  return make_double2 (x, l - (x - h));
+}
+
+/* ln of a Student-t term at a large nu: kappa log (1 + t) + c.  ncg_log_ge1 sees 1 + t
+ * rounded, so kappa = -(nu + d) / 2 times 1.5 2^-53 is lost there: less than the
+ * rounding of the result up to nu = d, 1e-9 of it at nu = 1e9. */
+static __device__ __noinline__ double
+ncg_lnt_wide (double t, double kappa, double c)
+{
+  const double2 g = ncg_log1p_dd (t, 0.0);
+
+  return fma (kappa, g.x, fma (kappa, g.y, c));
+}
+
+/* The nu that take it, by a kernel of their own (KERN = NCG_KERNEL_ST_WIDE): as a branch on
+ * a launch constant in the one for small nu it cost that one 2 % (d = 16, 8192 x 8192
+ * 3.18 -> 3.25 ms), although it never ran. */
+#define NCG_KERNEL_ST_WIDE 2
+
+static __host__ __device__ __forceinline__ bool
+ncg_nu_wide (double nu, int d)
+{
+  return nu > 8.0 && nu > (double) d;
+}
+
 /* One sum over kernels kept as (g, s): the terms added so far are
  * s exp(g).  g follows the largest term closely enough (within 4) that
  * g + log s loses nothing against the maximum itself; it starts at -1e300
