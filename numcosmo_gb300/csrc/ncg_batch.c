@@ -35,6 +35,11 @@ enum { BP_FP64 = 0, BP_MIXED = 1 };
  * 1024 keeps the sum's relative rounding near 1e-6 worst case. */
 #define NCG_BATCH_MIXED_KMAX 1024
 
+/* streams the tensor-core launches of a plan are spread over */
+#define NCG_BATCH_TC_STREAMS 4
+/* streams the branch schedule's launches are spread over */
+#define NCG_BATCH_BR_STREAMS 16
+
 typedef struct ncg_bplan
 {
   int valid;                   /* built for the current problem list and generations */
@@ -60,15 +65,17 @@ typedef struct ncg_bplan
   int ntcp, cap_tcp;
   int32_t *brp;                /* branch schedule (tc = 2): every problem, largest first */
   int8_t *brk;                 /* its launch: 0 FP64 tiles, 1 FP32 SIMT tiles, 2 tensor cores */
+  int8_t *brs;                 /* its stream */
   int nbrp, cap_brp;
+  /* scratch of the one-problem launches, a region per stream (the launches of a
+   * stream follow one another): the graph records its address, so it is the
+   * plan's own and moves only when the plan is built */
+  void *dscr;
+  size_t cap_scr;
+  size_t scr_off[NCG_BATCH_BR_STREAMS];
   int64_t pairs;
   int64_t captures, launches;
 } ncg_bplan_t;
-
-/* streams the tensor-core launches of a plan are spread over */
-#define NCG_BATCH_TC_STREAMS 4
-/* streams the branch schedule's launches are spread over */
-#define NCG_BATCH_BR_STREAMS 16
 
 struct ncg_batch
 {
@@ -105,6 +112,10 @@ _plan_free (ncg_bplan_t *p)
   free (p->tcp);
   free (p->brp);
   free (p->brk);
+  free (p->brs);
+
+  if (p->dscr)
+    cudaFree (p->dscr);
 
   if (p->dp)
     cudaFree (p->dp);
@@ -379,6 +390,130 @@ _is_tc (const ncg_bplan_t *P, int i)
   return 0;
 }
 
+typedef struct { double cost; int32_t k; } _brc_t;
+
+static int
+_brc_desc (const void *x, const void *y)
+{
+  const _brc_t *a = x, *c = y;
+
+  if (a->cost > c->cost) return -1;
+  if (a->cost < c->cost) return 1;
+  return (a->k < c->k) ? -1 : (a->k > c->k);
+}
+
+/* the branch schedule's order, largest problem first, each to the stream with the
+ * least work so far (longest processing time first) */
+static ncg_status_t
+_branch_streams (ncg_batch_t *b, ncg_bplan_t *P)
+{
+  double load[NCG_BATCH_BR_STREAMS] = { 0.0 };
+  _brc_t *ord;
+  int32_t *p;
+  int8_t *k8;
+
+  if (P->nbrp == 0)
+    return NCG_OK;
+
+  ord = malloc (sizeof (_brc_t) * P->nbrp);
+  p   = malloc (sizeof (int32_t) * P->nbrp);
+  k8  = malloc (sizeof (int8_t) * P->nbrp);
+
+  if (ord == NULL || p == NULL || k8 == NULL)
+  {
+    free (ord);
+    free (p);
+    free (k8);
+
+    return NCG_ERR_OUT_OF_MEMORY;
+  }
+
+  for (int k = 0; k < P->nbrp; k++)
+  {
+    const int i = P->brp[k];
+
+    /* tensor-core pairs at about a quarter of the FP32 SIMT pair time */
+    ord[k].cost = (double) b->m[i] * (double) b->sd[i]->nk * _pair_cost (b->sd[i]) * ((P->brk[k] == 2) ? 0.25 : 1.0);
+    ord[k].k    = k;
+  }
+
+  qsort (ord, P->nbrp, sizeof (_brc_t), _brc_desc);
+
+  for (int q = 0; q < P->nbrp; q++)
+  {
+    int best = 0;
+
+    for (int t = 1; t < NCG_BATCH_BR_STREAMS && t < P->nbrp; t++)
+      if (load[t] < load[best])
+        best = t;
+
+    load[best] += ord[q].cost;
+    p[q]        = P->brp[ord[q].k];
+    k8[q]       = P->brk[ord[q].k];
+    P->brs[q]   = (int8_t) best;
+  }
+
+  memcpy (P->brp, p, sizeof (int32_t) * P->nbrp);
+  memcpy (P->brk, k8, sizeof (int8_t) * P->nbrp);
+  free (ord);
+  free (p);
+  free (k8);
+
+  return NCG_OK;
+}
+
+/* scratch of problem i's own launch of kind k (ncg_bplan_t's brk) */
+static size_t
+_launch_scratch (ncg_batch_t *b, int i, int k)
+{
+  ncg_sd_t *sd = b->sd[i];
+  ncg_eval_args_t a;
+
+  if (k == 2)
+    return ncg_tc_scratch_bytes ((int64_t) b->m[i], (int) sd->nk, sd->dp);
+
+  ncg_sd_fill_args (sd, b->m[i], &a);
+
+  return ncg_eval_scratch_bytes (&a, k == 1 ? NCG_PREC_MIXED_SIMT : NCG_PREC_FP64);
+}
+
+/* the plan's scratch: per stream the largest need of its launches */
+static ncg_status_t
+_plan_scratch (ncg_batch_t *b, ncg_bplan_t *P)
+{
+  const int ntc = (P->ntcp < NCG_BATCH_TC_STREAMS) ? P->ntcp : NCG_BATCH_TC_STREAMS;
+  size_t need[NCG_BATCH_BR_STREAMS] = { 0 }, total = 0;
+
+  if (P->prm.tc == 2)
+  {
+    for (int k = 0; k < P->nbrp; k++)
+    {
+      const size_t s = _launch_scratch (b, P->brp[k], P->brk[k]);
+
+      if (s > need[P->brs[k]])
+        need[P->brs[k]] = s;
+    }
+  }
+  else
+  {
+    for (int k = 0; k < P->ntcp; k++)
+    {
+      const size_t s = _launch_scratch (b, P->tcp[k], 2);
+
+      if (s > need[k % ntc])
+        need[k % ntc] = s;
+    }
+  }
+
+  for (int t = 0; t < NCG_BATCH_BR_STREAMS; t++)
+  {
+    P->scr_off[t] = total;
+    total        += (need[t] + 255) & ~(size_t) 255;
+  }
+
+  return _reserve (&P->dscr, &P->cap_scr, total);
+}
+
 static ncg_status_t
 _build_plan (ncg_batch_t *b, int mixed)
 {
@@ -424,14 +559,18 @@ _build_plan (ncg_batch_t *b, int mixed)
   {
     int32_t *t = realloc (P->brp, sizeof (int32_t) * b->n);
     int8_t *k8 = t ? realloc (P->brk, sizeof (int8_t) * b->n) : NULL;
+    int8_t *s8 = k8 ? realloc (P->brs, sizeof (int8_t) * b->n) : NULL;
 
     if (t)
       P->brp = t;
 
-    if (k8 == NULL)
+    if (k8)
+      P->brk = k8;
+
+    if (s8 == NULL)
       return NCG_ERR_OUT_OF_MEMORY;
 
-    P->brk     = k8;
+    P->brs     = s8;
     P->cap_brp = b->n;
   }
 
@@ -456,23 +595,14 @@ _build_plan (ncg_batch_t *b, int mixed)
 
       tmix = (sd->mixed_kappa <= NCG_MIXED_KAPPA_MAX);
 
-      /* a tensor-core problem: its operand passes its check; its scratch is
-       * reserved now, since nothing may allocate inside the captured graph */
+      /* a tensor-core problem: its operand passes its check */
       if (tmix && prm->tc && ncg_tc_supported (sd->kind, sd->dp))
       {
         if ((r = ncg_sd_ensure_tc (sd)) != NCG_OK)
           return r;
 
         if (sd->tc_ok)
-        {
-          if ((r = ncg_sd_reserve (sd, (void **) &sd->dscratch, &sd->cap.scratch,
-                                   ncg_tc_scratch_bytes ((int64_t) b->m[i], (int) sd->nk, sd->dp))) != NCG_OK)
-            return r;
-
-          CK (cudaStreamSynchronize (sd->stream), "sync");
-
           P->tcp[P->ntcp++] = i;
-        }
       }
     }
 
@@ -480,29 +610,17 @@ _build_plan (ncg_batch_t *b, int mixed)
       P->n_fp64_tiles++;
 
     /* the branch schedule: a problem off the tensor cores runs its own
-     * specialised tile kernel (FP32 SIMT, or FP64), whose scratch is
-     * reserved now */
+     * specialised tile kernel (FP32 SIMT, or FP64) */
     if (prm->tc == 2)
     {
       const int on_tc = (P->ntcp > 0 && P->tcp[P->ntcp - 1] == i);
 
       P->brk[P->nbrp]   = on_tc ? 2 : ((mixed && tmix) ? 1 : 0);
       P->brp[P->nbrp++] = i;
-
-      if (!on_tc)
-      {
-        ncg_eval_args_t a;
-
-        ncg_sd_fill_args (sd, b->m[i], &a);
-
-        if ((r = ncg_sd_reserve (sd, (void **) &sd->dscratch, &sd->cap.scratch,
-                                 ncg_eval_scratch_bytes (&a, (mixed && tmix) ? NCG_PREC_MIXED_SIMT : NCG_PREC_FP64)))
-            != NCG_OK)
-          return r;
-
-        CK (cudaStreamSynchronize (sd->stream), "sync");
-      }
     }
+
+    /* what was built above was built on the handle's stream */
+    CK (cudaStreamSynchronize (sd->stream), "sync");
 
     memset (q, 0, sizeof (*q));
     ncg_sd_fill_args (sd, b->m[i], &q->a);
@@ -520,6 +638,9 @@ _build_plan (ncg_batch_t *b, int mixed)
     P->pairs  += (int64_t) b->m[i] * (int64_t) sd->nk;
     b->gen[i]  = sd->gen;
   }
+
+  if ((r = _branch_streams (b, P)) != NCG_OK || (r = _plan_scratch (b, P)) != NCG_OK)
+    return r;
 
   /* launches and grids */
   P->nlaunch = prm->split ? 2 : 1;
@@ -701,8 +822,9 @@ _enqueue_tc (ncg_batch_t *b, ncg_bplan_t *P, const double *dX, double *dout)
 
     ncg_sd_fill_args (sd, b->m[i], &a);
     CK (ncg_launch_eval_tc (&a, dX + b->x_off[i], sd->dtcB, sd->dmu, sd->dVg,
-                            ncg_packmx_cshift (sd->dpackmx, sd->kind, (int) sd->nk, sd->dp), sd->dscratch,
-                            dout + b->out_off[i], sd->d_flag_alias, NULL, b->stc[k % ns]), "batch eval_tc");
+                            ncg_packmx_cshift (sd->dpackmx, sd->kind, (int) sd->nk, sd->dp),
+                            (char *) P->dscr + P->scr_off[k % ns], dout + b->out_off[i], sd->d_flag_alias, NULL,
+                            b->stc[k % ns]), "batch eval_tc");
   }
 
   for (int k = 0; k < ns; k++)
@@ -714,83 +836,45 @@ _enqueue_tc (ncg_batch_t *b, ncg_bplan_t *P, const double *dX, double *dout)
   return NCG_OK;
 }
 
-typedef struct { double cost; int32_t k; } _brc_t;
-
-static int
-_brc_desc (const void *x, const void *y)
-{
-  const _brc_t *a = x, *c = y;
-
-  if (a->cost > c->cost) return -1;
-  if (a->cost < c->cost) return 1;
-  return (a->k < c->k) ? -1 : (a->k > c->k);
-}
-
 /* The branch schedule (tc = 2): every problem is one launch of the kernel its
  * own eval would use (tensor cores, FP32 SIMT tiles or FP64 tiles), the
- * problems spread over NCG_BATCH_BR_STREAMS streams forked from s1, largest
- * first, each to the stream with the least work so far (longest processing
- * time first); captured, the streams are parallel branches of the graph. */
+ * problems spread over NCG_BATCH_BR_STREAMS streams forked from s1
+ * (_branch_streams); captured, the streams are parallel branches of the graph. */
 static ncg_status_t
 _enqueue_branches (ncg_batch_t *b, ncg_bplan_t *P, const double *dX, double *dout)
 {
   const int ns = (P->nbrp < NCG_BATCH_BR_STREAMS) ? P->nbrp : NCG_BATCH_BR_STREAMS;
-  double load[NCG_BATCH_BR_STREAMS];
-  _brc_t *ord;
 
   if (ns == 0)
     return NCG_OK;
-
-  if ((ord = malloc (sizeof (_brc_t) * P->nbrp)) == NULL)
-    return NCG_ERR_OUT_OF_MEMORY;
-
-  for (int k = 0; k < P->nbrp; k++)
-  {
-    const int i = P->brp[k];
-
-    /* tensor-core pairs at about a quarter of the FP32 SIMT pair time */
-    ord[k].cost = (double) b->m[i] * (double) b->sd[i]->nk * _pair_cost (b->sd[i]) * ((P->brk[k] == 2) ? 0.25 : 1.0);
-    ord[k].k    = k;
-  }
-
-  qsort (ord, P->nbrp, sizeof (_brc_t), _brc_desc);
 
   {
     ncg_status_t r = ncg_cuda_status (cudaEventRecord (b->ev_fork, b->s1), "record");
 
     for (int k = 0; k < ns && r == NCG_OK; k++)
-    {
-      load[k] = 0.0;
-      r       = ncg_cuda_status (cudaStreamWaitEvent (b->sbr[k], b->ev_fork, 0), "wait");
-    }
+      r = ncg_cuda_status (cudaStreamWaitEvent (b->sbr[k], b->ev_fork, 0), "wait");
 
-    for (int q = 0; q < P->nbrp && r == NCG_OK; q++)
+    for (int k = 0; k < P->nbrp && r == NCG_OK; k++)
     {
-      const int k   = ord[q].k, i = P->brp[k];
-      ncg_sd_t *sd  = b->sd[i];
-      int best      = 0;
+      const int i    = P->brp[k];
+      ncg_sd_t *sd   = b->sd[i];
+      cudaStream_t s = b->sbr[P->brs[k]];
+      void *scratch  = (char *) P->dscr + P->scr_off[P->brs[k]];
       ncg_eval_args_t a;
 
-      for (int t = 1; t < ns; t++)
-        if (load[t] < load[best])
-          best = t;
-
-      load[best] += ord[q].cost;
       ncg_sd_fill_args (sd, b->m[i], &a);
 
       if (P->brk[k] == 2)
         r = ncg_cuda_status (ncg_launch_eval_tc (&a, dX + b->x_off[i], sd->dtcB, sd->dmu, sd->dVg,
                                                  ncg_packmx_cshift (sd->dpackmx, sd->kind, (int) sd->nk, sd->dp),
-                                                 sd->dscratch, dout + b->out_off[i], sd->d_flag_alias, NULL,
-                                                 b->sbr[best]), "batch eval_tc");
+                                                 scratch, dout + b->out_off[i], sd->d_flag_alias, NULL, s),
+                             "batch eval_tc");
       else if (P->brk[k] == 1)
         r = ncg_cuda_status (ncg_launch_eval_m2lnp_mixed (&a, dX + b->x_off[i], sd->dpackmx, sd->dmu, sd->dVg,
-                                                          dout + b->out_off[i], sd->dscratch, b->sbr[best]),
-                             "batch eval_mixed");
+                                                          dout + b->out_off[i], scratch, s), "batch eval_mixed");
       else
         r = ncg_cuda_status (ncg_launch_eval_m2lnp_fp64 (&a, dX + b->x_off[i], sd->dpack64, sd->dc, sd->dVg,
-                                                         dout + b->out_off[i], sd->dscratch, 0, b->sbr[best]),
-                             "batch eval_fp64");
+                                                         dout + b->out_off[i], scratch, 0, s), "batch eval_fp64");
     }
 
     for (int k = 0; k < ns && r == NCG_OK; k++)
@@ -800,8 +884,6 @@ _enqueue_branches (ncg_batch_t *b, ncg_bplan_t *P, const double *dX, double *dou
       if (r == NCG_OK)
         r = ncg_cuda_status (cudaStreamWaitEvent (b->s1, b->ev_br[k], 0), "wait");
     }
-
-    free (ord);
 
     return r;
   }
