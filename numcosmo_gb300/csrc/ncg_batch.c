@@ -42,7 +42,9 @@ enum { BP_FP64 = 0, BP_MIXED = 1 };
 
 typedef struct ncg_bplan
 {
-  int valid;                   /* built for the current problem list and generations */
+  int valid;                   /* built for the current problem list */
+  uint64_t *gen;               /* and for these generations of its handles (each plan has its own) */
+  int cap_gen;
   ncg_batch_params_t prm;
   int tuned;
   int nlaunch;                 /* 1, or 2 for the split schedule */
@@ -84,7 +86,7 @@ struct ncg_batch
   cudaEvent_t ev_in, ev_fork, ev_join, ev_out, t0, t1, ev_tc[NCG_BATCH_TC_STREAMS], ev_br[NCG_BATCH_BR_STREAMS];
   int n, cap;
   ncg_sd_t **sd;
-  uint64_t *m, *gen;
+  uint64_t *m;
   int64_t *x_off, *out_off;
   int64_t x_total, out_total;
   ncg_bplan_t plan[2];
@@ -107,6 +109,7 @@ static void
 _plan_free (ncg_bplan_t *p)
 {
   _plan_release (p);
+  free (p->gen);
   free (p->hp);
   free (p->hitems);
   free (p->tcp);
@@ -245,7 +248,6 @@ ncg_batch_free (ncg_batch_t *b)
   cudaStreamDestroy (b->s2);
   free (b->sd);
   free (b->m);
-  free (b->gen);
   free (b->x_off);
   free (b->out_off);
   free (b);
@@ -277,18 +279,17 @@ ncg_batch_add (ncg_batch_t *b, ncg_sd_t *sd, uint64_t m, int32_t *slot)
   if (b->n == b->cap)
   {
     const int nc = b->cap ? 2 * b->cap : 64;
-    void *p[5] = {
-      realloc (b->sd, sizeof (*b->sd) * nc), realloc (b->m, sizeof (*b->m) * nc), realloc (b->gen, sizeof (*b->gen) * nc),
+    void *p[4] = {
+      realloc (b->sd, sizeof (*b->sd) * nc), realloc (b->m, sizeof (*b->m) * nc),
       realloc (b->x_off, sizeof (*b->x_off) * nc), realloc (b->out_off, sizeof (*b->out_off) * nc),
     };
 
     if (p[0]) b->sd = p[0];
     if (p[1]) b->m = p[1];
-    if (p[2]) b->gen = p[2];
-    if (p[3]) b->x_off = p[3];
-    if (p[4]) b->out_off = p[4];
+    if (p[2]) b->x_off = p[2];
+    if (p[3]) b->out_off = p[3];
 
-    if (!p[0] || !p[1] || !p[2] || !p[3] || !p[4])
+    if (!p[0] || !p[1] || !p[2] || !p[3])
       return NCG_ERR_OUT_OF_MEMORY;
 
     b->cap = nc;
@@ -296,7 +297,6 @@ ncg_batch_add (ncg_batch_t *b, ncg_sd_t *sd, uint64_t m, int32_t *slot)
 
   b->sd[b->n]      = sd;
   b->m[b->n]       = m;
-  b->gen[b->n]     = 0;
   b->x_off[b->n]   = b->x_total;
   b->out_off[b->n] = b->out_total;
   b->x_total      += (int64_t) m * sd->d;
@@ -541,6 +541,17 @@ _build_plan (ncg_batch_t *b, int mixed)
     P->hp = hp;
   }
 
+  if (P->cap_gen < b->n)
+  {
+    uint64_t *g = realloc (P->gen, sizeof (uint64_t) * b->n);
+
+    if (g == NULL)
+      return NCG_ERR_OUT_OF_MEMORY;
+
+    P->gen     = g;
+    P->cap_gen = b->n;
+  }
+
   if (P->cap_tcp < b->n)
   {
     int32_t *t = realloc (P->tcp, sizeof (int32_t) * b->n);
@@ -636,7 +647,7 @@ _build_plan (ncg_batch_t *b, int mixed)
     q->bx      = (int32_t) ((b->m[i] + 127) / 128);
     total     += (double) b->m[i] * (double) sd->nk * _pair_cost (sd);
     P->pairs  += (int64_t) b->m[i] * (int64_t) sd->nk;
-    b->gen[i]  = sd->gen;
+    P->gen[i]  = sd->gen;
   }
 
   if ((r = _branch_streams (b, P)) != NCG_OK || (r = _plan_scratch (b, P)) != NCG_OK)
@@ -933,7 +944,7 @@ _stale (ncg_batch_t *b, const ncg_bplan_t *P)
     return 1;
 
   for (int i = 0; i < b->n; i++)
-    if (b->sd[i]->gen != b->gen[i] || !b->sd[i]->prepared)
+    if (b->sd[i]->gen != P->gen[i] || !b->sd[i]->prepared)
       return 1;
 
   return 0;

@@ -55,3 +55,25 @@ def test_one_handle_twice(gpu, precision, tc):
         assert np.max(np.abs(one[:333] - two)) <= 1e-6 * np.max(np.abs(two))
         if precision == 0:
             assert np.max(np.abs(one[:333] - two)) <= 1e-13 * np.max(np.abs(two))
+
+
+def test_both_plans_follow_a_new_prepare(gpu):
+    """The FP64 and the mixed plan are each rebuilt after their handles were prepared again."""
+    ng = gpu
+    F, M = ng.Precision.FP64, ng.Precision.MIXED
+    probs = [_problem(ng, *s, seed=60 + i) for i, s in enumerate(SHAPES)]
+    pts = [P for _, _, P in probs]
+    b = ng.Batch()
+    for sd, _, P in probs:
+        b.add(sd, len(P))
+    b.eval_m2lnp(pts, F)
+    b.eval_m2lnp(pts, M)
+    for sd, X, _ in probs:
+        sd.set_sample(X[::-1] * 1.3 + 0.2)
+        sd.prepare()
+    got = b.eval_m2lnp(pts, F), b.eval_m2lnp(pts, M)
+    fresh = ng.Batch()
+    for sd, _, P in probs:
+        fresh.add(sd, len(P))
+    for g, p in zip(got, (F, M)):
+        assert all(np.array_equal(x, y) for x, y in zip(g, fresh.eval_m2lnp(pts, p)))
