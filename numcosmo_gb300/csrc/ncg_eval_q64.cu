@@ -77,6 +77,7 @@
 #define Q_S 4.0                       /* the homogeneous coordinate         */
 #define Q_CHUNK 8192                  /* points per launch (scratch)        */
 #define Q_BAD_E 0x7fffffff            /* a point with a non-finite coordinate */
+#define Q_BAD_F 0x3fffffff            /* f of a kernel whose operand is not finite */
 
 __host__ __device__ static inline int
 q_bits (int d)
@@ -150,6 +151,13 @@ __device__ __forceinline__ int
 _exp_above (double x)
 {
   return (int) (((uint32_t) __double2hiint (x) >> 20) & 0x7ffu) - 1022;
+}
+
+/* inf or NaN */
+__device__ __forceinline__ bool
+_not_finite (double x)
+{
+  return ((uint32_t) __double2hiint (x) >> 20 & 0x7ffu) == 0x7ffu;
 }
 
 /* 2^e, e clamped to the normal range */
@@ -372,8 +380,10 @@ _q_build_B_kernel (const double *__restrict__ X, const double *__restrict__ pack
 
   __syncwarp ();
 
-  /* P = W'^T W', packed as its lower triangle (b, a), a <= b */
+  /* P = W'^T W', packed as its lower triangle (b, a), a <= b; a maximum leaves
+   * a NaN out, so what is not finite is noted beside it */
   double mx = 0.0;
+  bool bad  = false;
 
   for (int e = lane; e < T; e += 32)
   {
@@ -396,6 +406,7 @@ _q_build_B_kernel (const double *__restrict__ X, const double *__restrict__ pack
     Ph[e] = acc.h;
     Pl[e] = acc.l;
     mx    = fmax (mx, (a == b) ? acc.h : 2.0 * fabs (acc.h));
+    bad   = bad || _not_finite (acc.h);
   }
 
   __syncwarp ();
@@ -431,6 +442,7 @@ _q_build_B_kernel (const double *__restrict__ X, const double *__restrict__ pack
   cst.h *= -0.5 / Q_S;
   cst.l *= -0.5 / Q_S;
   mx     = fmax (fmax (mx, fabs (lin.h)), fabs (cst.h));
+  bad    = __any_sync (0xffffffffu, bad || _not_finite (lin.h) || _not_finite (cst.h) || _not_finite (mx));
 
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1)
@@ -444,7 +456,7 @@ _q_build_B_kernel (const double *__restrict__ X, const double *__restrict__ pack
   if (lane == 0)
   {
     sck[i] = fac * _pow2 (f - 2 * (bits - 1) - 9 * bits);
-    atomicMax (fmax_, f);
+    atomicMax (fmax_, bad ? Q_BAD_F : f);
   }
 
   /* lin and cst beside theta' (which is done with) */
