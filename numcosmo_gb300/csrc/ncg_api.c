@@ -1614,8 +1614,8 @@ _eval_device (ncg_sd_t *sd, const double *dXq, uint64_t m, double *dout, int lin
     if (sd->q64_ready == 1)
     {
       RESERVE (dscratch, scratch, ncg_q64_scratch_bytes (&a));
-      CK (ncg_launch_eval_q64 (&a, dXq, sd->dq64, sd->dc, sd->dmu, sd->dVg, dout, sd->dscratch, linear,
-                               sd->d_flag_alias, sd->stream), "eval_q64");
+      CK (ncg_launch_eval_q64 (&a, dXq, sd->dq64, sd->dpack64, sd->dc, sd->dmu, sd->dVg, dout, sd->dscratch,
+                               linear, sd->d_flag_alias, sd->stream), "eval_q64");
 
       return NCG_OK;
     }

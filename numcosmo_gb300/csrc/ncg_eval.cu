@@ -879,17 +879,6 @@ ncg_launch_merge_f2 (const void *part, int nparts, int64_t m, double shift, cons
   return cudaGetLastError ();
 }
 
-/* merge of FP64 (g, s) pairs written by another kernel */
-extern "C" cudaError_t
-ncg_launch_merge_d2 (const double2 *part, int nparts, int64_t m, double shift, double d_ln_href, int linear,
-                     double *out, cudaStream_t s)
-{
-  _merge_kernel<double2><<<(unsigned) ((m + 31) / 32), MG_TH, 0, s>>> (part, nparts, m, shift, NULL, d_ln_href, linear,
-                                                                      out);
-
-  return cudaGetLastError ();
-}
-
 /* device address of the constant C0 = max_i c_i stored behind the mixed pack */
 extern "C" const double *
 ncg_packmx_cshift (const float *packmx, int kind, int n, int dp)

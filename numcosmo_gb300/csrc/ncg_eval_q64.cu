@@ -28,9 +28,11 @@
  * o <= 6); sums of higher orders would have to align hundreds of extreme
  * digits to round, by a unit of 2^-61 or less.  Orders above 9 are dropped.
  * The fixed point is absolute: chi^2 is off by about sqrt(K) 2^(2e + f - 10 B),
- * against roughly 2^-52 chi^2 |W| |x| / |y| of the plain form's own roundings,
- * so the operand is used only where the largest f is at most Q64_FMAX(B)
- * (narrower kernels keep the plain form); x', W', P and theta' are formed in
+ * against roughly 2^-52 chi^2 |W| |x| / |y| of the plain form's own roundings.
+ * So a point with 2e + f above 10 B - 52, f the largest of the kernels (q_range:
+ * points far outside the sample, or any in the presence of very narrow kernels), is
+ * left to the merge, which evaluates it in the plain form; and where the largest f is above
+ * q_fmax, which leaves no room for points, all are.  x', W', P and theta' are formed in
  * double-double, so nothing else enters.
  *
  * Kernel.  Tiles of 128 points x 48 kernels.  Per 16 features (a K step) the
@@ -55,6 +57,7 @@
 #include <stdint.h>
 
 #include "ncg_internal.h"
+#include "ncg_eval_tiles.cuh"
 #include "ncg_fastmath.cuh"
 #include "ncg_tc_ptx.cuh"
 
@@ -76,7 +79,7 @@
 #define Q_KPW (Q_NK / Q_WG)           /* kernels per epilogue warp          */
 #define Q_S 4.0                       /* the homogeneous coordinate         */
 #define Q_CHUNK 8192                  /* points per launch (scratch)        */
-#define Q_BAD_E 0x7fffffff            /* a point with a non-finite coordinate */
+#define Q_FAR 0x7fffffff              /* exponent of a point that takes the plain form */
 #define Q_BAD_F 0x3fffffff            /* f of a kernel whose operand is not finite */
 
 __host__ __device__ static inline int
@@ -85,8 +88,15 @@ q_bits (int d)
   return d <= 16 ? 8 : 7;
 }
 
-/* largest f: chi^2 then stays within about 2^-47 absolute for points inside
- * the sample (2e = 6) */
+/* largest 2e + f: the rounding of chi^2 stays within sqrt (K) 2^-52 (3e-15 at d = 16,
+ * 5e-15 at d = 32) */
+__host__ __device__ static inline int
+q_range (int d)
+{
+  return 10 * q_bits (d) - 52;
+}
+
+/* largest f, for points inside the sample (2e = 6 or 8) */
 __host__ __device__ static inline int
 q_fmax (int d)
 {
@@ -507,10 +517,12 @@ q_build_a_warp (int d)
   return (size_t) (4 * NCG_DMAX + 4) * 8 + (size_t) Q_NS * q_steps (d) * 16 * 2;
 }
 
-/* one warp per point; rows past m are zero.  Also clears the error word. */
+/* one warp per point; rows past m are zero, and those of points past q_range.  Also
+ * clears the error word. */
 __global__ void __launch_bounds__ (QA_WARPS * 32)
 _q_build_A_kernel (const double *__restrict__ Xq, int64_t m, int d, const double *__restrict__ Vg,
-                   const double *__restrict__ mu, uint8_t *__restrict__ A, int32_t *__restrict__ pe2, int *err)
+                   const double *__restrict__ mu, const int32_t *__restrict__ fmax_, uint8_t *__restrict__ A,
+                   int32_t *__restrict__ pe2, int *err)
 {
   extern __shared__ __align__ (16) uint8_t q_smem[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -561,7 +573,10 @@ _q_build_A_kernel (const double *__restrict__ Xq, int64_t m, int d, const double
   /* past 2^510 chi^2 leaves FP64 (or the coordinates did, NaN included) */
   finite = finite && mx < 0x1p510;
 
-  const int e      = finite ? _exp_above (fmax (mx, Q_S)) : 0;
+  const int f = *fmax_, e = finite ? _exp_above (fmax (mx, Q_S)) : 0;
+
+  finite = finite && f <= q_fmax (d) && 2 * e + f <= q_range (d);
+
   const double sc  = finite ? _pow2 (-e) : 0.0;
 
   if (lane < d)
@@ -574,7 +589,7 @@ _q_build_A_kernel (const double *__restrict__ Xq, int64_t m, int d, const double
   {
     zh[d]  = finite ? Q_S * sc : 0.0;
     zl[d]  = 0.0;
-    pe2[j] = finite ? 2 * e : Q_BAD_E;
+    pe2[j] = finite ? 2 * e : Q_FAR;
   }
 
   __syncwarp ();
@@ -603,12 +618,12 @@ _q_build_A_kernel (const double *__restrict__ Xq, int64_t m, int d, const double
 struct QParams
 {
   const uint8_t *A, *B;
-  const int32_t *pe2;
+  const int32_t *pe2, *f;
   const double *sck, *c;
   double2 *part;          /* [Q_WG nslices][m] */
   int *err, *flag_host;
   int64_t m;
-  int n, steps, npt, nkt, nslices, tps;
+  int n, steps, npt, nkt, nslices, tps, fmax_;
   double kappa;
   int fault;
 };
@@ -693,6 +708,10 @@ _eval_q64_kernel (const QParams p)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nunits = p.npt * p.nslices;
   volatile int *err = &sm.err;
+
+  /* every point is left to the merge */
+  if (*p.f > p.fmax_)
+    return;
 
   if (threadIdx.x == 0)
   {
@@ -888,11 +907,11 @@ _eval_q64_kernel (const QParams p)
           if (i0 + k >= p.n)
             break;
 
-          /* the kernel's scale times 2^(2e), on the exponent (NaN for a bad
-           * point: its terms are left out) */
+          /* the kernel's scale times 2^(2e), on the exponent (NaN for a point of the
+           * merge's: its terms are left out) */
           const double sk = __ldg (p.sck + i0 + k), c = __ldg (p.c + i0 + k);
           const int hs    = __double2hiint (sk), ex = ((hs >> 20) & 0x7ff) + e2;
-          const double sc = (e2 == Q_BAD_E) ? CUDART_NAN
+          const double sc = (e2 == Q_FAR)   ? CUDART_NAN
                             : (ex > 0x7fe)  ? __hiloint2double ((hs & 0x80000000) | 0x7ff00000, 0)
                                             : __hiloint2double ((hs & 0x800fffff) | (ex << 20), __double2loint (sk));
 
@@ -925,6 +944,153 @@ _eval_q64_kernel (const QParams p)
 
     if (p.flag_host != NULL)
       *(volatile int *) p.flag_host = 1;
+  }
+}
+
+/* --------------------------------------------------------------------- merge */
+
+#define QM_TH 256
+
+struct QMerge
+{
+  const double2 *part;
+  const int32_t *pe2;
+  const double *Xq, *pack, *c;
+  double *out;
+  int64_t m;
+  int nparts, n, d, dp, linear;
+  double kappa, inv_nu, shift, d_ln_href;
+};
+
+/* this thread's kernels against the point xs, by the plain form (a kernel per
+ * thread; the whitened difference in local memory, since d is not a constant here) */
+template <int KERN>
+__device__ __noinline__ double2
+_q_plain (const QMerge &p, const double *xs)
+{
+  const int S = ncg_pack64_stride (NCG_VKDE, p.dp);
+  double dl[NCG_DMAX];
+  double g = NCG_LSE_EMPTY, s = 0.0;
+
+  for (int i = threadIdx.x; i < p.n; i += QM_TH)
+  {
+    const double *pk = p.pack + (size_t) i * S, *W = pk + p.dp;
+    double chi2      = 0.0;
+
+    for (int c = 0; c < p.d; c++)
+      dl[c] = xs[c] - pk[c];
+
+    for (int r = 0; r < p.d; r++)
+    {
+      double y = 0.0;
+
+      for (int c = 0; c <= r; c++)
+        y = fma (*W++, dl[c], y);
+
+      chi2 = fma (y, y, chi2);
+    }
+
+    ncg_lse_add (ncg_lnt_64<KERN> (chi2, p.c[i], p.kappa, p.inv_nu, false), g, s);
+  }
+
+  return make_double2 (g, s);
+}
+
+/* The slices of 32 points, as the merge of the plain form (ncg_eval.cu) combines
+ * them; then, one after the other, those of the points that take the plain form,
+ * the CTA's threads sharing the kernels.  Nothing is left to do there in a call on points
+ * like the sample's. */
+template <int KERN>
+__global__ void __launch_bounds__ (QM_TH)
+_q_merge_kernel (const QMerge p)
+{
+  __shared__ double red[QM_TH / 32][33];
+  __shared__ double xs[NCG_DMAX];
+  __shared__ double2 ex[QM_TH / 32];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int64_t j = (int64_t) blockIdx.x * 32 + lane;
+  const bool far_ = j < p.m && p.pe2[j] == Q_FAR, in = j < p.m && !far_;
+  double G = NCG_LSE_EMPTY, S = 0.0;
+
+  if (in)
+    for (int s = w; s < p.nparts; s += QM_TH / 32)
+      G = fmax (G, p.part[(size_t) s * p.m + j].x);
+
+  red[w][lane] = G;
+  __syncthreads ();
+
+#pragma unroll
+  for (int q = 0; q < QM_TH / 32; q++)
+    G = fmax (G, red[q][lane]);
+
+  __syncthreads ();
+
+  if (in)
+    for (int s = w; s < p.nparts; s += QM_TH / 32)
+    {
+      const double2 q = p.part[(size_t) s * p.m + j];
+
+      S = fma (q.y, ncg_exp (q.x - G), S);
+    }
+
+  red[w][lane] = S;
+  __syncthreads ();
+
+  if (w == 0 && in)
+  {
+#pragma unroll
+    for (int q = 1; q < QM_TH / 32; q++)
+      S += red[q][lane];
+
+    const double lnp = ncg_lse_lnp (G, S, p.shift, NULL, p.d_ln_href);
+
+    p.out[j] = p.linear ? exp (lnp) : -2.0 * lnp;
+  }
+
+  /* the same 32 points in every warp */
+  for (uint32_t mask = __ballot_sync (0xffffffffu, far_); mask; mask &= mask - 1)
+  {
+    const int64_t jf = (int64_t) blockIdx.x * 32 + __ffs (mask) - 1;
+
+    __syncthreads ();
+
+    if (tid < p.d)
+      xs[tid] = p.Xq[jf * p.d + tid];
+
+    __syncthreads ();
+
+    const double2 q = _q_plain<KERN> (p, xs);
+    double M = q.x, T = q.y;
+
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      M = fmax (M, __shfl_xor_sync (0xffffffffu, M, o));
+
+    T *= ncg_exp (q.x - M);
+
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      T += __shfl_xor_sync (0xffffffffu, T, o);
+
+    if (lane == 0)
+      ex[w] = make_double2 (M, T);
+
+    __syncthreads ();
+
+    if (tid == 0)
+    {
+      for (int k = 1; k < QM_TH / 32; k++)
+      {
+        const double N = fmax (M, ex[k].x);
+
+        T = T * ncg_exp (M - N) + ex[k].y * ncg_exp (ex[k].x - N);
+        M = N;
+      }
+
+      const double lnp = ncg_lse_lnp (M, T, p.shift, NULL, p.d_ln_href);
+
+      p.out[jf] = p.linear ? exp (lnp) : -2.0 * lnp;
+    }
   }
 }
 
@@ -1063,15 +1229,22 @@ _run_q64 (const QParams &p, int grid, cudaStream_t s)
 
 template <int KERN>
 static cudaError_t
-_run_q64_bits (const QParams &p, int d, int grid, cudaStream_t s)
+_run_q64_bits (const QParams &p, const QMerge &q, int d, int grid, cudaStream_t s)
 {
-  return (d <= 16) ? _run_q64<KERN, 8> (p, grid, s) : _run_q64<KERN, 7> (p, grid, s);
+  const cudaError_t e = (d <= 16) ? _run_q64<KERN, 8> (p, grid, s) : _run_q64<KERN, 7> (p, grid, s);
+
+  if (e != cudaSuccess)
+    return e;
+
+  _q_merge_kernel<KERN><<<(unsigned) ((q.m + 31) / 32), QM_TH, 0, s>>> (q);
+
+  return cudaGetLastError ();
 }
 
 extern "C" cudaError_t
-ncg_launch_eval_q64 (const ncg_eval_args_t *a, const double *Xq, const uint8_t *op, const double *c,
-                     const double *mu, const double *Vg, double *out, void *scratch, int linear, int *flag_host,
-                     cudaStream_t s)
+ncg_launch_eval_q64 (const ncg_eval_args_t *a, const double *Xq, const uint8_t *op, const double *pack64,
+                     const double *c, const double *mu, const double *Vg, double *out, void *scratch, int linear,
+                     int *flag_host, cudaStream_t s)
 {
   static int limit[NCG_MAX_DEVICES];
   const q_scratch_t o = _q_scratch (a);
@@ -1093,6 +1266,8 @@ ncg_launch_eval_q64 (const ncg_eval_args_t *a, const double *Xq, const uint8_t *
   p.A         = (const uint8_t *) scratch;
   p.B         = op;
   p.pe2       = (const int32_t *) ((uint8_t *) scratch + o.pe2);
+  p.f         = (const int32_t *) (op + b.fmax);
+  p.fmax_     = q_fmax (a->d);
   p.sck       = (const double *) (op + b.sck);
   p.c         = c;
   p.part      = (double2 *) ((uint8_t *) scratch + o.part);
@@ -1114,19 +1289,19 @@ ncg_launch_eval_q64 (const ncg_eval_args_t *a, const double *Xq, const uint8_t *
     p.npt = (int) ((mc + Q_M - 1) / Q_M);
 
     _q_build_A_kernel<<<p.npt * (Q_M / QA_WARPS), QA_WARPS * 32, smem, s>>> (
-      Xq + j0 * a->d, mc, a->d, Vg, mu, (uint8_t *) scratch, (int32_t *) p.pe2, p.err);
+      Xq + j0 * a->d, mc, a->d, Vg, mu, p.f, (uint8_t *) scratch, (int32_t *) p.pe2, p.err);
 
     if ((e = cudaGetLastError ()) != cudaSuccess)
       return e;
 
     const int units = p.npt * p.nslices, grid = units < nsm ? units : nsm;
 
-    e = (a->kernel == NCG_KERNEL_GAUSS)  ? _run_q64_bits<NCG_KERNEL_GAUSS> (p, a->d, grid, s)
-        : ncg_nu_wide (a->nu, a->d)      ? _run_q64_bits<NCG_KERNEL_ST_WIDE> (p, a->d, grid, s)
-                                         : _run_q64_bits<NCG_KERNEL_ST> (p, a->d, grid, s);
+    const QMerge q = { p.part, p.pe2, Xq + j0 * a->d, pack64, c, out + j0, mc, Q_WG * o.ns, a->n, a->d, a->dp, linear,
+                       a->kappa, 1.0 / a->nu, a->final_shift, a->d_ln_href };
 
-    if (e == cudaSuccess)
-      e = ncg_launch_merge_d2 (p.part, Q_WG * o.ns, mc, a->final_shift, a->d_ln_href, linear, out + j0, s);
+    e = (a->kernel == NCG_KERNEL_GAUSS)  ? _run_q64_bits<NCG_KERNEL_GAUSS> (p, q, a->d, grid, s)
+        : ncg_nu_wide (a->nu, a->d)      ? _run_q64_bits<NCG_KERNEL_ST_WIDE> (p, q, a->d, grid, s)
+                                         : _run_q64_bits<NCG_KERNEL_ST> (p, q, a->d, grid, s);
 
     if (e != cudaSuccess)
       return e;

@@ -166,11 +166,9 @@ const int32_t *ncg_q64_operand_fmax (const uint8_t *op, int n, int d);
 cudaError_t ncg_launch_q64_operand (const ncg_eval_args_t *a, const double *X, const double *pack64, const double *U,
                                     const double *Vg, const double *mu, uint8_t *op, cudaStream_t s);
 size_t      ncg_q64_scratch_bytes (const ncg_eval_args_t *a);
-cudaError_t ncg_launch_eval_q64 (const ncg_eval_args_t *a, const double *Xq, const uint8_t *op, const double *c,
-                                 const double *mu, const double *Vg, double *out, void *scratch, int linear,
-                                 int *flag_host, cudaStream_t s);
-cudaError_t ncg_launch_merge_d2 (const double2 *part, int nparts, int64_t m, double shift, double d_ln_href,
-                                 int linear, double *out, cudaStream_t s);
+cudaError_t ncg_launch_eval_q64 (const ncg_eval_args_t *a, const double *Xq, const uint8_t *op, const double *pack64,
+                                 const double *c, const double *mu, const double *Vg, double *out, void *scratch,
+                                 int linear, int *flag_host, cudaStream_t s);
 cudaError_t ncg_launch_compute_IM (const ncg_eval_args_t *a, const double *X, const double *pack64,
                                    const double *lnnorm, double kernel_lnnorm, const double *f,
                                    double *IM, cudaStream_t s);
