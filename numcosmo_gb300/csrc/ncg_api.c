@@ -248,7 +248,7 @@ _dev_free_all (ncg_sd_t *sd)
     (void **) &sd->dVg, (void **) &sd->dpackmx, (void **) &sd->dknn, (void **) &sd->dflag, (void **) &sd->dids,
     (void **) &sd->dkeys, (void **) &sd->dst, (void **) &sd->dscratch, (void **) &sd->dq,
     (void **) &sd->dqo, (void **) &sd->dqi, (void **) &sd->df, (void **) &sd->dmu, (void **) &sd->dcal, (void **) &sd->dcv, (void **) &sd->dloo,
-    (void **) &sd->drq, (void **) &sd->dq64,
+    (void **) &sd->drq, (void **) &sd->dq64, &sd->dq64s,
   };
 
   for (size_t i = 0; i < sizeof (bufs) / sizeof (bufs[0]); i++)
@@ -1613,8 +1613,9 @@ _eval_device (ncg_sd_t *sd, const double *dXq, uint64_t m, double *dout, int lin
 
     if (sd->q64_ready == 1)
     {
-      RESERVE (dscratch, scratch, ncg_q64_scratch_bytes (&a));
-      CK (ncg_launch_eval_q64 (&a, dXq, sd->dq64, sd->dpack64, sd->dc, sd->dmu, sd->dVg, dout, sd->dscratch,
+      /* scratch of its own: a recorded plain eval keeps the other */
+      RESERVE (dq64s, q64s, ncg_q64_scratch_bytes (&a));
+      CK (ncg_launch_eval_q64 (&a, dXq, sd->dq64, sd->dpack64, sd->dc, sd->dmu, sd->dVg, dout, sd->dq64s,
                                linear, sd->d_flag_alias, sd->stream), "eval_q64");
 
       return NCG_OK;

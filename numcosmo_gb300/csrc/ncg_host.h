@@ -19,7 +19,7 @@
 typedef struct ncg_caps
 {
   size_t X, Y, cov, U, Ui, lnnorm, w, c, wcum, pack64, Vg, packmx, knn, flag, ids, keys, st, scratch, q, qo, qi, f,
-         mu, cal, rq, cv, loo, q64;
+         mu, cal, rq, cv, loo, q64, q64s;
 } ncg_caps_t;
 
 /* prepare_interp / NNLS device state (ncg_interp.c) */
@@ -84,7 +84,8 @@ struct ncg_sd
   double *d_io;           /* its device address */
   uint8_t *dtcB;          /* tensor-core kernel tiles */
   size_t cap_tcB;
-  uint8_t *dq64;          /* the FP64 form's tensor-core operand */
+  uint8_t *dq64;          /* the FP64 form's tensor-core operand, and the scratch of its evals */
+  void *dq64s;
   int q64_ready;          /* 0 not built for this operand state, 1 usable, -1 out of its range */
   uint32_t k;
   uint64_t n_fallback;
