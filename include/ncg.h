@@ -169,7 +169,14 @@ ncg_status_t ncg_sd_prepare_interp (ncg_sd_t *sd, const double *m2lnp);
 ncg_status_t ncg_sd_eval_m2lnp (ncg_sd_t *sd, const double *x, double *m2lnp);
 /* the same at m points X (m x dim, host memory) in one launch */
 ncg_status_t ncg_sd_eval_m2lnp_batch (ncg_sd_t *sd, const double *X, uint64_t m, double *m2lnp);
-/* the same with device pointers, asynchronous on the handle's stream */
+/* the same with device pointers, asynchronous on the handle's stream.  It may
+ * be recorded in a CUDA graph once a call with as many points has made its
+ * buffers; replays then follow the handle's later fits of the same size.  (In
+ * the FP64 form a VKDE call of 640 points or more, d >= 5, first builds a
+ * tensor-core operand of the current fit, and where kernels turn out too
+ * narrow for it evaluates in the plain form; a capture before which that
+ * operand was not built records the plain form.  The mixed form wants a call
+ * after the last prepare.) */
 ncg_status_t ncg_sd_eval_m2lnp_device (ncg_sd_t *sd, const double *d_X, uint64_t m, double *d_m2lnp);
 
 /* eval_m2lnp in the FP64 form on device pointers, for callers that must not

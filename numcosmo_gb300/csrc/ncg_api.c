@@ -334,7 +334,7 @@ ncg_sd_new (ncg_kind_t kind, ncg_kernel_t kernel, uint32_t dim, double nu, const
       return s;
     }
 
-    sd->h_flag[0] = 0;
+    memset (sd->h_flag, 0, NCG_IO_OFFSET);
     sd->h_io      = (double *) ((char *) sd->h_flag + NCG_IO_OFFSET);
     sd->d_io      = (double *) ((char *) sd->d_flag_alias + NCG_IO_OFFSET);
   }
@@ -1172,8 +1172,8 @@ _loo_fit (ncg_sd_t *sd)
   return r;
 }
 
-ncg_status_t
-ncg_sd_prepare (ncg_sd_t *sd)
+static ncg_status_t
+_prepare (ncg_sd_t *sd)
 {
   ncg_prep_status_t st;
   const int d = (int) (sd ? sd->d : 0);
@@ -1405,6 +1405,14 @@ ncg_sd_prepare (ncg_sd_t *sd)
   return NCG_OK;
 }
 
+ncg_status_t
+ncg_sd_prepare (ncg_sd_t *sd)
+{
+  const ncg_status_t r = _prepare (sd);
+
+  return (r == NCG_OK) ? ncg_sd_q64_refresh (sd) : r;
+}
+
 /* ---------------------------------------------------------------- eval */
 
 void
@@ -1563,29 +1571,91 @@ _eval_path (ncg_sd_t *sd, int linear, ncg_status_t *r)
   return NCG_PATH_SIMT;
 }
 
-/* The FP64 form's tensor-core operand, built at the first call that takes it
- * after the kernels or the bandwidth changed (the weights are not in it);
- * q64_ready = -1 where a kernel is too narrow for its fixed point. */
-static ncg_status_t
-_ensure_q64 (ncg_sd_t *sd, const ncg_eval_args_t *a)
+/* whether the stream records a graph (a stream that cannot say does) */
+static int
+_capturing (cudaStream_t s)
 {
-  int32_t f = 0;
+  enum cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
 
-  if (sd->q64_ready)
-    return NCG_OK;
+  if (cudaStreamIsCapturing (s, &st) != cudaSuccess)
+  {
+    cudaGetLastError ();
 
+    return 1;
+  }
+
+  return st != cudaStreamCaptureStatusNone;
+}
+
+static ncg_status_t
+_build_q64 (ncg_sd_t *sd, const ncg_eval_args_t *a)
+{
   RESERVE (dq64, q64, ncg_q64_operand_bytes (a->n, a->d));
-  CK (ncg_launch_q64_operand (a, sd->dX, sd->dpack64, sd->dU, sd->dVg, sd->dmu, sd->dq64, sd->stream), "q64 operand");
-  CK (cudaMemcpyAsync (&f, ncg_q64_operand_fmax (sd->dq64, a->n, a->d), sizeof (f), cudaMemcpyDeviceToHost, sd->stream),
-      "D2H q64 range");
-  CK (cudaStreamSynchronize (sd->stream), "sync");
-  sd->q64_ready = (f <= ncg_q64_fmax (a->d)) ? 1 : -1;
+  CK (ncg_launch_q64_operand (a, sd->dX, sd->dpack64, sd->dU, sd->dVg, sd->dmu, sd->dq64,
+                              (unsigned long long *) (sd->d_flag_alias + 2), ++sd->q64_epoch, sd->stream), "q64 operand");
+  sd->q64_ready = 1;
 
   return NCG_OK;
 }
 
+/* Whether the FP64 eval of a takes the sliced products.  Their operand is built at the
+ * first call that wants it after the kernels or the bandwidth changed (the weights are not
+ * in it), without waiting: the kernels themselves look at its range, and the host
+ * learns of it from a word of mapped memory (with `wait`, for callers that
+ * synchronise anyway, at once), to go to the plain tiles where it is exceeded.
+ * The plain form also serves where there is no memory for the operand, and a
+ * capture before which it was not built. */
+int
+ncg_sd_q64_usable (ncg_sd_t *sd, const ncg_eval_args_t *a, int wait)
+{
+  if (!ncg_q64_wanted (a))
+    return 0;
+
+  if (sd->q64_ready == 0)
+  {
+    if (_capturing (sd->stream))
+      return 0;
+
+    if (_build_q64 (sd, a) != NCG_OK)
+    {
+      cudaGetLastError ();
+      sd->q64_ready = -1;
+    }
+  }
+
+  if (sd->q64_ready == 1)
+  {
+    unsigned long long w;
+
+    if (wait && cudaStreamSynchronize (sd->stream) != cudaSuccess)
+      return 0;
+
+    w = *(volatile unsigned long long *) (sd->h_flag + 2);
+
+    if ((uint32_t) (w >> 32) == sd->q64_epoch)
+      sd->q64_ready = (w & 1) ? 2 : -1;
+  }
+
+  return sd->q64_ready > 0;
+}
+
+/* a graph holds the operand's address: build it with the kernels, as the plain
+ * operand that such a graph would read otherwise */
+ncg_status_t
+ncg_sd_q64_refresh (ncg_sd_t *sd)
+{
+  ncg_eval_args_t a;
+
+  if (!sd->q64_graph || sd->q64_ready != 0)
+    return NCG_OK;
+
+  ncg_sd_fill_args (sd, 1, &a);
+
+  return _build_q64 (sd, &a);
+}
+
 static ncg_status_t
-_eval_device (ncg_sd_t *sd, const double *dXq, uint64_t m, double *dout, int linear)
+_eval_device (ncg_sd_t *sd, const double *dXq, uint64_t m, double *dout, int linear, int wait)
 {
   ncg_eval_args_t a;
   ncg_status_t r;
@@ -1606,20 +1676,27 @@ _eval_device (ncg_sd_t *sd, const double *dXq, uint64_t m, double *dout, int lin
 
   /* (a mixed request that its conditioning guard sends here keeps the plain
    * form, as in a batch) */
-  if (path == NCG_PATH_FP64 && sd->cfg.precision == NCG_PREC_FP64 && ncg_q64_wanted (&a))
+  if (path == NCG_PATH_FP64 && sd->cfg.precision == NCG_PREC_FP64 && ncg_sd_q64_usable (sd, &a, wait))
   {
-    if ((r = _ensure_q64 (sd, &a)) != NCG_OK)
-      return r;
+    const size_t need = ncg_q64_scratch_bytes (&a);
+    const int graph   = !wait && _capturing (sd->stream);
 
-    if (sd->q64_ready == 1)
+    /* scratch of its own, so that a recorded plain eval keeps the other, which is made
+     * here too: a capture after the next prepare takes the plain form; without room
+     * for it (which a capture does not make) the plain form */
+    if (!graph && ncg_sd_reserve (sd, &sd->dscratch, &sd->cap.scratch, ncg_eval_scratch_bytes (&a, NCG_PREC_FP64)) != NCG_OK)
+      cudaGetLastError ();
+
+    if (sd->cap.q64s >= need || (!graph && ncg_sd_reserve (sd, &sd->dq64s, &sd->cap.q64s, need) == NCG_OK))
     {
-      /* scratch of its own: a recorded plain eval keeps the other */
-      RESERVE (dq64s, q64s, ncg_q64_scratch_bytes (&a));
+      sd->q64_graph |= graph;
       CK (ncg_launch_eval_q64 (&a, dXq, sd->dq64, sd->dpack64, sd->dc, sd->dmu, sd->dVg, dout, sd->dq64s,
                                linear, sd->d_flag_alias, sd->stream), "eval_q64");
 
       return NCG_OK;
     }
+
+    cudaGetLastError ();
   }
 
   if (path == NCG_PATH_FP64)
@@ -1721,7 +1798,7 @@ ncg_sd_eval_m2lnp_device (ncg_sd_t *sd, const double *d_X, uint64_t m, double *d
   if (sd == NULL || (m > 0 && (d_X == NULL || d_m2lnp == NULL)))
     return NCG_ERR_INVALID_ARG;
 
-  return _eval_device (sd, d_X, m, d_m2lnp, 0);
+  return _eval_device (sd, d_X, m, d_m2lnp, 0, 0);
 }
 
 /* The FP64 eval with its per-call scratch in a static device array (see
@@ -1790,7 +1867,7 @@ _eval_host_mapped (ncg_sd_t *sd, const double *X, uint64_t m, double *out, int l
     dXq = sd->dq;
   }
 
-  r = _eval_device (sd, dXq, m, dout, linear);
+  r = _eval_device (sd, dXq, m, dout, linear, 1);
 
   /* nothing of this call may be reading the memory when the next one fills it */
   CK (cudaStreamSynchronize (sd->stream), "sync");
@@ -1835,7 +1912,7 @@ _eval_host (ncg_sd_t *sd, const double *X, uint64_t m, double *out, int linear)
   CK (ncg_launch_nonfinite (sd->dq, (int64_t) (m * sd->d), sd->d_flag_alias + 1, sd->stream), "nonfinite");
 
   {
-    ncg_status_t r = _eval_device (sd, sd->dq, m, sd->dqo, linear);
+    ncg_status_t r = _eval_device (sd, sd->dq, m, sd->dqo, linear, 1);
 
     if (r != NCG_OK)
       return r;

@@ -509,6 +509,12 @@ _q_build_B_kernel (const double *__restrict__ X, const double *__restrict__ pack
   _store_row (dig, Kp, steps, row, Q_B_STEP, Q_NK * 16, Q_B_LBO, lane);
 }
 
+__global__ void
+_q_tell_kernel (const int32_t *f, int fmax_, uint32_t epoch, unsigned long long *word)
+{
+  *(volatile unsigned long long *) word = (unsigned long long) epoch << 32 | (*f <= fmax_ ? 1u : 0u);
+}
+
 #define QA_WARPS 4
 
 __host__ __device__ static inline size_t
@@ -1109,12 +1115,6 @@ ncg_q64_wanted (const ncg_eval_args_t *a)
   return a->kind == NCG_VKDE && a->d >= 5 && a->m >= 640 && a->n >= 384 && a->n <= (1 << 24);
 }
 
-extern "C" int
-ncg_q64_fmax (int d)
-{
-  return q_fmax (d);
-}
-
 /* operand of n kernels: digits | scales (n padded) | Zl | largest f */
 typedef struct { size_t sck, zl, fmax, total; } q_operand_t;
 
@@ -1138,16 +1138,12 @@ ncg_q64_operand_bytes (int n, int d)
   return _q_operand (n, d).total;
 }
 
-/* device address of the largest f of the operand */
-extern "C" const int32_t *
-ncg_q64_operand_fmax (const uint8_t *op, int n, int d)
-{
-  return (const int32_t *) (op + _q_operand (n, d).fmax);
-}
-
+/* the operand of a's kernels; *word (mapped host memory) gets `epoch` in its upper half and
+ * whether their range leaves room for points in bit 0 */
 extern "C" cudaError_t
 ncg_launch_q64_operand (const ncg_eval_args_t *a, const double *X, const double *pack64, const double *U,
-                        const double *Vg, const double *mu, uint8_t *op, cudaStream_t s)
+                        const double *Vg, const double *mu, uint8_t *op, unsigned long long *word, uint32_t epoch,
+                        cudaStream_t s)
 {
   static int limit[NCG_MAX_DEVICES];
   const q_operand_t o = _q_operand (a->n, a->d);
@@ -1165,6 +1161,7 @@ ncg_launch_q64_operand (const ncg_eval_args_t *a, const double *X, const double 
   _q_build_B_kernel<<<npad / QB_WARPS, QB_WARPS * 32, smem, s>>> (
     X, pack64, ncg_pack64_stride (NCG_VKDE, a->dp), a->dp, a->n, a->d, U, Vg, (const double *) (op + o.zl), mu,
     (a->kernel == NCG_KERNEL_ST) ? 1.0 / a->nu : -0.5, op, (double *) (op + o.sck), (int32_t *) (op + o.fmax));
+  _q_tell_kernel<<<1, 1, 0, s>>> ((const int32_t *) (op + o.fmax), q_fmax (a->d), epoch, word);
 
   return cudaGetLastError ();
 }

@@ -86,7 +86,9 @@ struct ncg_sd
   size_t cap_tcB;
   uint8_t *dq64;          /* the FP64 form's tensor-core operand, and the scratch of its evals */
   void *dq64s;
-  int q64_ready;          /* 0 not built for this operand state, 1 usable, -1 out of its range */
+  int q64_ready;          /* 0 not built for this operand state, 1 built, 2 and known to be in range, -1 not usable */
+  uint32_t q64_epoch;     /* builds of it: the mapped word behind the flags tells of this one's range */
+  int q64_graph;          /* a recorded graph reads it */
   uint32_t k;
   uint64_t n_fallback;
   double href, kernel_lnnorm, rnorm;
@@ -135,5 +137,7 @@ void         ncg_sd_prepare_reserve (ncg_sd_t *sd);
 void         ncg_sd_interp_reserve (ncg_sd_t *sd);
 ncg_status_t ncg_sd_ensure_packmx (ncg_sd_t *sd);
 ncg_status_t ncg_sd_ensure_tc (ncg_sd_t *sd);      /* tensor-core operand + its check (VKDE) */
+int          ncg_sd_q64_usable (ncg_sd_t *sd, const ncg_eval_args_t *a, int wait);
+ncg_status_t ncg_sd_q64_refresh (ncg_sd_t *sd);
 
 #endif /* NCG_HOST_H */

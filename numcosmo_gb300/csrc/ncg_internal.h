@@ -160,11 +160,10 @@ cudaError_t ncg_launch_eval_tc (const ncg_eval_args_t *a, const double *Xq, cons
 
 /* ---- FP64 eval with chi^2 from the tensor cores (ncg_eval_q64.cu, VKDE) ---- */
 int         ncg_q64_wanted (const ncg_eval_args_t *a);
-int         ncg_q64_fmax (int d);
 size_t      ncg_q64_operand_bytes (int n, int d);
-const int32_t *ncg_q64_operand_fmax (const uint8_t *op, int n, int d);
 cudaError_t ncg_launch_q64_operand (const ncg_eval_args_t *a, const double *X, const double *pack64, const double *U,
-                                    const double *Vg, const double *mu, uint8_t *op, cudaStream_t s);
+                                    const double *Vg, const double *mu, uint8_t *op, unsigned long long *word,
+                                    uint32_t epoch, cudaStream_t s);
 size_t      ncg_q64_scratch_bytes (const ncg_eval_args_t *a);
 cudaError_t ncg_launch_eval_q64 (const ncg_eval_args_t *a, const double *Xq, const uint8_t *op, const double *pack64,
                                  const double *c, const double *mu, const double *Vg, double *out, void *scratch,

@@ -1207,8 +1207,8 @@ _split_fit (ncg_sd_t *sd, int n, int nk, const double *m2lnp, double min_m2lnp, 
   return _fit_at (sd, n, nk, ln_os, rnorm);
 }
 
-ncg_status_t
-ncg_sd_prepare_interp (ncg_sd_t *sd, const double *m2lnp)
+static ncg_status_t
+_prepare_interp (ncg_sd_t *sd, const double *m2lnp)
 {
   const double dbl_limit = 2.0;
   const double thr       = -2.0 * dbl_limit * NCG_LOG_DBL_EPSILON;
@@ -1399,6 +1399,14 @@ ncg_sd_prepare_interp (ncg_sd_t *sd, const double *m2lnp)
   }
 
   return NCG_OK;
+}
+
+ncg_status_t
+ncg_sd_prepare_interp (ncg_sd_t *sd, const double *m2lnp)
+{
+  const ncg_status_t r = _prepare_interp (sd, m2lnp);
+
+  return (r == NCG_OK) ? ncg_sd_q64_refresh (sd) : r;
 }
 
 /* the interpolation matrix with unit f (n_obs x n_kernels) into sd->nn.IM,
