@@ -66,7 +66,7 @@ typedef struct ncg_bplan
   int32_t *tcp;                /* problems on the tensor-core kernel */
   int ntcp, cap_tcp;
   int32_t *brp;                /* branch schedule (tc = 2): every problem, largest first */
-  int8_t *brk;                 /* its launch: 0 FP64 tiles, 1 FP32 SIMT tiles, 2 tensor cores */
+  int8_t *brk;                 /* its launch: 0 FP64 tiles, 1 FP32 SIMT tiles, 2 tensor cores, 3 FP64 sliced products */
   int8_t *brs;                 /* its stream */
   int nbrp, cap_brp;
   /* scratch of the one-problem launches, a region per stream (the launches of a
@@ -432,8 +432,10 @@ _branch_streams (ncg_batch_t *b, ncg_bplan_t *P)
   {
     const int i = P->brp[k];
 
-    /* tensor-core pairs at about a quarter of the FP32 SIMT pair time */
-    ord[k].cost = (double) b->m[i] * (double) b->sd[i]->nk * _pair_cost (b->sd[i]) * ((P->brk[k] == 2) ? 0.25 : 1.0);
+    /* tensor-core pairs at about a quarter of the FP32 SIMT pair time, sliced
+     * products at a sixth or so of the FP64 tiles' */
+    ord[k].cost = (double) b->m[i] * (double) b->sd[i]->nk * _pair_cost (b->sd[i]) *
+                  ((P->brk[k] == 2) ? 0.25 : (P->brk[k] == 3) ? 0.15 : 1.0);
     ord[k].k    = k;
   }
 
@@ -473,6 +475,9 @@ _launch_scratch (ncg_batch_t *b, int i, int k)
     return ncg_tc_scratch_bytes ((int64_t) b->m[i], (int) sd->nk, sd->dp);
 
   ncg_sd_fill_args (sd, b->m[i], &a);
+
+  if (k == 3)
+    return ncg_q64_scratch_bytes (&a);
 
   return ncg_eval_scratch_bytes (&a, k == 1 ? NCG_PREC_MIXED_SIMT : NCG_PREC_FP64);
 }
@@ -621,12 +626,16 @@ _build_plan (ncg_batch_t *b, int mixed)
       P->n_fp64_tiles++;
 
     /* the branch schedule: a problem off the tensor cores runs its own
-     * specialised tile kernel (FP32 SIMT, or FP64) */
+     * specialised tile kernel (FP32 SIMT, or FP64), or the FP64 form's sliced
+     * products where its own eval takes them (in the FP64 precision: a mixed
+     * problem that its guard sends to FP64 keeps the tiles, there and here) */
     if (prm->tc == 2)
     {
       const int on_tc = (P->ntcp > 0 && P->tcp[P->ntcp - 1] == i);
+      ncg_eval_args_t a;
 
-      P->brk[P->nbrp]   = on_tc ? 2 : ((mixed && tmix) ? 1 : 0);
+      ncg_sd_fill_args (sd, b->m[i], &a);
+      P->brk[P->nbrp]   = on_tc ? 2 : (mixed && tmix) ? 1 : (!mixed && ncg_sd_q64_usable (sd, &a, 1)) ? 3 : 0;
       P->brp[P->nbrp++] = i;
     }
 
@@ -848,8 +857,8 @@ _enqueue_tc (ncg_batch_t *b, ncg_bplan_t *P, const double *dX, double *dout)
 }
 
 /* The branch schedule (tc = 2): every problem is one launch of the kernel its
- * own eval would use (tensor cores, FP32 SIMT tiles or FP64 tiles), the
- * problems spread over NCG_BATCH_BR_STREAMS streams forked from s1
+ * own eval would use (tensor cores, FP32 SIMT tiles, FP64 tiles or the FP64
+ * form's sliced products), the problems spread over NCG_BATCH_BR_STREAMS streams forked from s1
  * (_branch_streams); captured, the streams are parallel branches of the graph. */
 static ncg_status_t
 _enqueue_branches (ncg_batch_t *b, ncg_bplan_t *P, const double *dX, double *dout)
@@ -883,6 +892,10 @@ _enqueue_branches (ncg_batch_t *b, ncg_bplan_t *P, const double *dX, double *dou
       else if (P->brk[k] == 1)
         r = ncg_cuda_status (ncg_launch_eval_m2lnp_mixed (&a, dX + b->x_off[i], sd->dpackmx, sd->dmu, sd->dVg,
                                                           dout + b->out_off[i], scratch, s), "batch eval_mixed");
+      else if (P->brk[k] == 3)
+        r = ncg_cuda_status (ncg_launch_eval_q64 (&a, dX + b->x_off[i], sd->dq64, sd->dpack64, sd->dc, sd->dmu, sd->dVg,
+                                                  dout + b->out_off[i], scratch, 0, sd->d_flag_alias, s),
+                             "batch eval_q64");
       else
         r = ncg_cuda_status (ncg_launch_eval_m2lnp_fp64 (&a, dX + b->x_off[i], sd->dpack64, sd->dc, sd->dVg,
                                                          dout + b->out_off[i], scratch, 0, s), "batch eval_fp64");
@@ -1076,6 +1089,14 @@ ncg_batch_eval_m2lnp (ncg_batch_t *b, int32_t precision, const double *X, double
       if (*(volatile int32_t *) b->sd[P->tcp[k]]->h_flag != 0)
       {
         ncg_set_error ("ncg_batch: the tensor-core eval of problem %d timed out", P->tcp[k]);
+
+        return NCG_ERR_TIMEOUT;
+      }
+
+    for (int k = 0; k < P->nbrp; k++)
+      if (P->brk[k] == 3 && *(volatile int32_t *) b->sd[P->brp[k]]->h_flag != 0)
+      {
+        ncg_set_error ("ncg_batch: the sliced-product eval of problem %d timed out", P->brp[k]);
 
         return NCG_ERR_TIMEOUT;
       }

@@ -5,7 +5,8 @@
  * pair of the slice.  Shared by the
  * one-problem launches (ncg_eval.cu, grid = point tiles x slices) and the
  * persistent multi-problem launch (ncg_batch.cu, tiles taken from a work
- * list), so a problem gets the same arithmetic in both.
+ * list), so a pair gets the same arithmetic in both (the sums over the kernels
+ * are cut differently).
  *
  * Restates, batched over points, _ncm_stats_dist_vkde_eval_weights_m2lnp
  * (numcosmo/ncm/stats/ncm_stats_dist_vkde.c:682-723) and
