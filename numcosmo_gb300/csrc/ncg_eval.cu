@@ -66,6 +66,7 @@ _eval64_kernel (const ncg_eval_args_t a, const double *__restrict__ Xq, const do
   pack += pdl0;
   cvec += pdl0;
   Vg   += pdl0;
+  part += pdl0;
 
   ncg_tile_eval64<DP, KIND, KERN, KC, EV64_WK> (a, Xq, pack, cvec, Vg, part, kper, blockIdx.x, blockIdx.y, sm, sc);
 }
@@ -94,6 +95,7 @@ _eval64_few_kernel (const ncg_eval_args_t a, const double *__restrict__ Xq, cons
   pack += pdl0;
   cvec += pdl0;
   Vg   += pdl0;
+  part += pdl0;
 
   if (tid < DP)
     xs[tid] = (tid < a.d) ? Xq[j * a.d + tid] : 0.0;
@@ -179,7 +181,10 @@ _merge_kernel (const T2 *__restrict__ part, int nslices, int64_t m, double shift
   const bool in   = j < m;
   double G = NCG_LSE_EMPTY, S = 0.0;
 
-  part += ncg_pdl_enter ();
+  const size_t pdl0 = ncg_pdl_enter ();
+
+  part += pdl0;
+  out += pdl0;
 
   if (in)
     for (int s = w; s < nslices; s += MG_TH / 32)

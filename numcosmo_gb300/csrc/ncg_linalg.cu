@@ -165,6 +165,7 @@ _gemv_n_kernel (const double *__restrict__ A, int nrows, int lda, const int32_t 
   A += pdl0;
   P += pdl0;
   x += pdl0;
+  y += pdl0;
 
   const int lane = threadIdx.x & 31;
   const int r    = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -209,6 +210,7 @@ _gemv_t_partial_kernel (const double *__restrict__ A, int nrows, int lda, const 
   A += pdl0;
   P += pdl0;
   x += pdl0;
+  part += pdl0;
 
   const int a  = blockIdx.x * blockDim.x + threadIdx.x;
   const int rb = blockIdx.y;
@@ -240,6 +242,7 @@ _gemv_t_final_kernel (const double *__restrict__ part, int nrb, int np, const do
 
   part += pdl0;
   b += pdl0;
+  y += pdl0;
 
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
 
@@ -349,6 +352,8 @@ _scale_vec_kernel (const int32_t *__restrict__ P, int np, const double *__restri
   P += pdl0;
   diagM += pdl0;
   b += pdl0;
+  Dsub += pdl0;
+  bsub += pdl0;
 
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
 
@@ -371,6 +376,8 @@ _gather_scaled_kernel (const float *__restrict__ M32, int n, const int32_t *__re
   M32 += pdl0;
   P += pdl0;
   Dsub += pdl0;
+  Msub += pdl0;
+  dg += pdl0;
 
   const int a = blockIdx.y;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -663,7 +670,9 @@ __global__ void __launch_bounds__ (256)
 _potrf_update_f32_kernel (float *A, int ld, int kb, int nb, int off, int nn, float *__restrict__ dg,
                           const int32_t *info)
 {
-  (void) ncg_pdl_wait ();
+  const size_t pdl0 = ncg_pdl_wait ();
+
+  dg += pdl0;
 
   __shared__ __align__ (16) float As[PB][PB];
   __shared__ __align__ (16) float Bs[PB][PB];
@@ -987,6 +996,10 @@ _pcg_dots_kernel (const double *__restrict__ u, const double *__restrict__ v, co
   v += pdl0;
   w += pdl0;
   D += pdl0;
+  p += pdl0;
+  sc += pdl0;
+  part += pdl0;
+  count += pdl0;
 
   double s[3] = { 0.0, 0.0, 0.0 };
 
@@ -1052,6 +1065,12 @@ _pcg_step_kernel (double *__restrict__ x, double *__restrict__ r, double *__rest
   p += pdl0;
   q += pdl0;
   D += pdl0;
+  x += pdl0;
+  r += pdl0;
+  rprev += pdl0;
+  sc += pdl0;
+  part += pdl0;
+  count += pdl0;
 
   const double rz = sc[NCG_PCG_RZ], al = (rz > 0.0) ? rz / sc[NCG_PCG_PQ] : 0.0;
   double s[3] = { 0.0, 0.0, 0.0 };
@@ -1077,6 +1096,7 @@ _pcg_dir_kernel (double *__restrict__ p, const double *__restrict__ z, int n, co
   const size_t pdl0 = ncg_pdl_enter ();
 
   z += pdl0;
+  p += pdl0;
 
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
 
@@ -1238,6 +1258,7 @@ _trinv_diag_kernel (const float *__restrict__ U, int n, float *__restrict__ V)
   const size_t pdl0 = ncg_pdl_enter ();
 
   U += pdl0;
+  V += pdl0;
 
   __shared__ __align__ (16) float S[2][TI][TI];   /* U11, U22, then V11, V22^T */
   __shared__ __align__ (16) float T[TI][TI];      /* 1 / diagonal, then U12, then U12^T V11 */
@@ -1400,6 +1421,9 @@ _fsolve_chain_kernel (const float *__restrict__ U, const float *__restrict__ V, 
   V += pdl0;
   D += pdl0;
   r += pdl0;
+  y += pdl0;
+  sync += pdl0;
+  err += pdl0;
 
   __shared__ float part[CS_TH / 32][SB];
   __shared__ __align__ (16) float sv[SB];
@@ -1502,6 +1526,10 @@ _bsolve_chain_kernel (const float *__restrict__ U, const float *__restrict__ V, 
   V += pdl0;
   D += pdl0;
   y += pdl0;
+  x += pdl0;
+  z += pdl0;
+  sync += pdl0;
+  err += pdl0;
 
   __shared__ __align__ (16) float sv[SB];
   __shared__ float half[SB];

@@ -13,9 +13,9 @@
  * A kernel launched by ncg_pdl_launch begins with ncg_pdl_enter or ncg_pdl_wait
  * (before any access to global memory): it returns once every kernel before it in
  * the stream has finished and its writes can be seen, since each of those waited in
- * the same way before it let the next one start.  Loads through `const T *__restrict__` may be
- * moved by the compiler as if nothing could write there, also ahead of that wait:
- * the zero that they return, added to such a pointer, ties its loads to
+ * the same way before it let the next one start.  Loads through a `__restrict__` pointer, const or not, may be
+ * moved by the compiler as if nothing else wrote there, also ahead of that wait:
+ * the zero that they return, added to every such parameter, ties its loads to
  * the wait and leaves the pointer what it is to the compiler (hidden pointers cost
  * the inverses' kernel twice its time, its loads no longer ran ahead of its stores).
  */

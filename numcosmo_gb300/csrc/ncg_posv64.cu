@@ -859,6 +859,11 @@ _posv_panel_kernel (double *__restrict__ A, int n, double *__restrict__ b, int k
 
   Lt   += pdl0;
   root += pdl0;
+  A += pdl0;
+  b += pdl0;
+  pk += pdl0;
+  ex += pdl0;
+  info += pdl0;
 
   if (*(volatile const int32_t *) info)
     return;

@@ -144,7 +144,12 @@ _syrk_tc_kernel (const uint8_t *__restrict__ pk, int nkc, int nn, float *__restr
     asm volatile ("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
 
-  pk += ncg_pdl_wait ();
+  const size_t pdl0 = ncg_pdl_wait ();
+
+  pk += pdl0;
+  C += pdl0;
+  dg += pdl0;
+  err_out += pdl0;
 
   /* a factorisation that already failed (or timed out) needs no more updates */
   const bool skip = *(volatile int *) err_out != 0;
