@@ -43,6 +43,7 @@
 #define P_BITS 9
 #define P_FIX 62                      /* |v| < 2^ex is held as v 2^(62 - ex) */
 #define P_K 32                        /* rows of a chunk (and of a panel)    */
+#define P_SLAB (1 << 13)              /* chunks of a launch at most: the orders' sums stay below 2^62 */
 #define P_T 128                       /* columns of a pack tile (MMA M)      */
 #define P_N 32                        /* output columns of a tile            */
 #define P_UNIT (P_T * 16)             /* 8 rows of one slice of a tile       */
@@ -492,9 +493,10 @@ _s_tile (int u, int T_, int ncol, int *ti, int *tj)
   return false;
 }
 
-/* hi 2^27 + lo rounded once (|hi| < 2^50, |lo| < 2^51), in integer
- * instructions: two FP64 additions on biased mantissas did the same at 128
- * cycles of the FP64 pipe, which the update then waited for */
+/* hi 2^27 + lo rounded once (|hi| < 2^62, |lo| < 2^62: a chunk adds up to 2^48.1 to hi and
+ * 2^42.4 to lo, and P_SLAB bounds their number), in integer instructions: two FP64
+ * additions on biased mantissas did the same at 128 cycles of the FP64 pipe, which the
+ * update then waited for */
 __device__ __forceinline__ double
 _join (long long hi, long long lo)
 {
@@ -1260,7 +1262,7 @@ ncg_launch_syrk_upper64 (const double *A, int nrows, int ncols, double *M, void 
                          int32_t *err, cudaStream_t s)
 {
   const int T_ = (ncols + P_T - 1) / P_T;
-  int slab     = (int) (cap / ((size_t) T_ * P_CHUNK) < (size_t) (1 << 20) ? cap / ((size_t) T_ * P_CHUNK) : (1 << 20));
+  int slab     = (int) (cap / ((size_t) T_ * P_CHUNK) < (size_t) P_SLAB ? cap / ((size_t) T_ * P_CHUNK) : P_SLAB);
   cudaError_t e;
   int nsm;
 
