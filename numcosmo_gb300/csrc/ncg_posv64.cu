@@ -437,7 +437,7 @@ struct S64Smem
   uint64_t full[S_STAGES], empty[S_STAGES], t_full[2], t_empty[2], done;
   DiagSmem diag;
   uint32_t tmem_base;
-  int err, ndiag;       /* ndiag: epilogue warps that stored tile 0 */
+  int err, skip, ndiag; /* skip: nothing to do; ndiag: epilogue warps that stored tile 0 */
 };
 
 #define S64_SMEM_BYTES (sizeof (S64Smem) + 1024)
@@ -577,7 +577,7 @@ _syrk64_kernel (const S64Params p)
   const bool skip = *(volatile int32_t *) p.err != 0;
 
   if (threadIdx.x == 0)
-    sm.err = skip ? 1 : 0;
+    sm.err = sm.skip = skip ? 1 : 0;
 
   _tc_fence_before ();
   __syncthreads ();
@@ -682,10 +682,9 @@ _syrk64_kernel (const S64Params p)
     const int q  = warp & 3;                      /* TMEM lane quarter (hardware: warp id mod 4) */
     const uint32_t base = tmem + ((uint32_t) (q * 32) << 16) + (uint32_t) (wg * 8);
     int tc = 0;
-    bool ok = !*err;
-
-    /* the warps agree before the warp-collective loads */
-    ok = __all_sync (0xffffffffu, ok);
+    /* the same answer in every warp (the error flag may go up before the last of them
+     * looks): all of them come to tile 0's barrier, or none */
+    bool ok = !sm.skip;
 
     for (int u = blockIdx.x; ok && _s_tile (u, T_, ncol, &ti, &tj); u += ustep)
     {
