@@ -284,15 +284,6 @@ _ev64 (const ncg_eval_args_t *a)
   return (a->kind == NCG_VKDE) ? _pick64<NCG_VKDE, NCG_KERNEL_ST> (a->dp, few) : _pick64_kde<NCG_KERNEL_ST> (a->d, few);
 }
 
-/* NcgEv64::KC */
-static int
-_kc64 (int kind, int dp)
-{
-  const int kc = 36864 / ((ncg_pack64_stride (kind, dp) + 1) * 8) / 4 * 4;
-
-  return kc < 4 ? 4 : (kc > 256 ? 256 : kc);
-}
-
 /* Slices of the FP64 forms.  The work is cut until there are about 48 CTAs
  * per SM (the last wave then costs a few per cent) but no finer than 8
  * kernels per warp, where the tile's own set-up and merge reach a tenth of the
@@ -814,7 +805,7 @@ _im64_kernel (const ncg_eval_args_t a, const double *__restrict__ X, const doubl
     for (int kk = 0; kk < kc; kk++)
     {
       const double chi2 = ncg_chi2_64<DP, KIND> (sm + kk * S, x);
-      const double K    = (KERN == NCG_KERNEL_ST) ? ncg_exp_full (-0.5 * (a.nu + a.d) * ncg_log_ge1 (fma (chi2, inv_nu, 1.0)))
+      const double K    = (KERN == NCG_KERNEL_ST) ? ncg_st_power (chi2, a.nu, inv_nu, -0.5 * (a.nu + a.d))
                                                   : ncg_exp_full (-0.5 * chi2);
 
       IM[(size_t) j * n + ic + kk] = (K * sn[kk]) * inv_f;
@@ -859,7 +850,10 @@ ncg_launch_compute_IM (const ncg_eval_args_t *a, const double *X, const double *
 
   int ns, kp;
 
-  _slicing (a->m, a->n, _kc64 (a->kind, a->dp), &ns, &kp);
+  /* slices down to 8 kernels: a thread's elements are one chain of FP64 instructions
+   * after the other, and whole staged chunks (100 kernels at d = 8) would leave 24 CTAs at
+   * n = 512: Student-t 400 us, 65 us so */
+  _slicing (a->m, a->n, 8, &ns, &kp);
 
   ncg_eval_args_t b = *a;
 

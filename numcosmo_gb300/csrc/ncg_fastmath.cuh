@@ -282,9 +282,10 @@ ncg_exp (double t)
   return fma (T, p, T);
 }
 
-/* exp(t) to about an ulp down to the subnormals, t <= 700: ln2/256 as two doubles, the scaling in two steps */
+/* exp(t + tl), tl far below 1, to about an ulp down to the subnormals, t <= 700: ln2/256 as two
+ * doubles, the scaling in two steps */
 static __device__ __forceinline__ double
-ncg_exp_full (double t)
+ncg_exp_full (double t, double tl = -0.0)
 {
   const uint32_t hi = (uint32_t) __double2hiint (t);
 
@@ -297,7 +298,7 @@ ncg_exp_full (double t)
   const double z  = fma (t, 0x1.71547652b82fep+8, 0x1.8p+52);
   const int k     = __double2loint (z);
   const double kd = z - 0x1.8p+52;
-  const double f  = fma (kd, -0x1.abc9e3b39803fp-64, fma (kd, -0x1.62e42fefa39efp-9, t));
+  const double f  = fma (kd, -0x1.abc9e3b39803fp-64, fma (kd, -0x1.62e42fefa39efp-9, t)) + tl;
   const double q  = f * f;
   const double h  = fma (f, fma (f, 0x1.5555555555555p-5, 0x1.5555555555555p-3), 0.5);
   const double tj = __ldg (ncg_exp2_tab + (k & 255));
@@ -457,7 +458,21 @@ ncg_lnt_wide (double t, double kappa, double c)
   return fma (kappa, g.x, fma (kappa, g.y, c));
 }
 
-/* The nu that take it, by a kernel of their own (KERN = NCG_KERNEL_ST_WIDE): as a branch on
+/* A Student-t kernel by itself, (1 + chi^2 / nu)^kappa, for the interpolation matrix:
+ * pow's accuracy, since an error of the logarithm counts kappa log u times there.  The
+ * quotient's remainder and the logarithm's and the product's low parts are kept (the
+ * rounded logarithm cost up to kappa (1 + 1.5 log u) units of 2^-53, pow's base kappa). */
+static __device__ __noinline__ double
+ncg_st_power (double chi2, double nu, double inv_nu, double kappa)
+{
+  const double t  = chi2 * inv_nu;
+  const double2 g = ncg_log1p_dd (t, fma (-t, nu, chi2) * inv_nu);
+  const double p  = kappa * g.x;
+
+  return ncg_exp_full (p, fma (kappa, g.x, -p) + kappa * g.y);
+}
+
+/* The nu that take ncg_lnt_wide, by a kernel of their own (KERN = NCG_KERNEL_ST_WIDE): as a branch on
  * a launch constant in the one for small nu it cost that one 2 % (d = 16, 8192 x 8192
  * 3.18 -> 3.25 ms), although it never ran. */
 #define NCG_KERNEL_ST_WIDE 2
