@@ -1600,9 +1600,9 @@ _build_q64 (ncg_sd_t *sd, const ncg_eval_args_t *a)
 
 /* Whether the FP64 eval of a takes the sliced products.  Their operand is built at the
  * first call that wants it after the kernels or the bandwidth changed (the weights are not
- * in it), without waiting: the kernels themselves look at its range, and the host
- * learns of it from a word of mapped memory (with `wait`, for callers that
- * synchronise anyway, at once), to go to the plain tiles where it is exceeded.
+ * in it), without waiting: the host learns of its range from a word of mapped memory
+ * (with `wait`, for callers that synchronise anyway, at once), and until then, and
+ * in a graph, the plain tiles follow the products and run where the range is exceeded.
  * The plain form also serves where there is no memory for the operand, and a
  * capture before which it was not built. */
 int
@@ -1682,21 +1682,27 @@ _eval_device (ncg_sd_t *sd, const double *dXq, uint64_t m, double *dout, int lin
     const int graph   = !wait && _capturing (sd->stream);
 
     /* scratch of its own, so that a recorded plain eval keeps the other, which is made
-     * here too: a capture after the next prepare takes the plain form; without room
-     * for it (which a capture does not make) the plain form */
-    if (!graph && ncg_sd_reserve (sd, &sd->dscratch, &sd->cap.scratch, ncg_eval_scratch_bytes (&a, NCG_PREC_FP64)) != NCG_OK)
+     * here too, for the tiles behind the products and for a capture after the next
+     * prepare; without room for it (which a capture does not make) the plain form */
+    const size_t plain = ncg_eval_scratch_bytes (&a, NCG_PREC_FP64);
+
+    if (!graph && (ncg_sd_reserve (sd, &sd->dscratch, &sd->cap.scratch, plain) != NCG_OK ||
+                   ncg_sd_reserve (sd, &sd->dq64s, &sd->cap.q64s, need) != NCG_OK))
       cudaGetLastError ();
 
-    if (sd->cap.q64s >= need || (!graph && ncg_sd_reserve (sd, &sd->dq64s, &sd->cap.q64s, need) == NCG_OK))
+    if (sd->cap.q64s >= need && sd->cap.scratch >= plain)
     {
       sd->q64_graph |= graph;
       CK (ncg_launch_eval_q64 (&a, dXq, sd->dq64, sd->dpack64, sd->dc, sd->dmu, sd->dVg, dout, sd->dq64s,
                                linear, sd->d_flag_alias, sd->stream), "eval_q64");
 
+      if (graph || sd->q64_ready == 1)
+        CK (ncg_launch_eval_m2lnp_fp64_if (&a, dXq, sd->dpack64, sd->dc, sd->dVg, dout, sd->dscratch, linear,
+                                           ncg_q64_operand_fmax (sd->dq64, a.n, a.d), ncg_q64_fmax (a.d), sd->stream),
+            "eval_fp64");
+
       return NCG_OK;
     }
-
-    cudaGetLastError ();
   }
 
   if (path == NCG_PATH_FP64)

@@ -54,7 +54,7 @@ template <int DP, int KIND, int KERN>
 __global__ void __launch_bounds__ (EV_THREADS)
 _eval64_kernel (const ncg_eval_args_t a, const double *__restrict__ Xq, const double *__restrict__ pack,
                 const double *__restrict__ cvec, const double *__restrict__ Vg, double2 *__restrict__ part,
-                int kper)
+                int kper, const int32_t *guard, int gmax)
 {
   constexpr int S  = NcgEv64<DP, KIND>::S;
   constexpr int KC = NcgEv64<DP, KIND>::KC;
@@ -68,6 +68,10 @@ _eval64_kernel (const ncg_eval_args_t a, const double *__restrict__ Xq, const do
   Vg   += pdl0;
   part += pdl0;
 
+  /* the sliced products served the call */
+  if (guard != NULL && *guard <= gmax)
+    return;
+
   ncg_tile_eval64<DP, KIND, KERN, KC, EV64_WK> (a, Xq, pack, cvec, Vg, part, kper, blockIdx.x, blockIdx.y, sm, sc);
 }
 
@@ -80,7 +84,7 @@ template <int DP, int KIND, int KERN>
 __global__ void __launch_bounds__ (EV_THREADS)
 _eval64_few_kernel (const ncg_eval_args_t a, const double *__restrict__ Xq, const double *__restrict__ pack,
                     const double *__restrict__ cvec, const double *__restrict__ Vg, double2 *__restrict__ part,
-                    int kper)
+                    int kper, const int32_t *, int)
 {
   constexpr int S   = NcgEv64<DP, KIND>::S;
   __shared__ double xs[DP], v[DP];
@@ -173,7 +177,7 @@ _eval64_few_kernel (const ncg_eval_args_t a, const double *__restrict__ Xq, cons
 template <typename T2>
 __global__ void __launch_bounds__ (MG_TH)
 _merge_kernel (const T2 *__restrict__ part, int nslices, int64_t m, double shift, const double *dshift,
-               double d_ln_href, int linear, double *__restrict__ out)
+               double d_ln_href, int linear, double *__restrict__ out, const int32_t *guard, int gmax)
 {
   __shared__ double red[MG_TH / 32][33];
   const int lane  = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -185,6 +189,9 @@ _merge_kernel (const T2 *__restrict__ part, int nslices, int64_t m, double shift
 
   part += pdl0;
   out += pdl0;
+
+  if (guard != NULL && *guard <= gmax)
+    return;
 
   if (in)
     for (int s = w; s < nslices; s += MG_TH / 32)
@@ -223,7 +230,7 @@ _merge_kernel (const T2 *__restrict__ part, int nslices, int64_t m, double shift
 }
 
 typedef void (*ev64_fn) (const ncg_eval_args_t, const double *, const double *, const double *,
-                         const double *, double2 *, int);
+                         const double *, double2 *, int, const int32_t *, int);
 
 #define EV64_PICK(DP) return few ? _eval64_few_kernel<DP, KIND, KERN> : _eval64_kernel<DP, KIND, KERN>
 
@@ -317,7 +324,7 @@ _slicing64 (const ncg_eval_args_t *a, int64_t ns_max, int *nslices, int *kper)
 
 static cudaError_t
 _run64 (const ncg_eval_args_t *a, const double *Xq, const double *pack64, const double *c, const double *Vg,
-        double *out, double2 *part, int64_t ns_max, int linear, cudaStream_t s)
+        double *out, double2 *part, int64_t ns_max, int linear, const int32_t *guard, int gmax, cudaStream_t s)
 {
   ev64_fn fn = _ev64 (a);
   int ns, kp;
@@ -330,13 +337,13 @@ _run64 (const ncg_eval_args_t *a, const double *Xq, const double *pack64, const 
   const int64_t bx = (a->m + EV_THREADS / EV64_WK - 1) / (EV_THREADS / EV64_WK);
   const dim3 grid  = (a->m <= EV64_FEW) ? dim3 ((unsigned) ns, (unsigned) a->m) : dim3 ((unsigned) bx, (unsigned) ns);
 
-  cudaError_t e = ncg_pdl_launch (fn, grid, EV_THREADS, 0, s, *a, Xq, pack64, c, Vg, part, kp);
+  cudaError_t e = ncg_pdl_launch (fn, grid, EV_THREADS, 0, s, *a, Xq, pack64, c, Vg, part, kp, guard, gmax);
 
   if (e != cudaSuccess)
     return e;
 
   return ncg_pdl_launch (_merge_kernel<double2>, (unsigned) ((a->m + 31) / 32), MG_TH, 0, s, part, ns, a->m,
-                         a->final_shift, (const double *) NULL, a->d_ln_href, linear, out);
+                         a->final_shift, (const double *) NULL, a->d_ln_href, linear, out, guard, gmax);
 }
 
 #define EV64_NS_MAX 4096
@@ -389,7 +396,16 @@ extern "C" cudaError_t
 ncg_launch_eval_m2lnp_fp64 (const ncg_eval_args_t *a, const double *Xq, const double *pack64, const double *c,
                             const double *Vg, double *out, void *scratch, int linear, cudaStream_t s)
 {
-  return _run64 (a, Xq, pack64, c, Vg, out, (double2 *) scratch, EV64_NS_MAX, linear, s);
+  return _run64 (a, Xq, pack64, c, Vg, out, (double2 *) scratch, EV64_NS_MAX, linear, NULL, 0, s);
+}
+
+/* the same for more than EV64_FEW points if *guard > gmax on the device, else nothing */
+extern "C" cudaError_t
+ncg_launch_eval_m2lnp_fp64_if (const ncg_eval_args_t *a, const double *Xq, const double *pack64, const double *c,
+                               const double *Vg, double *out, void *scratch, int linear, const int32_t *guard, int gmax,
+                               cudaStream_t s)
+{
+  return _run64 (a, Xq, pack64, c, Vg, out, (double2 *) scratch, EV64_NS_MAX, linear, guard, gmax, s);
 }
 
 /* ------------------------------------------------------------------------ */
@@ -739,7 +755,7 @@ ncg_launch_eval_m2lnp_mixed (const ncg_eval_args_t *a, const double *Xq, const f
     return e;
 
   _merge_kernel<float2><<<(unsigned) ((a->m + 31) / 32), MG_TH, 0, s>>> (
-    (const float2 *) scratch, ns, a->m, a->final_shift, cshift, a->d_ln_href, 0, out);
+    (const float2 *) scratch, ns, a->m, a->final_shift, cshift, a->d_ln_href, 0, out, NULL, 0);
 
   return cudaGetLastError ();
 }
@@ -873,7 +889,7 @@ ncg_launch_merge_f2 (const void *part, int nparts, int64_t m, double shift, cons
                      double *out, cudaStream_t s)
 {
   _merge_kernel<float2><<<(unsigned) ((m + 31) / 32), MG_TH, 0, s>>> ((const float2 *) part, nparts, m, shift, dshift,
-                                                                     d_ln_href, 0, out);
+                                                                     d_ln_href, 0, out, NULL, 0);
 
   return cudaGetLastError ();
 }
@@ -954,7 +970,7 @@ ncg_launch_eval_m2lnp_fp64_noalloc (const ncg_eval_args_t *a, const double *Xq, 
   /* the regular slicing, with the slice count capped by the static size */
   const int64_t fit = (int64_t) (NCG_NOALLOC_SCRATCH_BYTES / ((size_t) a->m * sizeof (double2)));
 
-  return _run64 (a, Xq, pack64, c, Vg, out, (double2 *) addr, fit < EV64_NS_MAX ? fit : EV64_NS_MAX, 0, s);
+  return _run64 (a, Xq, pack64, c, Vg, out, (double2 *) addr, fit < EV64_NS_MAX ? fit : EV64_NS_MAX, 0, NULL, 0, s);
 }
 
 /* ------------------------------------------------- FP64 pipe measurement */

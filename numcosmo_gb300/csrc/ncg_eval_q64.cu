@@ -32,7 +32,8 @@
  * So a point with 2e + f above 10 B - 52, f the largest of the kernels (q_range:
  * points far outside the sample, or any in the presence of very narrow kernels), is
  * left to the merge, which evaluates it in the plain form; and where the largest f is above
- * q_fmax, which leaves no room for points, all are.  x', W', P and theta' are formed in
+ * q_fmax, which leaves no room for points, these kernels do nothing and the caller's plain
+ * form serves the call.  x', W', P and theta' are formed in
  * double-double, so nothing else enters.
  *
  * Kernel.  Tiles of 128 points x 48 kernels.  Per 16 features (a K step) the
@@ -715,7 +716,7 @@ _eval_q64_kernel (const QParams p)
   const int nunits = p.npt * p.nslices;
   volatile int *err = &sm.err;
 
-  /* every point is left to the merge */
+  /* the plain form serves the call */
   if (*p.f > p.fmax_)
     return;
 
@@ -960,11 +961,11 @@ _eval_q64_kernel (const QParams p)
 struct QMerge
 {
   const double2 *part;
-  const int32_t *pe2;
+  const int32_t *pe2, *f;
   const double *Xq, *pack, *c;
   double *out;
   int64_t m;
-  int nparts, n, d, dp, linear;
+  int nparts, n, d, dp, linear, fmax_;
   double kappa, inv_nu, shift, d_ln_href;
 };
 
@@ -1017,6 +1018,9 @@ _q_merge_kernel (const QMerge p)
   const int64_t j = (int64_t) blockIdx.x * 32 + lane;
   const bool far_ = j < p.m && p.pe2[j] == Q_FAR, in = j < p.m && !far_;
   double G = NCG_LSE_EMPTY, S = 0.0;
+
+  if (*p.f > p.fmax_)
+    return;
 
   if (in)
     for (int s = w; s < p.nparts; s += QM_TH / 32)
@@ -1115,6 +1119,12 @@ ncg_q64_wanted (const ncg_eval_args_t *a)
   return a->kind == NCG_VKDE && a->d >= 5 && a->m >= 640 && a->n >= 384 && a->n <= (1 << 24);
 }
 
+extern "C" int
+ncg_q64_fmax (int d)
+{
+  return q_fmax (d);
+}
+
 /* operand of n kernels: digits | scales (n padded) | Zl | largest f */
 typedef struct { size_t sck, zl, fmax, total; } q_operand_t;
 
@@ -1136,6 +1146,13 @@ extern "C" size_t
 ncg_q64_operand_bytes (int n, int d)
 {
   return _q_operand (n, d).total;
+}
+
+/* device address of the largest f of the operand */
+extern "C" const int32_t *
+ncg_q64_operand_fmax (const uint8_t *op, int n, int d)
+{
+  return (const int32_t *) (op + _q_operand (n, d).fmax);
 }
 
 /* the operand of a's kernels; *word (mapped host memory) gets `epoch` in its upper half and
@@ -1293,8 +1310,8 @@ ncg_launch_eval_q64 (const ncg_eval_args_t *a, const double *Xq, const uint8_t *
 
     const int units = p.npt * p.nslices, grid = units < nsm ? units : nsm;
 
-    const QMerge q = { p.part, p.pe2, Xq + j0 * a->d, pack64, c, out + j0, mc, Q_WG * o.ns, a->n, a->d, a->dp, linear,
-                       a->kappa, 1.0 / a->nu, a->final_shift, a->d_ln_href };
+    const QMerge q = { p.part, p.pe2, p.f, Xq + j0 * a->d, pack64, c, out + j0, mc, Q_WG * o.ns, a->n, a->d, a->dp,
+                       linear, p.fmax_, a->kappa, 1.0 / a->nu, a->final_shift, a->d_ln_href };
 
     e = (a->kernel == NCG_KERNEL_GAUSS)  ? _run_q64_bits<NCG_KERNEL_GAUSS> (p, q, a->d, grid, s)
         : ncg_nu_wide (a->nu, a->d)      ? _run_q64_bits<NCG_KERNEL_ST_WIDE> (p, q, a->d, grid, s)

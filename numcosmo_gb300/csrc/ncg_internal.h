@@ -158,9 +158,15 @@ cudaError_t ncg_launch_eval_tc (const ncg_eval_args_t *a, const double *Xq, cons
                                 const double *Vg, const double *cshift, void *scratch, double *out, int *flag_host,
                                 cudaEvent_t *ev, cudaStream_t s);
 
+cudaError_t ncg_launch_eval_m2lnp_fp64_if (const ncg_eval_args_t *a, const double *Xq, const double *pack64,
+                                           const double *c, const double *Vg, double *out, void *scratch, int linear,
+                                           const int32_t *guard, int gmax, cudaStream_t s);
+
 /* ---- FP64 eval with chi^2 from the tensor cores (ncg_eval_q64.cu, VKDE) ---- */
 int         ncg_q64_wanted (const ncg_eval_args_t *a);
+int         ncg_q64_fmax (int d);
 size_t      ncg_q64_operand_bytes (int n, int d);
+const int32_t *ncg_q64_operand_fmax (const uint8_t *op, int n, int d);
 cudaError_t ncg_launch_q64_operand (const ncg_eval_args_t *a, const double *X, const double *pack64, const double *U,
                                     const double *Vg, const double *mu, uint8_t *op, unsigned long long *word,
                                     uint32_t epoch, cudaStream_t s);

@@ -118,6 +118,20 @@ def test_operand_out_of_range(gpu, kernel):
     torch.cuda.synchronize()
     sd.eval_m2lnp_device(x.data_ptr(), len(P), out.data_ptr())
     sd.synchronize()
-    plain = _plain(sd, P)
-    assert rel_err(out.cpu().numpy(), plain, floor=1.0) < PLAIN_TOL
-    assert np.array_equal(sd.eval_m2lnp(P), plain)
+    first, host = out.cpu().numpy(), sd.eval_m2lnp(P)
+    assert np.array_equal(first, host)
+    assert rel_err(host, _plain(sd, P), floor=1.0) < PLAIN_TOL
+
+
+def test_replay_with_an_operand_out_of_range(gpu):
+    """Recorded within the range, replayed after a fit that leaves it, and back."""
+    rng, sd, s, P, x, out = _setup(gpu, 6, 500, 700)
+    sd.eval_m2lnp_device(x.data_ptr(), 700, out.data_ptr())
+    torch.cuda.synchronize()
+    g = _capture(sd, s, x, out)
+    for scale in (1e-7, 1.0):
+        X = rng.standard_normal((500, 6))
+        X[:250] = 3.0 + scale * X[:250]
+        sd.set_sample(X)
+        sd.prepare()
+        assert np.array_equal(_replay(g, out), sd.eval_m2lnp(P))
