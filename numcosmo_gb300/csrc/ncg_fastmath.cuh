@@ -485,9 +485,9 @@ ncg_nu_wide (double nu, int d)
 
 /* One sum over kernels kept as (g, s): the terms added so far are
  * s exp(g).  g follows the largest term closely enough (within 4) that
- * g + log s loses nothing against the maximum itself; it starts at -1e300
- * with s = 0, where an empty sum or one of -inf terms stays. */
-#define NCG_LSE_EMPTY (-1.0e300)
+ * g + log s loses nothing against the maximum itself; it starts at the lowest
+ * double with s = 0, where an empty sum or one of -inf terms stays. */
+#define NCG_LSE_EMPTY (-0x1.fffffffffffffp+1023)
 
 static __device__ __forceinline__ void
 ncg_lse_add (double lnt, double &g, double &s)
