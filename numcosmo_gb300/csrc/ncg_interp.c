@@ -619,9 +619,11 @@ _add_largest (char *inP, int n, const double *v, double vmin, double add_frac)
   return adds;
 }
 
-/* A^T A of the mixed form goes to the tensor cores from this many columns (n =
- * 512: 115 us on the CUDA cores) */
-#define NCG_SYRK_TC_MIN 128
+/* A^T A of the mixed form goes to the tensor cores from this many columns: whole
+ * VKDE fits at d = 4 take 833 us on the CUDA cores against 857 us on the tensor cores
+ * at n = 200 (553 against 591 at n = 130), 935 against 919 at n = 300, 2163
+ * against 2093 at n = 512 */
+#define NCG_SYRK_TC_MIN 256
 
 /* every device buffer the NNLS of an nr x n system reserves (the large
  * matrices from the caller's arena when one is set, after the interpolation
