@@ -1639,8 +1639,8 @@ ncg_sd_q64_usable (ncg_sd_t *sd, const ncg_eval_args_t *a, int wait)
   return sd->q64_ready > 0;
 }
 
-/* a graph holds the operand's address: build it with the kernels, as the plain
- * operand that such a graph would read otherwise */
+/* a graph holds the operand's address: build it with the kernels, complete when the
+ * prepare returns (a replay may be on any stream), as the plain operand is */
 ncg_status_t
 ncg_sd_q64_refresh (ncg_sd_t *sd)
 {
@@ -1649,9 +1649,16 @@ ncg_sd_q64_refresh (ncg_sd_t *sd)
   if (!sd->q64_graph || sd->q64_ready != 0)
     return NCG_OK;
 
+  ncg_status_t r;
+
   ncg_sd_fill_args (sd, 1, &a);
 
-  return _build_q64 (sd, &a);
+  if ((r = _build_q64 (sd, &a)) != NCG_OK)
+    return r;
+
+  CK (cudaStreamSynchronize (sd->stream), "sync");
+
+  return NCG_OK;
 }
 
 static ncg_status_t

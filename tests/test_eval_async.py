@@ -90,6 +90,23 @@ def test_replay_follows_the_handle(gpu, warm):
             sd.eval_m2lnp(P[:300])                                 # tiles
 
 
+def test_replay_on_another_stream_after_prepare(gpu):
+    """The operand of a recorded eval is complete when a prepare returns."""
+    rng, sd, s, P, x, out = _setup(gpu, 16, 4000, 1500)
+    sd.eval_m2lnp_device(x.data_ptr(), 1500, out.data_ptr())
+    torch.cuda.synchronize()
+    g = _capture(sd, s, x, out)
+    other = torch.cuda.Stream()
+    for _ in range(3):
+        sd.set_sample(rng.standard_normal((4000, 16)))
+        torch.cuda.synchronize()
+        sd.prepare()
+        with torch.cuda.stream(other):
+            g.replay()
+        torch.cuda.synchronize()
+        assert rel_err(out.cpu().numpy(), _plain(sd, P)) < PLAIN_TOL
+
+
 def test_plain_capture_keeps_its_scratch(gpu):
     """A recorded tile eval and later sliced-product evals of the same handle."""
     _, sd, s, P, x, out = _setup(gpu, 6, 500, 300)
