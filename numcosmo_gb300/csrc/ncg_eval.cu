@@ -864,12 +864,19 @@ ncg_launch_compute_IM (const ncg_eval_args_t *a, const double *X, const double *
   if (fn == NULL || a->n <= 0 || a->m < a->n || a->m > INT32_MAX)
     return cudaErrorInvalidValue;
 
+  /* NcgEv64::KC */
+  const int raw = 36864 / ((ncg_pack64_stride (a->kind, a->dp) + 1) * 8) / 4 * 4;
+  const int kc  = raw < 4 ? 4 : (raw > 256 ? 256 : raw);
   int ns, kp;
 
-  /* slices down to 8 kernels: a thread's elements are one chain of FP64 instructions
-   * after the other, and whole staged chunks (100 kernels at d = 8) would leave 24 CTAs at
-   * n = 512: Student-t 400 us, 65 us so */
-  _slicing (a->m, a->n, 8, &ns, &kp);
+  /* whole staged chunks, or slices of 8 kernels and more where those leave too few CTAs: a
+   * thread's elements are one chain of FP64 instructions after the other (24 CTAs at
+   * n = 512, d = 8: Student-t 400 us, 65 us so; 430 at n = 1200, d = 16: 505 and 484 us;
+   * 1155 at n = 2600, d = 20: 3.27 ms, against 3.76 with the chunks cut) */
+  _slicing (a->m, a->n, kc, &ns, &kp);
+
+  if (ns * ((a->m + EV_THREADS - 1) / EV_THREADS) < 152 * 5)
+    _slicing (a->m, a->n, 8, &ns, &kp);
 
   ncg_eval_args_t b = *a;
 
