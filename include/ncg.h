@@ -171,12 +171,14 @@ ncg_status_t ncg_sd_eval_m2lnp (ncg_sd_t *sd, const double *x, double *m2lnp);
 ncg_status_t ncg_sd_eval_m2lnp_batch (ncg_sd_t *sd, const double *X, uint64_t m, double *m2lnp);
 /* the same with device pointers, asynchronous on the handle's stream.  It may
  * be recorded in a CUDA graph once a call with as many points has made its
- * buffers; replays then follow the handle's later fits of the same size.  (In
- * the FP64 form a VKDE call of 640 points or more, d >= 5, first builds a
+ * buffers.  A recorded FP64 eval of a VKDE follows the handle's later fits of
+ * the same size and bandwidth; a KDE's normalisation, the bandwidth and the
+ * mixed form's operand are those of the capture: record again after a fit.
+ * (An FP64 VKDE call of 640 points or more, d >= 5, first builds a
  * tensor-core operand of the current fit, and where kernels turn out too
  * narrow for it evaluates in the plain form; a capture before which that
  * operand was not built records the plain form.  The mixed form wants a call
- * after the last prepare.) */
+ * between the last prepare and the capture.) */
 ncg_status_t ncg_sd_eval_m2lnp_device (ncg_sd_t *sd, const double *d_X, uint64_t m, double *d_m2lnp);
 
 /* eval_m2lnp in the FP64 form on device pointers, for callers that must not
@@ -343,8 +345,10 @@ ncg_status_t ncg_rng_sample2_stream (ncg_rng_t *rng, ncg_kernel_t kernel, uint32
  * state: re-preparing a handle or refitting its weights re-plans the batch
  * on the next call.  precision: NCG_PREC_FP64, or NCG_PREC_MIXED (FP32 SIMT
  * tiles; a problem whose whitening is ill-conditioned gets FP64 tiles).
- * Each problem's result equals its one-problem eval with the same tile
- * arithmetic up to the slicing of its kernel range. */
+ * Each problem's result equals its one-problem eval up to rounding (the same
+ * arithmetic per pair in tiles, the kernel range sliced differently; an own FP64
+ * VKDE eval of 640 points or more goes by sliced products), or bit for bit in
+ * the branch schedule (tc = 2 below). */
 typedef struct ncg_batch ncg_batch_t;
 
 /* plan parameters (chosen by ncg_batch_autotune, or set) */

@@ -24,6 +24,11 @@
  * FP64 pipes leave room for and fewer points per CTA fill the last wave and
  * the last tile better */
 #define EV64_WK 4
+/* Up to here a kernel per thread (_eval64_few_kernel).  Measured on both sides, few-point kernel |
+ * tiles, us: KDE d = 4, n = 1000 at 16 points 12 | 24, at 64 18 | 24; KDE d = 16, n = 8000 42 |
+ * 76 and 119 | 120; VKDE d = 6, n = 500 13 | 34 and 16 | 34; VKDE d = 16, n = 8192 88 | 139 and
+ * 264 | 246: the kernels are walked again for every point, so from about 48 points the
+ * tiles win at the largest sizes, and at 16 the few-point kernel does at all. */
 #define EV64_FEW 16
 
 __device__ __forceinline__ double2

@@ -21,12 +21,12 @@
 #include "ncg_pdl.cuh"
 #include "ncg_syrk_tc.cuh"
 
-/* FP32 products (the mixed solver's A^T A below 1024 columns):
+/* FP32 products (the mixed solver's A^T A below 256 columns):
  * 128 x 128 upper tiles, 256 threads of 8 x 8 outputs (rows ty*4 + {0..3} and
  * 64 + ty*4 + {0..3}, columns likewise by tx), contraction rows staged 8 at a
  * time in double-buffered shared memory (the next chunk is loaded into
  * registers while the current one is used).  Each output is still one FMA
- * chain over the rows in ascending order, as in _syrk_tile_kernel. */
+ * chain over the rows in ascending order. */
 #define SY_T 128
 #define SY_KB 8
 
