@@ -1608,7 +1608,7 @@ _build_q64 (ncg_sd_t *sd, const ncg_eval_args_t *a)
 int
 ncg_sd_q64_usable (ncg_sd_t *sd, const ncg_eval_args_t *a, int wait)
 {
-  if (!ncg_q64_wanted (a))
+  if (sd->q64_off || !ncg_q64_wanted (a))
     return 0;
 
   if (sd->q64_ready == 0)

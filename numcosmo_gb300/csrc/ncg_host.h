@@ -89,6 +89,7 @@ struct ncg_sd
   int q64_ready;          /* 0 not built for this operand state, 1 built, 2 and known to be in range, -1 not usable */
   uint32_t q64_epoch;     /* builds of it: the mapped word behind the flags tells of this one's range */
   int q64_graph;          /* a recorded graph reads it */
+  int q64_off;            /* kept to the plain form (a server's memory budget) */
   uint32_t k;
   uint64_t n_fallback;
   double href, kernel_lnnorm, rnorm;

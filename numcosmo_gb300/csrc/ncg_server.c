@@ -53,6 +53,7 @@ typedef struct
   int state, running;
   int64_t npending;
   uint64_t steps, last_used, bytes;
+  int q64_off;                        /* the budget holds it without the sliced products only */
   ncg_sd_t *sd;
   cudaStream_t stream;                /* the handle's stream while resident */
   void *dbuf;                         /* step buffers, one allocation */
@@ -144,9 +145,9 @@ _dbuf_doubles (const ncg_chain_desc_t *c)
 
 /* device bytes a resident chain holds (its handle's state and scratch, and
  * the step buffers): an estimate from the layouts of the handle's buffers,
- * with 10 % and 4 MiB of slack */
+ * with 10 % and 4 MiB of slack; with or without the FP64 eval's sliced products */
 static uint64_t
-_chain_bytes (const ncg_chain_desc_t *c, int mixed)
+_chain_bytes (const ncg_chain_desc_t *c, int mixed, int q64)
 {
   const double n = (double) (c->n / 2), d = c->dim;   /* the fit's kernels */
   const int dp   = ncg_pad_dim ((int) c->dim);
@@ -167,7 +168,7 @@ _chain_bytes (const ncg_chain_desc_t *c, int mixed)
     if (!mixed)
       b += (double) ncg_posv_work_bytes (a.n);
 
-    if (!mixed && ncg_q64_wanted (&a))
+    if (!mixed && q64 && ncg_q64_wanted (&a))
       b += (double) ncg_q64_operand_bytes (a.n, a.d) + (double) ncg_q64_scratch_bytes (&a);
   }
 
@@ -491,7 +492,18 @@ _add_chain (ncg_server_t *s, const ncg_chain_desc_t *c, const double *m2, const 
   ch.desc.target_L = NULL;
   ch.desc.lb       = NULL;
   ch.desc.ub       = NULL;
-  ch.bytes         = _chain_bytes (&ch.desc, s->cfg.precision != NCG_PREC_FP64);
+
+  {
+    const int mixed = s->cfg.precision != NCG_PREC_FP64;
+
+    /* a chain that the budget holds without the sliced products' operand only
+     * keeps the plain form */
+    ch.bytes   = _chain_bytes (&ch.desc, mixed, 1);
+    ch.q64_off = !mixed && ch.bytes + ncg_sd_workspace_bytes_for (n / 2, 0) > s->cfg.hbm_budget;
+
+    if (ch.q64_off)
+      ch.bytes = _chain_bytes (&ch.desc, mixed, 0);
+  }
 
   pthread_mutex_lock (&s->mu);
 
@@ -1101,7 +1113,8 @@ _chain_load (ncg_server_t *s, chain_t *c)
 
   cfg.async_alloc = 1;
   SK (ncg_sd_new ((ncg_kind_t) dsc->kind, (ncg_kernel_t) dsc->kernel, dsc->dim, dsc->nu, &cfg, &c->sd));
-  c->sd->pool = s->pool;
+  c->sd->pool    = s->pool;
+  c->sd->q64_off = c->q64_off;
 
   /* Stream priority by step size: the chains of more than half the largest
    * size (the tail of the latency distribution) run on high-priority streams,
